@@ -197,6 +197,7 @@ struct Ctx {
   bool lj_uniform = false;   // every type pair has the same parameters
   float lj_single[3] = {0, 0, 0};
   double lj_single_cutsq_d = 0;
+  double lj_cutsq_max = 0;   // over the type pairs
   double lj_single_d[2] = {0, 0};  // lj1, lj2 of the uniform type pair in FP64
   // the mixed form's thermo-step energy, computed by the force call of the
   // positions it used: asked for before a compute (emd_lj_request_energy),

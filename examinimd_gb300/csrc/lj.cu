@@ -1,12 +1,13 @@
 // ForceLJNeigh on the device, FP64 drop-in (force_lj_neigh_impl.h:57-343).
 //
-// Full list: one thread per owned atom accumulates its row in list order and
-// adds the sum to f(i) once -- the same operations in the same order as the
-// serial reference, so with -fmad=false the forces are bit-identical.
+// Full list: every force component is summed over its row in list order from
+// pair forces rounded as the reference rounds them, so with -fmad=false the
+// forces are bit-identical (lj_fp64.cuh).
 // Half list: the partner's force is scattered with FP64 atomics (as the
 // reference's Atomic-trait view does on a GPU); the order of those adds is
 // not fixed, so half-list forces agree to rounding only.
-// Energy: per-atom shifted-LJ sums, deterministic block + device reduction.
+// Energy: shifted-LJ sums in a fixed order (lane, CTA, device reduction).
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 #include <vector>
@@ -15,161 +16,63 @@
 
 #include "emd_device.cuh"
 #include "emd_internal.h"
+#include "lj_fp64.cuh"
 #include "neigh_rows.cuh"
 
 namespace emd {
 namespace {
 
-struct LJParams {
-  const double* lj1;
-  const double* lj2;
-  const double* cutsq;
-  int ntypes;
-  const double* intensity;  // lj/cut/idial: repeat count per type pair (as doubles)
-};
-
-// pair force over r: the plain LJ term, or (IDIAL) ForceLJIDialNeigh's
-// repeated evaluation, each repeat adding 1/intensity of the term
-// (force_lj_idial_neigh_impl.h:137-149)
-template <bool IDIAL>
-__device__ __forceinline__ double lj_fpair(double rsq, double lj1, double lj2, double inten) {
-  if (!IDIAL) {
-    const double r2inv = 1.0 / rsq;
-    const double r6inv = r2inv * r2inv * r2inv;
-    return (r6inv * (lj1 * r6inv - lj2)) * r2inv;
-  }
-  double fpair = 0.0;
-  for (int repeat = 0; repeat < inten; repeat++) {
-    const double r2inv = 1.0 / rsq;
-    const double r6inv = r2inv * r2inv * r2inv;
-    fpair += (r6inv * (lj1 * r6inv - lj2)) * r2inv / inten;
-  }
-  return fpair;
-}
-
 __device__ __forceinline__ int entry_j(int e, bool packed) { return packed ? (e >> 6) : e; }
 
-// TagFullNeigh (force_lj_neigh_impl.h:164-206).  ZERO folds the pending
-// deep_copy(f, 0) into the store as 0.0 + sum, the reference's exact result.
-template <bool TWO_D, bool ZERO, bool IDIAL = false>
-__global__ void __launch_bounds__(128) k_lj_full_fp64(const double4_32a* __restrict__ x4, double* __restrict__ f,
-                                                      ListView L, LJParams P, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double4_32a xi = x4[i];
-  const int ti = int(xi.w);
-  const Row<TWO_D> row(L, i);
-  double fxi = 0.0, fyi = 0.0, fzi = 0.0;
-  for (int jj = 0; jj < row.n; ++jj) {
-    const int j = row[jj];
-    const double4_32a xj = x4[j];
-    const double dx = xi.x - xj.x;
-    const double dy = xi.y - xj.y;
-    const double dz = xi.z - xj.z;
-    const int tj = int(xj.w);
-    const double rsq = dx * dx + dy * dy + dz * dz;
-    const int tp = ti * P.ntypes + tj;
-    const double cutsq_ij = __ldg(P.cutsq + tp);
-    if (rsq < cutsq_ij) {
-      const double fpair = lj_fpair<IDIAL>(rsq, __ldg(P.lj1 + tp), __ldg(P.lj2 + tp),
-                                           IDIAL ? __ldg(P.intensity + tp) : 1.0);
-      fxi += dx * fpair;
-      fyi += dy * fpair;
-      fzi += dz * fpair;
+// Rows per warp of the FP64 tiles (lj_fp64.cuh).  A row costs about 38 FP64
+// instructions for its pairs and a tile 62 more for its sums (half of both for
+// a half list); the 608 warp schedulers work through ceil(tiles / 608) tiles
+// each, so the rows are the count that makes the busiest scheduler's share
+// smallest.  At most seven rows of a full list: larger tiles leave fewer warps
+// on the SM to run beside the ones that are filtering (256,000 atoms: 771 us
+// with 7 rows, 800 with 9, 1154 with 2; 32,000: 114 with the 6 this picks, 135
+// with 9; 2,048: 19 with 4, 30 with 9).  Half lists fill nine rows' lists half
+// as far (143,748 atoms: 256 us with 9 rows, 272 with 7).
+int lj_tile_rows(int n, bool half) {
+  const int most = half ? LJT_ROWS : 7, pairs = half ? 19 : 38, sums = half ? 31 : 62;
+  int best = 1;
+  long long best_cost = -1;
+  for (int r = 1; r <= most; ++r) {
+    const long long tiles = (n + r - 1) / r, cost = (tiles + 607) / 608 * (pairs * r + sums);
+    if (best_cost < 0 || cost <= best_cost) {
+      best = r;
+      best_cost = cost;
     }
   }
-  if (ZERO) {
-    f[3 * i] = 0.0 + fxi;
-    f[3 * i + 1] = 0.0 + fyi;
-    f[3 * i + 2] = 0.0 + fzi;
+  return best;
+}
+
+// Energy tiles are taken by a fixed number of CTAs, one partial each, so that
+// the sum depends on the atom count only and its scratch is bounded
+constexpr int LJE_BLOCKS = 152 * 6;
+
+template <int MODE, bool TWO_D, bool UNI, bool IDIAL = false, bool ZERO = false>
+void launch_lj_fp64(LJTile T, cudaStream_t s) {
+  T.rows = lj_tile_rows(T.n, T.half);
+  T.cap = ljt_cap(T.rows, T.half);
+  const size_t smem = LJT_WARPS * ljt_warp_bytes(T.cap, T.half, UNI);
+  auto k = k_lj_fp64<MODE, TWO_D, UNI, IDIAL, ZERO>;
+  EMD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  const int tiles = (T.n + T.rows - 1) / T.rows;
+  const int grid = MODE == LJ_ENERGY ? LJE_BLOCKS : (tiles + LJT_WARPS - 1) / LJT_WARPS;
+  k<<<grid, LJT_THREADS, smem, s>>>(T);
+  EMD_CHECK_LAUNCH();
+}
+
+template <int MODE, bool IDIAL = false, bool ZERO = false>
+void launch_lj_fp64(const LJTile& T, bool two_d, bool uniform, cudaStream_t s) {
+  if (two_d) {
+    if (uniform) launch_lj_fp64<MODE, true, true, IDIAL, ZERO>(T, s);
+    else launch_lj_fp64<MODE, true, false, IDIAL, ZERO>(T, s);
   } else {
-    f[3 * i] += fxi;
-    f[3 * i + 1] += fyi;
-    f[3 * i + 2] += fzi;
+    if (uniform) launch_lj_fp64<MODE, false, true, IDIAL, ZERO>(T, s);
+    else launch_lj_fp64<MODE, false, false, IDIAL, ZERO>(T, s);
   }
-}
-
-// TagHalfNeigh (force_lj_neigh_impl.h:211-254)
-// IDIAL: ForceLJIDialNeigh's half form scatters to owned partners only
-// (force_lj_idial_neigh_impl.h:199-203)
-template <bool TWO_D, bool IDIAL = false>
-__global__ void __launch_bounds__(128) k_lj_half_fp64(const double4_32a* __restrict__ x4, double* __restrict__ f,
-                                                      ListView L, LJParams P, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double4_32a xi = x4[i];
-  const int ti = int(xi.w);
-  const Row<TWO_D> row(L, i);
-  double fxi = 0.0, fyi = 0.0, fzi = 0.0;
-  for (int jj = 0; jj < row.n; ++jj) {
-    const int j = row[jj];
-    const double4_32a xj = x4[j];
-    const double dx = xi.x - xj.x;
-    const double dy = xi.y - xj.y;
-    const double dz = xi.z - xj.z;
-    const int tj = int(xj.w);
-    const double rsq = dx * dx + dy * dy + dz * dz;
-    const int tp = ti * P.ntypes + tj;
-    if (rsq < __ldg(P.cutsq + tp)) {
-      const double fpair = lj_fpair<IDIAL>(rsq, __ldg(P.lj1 + tp), __ldg(P.lj2 + tp),
-                                           IDIAL ? __ldg(P.intensity + tp) : 1.0);
-      fxi += dx * fpair;
-      fyi += dy * fpair;
-      fzi += dz * fpair;
-      if (!IDIAL || j < n) {
-        atomicAdd(f + 3 * j, -(dx * fpair));
-        atomicAdd(f + 3 * j + 1, -(dy * fpair));
-        atomicAdd(f + 3 * j + 2, -(dz * fpair));
-      }
-    }
-  }
-  atomicAdd(f + 3 * i, fxi);
-  atomicAdd(f + 3 * i + 1, fyi);
-  atomicAdd(f + 3 * i + 2, fzi);
-}
-
-// TagFullNeighPE / TagHalfNeighPE (force_lj_neigh_impl.h:259-343), one
-// partial per block.
-template <bool TWO_D>
-__global__ void __launch_bounds__(256) k_lj_energy(const double4_32a* __restrict__ x4, ListView L, LJParams P, int n,
-                                                   int half, int packed, double* __restrict__ part) {
-  __shared__ double sh[8];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double pe = 0.0;
-  if (i < n) {
-    const double4_32a xi = x4[i];
-    const int ti = int(xi.w);
-    const Row<TWO_D> row(L, i);
-    for (int jj = 0; jj < row.n; ++jj) {
-      const int j = entry_j(row[jj], packed);
-      const double4_32a xj = x4[j];
-      const double dx = xi.x - xj.x;
-      const double dy = xi.y - xj.y;
-      const double dz = xi.z - xj.z;
-      const int tj = int(xj.w);
-      const double rsq = dx * dx + dy * dy + dz * dz;
-      const int tp = ti * P.ntypes + tj;
-      const double cutsq_ij = __ldg(P.cutsq + tp);
-      if (rsq < cutsq_ij) {
-        const double lj1_ij = __ldg(P.lj1 + tp);
-        const double lj2_ij = __ldg(P.lj2 + tp);
-        const double r2inv = 1.0 / rsq;
-        const double r6inv = r2inv * r2inv * r2inv;
-        const double r2invc = 1.0 / cutsq_ij;
-        const double r6invc = r2invc * r2invc * r2invc;
-        if (!half) {
-          pe += 0.5 * r6inv * (0.5 * lj1_ij * r6inv - lj2_ij) / 6.0;
-          pe -= 0.5 * r6invc * (0.5 * lj1_ij * r6invc - lj2_ij) / 6.0;
-        } else {
-          const double fac = j < n ? 1.0 : 0.5;
-          pe += fac * r6inv * (0.5 * lj1_ij * r6inv - lj2_ij) / 6.0;
-          pe -= fac * r6invc * (0.5 * lj1_ij * r6invc - lj2_ij) / 6.0;
-        }
-      }
-    }
-  }
-  const double t = block_sum(pe, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
 }  // namespace
@@ -233,10 +136,26 @@ ListView list_view(Ctx& c) {
   return L;
 }
 
-static LJParams lj_params(Ctx& c) {
+static LJTile lj_tile(Ctx& c) {
   const size_t nt2 = size_t(c.lj_ntypes) * c.lj_ntypes;
-  return LJParams{c.lj_params.p, c.lj_params.p + nt2, c.lj_params.p + 2 * nt2, c.lj_ntypes,
-                  c.lj_idial ? c.lj_intensity.p : nullptr};
+  LJTile T{};
+  T.x4 = c.x4.p;
+  T.f = c.f.p;
+  T.L = list_view(c);
+  T.P = LJParams{c.lj_params.p, c.lj_params.p + nt2, c.lj_params.p + 2 * nt2, c.lj_ntypes,
+                 c.lj_idial ? c.lj_intensity.p : nullptr, c.type.p, c.lj_single_d[0], c.lj_single_d[1],
+                 c.lj_single_cutsq_d, c.lj_cutsq_max};
+  T.n = c.N_local;
+  T.half = c.lj_half;
+  T.packed = c.neigh_packed;
+  return T;
+}
+
+// one energy partial per CTA into part[0 .. LJE_BLOCKS)
+static void launch_lj_energy(Ctx& c, double* part) {
+  LJTile T = lj_tile(c);
+  T.part = part;
+  launch_lj_fp64<LJ_ENERGY>(T, c.neigh_layout_2d, c.lj_uniform, c.stream);
 }
 
 // ---- scratch of emd_lj_energy_noalloc
@@ -245,13 +164,13 @@ static LJParams lj_params(Ctx& c) {
 // would fail or fragment it), or a latency-bound loop that must not meet the
 // device-wide synchronisation a cudaFree implies.  For them the energy
 // reduction runs on a fixed array compiled into this library: one partial per
-// 256-atom block of k_lj_energy, then the deterministic two-stage sum.
+// CTA of the energy kernel, then the deterministic two-stage sum.
 // Nothing in it has to start at zero: every element a call reads was written
 // earlier in that same call.  The array is one per device and per process, so
 // calls that can overlap on one device (two contexts, two host threads, two
 // streams) race on it and must be serialised by the caller.
-constexpr int kNoAllocBlocks = EMD_LJ_ENERGY_NOALLOC_MAX_LOCAL / 256;  // 16,384 partials
-static_assert(kNoAllocBlocks * 256 == EMD_LJ_ENERGY_NOALLOC_MAX_LOCAL, "whole blocks");
+constexpr int kNoAllocBlocks = EMD_LJ_ENERGY_NOALLOC_MAX_LOCAL / 256;  // 16,384 doubles
+static_assert(kNoAllocBlocks >= LJE_BLOCKS, "room for every CTA's partial");
 constexpr int kNoAllocDoubles = kNoAllocBlocks + kSumScratchDoubles;  // 133,512 bytes
 static __device__ __align__(256) double g_lj_energy_scratch[kNoAllocDoubles];
 
@@ -333,6 +252,17 @@ emd_status emd_lj_init(emd_ctx* ctx, int ntypes, const double* lj1, const double
   EMD_CUDA(cudaMemcpyAsync(c.lj_params.p, h.data(), sizeof(double) * 3 * nt2, cudaMemcpyHostToDevice, c.stream));
   EMD_CUDA(cudaStreamSynchronize(c.stream));
   c.lj_ntypes = ntypes;
+  // every type pair identical (ExaMiniMD's stack parameters for <= 12 types
+  // always are): kernels keep the values in registers
+  c.lj_uniform = true;
+  c.lj_cutsq_max = cutsq[0];
+  for (size_t k = 1; k < nt2; ++k) {
+    c.lj_uniform = c.lj_uniform && lj1[k] == lj1[0] && lj2[k] == lj2[0] && cutsq[k] == cutsq[0];
+    c.lj_cutsq_max = std::max(c.lj_cutsq_max, cutsq[k]);
+  }
+  c.lj_single_d[0] = lj1[0];
+  c.lj_single_d[1] = lj2[0];
+  c.lj_single_cutsq_d = cutsq[0];
   c.lj_idial = false;  // emd_lj_set_intensity after this call selects lj/cut/idial
   c.lj_half = half_neigh ? 1 : 0;
   c.lj_prec = precision;
@@ -365,42 +295,26 @@ emd_status emd_lj_compute(emd_ctx* ctx) {
     return EMD_OK;
   }
   require(!c.neigh_packed, EMD_ERR_STATE, "emd_lj_compute: list was built for the mixed form");
-  const ListView L = list_view(c);
-  const LJParams P = lj_params(c);
+  const LJTile T = lj_tile(c);
   const bool two_d = c.neigh_layout_2d;
-  const int grid = blocks_for(n, 128);
+  const bool uniform = c.lj_uniform && (!c.lj_idial || c.lj_ntypes == 1);
   if (c.lj_half) materialize_zero(c, true, true);
   const bool zero = c.f_zero_pending & 1;
   TimedLaunch t(c, c.lj_half ? "lj_half_fp64" : "lj_full_fp64");
   if (!c.lj_half) {
-    if (two_d) {
-      if (c.lj_idial) {
-        if (zero) k_lj_full_fp64<true, true, true><<<grid, 128, 0, c.stream>>>(c.x4.p, c.f.p, L, P, n);
-        else k_lj_full_fp64<true, false, true><<<grid, 128, 0, c.stream>>>(c.x4.p, c.f.p, L, P, n);
-      } else {
-        if (zero) k_lj_full_fp64<true, true><<<grid, 128, 0, c.stream>>>(c.x4.p, c.f.p, L, P, n);
-        else k_lj_full_fp64<true, false><<<grid, 128, 0, c.stream>>>(c.x4.p, c.f.p, L, P, n);
-      }
+    if (c.lj_idial) {
+      if (zero) launch_lj_fp64<LJ_FULL, true, true>(T, two_d, uniform, c.stream);
+      else launch_lj_fp64<LJ_FULL, true, false>(T, two_d, uniform, c.stream);
     } else {
-      if (c.lj_idial) {
-        if (zero) k_lj_full_fp64<false, true, true><<<grid, 128, 0, c.stream>>>(c.x4.p, c.f.p, L, P, n);
-        else k_lj_full_fp64<false, false, true><<<grid, 128, 0, c.stream>>>(c.x4.p, c.f.p, L, P, n);
-      } else {
-        if (zero) k_lj_full_fp64<false, true><<<grid, 128, 0, c.stream>>>(c.x4.p, c.f.p, L, P, n);
-        else k_lj_full_fp64<false, false><<<grid, 128, 0, c.stream>>>(c.x4.p, c.f.p, L, P, n);
-      }
+      if (zero) launch_lj_fp64<LJ_FULL, false, true>(T, two_d, uniform, c.stream);
+      else launch_lj_fp64<LJ_FULL, false, false>(T, two_d, uniform, c.stream);
     }
     c.f_zero_pending &= ~1;
+  } else if (c.lj_idial) {
+    launch_lj_fp64<LJ_HALF, true>(T, two_d, uniform, c.stream);
   } else {
-    if (c.lj_idial) {
-      if (two_d) k_lj_half_fp64<true, true><<<grid, 128, 0, c.stream>>>(c.x4.p, c.f.p, L, P, n);
-      else k_lj_half_fp64<false, true><<<grid, 128, 0, c.stream>>>(c.x4.p, c.f.p, L, P, n);
-    } else {
-      if (two_d) k_lj_half_fp64<true><<<grid, 128, 0, c.stream>>>(c.x4.p, c.f.p, L, P, n);
-      else k_lj_half_fp64<false><<<grid, 128, 0, c.stream>>>(c.x4.p, c.f.p, L, P, n);
-    }
+    launch_lj_fp64<LJ_HALF, false>(T, two_d, uniform, c.stream);
   }
-  EMD_CHECK_LAUNCH();
   EMD_API_END
 }
 
@@ -429,19 +343,12 @@ emd_status emd_lj_energy(emd_ctx* ctx, double* pe) {
     *pe = 0.0;
     return EMD_OK;
   }
-  const int grid = blocks_for(n, 256);
-  c.red2.reserve(size_t(grid), c.stream);
-  const ListView L = list_view(c);
-  const LJParams P = lj_params(c);
+  c.red2.reserve(LJE_BLOCKS, c.stream);
   {
     TimedLaunch t(c, "lj_energy");
-    if (c.neigh_layout_2d)
-      k_lj_energy<true><<<grid, 256, 0, c.stream>>>(c.x4.p, L, P, n, c.lj_half, c.neigh_packed, c.red2.p);
-    else
-      k_lj_energy<false><<<grid, 256, 0, c.stream>>>(c.x4.p, L, P, n, c.lj_half, c.neigh_packed, c.red2.p);
-    EMD_CHECK_LAUNCH();
+    launch_lj_energy(c, c.red2.p);
   }
-  *pe = device_sum(c, c.red2.p, grid);
+  *pe = device_sum(c, c.red2.p, LJE_BLOCKS);
   EMD_API_END
 }
 
@@ -505,16 +412,9 @@ emd_status emd_lj_energy_noalloc(emd_ctx* ctx, double* pe) {
     return EMD_OK;
   }
   // the kernels and partition of emd_lj_energy, so both return the same bits
-  const int grid = blocks_for(n, 256);
-  const ListView L = list_view(c);
-  const LJParams P = lj_params(c);
-  if (c.neigh_layout_2d)
-    k_lj_energy<true><<<grid, 256, 0, c.stream>>>(c.x4.p, L, P, n, c.lj_half, c.neigh_packed, scratch);
-  else
-    k_lj_energy<false><<<grid, 256, 0, c.stream>>>(c.x4.p, L, P, n, c.lj_half, c.neigh_packed, scratch);
-  EMD_CHECK_LAUNCH();
+  launch_lj_energy(c, scratch);
   double* sum = scratch + kNoAllocBlocks;
-  device_sum_launch(c, scratch, grid, sum);
+  device_sum_launch(c, scratch, LJE_BLOCKS, sum);
   EMD_CUDA(cudaMemcpyAsync(c.h_scalar, sum + kSumScratchDoubles - 1, sizeof(double), cudaMemcpyDeviceToHost,
                            c.stream));
   EMD_CUDA(cudaStreamSynchronize(c.stream));

@@ -453,18 +453,9 @@ void lj_mixed_prepare(Ctx& c) {
   EMD_CUDA(cudaStreamSynchronize(c.stream));
   std::vector<float> hf(3 * nt2);
   for (size_t k = 0; k < 3 * nt2; ++k) hf[k] = float(h[k]);
-  // every type pair identical (ExaMiniMD's stack parameters for <= 12 types
-  // always are): keep the values in registers
-  bool uniform = true;
-  for (size_t k = 1; k < nt2; ++k)
-    uniform = uniform && h[k] == h[0] && h[nt2 + k] == h[nt2] && h[2 * nt2 + k] == h[2 * nt2];
-  c.lj_uniform = uniform;
   c.lj_single[0] = hf[0];
   c.lj_single[1] = hf[nt2];
   c.lj_single[2] = hf[2 * nt2];
-  c.lj_single_cutsq_d = h[2 * nt2];
-  c.lj_single_d[0] = h[0];
-  c.lj_single_d[1] = h[nt2];
   c.lj_params_f.reserve(3 * nt2, c.stream);
   EMD_CUDA(cudaMemcpyAsync(c.lj_params_f.p, hf.data(), sizeof(float) * 3 * nt2, cudaMemcpyHostToDevice, c.stream));
   EMD_CUDA(cudaStreamSynchronize(c.stream));
