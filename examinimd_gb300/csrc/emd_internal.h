@@ -258,6 +258,16 @@ struct TimedLaunch {
 void timing_collect(Ctx& c);
 void free_snap(Ctx& c);
 
+// Opts a kernel in to large dynamic shared memory.  The limit belongs to the
+// kernel, not to the launch, and several host threads launch the same kernel
+// with different sizes, so it is always the same: the whole 227 KB less room
+// for static shared memory.
+constexpr size_t kMaxDynSmem = 225 * 1024;
+template <typename K>
+inline void allow_dyn_smem(K kernel) {
+  EMD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMaxDynSmem)));
+}
+
 inline int blocks_for(long long n, int threads) {
   long long b = (n + threads - 1) / threads;
   return int(b < 1 ? 1 : b);

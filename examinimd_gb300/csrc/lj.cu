@@ -57,7 +57,7 @@ void launch_lj_fp64(LJTile T, cudaStream_t s) {
   T.cap = ljt_cap(T.rows, T.half);
   const size_t smem = LJT_WARPS * ljt_warp_bytes(T.cap, T.half, UNI);
   auto k = k_lj_fp64<MODE, TWO_D, UNI, IDIAL, ZERO>;
-  EMD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  allow_dyn_smem(k);
   const int tiles = (T.n + T.rows - 1) / T.rows;
   const int grid = MODE == LJ_ENERGY ? LJE_BLOCKS : (tiles + LJT_WARPS - 1) / LJT_WARPS;
   k<<<grid, LJT_THREADS, smem, s>>>(T);
