@@ -179,6 +179,17 @@ def snap_inside_mean(ctx, n_local: int, rcutsq: float) -> float:
     return float(np.count_nonzero(np.einsum("ij,ij->i", d, d) < rcutsq)) / n_local
 
 
+def snap_kernels(prec: str) -> list[str]:
+    """The kernels of one SNAP force call."""
+    return ["snap_pairs", "snap_u", f"snap_y_{prec}", f"snap_force_{prec}"]
+
+
+def snap_force_time(rep: dict, prec: str) -> tuple[float, int]:
+    """(total ms of the force calls' kernels, force calls) from a timing report."""
+    got = [rep.get(k, (0.0, 0)) for k in snap_kernels(prec)]
+    return sum(ms for ms, _ in got), got[-1][1]
+
+
 class ClockSampler:
     """nvidia-smi clocks / throttle reasons sampled every 200 ms."""
     Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,clocks_event_reasons.hw_slowdown,"
@@ -342,7 +353,7 @@ def run_gpu_arm(a, ws, rank, local):
     # (two per launch; the other launches are counted): the per-kernel
     # breakdown comes from a separate pass below
     ctx.timing(True)
-    ctx.timing_only(kname)
+    ctx.timing_only(snap_kernels(a.precision) if snap else kname)
     ctx.timing_reset()
     clocks = ClockSampler(local)
     e0 = torch.cuda.Event(enable_timing=True)
@@ -362,7 +373,7 @@ def run_gpu_arm(a, ws, rank, local):
     rep = ctx.timing_report()
     launches = sum(c for _, c in rep.values())
     value = ws * N * a.steps / (ms_max * 1e-3)
-    kms, kn = rep.get(kname, (0.0, 0))
+    kms, kn = snap_force_time(rep, a.precision) if snap else rep.get(kname, (0.0, 0))
     # per-kernel breakdown: every launch bracketed, over one more rebuild cycle
     # (20 steps; 3 for SNAP, which rebuilds every step) after the timed region
     ctx.timing_only(None)
@@ -611,8 +622,8 @@ def snap_measure(local: int, steps_mixed: int, steps_fp64: int, warm: int, cells
         ms = e0.elapsed_time(e1)
         rep = ctx.timing_report()
         ctx.timing(False)
-        kname = f"snap_{prec}"
-        kms, kn = rep.get(kname, (0.0, 0))
+        kname = f"snap_{prec}"  # the kernels of one force call together
+        kms, kn = snap_force_time(rep, prec)
         N = md.info()["N"]
         res[prec] = {"value": N * steps / (ms * 1e-3), "unit": METRIC, "ms_per_step": ms / steps, "steps": steps,
                      "warmup": warm, "kernel": kname, "kernel_ms_per_launch": (kms / kn) if kn else None,
@@ -623,10 +634,10 @@ def snap_measure(local: int, steps_mixed: int, steps_fp64: int, warm: int, cells
         # roofline: operations of the kernel's own formulation (snap_flops)
         # against the measured FP64 and FP32 pipe peaks
         if kn:
-            from examinimd_gb300.snap_flops import snap_flops
+            from examinimd_gb300.snap_flops import kernel_flops
             rc = 2.0 * 0.5 * 4.73442  # 2 radius rcutfac of the synthetic W coefficients
             nin = snap_inside_mean(ctx, md.info()["N_local"], rc * rc)
-            fl = snap_flops(8, nin)
+            fl = kernel_flops(8, nin)
             t = kms / kn * 1e-3
             n_loc = md.info()["N_local"]
             f64, f32 = fl["fp64"][prec] * n_loc, fl["fp32"][prec] * n_loc

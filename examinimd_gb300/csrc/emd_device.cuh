@@ -39,4 +39,25 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return t;
 }
 
+// ------------------------------------------------- FP32 view of a double
+// Truncation to FP32 by integer operations: magnitudes below 2^-126 become 0,
+// beyond the FP32 range (and NaN) infinity.  Within 2^-23 relative otherwise.
+__device__ __forceinline__ float f32_bits(double v) {
+  const unsigned hi = __double2hiint(v), lo = __double2loint(v);
+  const unsigned e = (hi >> 20) & 0x7ffu;
+  unsigned m = (((hi & 0x7fffffffu) << 3) | (lo >> 29)) - 0xc0000000u;  // exponent less 896
+  m = e < 897u ? 0u : (e > 1150u ? 0x7f800000u : m);
+  return __uint_as_float(m | (hi & 0x80000000u));
+}
+// Threshold for an FP32 r^2 formed from f32_bits positions: every partner with
+// r^2 < cutsq lies below it.  Such a partner has coordinates below M in
+// magnitude, so the FP32 differences are off by at most d = 2^-21 M per
+// dimension and r^2 by 2 sqrt(3) rc d + 3 d^2 plus the FP32 operations'
+// rounding.  Non-finite coordinates give a comparison that rejects nothing.
+__device__ __forceinline__ float f32_cut_threshold(float cutsq, float x, float y, float z) {
+  const float rc = sqrtf(cutsq);
+  const float d = (fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))) + rc) * 4.7683716e-7f;
+  return fmaf(cutsq, 1.00001f, fmaf(4.0f * rc, d, 3.0f * d * d));
+}
+
 }  // namespace emd

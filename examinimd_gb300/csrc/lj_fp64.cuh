@@ -42,16 +42,6 @@ struct LJParams {
   double cutsq_max;
 };
 
-// ------------------------------------------------- FP32 view of a double
-// Truncation to FP32 by integer operations: magnitudes below 2^-126 become 0,
-// beyond the FP32 range (and NaN) infinity.  Within 2^-23 relative otherwise.
-__device__ __forceinline__ float f32_bits(double v) {
-  const unsigned hi = __double2hiint(v), lo = __double2loint(v);
-  const unsigned e = (hi >> 20) & 0x7ffu;
-  unsigned m = (((hi & 0x7fffffffu) << 3) | (lo >> 29)) - 0xc0000000u;  // exponent less 896
-  m = e < 897u ? 0u : (e > 1150u ? 0x7f800000u : m);
-  return __uint_as_float(m | (hi & 0x80000000u));
-}
 __device__ __forceinline__ double f64_of_normal(float f) {  // exact for a normal f > 0
   const unsigned b = __float_as_uint(f);
   return __hiloint2double(int((b >> 3) + 0x38000000u), int(b << 29));
@@ -150,7 +140,6 @@ __global__ void __launch_bounds__(LJT_THREADS) k_lj_fp64(LJTile T) {
     ecut_0 = r6c * (c12_0 * r6c - c6_0);
   }
   const float cutsq_f = __double2float_ru(T.P.cutsq_max);
-  const float rc_f = sqrtf(cutsq_f);
   const int tiles = (T.n + T.rows - 1) / T.rows;
   double esum = 0.0;
   const int step = MODE == LJ_ENERGY ? gridDim.x * LJT_WARPS : tiles;
@@ -275,13 +264,7 @@ __global__ void __launch_bounds__(LJT_THREADS) k_lj_fp64(LJTile T) {
       load_entries(last ? a + 1 : a, last ? 0 : k0 + 32 * NB, en);
       const float xf = __shfl_sync(FULL_MASK, xf_l, a), yf = __shfl_sync(FULL_MASK, yf_l, a),
                   zf = __shfl_sync(FULL_MASK, zf_l, a);
-      // A partner inside the cutoff has coordinates below M in magnitude, so the
-      // FP32 differences are off by at most d = 2^-21 M per dimension: its FP32
-      // r^2 lies below the threshold (4 rc d >= 2 sqrt(3) rc d, 3 d^2 and the
-      // FP32 operations' rounding).  Non-finite coordinates reach the FP64 test.
-      const float M = fmaxf(fabsf(xf), fmaxf(fabsf(yf), fabsf(zf))) + rc_f;
-      const float d = M * 4.7683716e-7f;
-      const float thr = fmaf(cutsq_f, 1.00001f, fmaf(4.0f * rc_f, d, 3.0f * d * d));
+      const float thr = f32_cut_threshold(cutsq_f, xf, yf, zf);
       if (MODE != LJ_ENERGY && row_l == a && k0 == 0) seg_b = seg_e = cnt;
 #pragma unroll
       for (int h = 0; h < NB; ++h) {

@@ -3,13 +3,18 @@
 // snap_kernel.cuh; the mixed-form instantiation is compiled in snap_mixed.cu.
 #include <algorithm>
 #include <cmath>
+#include <memory>
+#include <mutex>
 #include <vector>
 
 #include "snap_kernel.cuh"
 
 namespace emd {
 
-void snap_mixed_launch(const snapk::SnapArgs& A, size_t smem, cudaStream_t s);
+void snap_mixed_pairs(const snapk::SnapArgs& A, cudaStream_t s);
+void snap_mixed_u(const snapk::SnapArgs& A, cudaStream_t s);
+void snap_mixed_y(const snapk::SnapArgs& A, cudaStream_t s);
+void snap_mixed_force(const snapk::SnapArgs& A, int threads, cudaStream_t s);
 
 namespace {
 
@@ -18,19 +23,29 @@ using namespace snapk;
 struct SnapHost {
   SnapDev d;
   int precision = EMD_PREC_FP64;
-  DevBuf<int> trip, cg_off, jobs, tjob_off, yred_off, yred_job, map;
-  DevBuf<int4> zord;
-  DevBuf<int> inside_max;  // k_snap_inside_max's result
-  DevBuf<double> cg, cY, beta0, radelem, wjelem, eatom, invf, yscale;
-  DevBuf<float> cg_f, cY_f, yscale_f;
+  // tables
+  DevBuf<Entry> ent;
+  DevBuf<ZTask> task;
+  DevBuf<ZRec> rec;
+  DevBuf<int> e0, map, zt0, tmask;
+  DevBuf<int2> xsum, half, zt, prod;
+  DevBuf<int4> hfull;
+  DevBuf<double> zc, cY, AB, beta0, wjelem, pr;
+  DevBuf<float> cY_f, AB_f;
+  DevBuf<float2> zc_f;
+  // per-chunk work arrays
+  DevBuf<double> pd, pr_f, U, Y, zk;
+  DevBuf<int> pj, cnt;
+  DevBuf<Cplx<double>> D, H;
+  DevBuf<double> eatom;
   // adjoint: per-atom columns, their per-element sums, the loss gradient dL/dF
   DevBuf<double> adj, adj_sum, adj_g;
   // coefficient k's three dB/dr terms: full triples and factors (the cY fold)
   std::vector<int> k_t1, k_t2, k_t3;
   std::vector<double> k_f2, k_f3;
   std::vector<int> k_j;  // (j1, j2, j) of coefficient k
-  // U_tot and Z jobs of the last FP64 force pass, kept for an adjoint on the
-  // same positions and list (emd_snap_keep_for_adjoint)
+  // U_tot and the Z of the last FP64 force pass, kept for an adjoint
+  // on the same positions and list (emd_snap_keep_for_adjoint)
   bool keep_on = false, keep_valid = false;
   unsigned long long keep_xver = 0;
   long long keep_builds = -1;
@@ -69,107 +84,193 @@ double clebsch_gordan(int j1, int j2, int j, int m1, int m2) {
                    factorial((j2 - bb2) / 2) * factorial((j + cc2) / 2) * factorial((j - cc2) / 2) * (j + 1));
 }
 
-// The Z jobs as descriptors (see SnapDev::zord), ordered for
-// balance: sorted by inner-loop count, longest first, in chunks of 32 (a warp
-// gets jobs of one length); chunk c goes to round c / 8 and, alternating
-// direction from round to round, to warp c % 8 or 7 - c % 8.
-std::vector<int4> zjob_order(const std::vector<int>& trip, const std::vector<int>& cg_off, const std::vector<int>& jobs) {
-  const int nj = int(jobs.size());
-  std::vector<int4> desc(static_cast<size_t>(nj));
-  std::vector<int> cost(static_cast<size_t>(nj));
-  for (int jb = 0; jb < nj; ++jb) {
-    const int code = jobs[size_t(jb)], t = code >> 8, ma = (code >> 4) & 15, mb = code & 15;
-    const int j1 = trip[3 * size_t(t)], j2 = trip[3 * size_t(t) + 1], j = trip[3 * size_t(t) + 2];
-    const int ma1lo = std::max(0, (2 * ma - j - j2 + j1) / 2), ma1hi = std::min(j1, (2 * ma - j + j2 + j1) / 2);
-    const int mb1lo = std::max(0, (2 * mb - j - j2 + j1) / 2), mb1hi = std::min(j1, (2 * mb - j + j2 + j1) / 2);
-    int na = std::max(0, ma1hi - ma1lo + 1), nb = std::max(0, mb1hi - mb1lo + 1);
-    const int ma2 = (2 * ma - j - (2 * ma1lo - j1) + j2) / 2, mb2 = (2 * mb - j - (2 * mb1lo - j1) + j2) / 2;
-    const int uo1 = j1 * (j1 + 1) * (2 * j1 + 1) / 6, uo2 = j2 * (j2 + 1) * (2 * j2 + 1) / 6;
-    int u1 = uo1 + ma1lo * (j1 + 1) + mb1lo, u2 = uo2 + ma2 * (j2 + 1) + mb2;
-    int ci = cg_off[size_t(t)] + mb1lo * (j2 + 1) + mb2, co = cg_off[size_t(t)] + ma1lo * (j2 + 1) + ma2;
-    if (na == 0 || nb == 0) na = nb = u1 = u2 = ci = co = 0;  // Z = 0, nothing read
-    require(u1 >= 0 && u2 >= 0 && ci >= 0 && co >= 0 && u1 < 65536 && u2 < 65536 && ci < 65536 && co < 65536 &&
-                na < 256 && nb < 256,
-            EMD_ERR_ARG,
-            "SNAP: Z job tables exceed their packed fields");
-    desc[size_t(jb)] = int4{jb, int(unsigned(u1) | (unsigned(u2) << 16)), int(unsigned(ci) | (unsigned(co) << 16)),
-                            int(unsigned(na) | (unsigned(nb) << 8) | (unsigned(j1 + 1) << 16) | (unsigned(j2 + 1) << 24))};
-    cost[size_t(jb)] = na * (nb + 1);
-  }
-  std::vector<int> idx(static_cast<size_t>(nj));
-  for (int k = 0; k < nj; ++k) idx[size_t(k)] = k;
-  // longest first; within one length, jobs of equal row counts together, so
-  // a warp's lanes run the same inner loops (no divergence between na x nb
-  // splits of one length)
-  std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) {
-    if (cost[size_t(x)] != cost[size_t(y)]) return cost[size_t(x)] > cost[size_t(y)];
-    return (desc[size_t(x)].w & 0xff) > (desc[size_t(y)].w & 0xff);
-  });
-  const int nchunk = (nj + 31) / 32, nround = (nchunk + SNAP_WARPS - 1) / SNAP_WARPS;
-  std::vector<int4> out(size_t(nround) * SNAP_THREADS, int4{-1, 0, 0, 0});
-  for (int c = 0; c < nchunk; ++c) {
-    const int r = c / SNAP_WARPS, p = c % SNAP_WARPS, w = (r & 1) ? SNAP_WARPS - 1 - p : p;
-    for (int l = 0; l < 32 && 32 * c + l < nj; ++l)
-      out[size_t(r) * SNAP_THREADS + 32 * size_t(w) + l] = desc[size_t(idx[size_t(32 * c + l)])];
-  }
-  return out;
+double jacobi_A(int al, int be, int k) {  // monic Jacobi P_k^(al, be): P_{k+1} = (x - A) P_k - B P_{k-1}
+  const double s = 2.0 * k + al + be;
+  if (k == 0) return (be - al) / (s + 2.0);
+  return (double(be) * be - double(al) * al) / (s * (s + 2.0));
+}
+double jacobi_B(int al, int be, int k) {
+  if (k == 0) return 0.0;
+  const double s = 2.0 * k + al + be;
+  return 4.0 * k * (k + al) * (k + be) * (k + al + be) / (s * s * (s + 1.0) * (s - 1.0));
 }
 
-// bytes of the `work` region: the neighbour slots' half layers (B), Z jobs
-// (C), the forward layers and adjoints of d_reverse (D), or the fitting
-// adjoint's per-warp U and dU layers
-size_t snap_work_bytes(const SnapDev& S, int real_bytes) {
-  const int L2 = S.L * S.L, J = S.twojmax;
-  const size_t wB = 2 * sizeof(double) * size_t(SNAP_WARPS) * BG * size_t(S.bh_even + S.bh_odd);
-  const size_t wC = 2 * size_t(real_bytes) * size_t(S.njobs);
-  size_t wD = 2 * size_t(real_bytes) * size_t(SNAP_WARPS) * 2 * size_t(drev_words(J));
-  if (real_bytes == int(sizeof(double)))  // the fitting adjoint's U and tangent layers
-    wD = std::max(wD, 2 * sizeof(double) * size_t(SNAP_WARPS) * 4 * L2);
-  return (std::max(wB, std::max(wC, wD)) + 15) & ~size_t(15);
-}
+// The tables of one twojmax (see the structures in snap_kernel.cuh)
+struct SnapTables {
+  std::vector<Entry> ent;
+  std::vector<int> e0, zt0, tmask;
+  std::vector<int2> xsum, half, zt, prod;
+  std::vector<int4> hfull;
+  std::vector<ZTask> task;
+  std::vector<ZRec> rec;
+  std::vector<double> zc, AB;
+  std::vector<float2> zc_f;
+  int nz = 0, nh = 0;
 
-// the adjoint's extra shared memory after `work`: kept Z, per-warp D partials, D
-size_t snap_adjoint_bytes(const SnapDev& S) {
-  return 2 * sizeof(double) * (size_t(S.njobs) + size_t(SNAP_WARPS + 1) * S.nyh);
-}
-
-// the kernel's shared-memory carve-up (k_snap), for `cap` inside neighbours
-size_t snap_smem_bytes(const SnapDev& S, int cap, int real_bytes) {
-  const bool f64 = real_bytes == int(sizeof(double));
-  const size_t nd = f64 ? size_t(ND_FIELDS) : size_t(ND_MIXED), nr = f64 ? 0 : size_t(NR_MIXED);
-  size_t b = 0;
-  b += sizeof(double) * 5 * size_t(cap);                                // r, w, rcut
-  b += 2 * sizeof(double) * size_t(S.nuf);                              // utot
-  b += 2 * size_t(real_bytes) * size_t(S.nyh);                          // ytot
-  if (!f64) b += 2 * size_t(real_bytes) * size_t(S.nuf);               // FP32 U_tot
-  b += sizeof(int) * size_t((cap + 3) & ~3);                            // inside j
-  b += sizeof(double) * 4 * SNAP_WARPS;                                 // reductions
-  b += sizeof(double) * nd * size_t(cap);                               // FP64 per-neighbour fields
-  b += sizeof(double) * ((nr * size_t(cap) + 1) / 2);                   // FP32 per-neighbour fields
-  b += snap_work_bytes(S, real_bytes);
-  return b + 64;
-}
-
-// the largest number of inside neighbours (r^2 < rcutmax^2) over the owned
-// atoms: the kernel's per-neighbour shared arrays are sized by it
-__global__ void __launch_bounds__(256) k_snap_inside_max(const double4_32a* __restrict__ x4, ListView L, int n,
-                                                         double cutsq, int* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int cnt = 0;
-  if (i < n) {
-    const double4_32a xi = x4[i];
-    const Row<false> rowc(L, i);
-    const Row<true> row2(L, i);
-    const bool two_d = L.stride != 0;
-    for (int k = 0; k < rowc.n; ++k) {
-      const int j = two_d ? row2[k] : rowc[k];
-      const double4_32a xj = x4[j];
-      const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-      cnt += (dx * dx + dy * dy + dz * dz) < cutsq;
+  SnapTables(int J, const std::vector<int>& trip) {
+    const int L = J + 1, ntrip = int(trip.size() / 3);
+    auto uidx = [](int j, int ma, int mb) { return j * (j + 1) * (2 * j + 1) / 6 + ma * (j + 1) + mb; };
+    // entries, real sums and their table columns (k_snap_u: powers of a, of b,
+    // then the products in (T, q, k) order)
+    e0.assign(size_t(L) * L, -1);
+    int col = 4 * L;
+    for (int T = 0; T <= J; ++T)
+      for (int q = 0; q <= J - T; ++q) {
+        e0[size_t(T) * L + q] = int(ent.size());
+        for (int k = 0; q + T + 2 * k <= J; ++k) {
+          const int j = q + T + 2 * k, ma = (j - q - T) / 2, mb = (j - q + T) / 2;
+          Entry E{};
+          E.N = std::ldexp(factorial(j) / std::sqrt(factorial(ma) * factorial(j - ma) * factorial(mb) * factorial(j - mb)),
+                           -k);
+          E.invN = 1.0 / E.N;
+          E.A = jacobi_A(T, q, k);
+          E.B = jacobi_B(T, q, k);
+          AB.push_back(E.A);
+          AB.push_back(E.B);
+          E.T = T;
+          E.q = q;
+          E.j = j;
+          E.ep = uidx(j, ma, mb);
+          E.em = uidx(j, mb, ma);
+          E.mp = uidx(j, j - ma, j - mb);
+          E.mm = uidx(j, j - mb, j - ma);
+          E.xo = int(xsum.size());
+          const int cu = k == 0 ? 2 * L + 2 * T : col, cv = cu + 1, cp = 2 * q, cr = 2 * q + 1;
+          if (k > 0) col += T > 0 ? 2 : 1;
+          xsum.push_back(int2{cp, cu});
+          if (q > 0) xsum.push_back(int2{cr, cu});
+          if (T > 0) xsum.push_back(int2{cp, cv});
+          if (q > 0 && T > 0) xsum.push_back(int2{cr, cv});
+          half.push_back(int2{nh, q > 0 && T > 0 ? nh + 1 : -1});
+          nh += q > 0 && T > 0 ? 2 : 1;
+          const int sign = T & 1 ? -1 : 1;  // (-1)^(ma + mb)
+          hfull.push_back(int4{E.ep, E.mp, sign, 0});
+          if (q > 0 && T > 0) hfull.push_back(int4{E.em, E.mm, sign, 0});
+          ent.push_back(E);
+        }
+      }
+    // Clebsch-Gordan coefficients of every (j1, j2): for each (m1, m2) the
+    // allowed j from the highest down
+    std::vector<int> cgo(size_t(L) * L), njt(size_t(L) * L), ttop(size_t(L) * L);
+    std::vector<double> cg;
+    for (int j1 = 0; j1 <= J; ++j1)
+      for (int j2 = 0; j2 <= j1; ++j2) {
+        const size_t pr = size_t(j1) * L + j2;
+        const int lo = j1 - j2, hi = std::min(J - ((J + j1 + j2) & 1), j1 + j2);
+        cgo[pr] = int(cg.size());
+        njt[pr] = (hi - lo) / 2 + 1;
+        for (int m1 = 0; m1 <= j1; ++m1)
+          for (int m2 = 0; m2 <= j2; ++m2)
+            for (int j = hi; j >= lo; j -= 2) cg.push_back(clebsch_gordan(j1, j2, j, m1, m2));
+        for (int t = 0; t < ntrip; ++t)
+          if (trip[3 * size_t(t)] == j1 && trip[3 * size_t(t) + 1] == j2 && trip[3 * size_t(t) + 2] == hi) ttop[pr] = t;
+      }
+    // Z tasks, longest first
+    struct Raw {
+      ZTask t;
+      std::vector<ZRec> r[2];
+      long long cost;
+    };
+    std::vector<int2> rp;    // products and coefficients in record order
+    std::vector<double> rc;  // before the tasks are sorted
+    std::vector<Raw> raw;
+    for (int T = 0; T <= J; ++T)
+      for (int q = 0; q <= J - T; ++q) {
+        Raw w{};
+        w.t.T = T;
+        w.t.q = q;
+        w.t.y0 = e0[size_t(T) * L + q];
+        w.t.kmax = (J - q - T) / 2;
+        const int top = q + T + 2 * w.t.kmax;
+        for (int s = 0; s < (T > 0 && q > 0 ? 2 : 1); ++s)
+          for (int j1 = 0; j1 <= J; ++j1)
+            for (int j2 = 0; j2 <= j1; ++j2) {
+              if ((j1 + j2 - q - T) & 1) continue;
+              const size_t pr = size_t(j1) * L + j2;
+              const int hi = j1 - j2 + 2 * (njt[pr] - 1), lo = std::max(j1 - j2, q + T);
+              if (hi < lo) continue;
+              const int sT = s ? -T : T, M = (j1 + j2 - q - sT) / 2, Mp = (j1 + j2 - q + sT) / 2;
+              ZRec z{};
+              z.nj = short((hi - lo) / 2 + 1);
+              z.d = short((top - hi) / 2);
+              z.t0 = ttop[pr];
+              z.p0 = int(rp.size());
+              z.c0 = int(rc.size());
+              for (int m1 = std::max(0, M - j2); m1 <= std::min(j1, M); ++m1)
+                for (int n1 = std::max(0, Mp - j2); n1 <= std::min(j1, Mp); ++n1) {
+                  const int m2 = M - m1, n2 = Mp - n1;
+                  // j1 = j2: (m1, n1)(m2, n2) and (m2, n2)(m1, n1) are one product
+                  if (j1 == j2 && (m2 < m1 || (m2 == m1 && n2 < n1))) continue;
+                  const double twice = j1 == j2 && !(m1 == m2 && n1 == n2) ? 2.0 : 1.0;
+                  rp.push_back(int2{uidx(j1, m1, n1), uidx(j2, m2, n2)});
+                  for (int j = 0; j < z.nj; ++j)
+                    rc.push_back(twice * cg[size_t(cgo[pr] + (m1 * (j2 + 1) + m2) * njt[pr] + j)] *
+                                 cg[size_t(cgo[pr] + (n1 * (j2 + 1) + n2) * njt[pr] + j)]);
+                }
+              z.np = int(rp.size()) - z.p0;
+              w.cost += (long long)z.np * (4 + 2 * z.nj);
+              w.r[s].push_back(z);
+            }
+        raw.push_back(std::move(w));
+      }
+    std::stable_sort(raw.begin(), raw.end(), [](const Raw& x, const Raw& y) { return x.cost > y.cost; });
+    std::vector<std::vector<int2>> by_t(static_cast<size_t>(ntrip));
+    for (Raw& w : raw) {
+      w.t.rec0 = int(rec.size());
+      for (int s = 0; s < 2; ++s) {
+        for (ZRec& z : w.r[s]) {
+          const int rp0 = z.p0, rc0 = z.c0;
+          z.p0 = int(prod.size());
+          z.c0 = int(zc.size());
+          z.cf = int(zc_f.size());
+          prod.insert(prod.end(), rp.begin() + rp0, rp.begin() + rp0 + z.np);
+          zc.insert(zc.end(), rc.begin() + rc0, rc.begin() + rc0 + z.np * z.nj);
+          for (int k = 0; k < z.np; ++k) {
+            for (int j = 0; j < z.nj; ++j) zc_f.push_back(make_float2(float(rc[rc0 + k * z.nj + j]), float(rc[rc0 + k * z.nj + j])));
+            if (z.nj & 1) zc_f.push_back(make_float2(0.f, 0.f));
+          }
+          z.z0 = nz;
+          for (int j = 0; j < z.nj; ++j) {  // highest j first: entry kmax - d - j of the task
+            const int2 h = half[size_t(w.t.y0 + w.t.kmax - z.d - j)];
+            by_t[size_t(z.t0 - j)].push_back(int2{nz, s ? h.y : h.x});
+            ++nz;
+          }
+          rec.push_back(z);
+        }
+        (s ? w.t.rec2 : w.t.rec1) = int(rec.size());
+      }
+      task.push_back(w.t);
+    }
+    for (const auto& v : by_t) {
+      zt0.push_back(int(zt.size()));
+      zt.insert(zt.end(), v.begin(), v.end());
+    }
+    zt0.push_back(int(zt.size()));
+    // four groups of T of about equal work (k_snap_force)
+    std::vector<long long> load(4, 0);
+    tmask.assign(4, 0);
+    std::vector<std::pair<long long, int>> tw;
+    for (int T = 0; T <= J; ++T) {
+      long long wk = 0;
+      for (int q = 0; q <= J - T; ++q) wk += (T ? 2 : 1) * (8 + 8 * ((J - T - q) / 2));
+      tw.push_back({-wk, T});
+    }
+    std::sort(tw.begin(), tw.end());
+    for (const auto& w : tw) {
+      const size_t g = size_t(std::min_element(load.begin(), load.end()) - load.begin());
+      load[g] -= w.first;
+      tmask[g] |= 1 << w.second;
     }
   }
-  cnt = __reduce_max_sync(FULL_MASK, cnt);
-  if ((threadIdx.x & 31) == 0 && cnt > 0) atomicMax(out, cnt);
+};
+
+// They depend on twojmax alone: built once per process, shared and read-only.
+const SnapTables& snap_tables(int J, const std::vector<int>& trip) {
+  static std::mutex mu;
+  static std::unique_ptr<const SnapTables> tables[15];
+  std::lock_guard<std::mutex> lock(mu);
+  if (!tables[J]) tables[J] = std::make_unique<const SnapTables>(J, trip);
+  return *tables[J];
 }
 
 // per-element column sums of the adjoint's per-atom outputs (fixed order)
@@ -191,21 +292,23 @@ __global__ void __launch_bounds__(256) k_adj_reduce(const double* __restrict__ a
 void free_snap(Ctx& c) {
   if (!c.snap) return;
   SnapHost* h = static_cast<SnapHost*>(c.snap);
-  for (auto* b : {&h->trip, &h->cg_off, &h->jobs, &h->tjob_off, &h->yred_off, &h->yred_job, &h->map}) b->release();
-  h->zord.release();
-  h->inside_max.release();
-  for (auto* b : {&h->cg, &h->cY, &h->beta0, &h->radelem, &h->wjelem, &h->eatom, &h->adj, &h->adj_sum,
-                  &h->adj_g, &h->invf, &h->yscale, &h->keep_u, &h->keep_z})
+  h->ent.release();
+  h->task.release();
+  h->rec.release();
+  h->D.release();
+  h->H.release();
+  h->hfull.release();
+  h->zc_f.release();
+  for (auto* b : {&h->e0, &h->map, &h->zt0, &h->tmask, &h->pj, &h->cnt}) b->release();
+  for (auto* b : {&h->xsum, &h->half, &h->zt, &h->prod}) b->release();
+  for (auto* b : {&h->zc, &h->cY, &h->AB, &h->beta0, &h->wjelem, &h->pr, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk,
+                  &h->eatom, &h->adj, &h->adj_sum, &h->adj_g, &h->keep_u, &h->keep_z})
     b->release();
-  for (auto* b : {&h->cg_f, &h->cY_f, &h->yscale_f}) b->release();
+  for (auto* b : {&h->cY_f, &h->AB_f}) b->release();
   delete h;
   c.snap = nullptr;
 }
 
-static void upload_i(Ctx& c, DevBuf<int>& b, const std::vector<int>& v) {
-  b.reserve(v.size() + 1, c.stream);
-  EMD_CUDA(cudaMemcpyAsync(b.p, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, c.stream));
-}
 template <class T>
 static void upload(Ctx& c, DevBuf<T>& b, const std::vector<T>& v) {
   b.reserve(v.size() + 1, c.stream);
@@ -232,94 +335,160 @@ void snap_fold_beta(const SnapHost& h, int nfull, int nelem, int ncoeffall, cons
   }
 }
 
-// cap for the kernel's per-neighbour arrays: the largest inside count
-static int snap_cap(Ctx& c, SnapHost* h) {
-  const int n = c.N_local;
-  h->inside_max.reserve(1, c.stream);
-  EMD_CUDA(cudaMemsetAsync(h->inside_max.p, 0, sizeof(int), c.stream));
-  {
-    TimedLaunch t(c, "snap_inside_max");
-    k_snap_inside_max<<<blocks_for(n, 256), 256, 0, c.stream>>>(c.x4.p, list_view(c), n, h->d.cutsq,
-                                                                 h->inside_max.p);
-    EMD_CHECK_LAUNCH();
+// Atoms are worked on in chunks so that the work arrays stay bounded: at most
+// kChunk atoms and about kChunkBytes of pair fields.
+constexpr int kChunk = 131072;
+constexpr size_t kChunkBytes = size_t(3) << 30;
+
+static int snap_chunk(int n, int cap, bool adjoint_z, const SnapDev& S) {
+  size_t per = size_t(cap) * (8 * (PD_N + PF_N) + 4);
+  if (adjoint_z) per += size_t(16) * S.nz;
+  const size_t most = std::max<size_t>(32, std::min<size_t>(kChunk, kChunkBytes / per));
+  const int chunks = int((size_t(n) + most - 1) / most);
+  return std::min(n, ((n + chunks - 1) / chunks + 31) & ~31);
+}
+
+// Atoms per tile of k_snap_y.  A tile costs the same whatever its lanes hold,
+// so 32 atoms where the tiles (and their tasks, split over up to four CTAs)
+// fill the 152 SMs, fewer atoms with the rows shared by lane groups (0.89,
+// 0.73, 0.53 of the lanes' work useful at 16, 8, 4) where they would not.
+static int snap_tile_atoms(const SnapDev& S, int n, size_t real, bool keep) {
+  int ta = 32;
+  if (!keep)
+    while (ta > 4 && (n + ta - 1) / ta * 4 < 152) ta /= 2;
+  while (ta > 1 && snap_y_smem(S, ta, real) > kMaxDynSmem) ta /= 2;
+  return ta;
+}
+// CTAs that share a tile's tasks: the number (up to four: the longest task is
+// 7% of a tile) that wastes least of the last wave
+static int snap_tile_split(int tiles, int resident) {
+  int best = 1;
+  double best_cost = 1e300;
+  for (int k = 1; k <= 4; ++k) {
+    const long long ctas = (long long)tiles * k, wave = 152LL * resident;
+    const double cost = double((ctas + wave - 1) / wave) / k + 0.01 * k;
+    if (cost < best_cost) {
+      best = k;
+      best_cost = cost;
+    }
   }
-  EMD_CUDA(cudaMemcpyAsync(c.h_int, h->inside_max.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-  EMD_CUDA(cudaStreamSynchronize(c.stream));
-  return std::max(1, c.h_int[0]);
+  return best;
+}
+
+// arguments of one chunk, work arrays reserved
+static SnapArgs snap_args(Ctx& c, SnapHost* h, int first, int n, bool fp64, bool keep) {
+  const SnapDev& S = h->d;
+  const size_t real = fp64 ? 8 : 4;
+  SnapArgs A{};
+  A.S = S;
+  A.x4 = c.x4.p;
+  A.type = c.type.p;
+  A.L = list_view(c);
+  A.first = first;
+  A.n = n;
+  A.n_local = c.N_local;
+  A.cap = std::max(1, c.neigh_maxrow);
+  A.rows = std::min(SP_ROWS, std::max(1, n / (152 * 8)));
+  const size_t np = size_t(n) * A.cap;
+  h->pd.reserve(PD_N * np, c.stream);
+  h->pr_f.reserve(fp64 ? PF_N * np : (PR_N * np + 1) / 2, c.stream);
+  h->pj.reserve(np, c.stream);
+  h->cnt.reserve(size_t(n), c.stream);
+  A.pd = h->pd.p;
+  A.pr = h->pr_f.p;
+  A.pj = h->pj.p;
+  A.cnt = h->cnt.p;
+  A.ta = snap_tile_atoms(S, c.N_local, real, keep);
+  const int tiles = (n + A.ta - 1) / A.ta;
+  A.nsplit = snap_tile_split(tiles, fp64 ? 1 : 2);
+  h->Y.reserve((size_t(tiles) * 4 * S.ne * A.ta * real + 7) / 8, c.stream);
+  A.Y = h->Y.p;
+  A.f = c.f.p;
+  A.tmask = h->tmask.p;
+  return A;
+}
+
+// U_tot and Y of a chunk
+static void snap_uy(Ctx& c, const SnapArgs& A, bool fp64) {
+  {
+    TimedLaunch t(c, "snap_pairs");
+    if (fp64) launch_pairs<double>(A, c.stream);
+    else snap_mixed_pairs(A, c.stream);
+  }
+  {
+    TimedLaunch t(c, "snap_u");
+    if (fp64) launch_u<double>(A, c.stream);
+    else snap_mixed_u(A, c.stream);
+  }
+  TimedLaunch t(c, fp64 ? "snap_y_fp64" : "snap_y_mixed");
+  if (!fp64) snap_mixed_y(A, c.stream);
+  else if (A.S.twojmax <= 9) launch_y<double, 5>(A, c.stream);
+  else launch_y<double, 8>(A, c.stream);
+}
+
+static void snap_require_list(Ctx& c, const char* what) {
+  require(c.neigh_ready && c.neigh_rows == c.N_local && !c.half_neigh, EMD_ERR_STATE, what);
+  require(!c.neigh_packed, EMD_ERR_STATE, "SNAP reads plain neighbour rows");
 }
 
 static void snap_launch(Ctx& c, bool energy) {
   SnapHost* h = static_cast<SnapHost*>(c.snap);
   require(h != nullptr, EMD_ERR_STATE, "SNAP not initialised");
-  require(c.neigh_ready && c.neigh_rows == c.N_local && !c.half_neigh, EMD_ERR_STATE,
-          "SNAP needs a current full neighbour list");
-  require(!c.neigh_packed, EMD_ERR_STATE, "SNAP reads plain neighbour rows");
+  snap_require_list(c, "SNAP needs a current full neighbour list");
   const int n = c.N_local;
   if (n == 0) return;
   if (!energy) {
     materialize_kick(c);  // the forces are about to be overwritten
     materialize_zero(c, true, true);
   }
-  SnapArgs A;
-  A.S = h->d;
-  A.x4 = c.x4.p;
-  A.type = c.type.p;
-  A.f = c.f.p;
-  A.L = list_view(c);
-  A.n_local = n;
-  A.cap = snap_cap(c, h);
-  A.status = c.d_status;
-  A.eatom = nullptr;
+  const SnapDev& S = h->d;
   const bool fp64 = h->precision == EMD_PREC_FP64 || energy;
-  const size_t smem = snap_smem_bytes(h->d, A.cap, fp64 ? 8 : 4);
-  require(smem <= 227 * 1024, EMD_ERR_ARG, "SNAP: neighbour rows too long for one atom's shared memory");
-  A.g = nullptr;
-  A.ghost_owner = nullptr;
-  A.newton = 0;
-  A.adj = nullptr;
-  A.work_bytes = snap_work_bytes(h->d, fp64 ? 8 : 4);
-  if (energy) {
-    h->eatom.reserve(size_t(n), c.stream);
-    A.eatom = h->eatom.p;
-    auto k = k_snap<double, 1>;
-    EMD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    TimedLaunch t(c, "snap_energy");
-    k<<<n, SNAP_THREADS, smem, c.stream>>>(A);
-    EMD_CHECK_LAUNCH();
-    return;
+  // asked for (emd_snap_request_energy): the per-atom energies in the same pass
+  const bool fused = !energy && fp64 && c.snap_energy_request;
+  const bool keep = !energy && fp64 && h->keep_on;
+  if (energy || fused) h->eatom.reserve(size_t(n), c.stream);
+  if (keep) {
+    h->keep_u.reserve(2 * size_t(S.nh) * n, c.stream);
+    h->keep_z.reserve(2 * size_t(S.nz) * ((size_t(n) + 31) & ~size_t(31)), c.stream);
   }
-  if (fp64) {
-    // asked for (emd_snap_request_energy): the per-atom energies in the same pass
-    const bool fused = c.snap_energy_request;
-    if (fused) {
-      h->eatom.reserve(size_t(n), c.stream);
+  const int chunk = snap_chunk(n, std::max(1, c.neigh_maxrow), false, S);
+  for (int first = 0; first < n; first += chunk) {
+    SnapArgs A = snap_args(c, h, first, std::min(chunk, n - first), fp64, fp64 && h->keep_on);
+    if (keep) {
+      A.U = h->keep_u.p + 2 * size_t(S.nh) * first;
+      A.zkeep = h->keep_z.p + 2 * size_t(S.nz) * first;
+    } else {
+      h->U.reserve(2 * size_t(S.nh) * A.n, c.stream);
+      A.U = h->U.p;
+    }
+    snap_uy(c, A, fp64);
+    if (energy || fused) {
       A.eatom = h->eatom.p;
+      TimedLaunch t(c, "snap_energy");
+      k_snap_energy<<<(A.n + 3) / 4, 128, 0, c.stream>>>(A);
+      EMD_CHECK_LAUNCH();
     }
-    if (h->keep_on) {
-      h->keep_u.reserve(2 * size_t(h->d.nuf) * n, c.stream);
-      h->keep_z.reserve(2 * size_t(h->d.njobs) * n, c.stream);
-      A.keep_u = reinterpret_cast<Cplx<double>*>(h->keep_u.p);
-      A.keep_z = reinterpret_cast<Cplx<double>*>(h->keep_z.p);
-    }
-    auto k = k_snap<double, 0>;
-    EMD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    TimedLaunch t(c, fused ? "snap_fp64_energy" : "snap_fp64");
-    k<<<n, SNAP_THREADS, smem, c.stream>>>(A);
-    if (fused) {
-      c.snap_pe_fused_valid = true;
-      c.snap_pe_fused_version = c.x_version;
-    }
-    if (h->keep_on) {
-      h->keep_valid = true;
-      h->keep_xver = c.x_version;
-      h->keep_builds = c.neigh_builds;
-      h->keep_n = n;
-    }
-  } else {
-    TimedLaunch t(c, "snap_mixed");
-    snap_mixed_launch(A, smem, c.stream);
+    if (energy) continue;
+    // Eight atoms pool about 208 pairs for 256 lanes; a small system takes one
+    // atom per CTA and spreads the T of a pair over four warps
+    A.apc = std::max(1, std::min(SF_ATOMS, A.n / 152));
+    A.tsplit = A.apc < 4 ? 4 : 1;
+    const int threads = A.tsplit == 4 ? 32 * 4 * std::max(1, std::min(2, A.apc)) : SF_THREADS;
+    TimedLaunch t(c, fp64 ? "snap_force_fp64" : "snap_force_mixed");
+    if (!fp64) snap_mixed_force(A, threads, c.stream);
+    else if (S.twojmax <= 8) launch_force<double, 9>(A, threads, c.stream);
+    else launch_force<double, 15>(A, threads, c.stream);
   }
-  EMD_CHECK_LAUNCH();
+  if (fused) {
+    c.snap_pe_fused_valid = true;
+    c.snap_pe_fused_version = c.x_version;
+  }
+  if (keep) {
+    h->keep_valid = true;
+    h->keep_xver = c.x_version;
+    h->keep_builds = c.neigh_builds;
+    h->keep_n = n;
+  }
 }
 
 // d/dbeta of (dL_dE * E + sum_i dL_dF_i . F_i) for a loss L(E, F) of the
@@ -337,34 +506,45 @@ static void snap_adjoint(Ctx& c, const double* dL_dF, double dL_dE, double* grad
     EMD_CUDA(cudaMemcpyAsync(h->adj_g.p, dL_dF, sizeof(double) * 3 * size_t(n), cudaMemcpyHostToDevice, c.stream));
     h->adj.reserve(size_t(ncols) * n, c.stream);
     h->adj_sum.reserve(size_t(nelem) * ncols, c.stream);
-    SnapArgs A;
-    A.S = S;
-    A.x4 = c.x4.p;
-    A.type = c.type.p;
-    A.f = nullptr;
-    A.L = list_view(c);
-    A.n_local = n;
-    A.cap = snap_cap(c, h);
-    A.status = c.d_status;
-    A.eatom = nullptr;
-    A.g = h->adj_g.p;
-    A.ghost_owner = c.ghost_owner.p;
-    A.newton = c.comm_newton;
-    A.adj = h->adj.p;
-    A.work_bytes = snap_work_bytes(S, 8);
-    // B and C from the last FP64 force pass, when it ran on these positions and this list
-    if (h->keep_on && h->keep_valid && h->keep_xver == c.x_version && h->keep_builds == c.neigh_builds &&
-        h->keep_n == n) {
-      A.keep_u = reinterpret_cast<Cplx<double>*>(h->keep_u.p);
-      A.keep_z = reinterpret_cast<Cplx<double>*>(h->keep_z.p);
-    }
-    const size_t smem = snap_smem_bytes(S, A.cap, 8) + snap_adjoint_bytes(S);
-    require(smem <= 227 * 1024, EMD_ERR_ARG, "SNAP adjoint: neighbour rows too long for shared memory");
-    auto k = k_snap<double, 2>;
-    EMD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    {
+    // U_tot and Z from the last FP64 force pass, when it ran on these positions and this list
+    const bool kept = h->keep_on && h->keep_valid && h->keep_xver == c.x_version && h->keep_builds == c.neigh_builds &&
+                      h->keep_n == n;
+    const int chunk = snap_chunk(n, std::max(1, c.neigh_maxrow), true, S);
+    for (int first = 0; first < n; first += chunk) {
+      SnapArgs A = snap_args(c, h, first, std::min(chunk, n - first), true, true);
+      const int tiles = (A.n + 31) / 32;
+      if (kept) {
+        A.U = h->keep_u.p + 2 * size_t(S.nh) * first;
+        A.zkeep = h->keep_z.p + 2 * size_t(S.nz) * first;
+        TimedLaunch t(c, "snap_pairs");
+        launch_pairs<double>(A, c.stream);
+      } else {
+        h->U.reserve(2 * size_t(S.nh) * A.n, c.stream);
+        h->zk.reserve(2 * size_t(S.nz) * tiles * 32, c.stream);
+        A.U = h->U.p;
+        A.zkeep = h->zk.p;
+        snap_uy(c, A, true);
+      }
+      h->D.reserve(size_t(S.nh) * A.n, c.stream);
+      h->H.reserve(size_t(tiles) * 2 * S.nh * 32, c.stream);
+      A.D = h->D.p;
+      A.H = h->H.p;
+      A.g = h->adj_g.p;
+      A.ghost_owner = c.ghost_owner.p;
+      A.newton = c.comm_newton;
+      A.adj = h->adj.p;
+      {
+        TimedLaunch t(c, "snap_dt");
+        const size_t smem = sizeof(double) * (size_t((S.nx + 1) & ~1) + 64 * size_t(S.cols));
+        require(smem <= kMaxDynSmem, EMD_ERR_ARG, "SNAP adjoint: twojmax too large for shared memory");
+        allow_dyn_smem(k_snap_dt);
+        k_snap_dt<<<A.n, 32, smem, c.stream>>>(A);
+        EMD_CHECK_LAUNCH();
+      }
       TimedLaunch t(c, "snap_adjoint");
-      k<<<n, SNAP_THREADS, smem, c.stream>>>(A);
+      k_snap_half<<<blocks_for((long long)tiles * S.nh * 32, 256), 256, 0, c.stream>>>(A);
+      EMD_CHECK_LAUNCH();
+      k_snap_pq<<<dim3(tiles, (S.nfull + 7) / 8), 256, 0, c.stream>>>(A);
       EMD_CHECK_LAUNCH();
     }
     {
@@ -415,8 +595,6 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   h->precision = precision;
   SnapDev& S = h->d;
   S.twojmax = twojmax;
-  S.L = twojmax + 1;
-  const int L = S.L;
   // index lists (SNA::build_indexlist, sna_impl.hpp:88-139, diagonalstyle 3)
   std::vector<int> trip;
   std::vector<int> idxj;  // positions of the idxj triples (j >= j1) in the full list
@@ -442,43 +620,14 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
       if (trip[3 * t] == a && trip[3 * t + 1] == b && trip[3 * t + 2] == cc) return t;
     throw Error(EMD_ERR_ARG, "SNAP: triple not found");
   };
-  // compact CG blocks
-  std::vector<int> cg_off(static_cast<size_t>(S.nfull));
-  std::vector<double> cg;
-  for (int t = 0; t < S.nfull; ++t) {
-    const int a = trip[3 * t], b = trip[3 * t + 1], cc = trip[3 * t + 2];
-    cg_off[size_t(t)] = int(cg.size());
-    for (int m1 = 0; m1 <= a; ++m1)
-      for (int m2 = 0; m2 <= b; ++m2) cg.push_back(clebsch_gordan(a, b, cc, m1, m2));
-  }
-  // Z jobs over the half grid of every triple, grouped by Y element
-  auto yoff_h = [](int j) {
-    int s = 0;
-    for (int k = 0; k < j; ++k) s += (k + 1) * (k / 2 + 1);
-    return s;
-  };
-  S.nyh = yoff_h(L);
-  S.nuf = L * (L + 1) * (2 * L + 1) / 6;
-  std::vector<std::vector<int>> by_y(static_cast<size_t>(S.nyh));
-  std::vector<int> jobs, tjob_off;
-  for (int t = 0; t < S.nfull; ++t) {
-    const int cc = trip[3 * t + 2];
-    tjob_off.push_back(int(jobs.size()));
-    for (int mb = 0; 2 * mb <= cc; ++mb)
-      for (int ma = 0; ma <= cc; ++ma) {
-        by_y[size_t(yoff_h(cc) + mb * (cc + 1) + ma)].push_back(int(jobs.size()));
-        jobs.push_back((t << 8) | (ma << 4) | mb);
-      }
-  }
-  S.njobs = int(jobs.size());
-  tjob_off.push_back(S.njobs);
-  const std::vector<int4> zord = zjob_order(trip, cg_off, jobs);
-  std::vector<int> yred_off(size_t(S.nyh) + 1, 0), yred_job;
-  for (int e = 0; e < S.nyh; ++e) {
-    yred_off[size_t(e)] = int(yred_job.size());
-    for (int jb : by_y[size_t(e)]) yred_job.push_back(jb);
-  }
-  yred_off[size_t(S.nyh)] = int(yred_job.size());
+  const SnapTables& tab = snap_tables(twojmax, trip);
+  S.ne = int(tab.ent.size());
+  S.nx = int(tab.xsum.size());
+  S.cols = su_cols(twojmax);
+  S.nuf = (twojmax + 1) * (twojmax + 2) * (2 * twojmax + 3) / 6;
+  S.ntask = int(tab.task.size());
+  S.nz = tab.nz;
+  S.nh = tab.nh;
   for (int k = 0; k < S.ncoeff; ++k) {
     const int j1 = idx3[3 * k], j2 = idx3[3 * k + 1], j = idx3[3 * k + 2];
     h->k_t1.push_back(find_full(j1, j2, j));
@@ -490,72 +639,65 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   }
   std::vector<double> cY, beta0;
   snap_fold_beta(*h, S.nfull, nelem, ncoeffall, beta, cY, beta0);
-  // over the half grid: 1 / f_j(ma, mb) of the rescaled recursion and the
-  // D contraction's Y scale (twice the half-grid weight over f); the largest
-  // half layer of even and odd j
-  std::vector<double> invf(static_cast<size_t>(S.nyh));
-  std::vector<double> yscale(static_cast<size_t>(S.nyh));
-  S.bh_even = S.bh_odd = 1;
-  for (int j = 0; j <= twojmax; ++j) {
-    const int nh = (j + 1) * (j / 2 + 1);
-    (j & 1 ? S.bh_odd : S.bh_even) = std::max(j & 1 ? S.bh_odd : S.bh_even, nh);
-    for (int mb = 0; 2 * mb <= j; ++mb)
-      for (int ma = 0; ma <= j; ++ma) {
-        const size_t e = size_t(yoff_h(j) + mb * (j + 1) + ma);
-        invf[e] = std::sqrt(factorial(j - ma) * factorial(ma) / (factorial(j - mb) * factorial(mb)));
-        // twice the half-grid contraction weight (sna_impl.hpp:384-413)
-        const double w2 = (2 * mb < j || 2 * ma < j) ? 2.0 : (2 * ma == j ? 1.0 : 0.0);
-        yscale[e] = w2 * invf[e];
-      }
-  }
   double rcutmax = 0.0;
   for (int e = 0; e < nelem; e++) rcutmax = std::max(2.0 * radelem[e] * rcutfac, rcutmax);
   S.rfac0 = rfac0;
   S.rmin0 = rmin0;
-  S.rcutfac = rcutfac;
   S.cutsq = rcutmax * rcutmax;
   S.wself = 1.0;
   S.switchflag = switchflag;
   S.nelem = nelem;
   S.ntypes = ntypes;
-  upload_i(c, h->trip, trip);
-  upload_i(c, h->cg_off, cg_off);
-  upload(c, h->cg, cg);
-  std::vector<float> cgf(cg.begin(), cg.end()), cYf(cY.begin(), cY.end());
-  upload(c, h->cg_f, cgf);
-  upload_i(c, h->jobs, jobs);
-  h->zord.reserve(zord.size(), c.stream);
-  EMD_CUDA(cudaMemcpyAsync(h->zord.p, zord.data(), sizeof(int4) * zord.size(), cudaMemcpyHostToDevice, c.stream));
-  S.nzo = int(zord.size());
-  upload_i(c, h->tjob_off, tjob_off);
-  upload_i(c, h->yred_off, yred_off);
-  upload_i(c, h->yred_job, yred_job);
+  // per element pair: cutoff, theta0 and switching slopes (compute_ui, compute_sfac)
+  std::vector<double> pr;
+  for (int a = 0; a < nelem; ++a)
+    for (int b = 0; b < nelem; ++b) {
+      const double rcut = (radelem[a] + radelem[b]) * rcutfac;
+      pr.push_back(rcut);
+      pr.push_back(rfac0 * MY_PI / (rcut - rmin0));
+      pr.push_back(MY_PI / (rcut - rmin0));
+    }
+  const std::vector<float> cYf(cY.begin(), cY.end()), ABf(tab.AB.begin(), tab.AB.end());
+  upload(c, h->ent, tab.ent);
+  upload(c, h->task, tab.task);
+  upload(c, h->rec, tab.rec);
+  upload(c, h->e0, tab.e0);
+  upload(c, h->xsum, tab.xsum);
+  upload(c, h->half, tab.half);
+  upload(c, h->zt0, tab.zt0);
+  upload(c, h->zt, tab.zt);
+  upload(c, h->tmask, tab.tmask);
+  upload(c, h->hfull, tab.hfull);
+  upload(c, h->prod, tab.prod);
+  upload(c, h->zc, tab.zc);
+  upload(c, h->zc_f, tab.zc_f);
+  upload(c, h->AB, tab.AB);
+  upload(c, h->AB_f, ABf);
   upload(c, h->cY, cY);
   upload(c, h->cY_f, cYf);
-  upload(c, h->invf, invf);
-  upload(c, h->yscale, yscale);
-  upload(c, h->yscale_f, std::vector<float>(yscale.begin(), yscale.end()));
   upload(c, h->beta0, beta0);
-  upload(c, h->radelem, std::vector<double>(radelem, radelem + nelem));
+  upload(c, h->pr, pr);
   upload(c, h->wjelem, std::vector<double>(wjelem, wjelem + nelem));
-  upload_i(c, h->map, std::vector<int>(map, map + ntypes));
+  upload(c, h->map, std::vector<int>(map, map + ntypes));
   EMD_CUDA(cudaStreamSynchronize(c.stream));
-  S.trip = h->trip.p;
-  S.cg_off = h->cg_off.p;
-  S.cg = h->cg.p;
-  S.cg_f = h->cg_f.p;
-  S.jobs = h->jobs.p;
-  S.zord = h->zord.p;
-  S.tjob_off = h->tjob_off.p;
-  S.yred_off = h->yred_off.p;
-  S.yred_job = h->yred_job.p;
+  S.ent = h->ent.p;
+  S.task = h->task.p;
+  S.rec = h->rec.p;
+  S.e0 = h->e0.p;
+  S.xsum = h->xsum.p;
+  S.half = h->half.p;
+  S.zt0 = h->zt0.p;
+  S.zt = h->zt.p;
+  S.hfull = h->hfull.p;
+  S.prod = h->prod.p;
+  S.zc = h->zc.p;
+  S.zc_f = h->zc_f.p;
+  S.AB = h->AB.p;
+  S.AB_f = h->AB_f.p;
   S.cY = h->cY.p;
   S.cY_f = h->cY_f.p;
-  S.invf = h->invf.p;
-  S.yscale = h->yscale.p;
-  S.yscale_f = h->yscale_f.p;
   S.beta0 = h->beta0.p;
-  S.radelem = h->radelem.p;
+  S.pr = h->pr.p;
   S.wjelem = h->wjelem.p;
   S.map = h->map.p;
   EMD_API_END

@@ -1,37 +1,38 @@
 // ForceSNAP on the device (force_snap_neigh_impl.h:160-724, sna_impl.hpp).
 //
-// One CTA per owned atom i, 8 warps, U / Y in shared memory:
-//   A. inside list: warp 0 compacts the neighbours with r^2 < rcutmax^2 in
-//      row order (ballot + popc), keeping r_ij = x_j - x_i, w_j, rcut_ij;
-//   B. U_tot = wself*I + sum_j sfac*w_j*U_j by the Cayley-Klein layer
-//      recursion (compute_uarray, sna_impl.hpp:642-720), in FP64 in both
-//      forms: the rescaled recursion (no square-root factors, b_stage), lanes
-//      over (neighbour, element) pairs of four neighbours per warp, one
-//      fixed-order block sum per layer, mirrored to the full matrices;
-//   C. adjoint contraction: Z_t(ma,mb) for the 125 (j1>=j2, j) triples
-//      (compute_zi, sna_impl.hpp:197-283) and Y_j = sum_t cY_t Z_t, where
-//      cY folds the linear coefficients with the (j+1)/(j1+1), (j+1)/(j2+1)
-//      weights of the three terms of compute_dbidrj (sna_impl.hpp:330-539);
-//   D. per inside neighbour (two per warp at a time):
-//      F_ij = sum_j 2 sum_half w Re(conj(dU'_j) Y_j) + (-1.5e6/r^14) r_ij,
-//      which equals sum_k beta_k dB_k/dr_ij of the reference, from one
-//      forward sweep of the rescaled U recursion and one adjoint sweep
-//      (d_reverse) in place of the dU/dr recursion of compute_duarray
-//      (sna_impl.hpp:729-893); then, one thread per neighbour, f_j -= F_ij
-//      with FP64 atomics (j may be a ghost; update_force follows) and
-//      f_i += sum_j F_ij in a fixed order.  The fitting adjoint (MODE 2)
-//      carries one directional derivative of the rescaled recursion per
-//      neighbour (dt_layer).
-// The energy variant adds E_i = beta_0 + (2/3) sum_j sum_half w Re(conj(U_j) Y_j)
-// (B is cubic in U, so <U, dB/dU> = 3B) plus 1.25e5/r^12 per inside pair.
+// The Wigner matrices of a neighbour depend on its Cayley-Klein pair (a, b)
+// alone, and every element separates:
+//   U_j(ma, mb) = N conj(a)^q b^T P_k(x)            (mb - ma = T >= 0)
+//   U_j(ma, mb) = N conj(a)^q (-conj(b))^T P_k(x)   (ma - mb = T > 0)
+// with q = j - ma - mb >= 0, j = q + T + 2k, x = |a|^2 - |b|^2, P_k the monic
+// Jacobi polynomial P_k^(T, q) (three-term recurrence) and
+// N = 2^-k j! / sqrt(ma! (j - ma)! mb! (j - mb)!).  q < 0 follows from the
+// inversion U_j(j - ma, j - mb) = (-1)^(ma + mb) conj U_j(ma, mb).  This
+// replaces the layer recursion of compute_uarray (sna_impl.hpp:642-720) and
+// its derivative (compute_duarray, 729-893): no layers to keep, one polynomial
+// for up to four elements, and lanes that all do the same thing.  An "entry"
+// below is one (T, q, k): 95 of them at twojmax 8 for 285 elements.
+//
+// Per force call, over chunks of atoms:
+//   k_snap_pairs  inside list and per-pair scalars (lanes = pairs)
+//   k_snap_u      U_tot = wself + sum over the neighbours of w_j sfac U, from the
+//                 four real products of conj(a)^q and b^T times P_k, FP64 in
+//                 both forms (one warp per atom; lanes = neighbours, then sums)
+//   k_snap_y      Z and Y (lanes = atoms, so the Clebsch-Gordan loops are
+//                 uniform and every operand load is coalesced)
+//   k_snap_force  pair forces (lanes = pairs): Phi = Re sum conj(U) Y and its
+//                 gradient in (a, b), chain rule, scatter
+// and for the energy k_snap_energy; for the fitting adjoint k_snap_dt (the
+// directional derivative of X) and k_snap_pq.
 //
 // Precision forms: FP64 (the drop-in; snap.cu, -fmad=false) and mixed
-// (snap_mixed.cu, contraction allowed), where U_tot stays FP64 (phase B) and
-// phases C/D run in FP32 with FP64 force sums.  The recursions and the Z
-// contraction use explicit fused multiply-adds in both forms.
+// (snap_mixed.cu), where the pair scalars and X stay FP64 and k_snap_y and the
+// sums of k_snap_force run in FP32, with FP64 force sums.  The recurrences and
+// contractions use explicit fused multiply-adds in both forms.
 #pragma once
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "emd_device.cuh"
 #include "emd_internal.h"
@@ -44,958 +45,1082 @@ ListView list_view(Ctx& c);
 namespace snapk {
 
 constexpr double MY_PI = 3.14159265358979323846;
-constexpr int SNAP_THREADS = 256;
-constexpr int SNAP_WARPS = SNAP_THREADS / 32;
-// per-neighbour scalar fields (structure of arrays, `cap` entries each)
-enum {
-  ND_AR_U, ND_AI_U, ND_BR_U, ND_BI_U,  // Cayley-Klein a, b of compute_uarray
-  ND_AR, ND_AI, ND_BR, ND_BI,          // a, b of compute_duarray
-  ND_DAR, ND_DAI = ND_DAR + 3, ND_DBR = ND_DAI + 3, ND_DBI = ND_DBR + 3, ND_UK = ND_DBI + 3,
-  ND_SFAC = ND_UK + 3, ND_DSFAC, ND_FP, ND_EP = ND_FP + 3, ND_FIELDS
-};
-// Slots of those fields.  The FP64 form keeps every field in nd (FP64).  The
-// mixed form keeps in nd only what phase B and the FP64 force tail read (a, b
-// of compute_uarray, sfac, the repulsion force) and the phase D inputs in ndr
-// (FP32, fields ND_AR .. ND_DSFAC).
-constexpr int ND_MIXED = 8;
-constexpr int NR_MIXED = ND_DSFAC + 1 - ND_AR;
-template <bool F64>
-__host__ __device__ constexpr int ndx(int f) {
-  return F64 ? f : (f < ND_AR ? f : (f == ND_SFAC ? 4 : 5 + (f - ND_FP)));
-}
-template <bool F64>
-__host__ __device__ constexpr int nrx(int f) {
-  return F64 ? f : f - ND_AR;
-}
-
-struct SnapDev {
-  int twojmax, L;         // L = twojmax + 1
-  int nfull, njobs, nyh;  // triples, Z jobs, half-grid Y size
-  int nuf;                // full U size
-  int ncoeff, ncoeffall, nelem, ntypes;
-  double rfac0, rmin0, rcutfac, cutsq, wself;
-  int switchflag;
-  const int* trip;      // nfull x 3
-  const int* cg_off;    // nfull
-  const double* cg;     // compact CG blocks (a+1) x (b+1)
-  const float* cg_f;
-  const int* jobs;      // njobs: (t << 8) | (ma << 4) | mb
-  const int* tjob_off;  // nfull + 1: the jobs of triple t are [tjob_off[t], tjob_off[t+1])
-  const int* yred_off;  // nyh + 1
-  const int* yred_job;  // njobs
-  const double* cY;     // nelem x nfull
-  const float* cY_f;
-  const double* beta0;   // nelem
-  const double* radelem;
-  const double* wjelem;
-  const int* map;  // ntypes
-  // rescaled recursion: V_j(ma, mb) = f_j(ma, mb) U_j(ma, mb); over the half
-  // grid (nyh): invf = 1 / f, yscale = 2 hw / f (the force contraction's
-  // weight folded into Y; FP64 and FP32); half-layer buffer sizes (even, odd j)
-  const double* invf;
-  const double* yscale;
-  const float* yscale_f;
-  int bh_even, bh_odd;
-  // the Z jobs as descriptors, longest first, in the order
-  // thread (warp w, lane l) takes them in round r: zord[r * SNAP_THREADS +
-  // 32 w + l] (x < 0: no job); see zjob_order in snap.cu
-  const int4* zord;
-  int nzo;
-};
-
-
-// ---- index helpers (device)
-__device__ __forceinline__ int yoff(int j) {  // sum_{j'<j} (j'+1)(j'/2+1)
-  int s = 0;
-  for (int k = 0; k < j; ++k) s += (k + 1) * (k / 2 + 1);
-  return s;
-}
-__device__ __forceinline__ int uoff(int j) {  // sum_{j'<j} (j'+1)^2
-  return j * (j + 1) * (2 * j + 1) / 6;
-}
 
 template <typename R>
 struct Cplx {
   R r, i;
 };
 
-// contraction weight of half-grid element (ma, mb) of layer j (sna_impl.hpp:384-413)
-__device__ __forceinline__ double hw(int j, int ma, int mb) {
-  if (2 * mb < j) return 1.0;
-  if (2 * ma < j) return 1.0;
-  if (2 * ma == j) return 0.5;
-  return 0.0;
-}
-
-template <typename R>
-__device__ __forceinline__ R warp_sum_r(R v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(FULL_MASK, v, o);
-  return v;
-}
-
-__device__ __forceinline__ double sfac_of(const SnapDev& S, double r, double rcut) {
-  if (S.switchflag == 0) return 1.0;
-  if (r <= S.rmin0) return 1.0;
-  if (r > rcut) return 0.0;
-  return 0.5 * (cos((r - S.rmin0) * (MY_PI / (rcut - S.rmin0))) + 1.0);
-}
-__device__ __forceinline__ double dsfac_of(const SnapDev& S, double r, double rcut) {
-  if (S.switchflag == 0) return 0.0;
-  if (r <= S.rmin0) return 0.0;
-  if (r > rcut) return 0.0;
-  const double rcutfac = MY_PI / (rcut - S.rmin0);
-  return -0.5 * sin((r - S.rmin0) * rcutfac) * rcutfac;
-}
-
-// ---- rescaled recursion (mixed form)
-// With V_j(ma, mb) = f_j(ma, mb) U_j(ma, mb), f_j(ma, mb)^2 = (j-mb)! mb! / ((j-ma)! ma!),
-// compute_uarray's recursion (sna_impl.hpp:664-690)
-//   U_j(ma, mb) = rootpq(j-ma, j-mb) a U_{j-1}(ma, mb) - rootpq(ma, j-mb) b U_{j-1}(ma-1, mb)
-// becomes V_j(ma, mb) = a V_{j-1}(ma, mb) - b V_{j-1}(ma-1, mb), because
-// f_j(ma, mb) sqrt((j-ma)/(j-mb)) = f_{j-1}(ma, mb) and
-// f_j(ma, mb) sqrt(ma/(j-mb)) = f_{j-1}(ma-1, mb).  f_j(ma, mb) = f_j(j-ma, j-mb),
-// so the inversion mirror holds for V as for U.  U = V / f is restored once
-// per atom (on the U_tot sums, and folded into Y for the dU contraction).
-
-__device__ __forceinline__ double flip_if(double x, bool f) {
-  const unsigned long long sign = f ? 0x8000000000000000ull : 0ull;
-  return __longlong_as_double(static_cast<long long>(static_cast<unsigned long long>(__double_as_longlong(x)) ^ sign));
-}
-
-// element (ma, mb) of half layer jp (index mb (jp + 1) + ma, 2 mb <= jp); the
-// column past the half by the mirror (-1)^(ma+mb) conj V(jp - ma, jp - mb)
-__device__ __forceinline__ Cplx<double> ld_half(const Cplx<double>* P, int jp, int ma, int mb) {
-  if (2 * mb <= jp) return P[mb * (jp + 1) + ma];
-  const Cplx<double> v = P[(jp - mb) * (jp + 1) + (jp - ma)];
-  const bool odd = (ma + mb) & 1;
-  return Cplx<double>{flip_if(v.r, odd), flip_if(v.i, !odd)};
-}
-
-// neighbour slots per warp in b_stage
-constexpr int BG = 4;
-
-// B: U_tot (FP64) and, for R = float, its FP32 copy.  Neighbours go in
-// rounds of SNAP_WARPS * BG; warp w holds neighbours w, w + SNAP_WARPS, ... of
-// the round, its lanes over (slot, half-layer element) pairs.  Layer 0 is
-// seeded with sfac * w_j, so each layer's sum over the neighbours is a plain
-// sum: one warp adds up layer j - 1 (in a fixed order) while the others run
-// layer j.  `work` holds SNAP_WARPS * BG slots of (bh_even + bh_odd) elements.
-// JF > 0: twojmax fixed at compile time (the layer loop unrolls and the
-// element index arithmetic divides by constants); 0: S.twojmax.
-template <typename R, int JF = 0>
-__device__ __forceinline__ void b_stage(const SnapDev& S, const double* nd, int cap, int ninside, Cplx<double>* work,
-                                        Cplx<double>* utot, Cplx<R>* utot_r) {
-  constexpr bool kCopy = sizeof(R) != sizeof(double);
-  constexpr int kUnroll = JF > 0 ? JF + 1 : 1;
-  const int J = JF > 0 ? JF : S.twojmax;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int sw = S.bh_even + S.bh_odd, per_round = SNAP_WARPS * BG;
-  Cplx<double>* mine = work + size_t(warp) * BG * sw;
-  const int rounds = max(1, (ninside + per_round - 1) / per_round);
-  for (int rd = 0; rd < rounds; ++rd) {
-    const int nb0 = rd * per_round;
-    const int nin = max(0, min(ninside - nb0, per_round));
-    const int gw = nin > warp ? (nin - warp + SNAP_WARPS - 1) / SNAP_WARPS : 0;  // this warp's slots
-    if (lane < gw) mine[lane * sw] = Cplx<double>{nd[ndx<!kCopy>(ND_SFAC) * cap + nb0 + lane * SNAP_WARPS + warp], 0.0};
-    __syncthreads();
-#pragma unroll kUnroll
-    for (int j = 1; j <= J + 1; ++j) {
-      if (j <= J) {
-        const int nh = (j + 1) * (j / 2 + 1);
-        const int po = ((j - 1) & 1) * S.bh_even, co = (j & 1) * S.bh_even;
-        for (int it = lane; it < gw * nh; it += 32) {
-          const int g = it / nh, e = it - g * nh;
-          const int mb = e / (j + 1), ma = e - mb * (j + 1);
-          const int nb = nb0 + g * SNAP_WARPS + warp;
-          const double ar = nd[ndx<!kCopy>(ND_AR_U) * cap + nb], ai = nd[ndx<!kCopy>(ND_AI_U) * cap + nb];
-          const double br = nd[ndx<!kCopy>(ND_BR_U) * cap + nb], bi = nd[ndx<!kCopy>(ND_BI_U) * cap + nb];
-          const Cplx<double>* P = mine + g * sw + po;
-          Cplx<double> u1{0.0, 0.0}, u2{0.0, 0.0};
-          if (ma > 0) u1 = ld_half(P, j - 1, ma - 1, mb);
-          if (ma < j) u2 = ld_half(P, j - 1, ma, mb);
-          const double vr = fma(ar, u2.r, fma(ai, u2.i, fma(-br, u1.r, -bi * u1.i)));
-          const double vi = fma(ar, u2.i, fma(-ai, u2.r, fma(-br, u1.i, bi * u1.r)));
-          // the centre element conjugated, as the reference's in-place mirror leaves it
-          mine[g * sw + co + e] = Cplx<double>{vr, flip_if(vi, 2 * ma == j && 2 * mb == j)};
-        }
-      }
-      const int jr = j - 1;
-      if (warp == jr % SNAP_WARPS) {
-        // elements in chunks of up to 32; a chunk of m elements spreads the
-        // neighbours over G = 32 / m (a power of two) lane groups, each summing
-        // a contiguous share, then the groups are added pairwise (fixed order)
-        const int nh = (jr + 1) * (jr / 2 + 1), ro = (jr & 1) * S.bh_even, yo = yoff(jr), uo = uoff(jr);
-        for (int c0 = 0; c0 < nh; c0 += 32) {
-          const int m = min(32, nh - c0);
-          int G = 1;
-          while (4 * G * m <= 64) G *= 2;
-          const int g = lane / m, e = c0 + lane - g * m;
-          const int per = (nin + G - 1) / G;
-          double sr = 0.0, si = 0.0;
-          if (g < G) {
-            const int k1 = min(nin, (g + 1) * per);
-            for (int k = g * per; k < k1; ++k) {
-              const Cplx<double> v = work[size_t((k % SNAP_WARPS) * BG + k / SNAP_WARPS) * sw + ro + e];
-              sr += v.r;
-              si += v.i;
-            }
-          }
-          for (int h = G / 2; h >= 1; h /= 2) {
-            const double ur = __shfl_down_sync(FULL_MASK, sr, h * m);
-            const double ui = __shfl_down_sync(FULL_MASK, si, h * m);
-            if (g < h) {
-              sr += ur;
-              si += ui;
-            }
-          }
-          if (g == 0) {
-            const int mb = e / (jr + 1), ma = e - mb * (jr + 1);
-            const double f = S.invf[yo + e];
-            Cplx<double>& t = utot[uo + ma * (jr + 1) + mb];
-            const double r0 = rd == 0 ? (ma == mb ? S.wself : 0.0) : t.r;
-            const double i0 = rd == 0 ? 0.0 : t.i;
-            t = Cplx<double>{fma(sr, f, r0), fma(si, f, i0)};
-          }
-        }
-      }
-      __syncthreads();
-    }
-  }
-  // mirror to the full matrices, FP32 copy
-  for (int e = tid; e < S.nyh; e += SNAP_THREADS) {
-    int j = 0;
-    while (yoff(j + 1) <= e) ++j;
-    const int q = e - yoff(j), mb = q / (j + 1), ma = q % (j + 1);
-    if (2 * mb == j && 2 * ma > j) continue;  // written as the mirror of (j - ma, mb)
-    const int uo = uoff(j);
-    const Cplx<double> u = utot[uo + ma * (j + 1) + mb];
-    if constexpr (kCopy) utot_r[uo + ma * (j + 1) + mb] = Cplx<R>{R(u.r), R(u.i)};
-    if (2 * mb < j || 2 * ma < j) {
-      const bool odd = (ma + mb) & 1;
-      const Cplx<double> m{flip_if(u.r, odd), flip_if(u.i, !odd)};
-      const int t = uo + (j - ma) * (j + 1) + (j - mb);
-      utot[t] = m;
-      if constexpr (kCopy) utot_r[t] = Cplx<R>{R(m.r), R(m.i)};
-    }
-  }
-  __syncthreads();
-}
-
-// Phase D of the force, in reverse mode, for NB neighbours at once (one per
-// register set, so each lane carries NB independent chains).  With
-// Phi = sum_j sum_half Re(conj(V_j) Y'_j), Y' = w Y / f (ytot of the force
-// kernel), the pair force needs only Phi and its gradient in a = (ar, ai),
-// b = (br, bi):  F_k = dsfac u_k Phi + sfac sum_p dPhi/dp dp/dr_k.  The
-// forward sweep runs the rescaled recursion and keeps layers 0..J-1 (full,
-// column-major, in F); the backward sweep carries the adjoint
-// lambda_j = dPhi/dV_j down the layers: from a mirrored element back to its
-// source (conjugated, with the mirror's sign), through the centre
-// conjugation, and through the recursion as
-//   lambda_{j-1}(ma, mb) = a lambda'_j(ma, mb) - b lambda'_j(ma + 1, mb),
-//   dPhi/d conj(a) += conj(V_{j-1}(ma, mb)) lambda'_j(ma, mb),
-//   dPhi/d conj(b) -= conj(V_{j-1}(ma - 1, mb)) lambda'_j(ma, mb).
-// One forward and one adjoint sweep replace the three dU/dr recursions of
-// compute_duarray (sna_impl.hpp:729-893) and their contraction with Y.
-// Outputs per-lane partials: phi, ga = sum conj(V) lambda' for a, gb for b
-// (dPhi/dar = ga.r, dPhi/dai = -ga.i, dPhi/dbr = -gb.r, dPhi/dbi = gb.i).
-// Neighbour n's buffers start at W + n * drev_words(J): F max(1, uoff(J)),
-// LA and LB max(1, J (J/2 + 1)) each, LP (J + 1)(J/2 + 1).
-template <typename R>
-struct DRevAB {
-  R ar, ai, br, bi;
+// One (T, q, k) entry
+struct Entry {
+  double N, invN;  // the elements' norm and its inverse
+  double A, B;     // P_{k+1} = (x - A) P_k - B P_{k-1}
+  int xo;          // first of its real sums: p u, [q>0] r u, [T>0] p v, [q>0, T>0] r v
+  int T, q, j;
+  int ep, em, mp, mm;  // full-grid elements (ma, mb) and (mb, ma), and their inversions
 };
-__host__ __device__ __forceinline__ int drev_words(int J) {
-  return (J * (J + 1) * (2 * J + 1) / 6 > 1 ? J * (J + 1) * (2 * J + 1) / 6 : 1) +
-         2 * (J * (J / 2 + 1) > 1 ? J * (J / 2 + 1) : 1) + (J + 1) * (J / 2 + 1);
-}
-// JF > 0: twojmax fixed at compile time (the layer loops unroll and the
-// element index arithmetic divides by constants); 0: twojmax = Jrt.
-template <typename R, int NB, int JF = 0>
-__device__ __forceinline__ void d_reverse(int Jrt, int lane, const DRevAB<R>* ab, const Cplx<R>* __restrict__ ytot,
-                                          Cplx<R>* W, R* phi, Cplx<R>* ga, Cplx<R>* gb) {
-  constexpr int kUnroll = JF > 0 ? JF : 1;
-  const int J = JF > 0 ? JF : Jrt;
-  const int nF = max(1, uoff(J)), nL = max(1, J * (J / 2 + 1)), stride = drev_words(J);
-#pragma unroll
-  for (int n = 0; n < NB; ++n) {
-    phi[n] = (lane == 0) ? ytot[0].r : R(0);
-    ga[n] = gb[n] = Cplx<R>{R(0), R(0)};
-    if (lane == 0) W[n * stride] = Cplx<R>{R(1), R(0)};
-  }
-  __syncwarp();
-#pragma unroll kUnroll
-  for (int j = 1; j <= J; ++j) {
-    const int nh = (j + 1) * (j / 2 + 1), yo = yoff(j), po = uoff(j - 1), co = uoff(j);
-    for (int e = lane; e < nh; e += 32) {
-      const int mb = e / (j + 1), ma = e - mb * (j + 1);
-      // the lower half of the middle column is the mirror of its upper half
-      // (written below by the lane that computes the source); its Y' is 0
-      if (2 * mb == j && 2 * ma > j) continue;
-      const Cplx<R> y = ytot[yo + e];
-      const bool centre = 2 * ma == j && 2 * mb == j;
-      const bool mirrored = 2 * mb < j || 2 * ma < j;
-      const bool even = ((ma + mb) & 1) == 0;
-      const int t = co + (j - mb) * (j + 1) + (j - ma);
-#pragma unroll
-      for (int n = 0; n < NB; ++n) {
-        const Cplx<R>* P = W + n * stride + po;
-        Cplx<R> u1{R(0), R(0)}, u2{R(0), R(0)};
-        if (ma > 0) u1 = P[mb * j + ma - 1];
-        if (ma < j) u2 = P[mb * j + ma];
-        const R vr = fma(ab[n].ar, u2.r, fma(ab[n].ai, u2.i, fma(-ab[n].br, u1.r, -ab[n].bi * u1.i)));
-        R vi = fma(ab[n].ar, u2.i, fma(-ab[n].ai, u2.r, fma(-ab[n].br, u1.i, ab[n].bi * u1.r)));
-        if (centre) vi = -vi;
-        phi[n] = fma(vr, y.r, fma(vi, y.i, phi[n]));
-        if (j < J) {
-          W[n * stride + co + e] = Cplx<R>{vr, vi};
-          if (mirrored) W[n * stride + t] = even ? Cplx<R>{vr, -vi} : Cplx<R>{-vr, vi};
-        }
-      }
-    }
-    __syncwarp();
-  }
-  int lam = nF, nxt = nF + nL;  // offsets of the current and next adjoint layers
-  const int lp = nF + 2 * nL;
-#pragma unroll kUnroll
-  for (int j = J; j >= 1; --j) {
-    const int nh = (j + 1) * (j / 2 + 1), yo = yoff(j), po = uoff(j - 1);
-    for (int e = lane; e < nh; e += 32) {
-      const int mb = e / (j + 1), ma = e - mb * (j + 1);
-      const bool dead = 2 * mb == j && 2 * ma > j;  // overwritten by the mirror: no adjoint
-      const bool mirrored = 2 * mb < j || 2 * ma < j;
-      // the mirror target (j - ma, j - mb) has an adjoint only where layer
-      // j + 1 read it (columns up to (j + 1) / 2)
-      const int tc = j - mb;
-      const bool from_t = mirrored && j < J && 2 * tc <= j + 1;
-      const bool even = ((ma + mb) & 1) == 0;
-      const Cplx<R> y = ytot[yo + e];
-#pragma unroll
-      for (int n = 0; n < NB; ++n) {
-        Cplx<R>* Wn = W + n * stride;
-        Cplx<R> l{R(0), R(0)};
-        if (!dead) {
-          l = (j == J) ? y : Wn[lam + e];
-          if (from_t) {
-            const Cplx<R> lt = Wn[lam + tc * (j + 1) + (j - ma)];
-            l.r += even ? lt.r : -lt.r;
-            l.i += even ? -lt.i : lt.i;
-          } else if (!mirrored && 2 * ma == j) {
-            l.i = -l.i;
-          }
-          if (ma < j) {
-            const Cplx<R> p = Wn[po + mb * j + ma];
-            ga[n].r = fma(p.r, l.r, fma(p.i, l.i, ga[n].r));
-            ga[n].i = fma(p.r, l.i, fma(-p.i, l.r, ga[n].i));
-          }
-          if (ma > 0) {
-            const Cplx<R> p = Wn[po + mb * j + ma - 1];
-            gb[n].r = fma(p.r, l.r, fma(p.i, l.i, gb[n].r));
-            gb[n].i = fma(p.r, l.i, fma(-p.i, l.r, gb[n].i));
-          }
-        }
-        Wn[lp + e] = l;
-      }
-    }
-    __syncwarp();
-    if (j > 1) {
-      // adjoint of layer j - 1 over the columns layer j reads (mb <= j / 2),
-      // plus its own Y' term on the half grid
-      const int n = j * (j / 2 + 1), nhp = j * ((j - 1) / 2 + 1), yop = yoff(j - 1);
-      for (int idx = lane; idx < n; idx += 32) {
-        const int mb = idx / j, mp = idx - mb * j;
-        Cplx<R> y{R(0), R(0)};
-        if (idx < nhp) y = ytot[yop + idx];
-#pragma unroll
-        for (int k = 0; k < NB; ++k) {
-          Cplx<R>* Wn = W + k * stride;
-          const Cplx<R> l1 = Wn[lp + mb * (j + 1) + mp], l0 = Wn[lp + mb * (j + 1) + mp + 1];
-          const DRevAB<R>& q = ab[k];
-          Wn[nxt + idx] = Cplx<R>{fma(q.ar, l1.r, fma(-q.ai, l1.i, fma(-q.br, l0.r, fma(q.bi, l0.i, y.r)))),
-                                  fma(q.ar, l1.i, fma(q.ai, l1.r, fma(-q.br, l0.i, fma(-q.bi, l0.r, y.i))))};
-        }
-      }
-      __syncwarp();
-      const int t = lam;
-      lam = nxt;
-      nxt = t;
-    }
-  }
-}
 
-// Layer j of the rescaled recursion and of its derivative along one
-// direction (the fitting adjoint's g_i - g_j):
-//   V_j = conj(a) V_{j-1}(ma) - conj(b) V_{j-1}(ma - 1),
-//   T_j = conj(ta) V_{j-1}(ma) + conj(a) T_{j-1}(ma) - conj(tb) V_{j-1}(ma - 1) - conj(b) T_{j-1}(ma - 1),
-// with du_layer's inversion mirror and centre conjugation.  Full layers,
-// column-major (element (ma, mb) at mb (j + 1) + ma).
-template <typename R>
-__device__ __forceinline__ void dt_layer(int j, int lane, R ar, R ai, R br, R bi, R tar, R tai, R tbr, R tbi,
-                                         const Cplx<R>* P, const Cplx<R>* TP, Cplx<R>* C, Cplx<R>* TC) {
-  const int nh = (j + 1) * (j / 2 + 1);
-  for (int e = lane; e < nh; e += 32) {
-    const int mb = e / (j + 1), ma = e - mb * (j + 1);
-    Cplx<R> u1{0, 0}, u2{0, 0}, t1{0, 0}, t2{0, 0};
-    if (ma > 0) {
-      u1 = P[mb * j + ma - 1];
-      t1 = TP[mb * j + ma - 1];
-    }
-    if (ma < j) {
-      u2 = P[mb * j + ma];
-      t2 = TP[mb * j + ma];
-    }
-    C[e] = Cplx<R>{fma(ar, u2.r, fma(ai, u2.i, fma(-br, u1.r, -bi * u1.i))),
-                   fma(ar, u2.i, fma(-ai, u2.r, fma(-br, u1.i, bi * u1.r)))};
-    const R tr = fma(tar, u2.r, fma(tai, u2.i, fma(ar, t2.r, fma(ai, t2.i,
-                 fma(-tbr, u1.r, fma(-tbi, u1.i, fma(-br, t1.r, -bi * t1.i)))))));
-    const R ti = fma(tar, u2.i, fma(-tai, u2.r, fma(ar, t2.i, fma(-ai, t2.r,
-                 fma(-tbr, u1.i, fma(tbi, u1.r, fma(-br, t1.i, bi * t1.r)))))));
-    TC[e] = Cplx<R>{tr, ti};
-  }
-  __syncwarp();
-  for (int e = lane; e < nh; e += 32) {
-    const int mb = e / (j + 1), ma = e - mb * (j + 1);
-    const bool even = ((ma + mb) & 1) == 0;
-    if (2 * mb < j || 2 * ma < j) {
-      const int t = (j - mb) * (j + 1) + (j - ma);
-      const Cplx<R> u = C[e], w = TC[e];
-      C[t] = even ? Cplx<R>{u.r, -u.i} : Cplx<R>{-u.r, u.i};
-      TC[t] = even ? Cplx<R>{w.r, -w.i} : Cplx<R>{-w.r, w.i};
-    } else if (2 * ma == j) {
-      C[e].i = -C[e].i;
-      TC[e].i = -TC[e].i;
-    }
-  }
-  __syncwarp();
-}
+// The products of one (j1, j2) at one (2m, 2m') = (-q -+ T, -q +- T) of a Z task
+struct ZRec {
+  int p0, np, c0, cf;  // products [p0, p0 + np); first coefficient, in zc and in zc_f
+  short nj, d;         // number of j, the highest first; its distance from the task's highest j over 2
+  int t0, z0;          // triple of the highest j; first kept Z
+};
+struct ZTask {
+  int T, q, rec0, rec1, rec2;  // records of the +T elements [rec0, rec1), of the -T ones [rec1, rec2)
+  int y0, kmax;                // first entry, last k
+};
 
-// C: the Z jobs, one per thread (compute_zi, sna_impl.hpp:197-283).  A
-// job's descriptor holds the U_tot offsets of its first U1 and U2 terms, its
-// first inner and outer Clebsch-Gordan offsets, its counts (ma1, mb1) and the
-// row strides j1 + 1, j2 + 1.  Along mb1 the U1 index rises by 1, the U2
-// index falls by 1 and the CG index rises by j2; along ma1 the rows move by
-// +(j1 + 1) and -(j2 + 1).  NBMAX > 0 (twojmax = NBMAX - 1): the inner
-// Clebsch-Gordan row, the same for every ma1, is read once into registers
-// and the inner loop unrolls over NBMAX slots (constant offsets); the
-// arithmetic and its order are the same either way.
-template <typename R, int NBMAX>
-__device__ __forceinline__ void z_jobs(const SnapDev& S, const Cplx<R>* __restrict__ utot_r, const R* __restrict__ cg,
-                                       Cplx<R>* __restrict__ zs) {
-  for (int k = threadIdx.x; k < S.nzo; k += SNAP_THREADS) {
-    const int4 d = S.zord[k];
-    if (d.x < 0) continue;
-    const int u1 = d.y & 0xffff, u2 = int(unsigned(d.y) >> 16);
-    const int ci = d.z & 0xffff, co = int(unsigned(d.z) >> 16);
-    const int na = d.w & 0xff, nbb = (d.w >> 8) & 0xff, s1 = (d.w >> 16) & 0xff, s2 = int(unsigned(d.w) >> 24);
-    const int cs = s2 - 1;
-    R zr = 0, zi = 0;
-    if constexpr (NBMAX > 0) {
-      R cb[NBMAX];
-#pragma unroll
-      for (int b = 0; b < NBMAX; ++b) cb[b] = b < nbb ? cg[ci + b * cs] : R(0);
-      for (int a = 0; a < na; ++a) {
-        const Cplx<R>* A1 = utot_r + u1 + a * s1;
-        const Cplx<R>* B2 = utot_r + u2 - a * s2;
-        R sr = 0, si = 0;
-#pragma unroll
-        for (int b = 0; b < NBMAX; ++b) {
-          if (b < nbb) {
-            const Cplx<R> x = A1[b], y = B2[-b];
-            sr = fma(cb[b], fma(x.r, y.r, -x.i * y.i), sr);
-            si = fma(cb[b], fma(x.r, y.i, x.i * y.r), si);
-          }
-        }
-        const R c = cg[co + a * cs];
-        zr = fma(sr, c, zr);
-        zi = fma(si, c, zi);
-      }
-    } else {
-      for (int a = 0; a < na; ++a) {
-        const Cplx<R>* A1 = utot_r + u1 + a * s1;
-        const Cplx<R>* B2 = utot_r + u2 - a * s2;
-        R sr = 0, si = 0;
-        for (int b = 0; b < nbb; ++b) {
-          const R c = cg[ci + b * cs];
-          const Cplx<R> x = A1[b], y = B2[-b];
-          sr = fma(c, fma(x.r, y.r, -x.i * y.i), sr);
-          si = fma(c, fma(x.r, y.i, x.i * y.r), si);
-        }
-        const R c = cg[co + a * cs];
-        zr = fma(sr, c, zr);
-        zi = fma(si, c, zi);
-      }
-    }
-    zs[d.x] = Cplx<R>{zr, zi};
-  }
-}
+struct SnapDev {
+  int twojmax, ne, nx, nuf;    // entries, real sums, elements of the full grid
+  int cols;                    // columns of a neighbour's table (su_cols)
+  int ntask, nfull, nz;        // Z tasks, (j1 >= j2, j) triples, kept Z values per atom
+  int ncoeff, ncoeffall, nelem, ntypes;
+  double rfac0, rmin0, cutsq, wself;
+  int switchflag;
+  const Entry* ent;
+  const int* e0;       // (J + 1) x (J + 1): first entry of (T, q)
+  const int2* xsum;    // nx: the two factors of a sum in a neighbour's table (k_snap_u)
+  const ZTask* task;
+  const ZRec* rec;
+  const int2* prod;    // the two U elements of a product
+  const double* zc;    // coefficients, nj per product
+  const float2* zc_f;  // the same, each twice and nj rounded up to an even number
+  const double* cY;    // nelem x nfull
+  const float* cY_f;
+  const double* AB;    // ne x 2
+  const float* AB_f;
+  const double* beta0;
+  const double* wjelem;
+  const double* pr;    // per element pair: rcut, rscale0, pi / (rcut - rmin0)
+  const int* map;      // ntypes
+  // half-grid elements of an entry, +T and -T (-1: none); the kept Z values of
+  // triple t with their elements, [zt0[t], zt0[t + 1]) of zt
+  int nh;
+  const int2* half;
+  const int4* hfull;   // per half-grid element: its full-grid index, its inversion's, sign
+  const int* zt0;
+  const int2* zt;
+};
+
+// ---- pair fields, one array each of stride `np` (pairs of the chunk)
+enum { PD_AR, PD_AI, PD_BR, PD_BI, PD_SF, PD_FX, PD_FY, PD_FZ, PD_EP, PD_N };  // FP64
+// force inputs, mixed form (FP32): a, b, sfac, dsfac, u, and the three numbers
+// da/dr and db/dr are made of; FP64 form: a and b as compute_duidrj rounds
+// them, dsfac, u and every derivative in the reference's operations
+enum { PR_AR, PR_AI, PR_BR, PR_BI, PR_DSF, PR_UX, PR_UY, PR_UZ, PR_SF, PR_C1, PR_GR, PR_R0, PR_N };
+enum { PF_DAR = PR_SF, PF_DAI = PF_DAR + 3, PF_DBR = PF_DAI + 3, PF_DBI = PF_DBR + 3, PF_N = PF_DBI + 3 };
 
 struct SnapArgs {
   SnapDev S;
   const double4_32a* x4;
   const int* type;
-  double* f;
   ListView L;
-  int n_local, cap;
-  double* eatom;  // energy variant
-  unsigned* status;
-  // adjoint variant
-  const double* g;           // dL/dF of the owned atoms (n_local x 3)
-  const int* ghost_owner;    // owned atom behind every ghost
-  int newton;                // ghost forces fold back to their owners
-  double* adj;               // column-major per-atom outputs, (2 nfull + 1) x n_local
-  size_t work_bytes;         // size of the shared `work` region
-  // U_tot (nuf) and the Z jobs (njobs) of every owned atom, FP64 form only:
-  // a force pass (MODE 0) writes them when non-null, and an adjoint (MODE 2)
-  // on the same positions and list reads them instead of running B and C
-  Cplx<double>* keep_u = nullptr;
-  Cplx<double>* keep_z = nullptr;
+  int first, n;        // atoms [first, first + n) of this chunk
+  int n_local, cap;    // owned atoms; pair slots per atom
+  int rows;            // k_snap_pairs: atoms per warp
+  double* pd;          // PD_N x (n cap)
+  void* pr;            // PR_N x (n cap), force type (the FP64 form reads a, b and sfac from pd)
+  int* pj;             // n cap
+  int* cnt;            // n
+  void* U;             // n x nh complex, force type
+  void* Y;             // tiles x (4 ne) x TA, force type
+  int ta, nsplit;      // atoms per tile, CTAs per tile
+  double* zkeep;       // tiles x nz x 32 complex, or null
+  double* f;
+  double* eatom;       // energy
+  // adjoint
+  const double* g;
+  const int* ghost_owner;
+  int newton;
+  Cplx<double>* D;     // n x nh
+  Cplx<double>* H;     // tiles x 2 nh x 32: weighted U and D elements
+  double* adj;         // (2 nfull + 1) x n_local
+  int tsplit;          // k_snap_force: T groups
+  int apc;             // k_snap_force: atoms per CTA
+  const int* tmask;    // tsplit masks of T
 };
 
-// MODE 0: forces; 1: per-atom energy; 2: adjoint columns (FP64 only).
-// Minimum resident CTAs: four for the mixed form (<= 64 registers; its
-// shared memory, sized by the largest inside count, fits four per SM up to
-// about 28 inside neighbours), two for the FP64 forms.
-template <typename R, int MODE>
-__global__ void __launch_bounds__(SNAP_THREADS, sizeof(R) == sizeof(float) ? 4 : 2) k_snap(SnapArgs A) {
-  const SnapDev& S = A.S;
-  const int i = blockIdx.x;
-  if (i >= A.n_local) return;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int L = S.L, L2 = L * L;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  // ---- shared memory carve-up (mirrored by snap_smem_bytes)
-  constexpr bool kF64 = sizeof(R) == sizeof(double);
-  constexpr int kNd = kF64 ? int(ND_FIELDS) : ND_MIXED, kNr = kF64 ? 0 : NR_MIXED;
-  double* in_r = reinterpret_cast<double*>(smem_raw);      // 3*cap
-  double* in_w = in_r + 3 * A.cap;                         // cap
-  double* in_rc = in_w + A.cap;                            // cap
-  Cplx<double>* utot = reinterpret_cast<Cplx<double>*>(in_rc + A.cap);  // nuf
-  Cplx<R>* ytot = reinterpret_cast<Cplx<R>*>(utot + S.nuf);            // nyh
-  // U_tot in the contraction type: the FP64 array itself, or an FP32 copy
-  // made once per atom (converting inside the Z loops would put an FP64-pipe
-  // conversion on every Clebsch-Gordan term)
-  Cplx<R>* utot_r = kF64 ? reinterpret_cast<Cplx<R>*>(utot) : ytot + S.nyh;      // nuf
-  int* in_j = reinterpret_cast<int*>(kF64 ? ytot + S.nyh : utot_r + S.nuf);     // cap
-  double* red = reinterpret_cast<double*>(in_j + ((A.cap + 3) & ~3));          // 4*SNAP_WARPS
-  double* nd = red + 4 * SNAP_WARPS;                                           // kNd*cap
-  // the phase D inputs in the contraction type (mixed form: FP32 fields)
-  R* ndr = kF64 ? reinterpret_cast<R*>(nd) : reinterpret_cast<R*>(nd + kNd * A.cap);
-  unsigned char* work = reinterpret_cast<unsigned char*>(nd + kNd * A.cap + (kNr * A.cap + 1) / 2);
-  __shared__ int s_ninside;
+// ------------------------------------------------------------------ pairs
+// One warp takes `rows` atoms: their rows are filtered in FP32 (conservative,
+// see f32_cut_threshold) into a shared list, then the lanes take listed pairs
+// 32 at a time and write the scalars.  A listed pair that the FP64 test puts
+// outside the cutoff is written with zero weight and force.
+constexpr int SP_ROWS = 8;
+constexpr int SP_CAP = 512;  // listed pairs per warp; a fuller list is emptied in between
 
-  // ---- A: inside list (force_snap_neigh_impl.h:612-656)
-  const double4_32a xi = A.x4[i];
-  const int ti = A.type[i];
-  const int ei = S.map[ti];
-  if (warp == 0) {
-    const double radi = S.radelem[ei];
+template <typename R>
+__global__ void __launch_bounds__(64) k_snap_pairs(SnapArgs A) {
+  const SnapDev& S = A.S;
+  __shared__ int s_j[2][SP_CAP];
+  __shared__ int s_a[2][SP_CAP];  // atom of the warp | slot << 4
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  const int a0 = (blockIdx.x * 2 + warp) * A.rows;
+  if (a0 >= A.n) return;
+  const int na = min(A.rows, A.n - a0);
+  int* lj = s_j[warp];
+  int* la = s_a[warp];
+  const size_t np = size_t(A.n) * A.cap;
+  constexpr bool kF64 = sizeof(R) == sizeof(double);
+  R* pr = static_cast<R*>(A.pr);
+  auto flush = [&](int cnt) {
+    __syncwarp();
+    for (int k = lane; k < cnt; k += 32) {
+      const int al = a0 + (la[k] & 15), slot = la[k] >> 4, j = lj[k];
+      const double4_32a pi = A.x4[A.first + al], pj = A.x4[j];
+      const double x = pj.x - pi.x, y = pj.y - pi.y, z = pj.z - pi.z;
+      const double rsq = x * x + y * y + z * z;
+      const size_t p = size_t(al) * A.cap + slot;
+      double* q = A.pd + p;
+      const bool in = rsq < S.cutsq;
+      const int ei = S.map[A.type[A.first + al]], ej = S.map[A.type[j]];
+      const double* t = S.pr + 3 * (ei * S.nelem + ej);
+      const double rcut = t[0], rscale0 = t[1], rsw = t[2];
+      const double wj = in ? S.wjelem[ej] : 0.0;
+      R* w = pr + p;
+      double sf = 1.0, dsf = 0.0;
+      if constexpr (kF64) {
+        const double r = in ? sqrt(rsq) : 1.0;
+        // compute_ui (sna_impl.hpp:174-187): a, b of compute_uarray
+        const double theta0 = (r - S.rmin0) * S.rfac0 * MY_PI / (rcut - S.rmin0);
+        const double z0u = r / tan(theta0);
+        const double r0u = 1.0 / sqrt(r * r + z0u * z0u);
+        q[PD_AR * np] = in ? r0u * z0u : 1.0;
+        q[PD_AI * np] = in ? -r0u * z : 0.0;
+        q[PD_BR * np] = in ? r0u * y : 0.0;
+        q[PD_BI * np] = in ? -r0u * x : 0.0;
+        // compute_duidrj + the prologue of compute_duarray (sna_impl.hpp:291-321, 729-778)
+        const double th = (r - S.rmin0) * rscale0;
+        const double cs = cos(th), sn = sin(th);
+        const double z0 = r * cs / sn;
+        const double dz0dr = z0 / r - (r * rscale0) * (rsq + z0 * z0) / rsq;
+        const double rinv = 1.0 / r;
+        const double uk[3] = {x * rinv, y * rinv, z * rinv};
+        const double r0inv = 1.0 / sqrt(r * r + z0 * z0);
+        w[PR_AR * np] = in ? z0 * r0inv : 1.0;
+        w[PR_AI * np] = in ? -z * r0inv : 0.0;
+        w[PR_BR * np] = in ? y * r0inv : 0.0;
+        w[PR_BI * np] = in ? -x * r0inv : 0.0;
+        const double dr0invdr = -(r0inv * r0inv * r0inv) * (r + z0 * dz0dr);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const double dr0inv = dr0invdr * uk[d], dz0 = dz0dr * uk[d];
+          w[(PF_DAR + d) * np] = in ? dz0 * r0inv + z0 * dr0inv : 0.0;
+          w[(PF_DAI + d) * np] = in ? -z * dr0inv + (d == 2 ? -r0inv : 0.0) : 0.0;
+          w[(PF_DBR + d) * np] = in ? y * dr0inv + (d == 1 ? r0inv : 0.0) : 0.0;
+          w[(PF_DBI + d) * np] = in ? -x * dr0inv + (d == 0 ? -r0inv : 0.0) : 0.0;
+          w[(PR_UX + d) * np] = in ? uk[d] : 0.0;
+        }
+        // compute_sfac, compute_dsfac (sna_impl.hpp:1099-1128)
+        if (S.switchflag != 0 && r > S.rmin0) {
+          sf = r > rcut ? 0.0 : 0.5 * (cos((r - S.rmin0) * rsw) + 1.0);
+          dsf = r > rcut ? 0.0 : -0.5 * sin((r - S.rmin0) * rsw) * rsw;
+        }
+        w[PR_DSF * np] = dsf * wj;
+        // extra repulsion of the reference (force_snap_neigh_impl.h:705-711) and
+        // its energy 1.25e5 / r^12 per ordered pair
+        const double r2 = rsq * rsq, r4 = r2 * r2;
+        const double fr = in ? -1.5e6 / (r4 * r2 * rsq) : 0.0;
+        q[PD_FX * np] = x * fr;
+        q[PD_FY * np] = y * fr;
+        q[PD_FZ * np] = z * fr;
+        q[PD_EP * np] = in ? 1.25e5 / (r4 * r2) : 0.0;
+      } else {
+        // The same quantities in closed form, once, in FP64.  With s =
+        // sin(theta0), c = cos(theta0): z0 = r c / s and r0inv = s / r, so
+        //   a = c - i z s / r, b = (y - i x) s / r,
+        //   da/dr_k = -s rscale0 u_k - i (g u_k z + r0inv [k = z]), db/dr_k likewise,
+        //   g = d(s / r)/dr = (c rscale0 r - s) / r^2 (the prologue of
+        //   compute_duarray without its cancelling terms)
+        const double rinv = in ? rsqrt(rsq) : 0.0;
+        const double r = rsq * rinv;
+        double sn, cs;
+        sincos((r - S.rmin0) * rscale0, &sn, &cs);
+        const double r0inv = sn * rinv;
+        if (S.switchflag != 0 && r > S.rmin0) {
+          if (r > rcut) {
+            sf = 0.0;
+          } else {
+            double ss, cc;
+            sincos((r - S.rmin0) * rsw, &ss, &cc);
+            sf = 0.5 * (cc + 1.0);
+            dsf = -0.5 * ss * rsw;
+          }
+        }
+        const double ar = in ? cs : 1.0, ai = -z * r0inv, br = y * r0inv, bi = -x * r0inv;
+        q[PD_AR * np] = ar;
+        q[PD_AI * np] = ai;
+        q[PD_BR * np] = br;
+        q[PD_BI * np] = bi;
+        // the r^-12 repulsion's force stays FP64: its pair terms are of the size
+        // of the net force and cancel in the sum over neighbours
+        const double ri2 = rinv * rinv, ri4 = ri2 * ri2;
+        const double fr = -1.5e6 * (ri4 * ri4 * ri4 * ri2);
+        q[PD_FX * np] = x * fr;
+        q[PD_FY * np] = y * fr;
+        q[PD_FZ * np] = z * fr;
+        w[PR_AR * np] = R(ar);
+        w[PR_AI * np] = R(ai);
+        w[PR_BR * np] = R(br);
+        w[PR_BI * np] = R(bi);
+        w[PR_DSF * np] = R(dsf * wj);
+        w[PR_UX * np] = R(x * rinv);
+        w[PR_UY * np] = R(y * rinv);
+        w[PR_UZ * np] = R(z * rinv);
+        w[PR_SF * np] = R(sf * wj);
+        w[PR_C1 * np] = R(-sn * rscale0);
+        w[PR_GR * np] = R(fma(cs, rscale0, -r0inv));
+        w[PR_R0 * np] = R(r0inv);
+      }
+      q[PD_SF * np] = sf * wj;
+      A.pj[p] = j;
+    }
+    __syncwarp();
+  };
+  const float cutsq_f = __double2float_ru(S.cutsq);
+  int cnt = 0;
+  for (int al = 0; al < na; ++al) {
+    const int i = A.first + a0 + al;
+    const double4_32a xi = A.x4[i];
+    const float xf = f32_bits(xi.x), yf = f32_bits(xi.y), zf = f32_bits(xi.z);
+    const float thr = f32_cut_threshold(cutsq_f, xf, yf, zf);
     const Row<false> rowc(A.L, i);
     const Row<true> row2(A.L, i);
     const bool two_d = A.L.stride != 0;
-    const int n = rowc.n;
-    const unsigned lt = (1u << lane) - 1u;
-    int cnt = 0;
-    for (int base = 0; base < n; base += 32) {
-      const int k = base + lane;
-      bool take = false;
+    int m = 0;  // pairs of this atom
+    for (int k0 = 0; k0 < rowc.n; k0 += 32) {
+      const int k = k0 + lane;
+      bool keep = false;
       int j = 0;
-      double dx = 0, dy = 0, dz = 0;
-      if (k < n) {
+      if (k < rowc.n) {
         j = two_d ? row2[k] : rowc[k];
-        const double4_32a xj = A.x4[j];
-        dx = xj.x - xi.x;
-        dy = xj.y - xi.y;
-        dz = xj.z - xi.z;
-        take = (dx * dx + dy * dy + dz * dz) < S.cutsq;
+        const double4_32a p = A.x4[j];
+        const float fx = xf - f32_bits(p.x), fy = yf - f32_bits(p.y), fz = zf - f32_bits(p.z);
+        keep = !(fmaf(fz, fz, fmaf(fy, fy, fx * fx)) > thr);
       }
-      const unsigned m = __ballot_sync(FULL_MASK, take);
-      const int pos = cnt + __popc(m & lt);
-      if (take && pos < A.cap) {
-        const int ej = S.map[A.type[j]];
-        in_j[pos] = j;
-        in_r[3 * pos] = dx;
-        in_r[3 * pos + 1] = dy;
-        in_r[3 * pos + 2] = dz;
-        in_w[pos] = S.wjelem[ej];
-        in_rc[pos] = (radi + S.radelem[ej]) * S.rcutfac;
+      const unsigned bal = __ballot_sync(FULL_MASK, keep);
+      if (cnt + __popc(bal) > SP_CAP) {
+        flush(cnt);
+        cnt = 0;
       }
-      cnt += __popc(m);
+      if (keep) {
+        const int s = __popc(bal & lt);
+        lj[cnt + s] = j;
+        la[cnt + s] = al | ((m + s) << 4);
+      }
+      cnt += __popc(bal);
+      m += __popc(bal);
     }
-    if (lane == 0) {
-      if (cnt > A.cap) latch_status(A.status, ST_BOUNDS);
-      s_ninside = min(cnt, A.cap);
-    }
+    if (lane == 0) A.cnt[a0 + al] = m;
   }
-  __syncthreads();
-  const int ninside = s_ninside;
+  flush(cnt);
+}
 
-  // ---- per-neighbour scalars, one thread per neighbour (every lane of a
-  // warp would otherwise repeat the FP64 transcendentals)
-  for (int nb = tid; nb < ninside; nb += SNAP_THREADS) {
-    const double x = in_r[3 * nb], y = in_r[3 * nb + 1], z = in_r[3 * nb + 2];
-    const double rcut = in_rc[nb], wj = in_w[nb];
-    const double rsq = x * x + y * y + z * z;
-    const double r = sqrt(rsq);
-    double* q = nd + nb;
-    if constexpr (kF64) {
-      // compute_ui (sna_impl.hpp:174-187): a, b of compute_uarray
-      {
-        const double theta0 = (r - S.rmin0) * S.rfac0 * MY_PI / (rcut - S.rmin0);
-        const double z0 = r / tan(theta0);
-        const double r0inv = 1.0 / sqrt(r * r + z0 * z0);
-        q[ND_AR_U * A.cap] = r0inv * z0;
-        q[ND_AI_U * A.cap] = -r0inv * z;
-        q[ND_BR_U * A.cap] = r0inv * y;
-        q[ND_BI_U * A.cap] = -r0inv * x;
-      }
-      q[ND_SFAC * A.cap] = sfac_of(S, r, rcut) * wj;
-      // compute_duidrj + the prologue of compute_duarray (sna_impl.hpp:291-321, 729-778)
-      const double rscale0 = S.rfac0 * MY_PI / (rcut - S.rmin0);
-      const double theta0 = (r - S.rmin0) * rscale0;
-      const double cs = cos(theta0), sn = sin(theta0);
-      const double z0 = r * cs / sn;
-      const double dz0dr = z0 / r - (r * rscale0) * (rsq + z0 * z0) / rsq;
-      const double rinv = 1.0 / r;
-      const double uk[3] = {x * rinv, y * rinv, z * rinv};
-      const double r0inv = 1.0 / sqrt(r * r + z0 * z0);
-      q[ND_AR * A.cap] = z0 * r0inv;
-      q[ND_AI * A.cap] = -z * r0inv;
-      q[ND_BR * A.cap] = y * r0inv;
-      q[ND_BI * A.cap] = -x * r0inv;
-      const double dr0invdr = -(r0inv * r0inv * r0inv) * (r + z0 * dz0dr);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const double dr0inv = dr0invdr * uk[k];
-        const double dz0 = dz0dr * uk[k];
-        q[(ND_DAR + k) * A.cap] = dz0 * r0inv + z0 * dr0inv + 0.0;
-        q[(ND_DAI + k) * A.cap] = -z * dr0inv + (k == 2 ? -r0inv : 0.0);
-        q[(ND_DBR + k) * A.cap] = y * dr0inv + (k == 1 ? r0inv : 0.0);
-        q[(ND_DBI + k) * A.cap] = -x * dr0inv + (k == 0 ? -r0inv : 0.0);
-        q[(ND_UK + k) * A.cap] = uk[k];
-      }
-      q[ND_DSFAC * A.cap] = dsfac_of(S, r, rcut) * wj;
-      // extra repulsion of the reference (force_snap_neigh_impl.h:705-711) and
-      // its energy 1.25e5 / r^12 per ordered pair
-      const double r2 = rsq * rsq, r4 = r2 * r2;
-      const double fdivr = -1.5e6 / (r4 * r2 * rsq);
-      q[ND_FP * A.cap] = x * fdivr;
-      q[(ND_FP + 1) * A.cap] = y * fdivr;
-      q[(ND_FP + 2) * A.cap] = z * fdivr;
-      q[ND_EP * A.cap] = 1.25e5 / (r4 * r2);
-    } else {
-      // Mixed form: the same quantities in closed form, once, in FP64.  With
-      // s = sin(theta0), c = cos(theta0): z0 = r c / s, r0inv = s / r, so
-      //   a = c - i z s / r,  b = (y - i x) s / r  (compute_ui and
-      //   compute_duidrj give these twice, sna_impl.hpp:174-187, 291-321),
-      //   da/dr_k = -s rscale0 u_k,  d(s / r)/dr_k = g u_k,
-      //   g = (c rscale0 r - s) / r^2  (the prologue of compute_duarray,
-      //   sna_impl.hpp:729-778, in a form without its cancelling terms).
-      // a, b and sfac feed phase B in FP64; the rest is rounded once to FP32
-      // for phase D.
-      R* qf = ndr + nb;
-      const double rscale0 = S.rfac0 * MY_PI / (rcut - S.rmin0);
-      double sn, cs;
-      sincos((r - S.rmin0) * rscale0, &sn, &cs);
-      const double rinv = 1.0 / r;
-      const double r0inv = sn * rinv;
-      const double uk[3] = {x * rinv, y * rinv, z * rinv};
-      const double g = (cs * rscale0 * r - sn) * (rinv * rinv);
-      q[ndx<false>(ND_AR_U) * A.cap] = cs;
-      q[ndx<false>(ND_AI_U) * A.cap] = -z * r0inv;
-      q[ndx<false>(ND_BR_U) * A.cap] = y * r0inv;
-      q[ndx<false>(ND_BI_U) * A.cap] = -x * r0inv;
-      qf[nrx<false>(ND_AR) * A.cap] = R(cs);
-      qf[nrx<false>(ND_AI) * A.cap] = R(-z * r0inv);
-      qf[nrx<false>(ND_BR) * A.cap] = R(y * r0inv);
-      qf[nrx<false>(ND_BI) * A.cap] = R(-x * r0inv);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const double dr0inv = g * uk[k];
-        qf[nrx<false>(ND_DAR + k) * A.cap] = R(-sn * rscale0 * uk[k]);
-        qf[nrx<false>(ND_DAI + k) * A.cap] = R(-z * dr0inv + (k == 2 ? -r0inv : 0.0));
-        qf[nrx<false>(ND_DBR + k) * A.cap] = R(y * dr0inv + (k == 1 ? r0inv : 0.0));
-        qf[nrx<false>(ND_DBI + k) * A.cap] = R(-x * dr0inv + (k == 0 ? -r0inv : 0.0));
-        qf[nrx<false>(ND_UK + k) * A.cap] = R(uk[k]);
-      }
-      // switching function and its derivative from one sincos (compute_sfac,
-      // compute_dsfac, sna_impl.hpp:1099-1128)
-      double sf = 1.0, dsf = 0.0;
-      if (S.switchflag != 0 && r > S.rmin0) {
-        if (r > rcut) {
-          sf = 0.0;
-        } else {
-          const double rcutfac = MY_PI / (rcut - S.rmin0);
-          double ss, cc;
-          sincos((r - S.rmin0) * rcutfac, &ss, &cc);
-          sf = 0.5 * (cc + 1.0);
-          dsf = -0.5 * ss * rcutfac;
-        }
-      }
-      q[ndx<false>(ND_SFAC) * A.cap] = sf * wj;
-      qf[nrx<false>(ND_SFAC) * A.cap] = R(sf * wj);
-      qf[nrx<false>(ND_DSFAC) * A.cap] = R(dsf * wj);
-      // the r^-12 repulsion's force stays FP64: its pair terms are of the size
-      // of the net force and cancel in the sum over neighbours
-      const double r2 = rsq * rsq, r4 = r2 * r2;
-      const double fdivr = -1.5e6 / (r4 * r2 * rsq);
-      q[ndx<false>(ND_FP) * A.cap] = x * fdivr;
-      q[ndx<false>(ND_FP + 1) * A.cap] = y * fdivr;
-      q[ndx<false>(ND_FP + 2) * A.cap] = z * fdivr;
-    }
-  }
-  __syncthreads();
+// ---------------------------------------------------------------------- U
+// One warp per atom, 32 neighbours at a time.  Lanes = neighbours: the powers
+// p_q + i r_q = a^q and u_T + i v_T = w b^T, the polynomials, and u P_k, v P_k
+// go to the neighbour's row of a shared table.  Lanes = sums: each of the nx
+// real sums is p or r times u P or v P over the neighbours, one FP64
+// multiply-add per neighbour.  Then the half-grid elements, once per atom, in
+// the contraction's type.  Bound by the FP64 pipe: about 240 instructions for
+// 32 neighbours and nx / 32 for each neighbour (480 per atom at twojmax 8 and
+// 26 neighbours, where the layer recursion and its sums took about 1,700).
+inline int su_cols(int J) {  // p, r; u, v; u P_k, v P_k (k >= 1)
+  int c = 2 * (J + 1) + 2 * (J + 1);
+  for (int T = 0; T <= J; ++T)
+    for (int q = 0; q <= J - T; ++q) c += (T ? 2 : 1) * ((J - T - q) / 2);
+  return c | 1;  // odd: rows start in different banks
+}
 
-  // (the adjoint keeps Z for its final contraction, beyond `work`)
-  Cplx<R>* zs = reinterpret_cast<Cplx<R>*>(MODE == 2 ? work + A.work_bytes : work);
-  const R* cg = sizeof(R) == 8 ? reinterpret_cast<const R*>(S.cg) : reinterpret_cast<const R*>(S.cg_f);
-  if (MODE == 2 && kF64 && A.keep_u != nullptr) {
-    // B and C as the force pass on the same positions and list left them
-    // (the same operations: the values are bit for bit those of a rerun)
-    const Cplx<double>* ku = A.keep_u + size_t(i) * S.nuf;
-    const Cplx<double>* kz = A.keep_z + size_t(i) * S.njobs;
-    for (int e = tid; e < S.nuf; e += SNAP_THREADS) utot[e] = ku[e];
-    for (int e = tid; e < S.njobs; e += SNAP_THREADS) zs[e] = Cplx<R>{R(kz[e].r), R(kz[e].i)};
-  } else {
-    // ---- B: U_tot (FP64, both forms); layer loops unrolled at the SNAP-W setting
-    if (S.twojmax == 8)
-      b_stage<R, 8>(S, nd, A.cap, ninside, reinterpret_cast<Cplx<double>*>(work), utot, utot_r);
-    else
-      b_stage<R>(S, nd, A.cap, ninside, reinterpret_cast<Cplx<double>*>(work), utot, utot_r);
-    // ---- C: Z jobs and Y = sum_t cY_t Z_t
-    if (S.twojmax == 8)
-      z_jobs<R, 9>(S, utot_r, cg, zs);
-    else
-      z_jobs<R, 0>(S, utot_r, cg, zs);
+// the neighbour's table row: powers, polynomials and products
+__device__ __forceinline__ void su_row(const SnapDev& S, double* t, double ar, double ai, double br, double bi,
+                                       double w) {
+  const int J = S.twojmax;
+  double* uT = t + 2 * (J + 1);  // u_T, v_T
+  double* prod = t + 4 * (J + 1);
+  t[0] = 1.0;
+  t[1] = 0.0;
+  uT[0] = w;
+  uT[1] = 0.0;
+  double p = ar, r = ai, u = w * br, v = w * bi;
+  for (int q = 1; q <= J; ++q) {
+    t[2 * q] = p;
+    t[2 * q + 1] = r;
+    uT[2 * q] = u;
+    uT[2 * q + 1] = v;
+    if (q == J) break;
+    const double pn = fma(p, ar, -r * ai), un = fma(u, br, -v * bi);
+    r = fma(p, ai, r * ar);
+    v = fma(u, bi, v * br);
+    p = pn;
+    u = un;
   }
-  __syncthreads();
-  if (MODE == 0 && kF64 && A.keep_u != nullptr) {  // kept for a following adjoint
-    Cplx<double>* ku = A.keep_u + size_t(i) * S.nuf;
-    Cplx<double>* kz = A.keep_z + size_t(i) * S.njobs;
-    for (int e = tid; e < S.nuf; e += SNAP_THREADS) ku[e] = utot[e];
-    for (int e = tid; e < S.njobs; e += SNAP_THREADS) kz[e] = Cplx<double>{double(zs[e].r), double(zs[e].i)};
-  }
-  const R* cY = (sizeof(R) == 8 ? reinterpret_cast<const R*>(S.cY) : reinterpret_cast<const R*>(S.cY_f)) +
-                (size_t)ei * S.nfull;
-  // FP64 forces with A.eatom set: the atom's energy in the same pass, the
-  // terms and order of the energy variant (MODE 1) below
-  const bool fuse_e = MODE == 0 && kF64 && A.eatom != nullptr;
-  double eacc = 0.0;
-  for (int e = tid; e < (MODE == 2 ? 0 : S.nyh); e += SNAP_THREADS) {
-    R yr = 0, yi = 0;
-    for (int k = S.yred_off[e]; k < S.yred_off[e + 1]; ++k) {
-      const int jb = S.yred_job[k];
-      const R cy = cY[S.jobs[jb] >> 8];
-      yr += cy * zs[jb].r;
-      yi += cy * zs[jb].i;
+  const double x = fma(ar, ar, ai * ai) - fma(br, br, bi * bi);
+  for (int T = 0; T <= J; ++T) {
+    const double uu = uT[2 * T], vv = uT[2 * T + 1];
+    for (int q = 0; q <= J - T - 2; ++q) {
+      const double2* ab = reinterpret_cast<const double2*>(S.AB) + S.e0[T * (J + 1) + q];
+      const int km = (J - T - q) / 2;
+      double pm = 1.0, pk = x - __ldg(ab).x;
+      *prod++ = uu * pk;
+      if (T > 0) *prod++ = vv * pk;
+      for (int k = 2; k <= km; ++k) {
+        const double2 c = __ldg(ab + k - 1);
+        const double pn = fma(x - c.x, pk, -c.y * pm);
+        pm = pk;
+        pk = pn;
+        *prod++ = uu * pk;
+        if (T > 0) *prod++ = vv * pk;
+      }
     }
-    if (fuse_e) {
-      int j = 0;
-      while (yoff(j + 1) <= e) ++j;
-      const int q = e - yoff(j), mb = q / (j + 1), ma = q % (j + 1);
-      const Cplx<double> u = utot[uoff(j) + ma * (j + 1) + mb];
-      eacc += hw(j, ma, mb) * (u.r * double(yr) + u.i * double(yi));
-    }
-    if constexpr (MODE == 0) {  // w Y / f: the force runs on V = f U (d_reverse)
-      const R f = sizeof(R) == sizeof(double) ? R(S.yscale[e]) : R(S.yscale_f[e]);
-      yr *= f;
-      yi *= f;
-    }
-    ytot[e] = Cplx<R>{yr, yi};
   }
-  __syncthreads();
-  if (fuse_e) {
-    for (int nb = tid; nb < ninside; nb += SNAP_THREADS) eacc += nd[ND_EP * A.cap + nb] * 1.5;  // x 2/3 below
-    const double t = block_sum(eacc, red);
-    if (tid == 0) A.eatom[i] = S.beta0[ei] + (2.0 / 3.0) * t;
-  }
+}
 
-  // ---- energy (optional): beta_0 + (2/3) sum_j sum_half w Re(conj(U) Y) + pair terms
-  if constexpr (MODE == 1) {
-    double acc = 0.0;
-    for (int e = tid; e < S.nyh; e += SNAP_THREADS) {
-      int j = 0;
-      while (yoff(j + 1) <= e) ++j;
-      const int q = e - yoff(j), mb = q / (j + 1), ma = q % (j + 1);
-      const Cplx<double> u = utot[uoff(j) + ma * (j + 1) + mb];
-      acc += hw(j, ma, mb) * (u.r * double(ytot[e].r) + u.i * double(ytot[e].i));
-    }
-    for (int nb = tid; nb < ninside; nb += SNAP_THREADS) acc += nd[ND_EP * A.cap + nb] * 1.5;  // x 2/3 below
-    const double t = block_sum(acc, red);
-    if (tid == 0) A.eatom[i] = S.beta0[ei] + (2.0 / 3.0) * t;
-    return;
+// the half-grid elements of entry e from its real sums: conj(a)^q b^T = (p u +
+// r v) + i (p v - r u); for -T: (-1)^T ((p u - r v) - i (p v + r u)); N scales,
+// the atom's own term is 1 on the diagonal (T = 0)
+template <typename R>
+__device__ __forceinline__ void su_store(const SnapDev& S, int e, const double* x, double self, Cplx<R>* U) {
+  const Entry& E = S.ent[e];
+  x += E.xo;
+  double pu = *x++, ru = 0.0, pv = 0.0, rv = 0.0;
+  if (E.q > 0) ru = *x++;
+  if (E.T > 0) pv = *x++;
+  if (E.q > 0 && E.T > 0) rv = *x;
+  const int2 h = S.half[e];
+  U[h.x] = Cplx<R>{R(fma(E.N, pu + rv, E.T == 0 ? self : 0.0)), R(E.N * (pv - ru))};
+  if (h.y >= 0) {
+    const double sg = E.T & 1 ? -E.N : E.N;
+    U[h.y] = Cplx<R>{R(sg * (pu - rv)), R(-sg * (pv + ru))};
   }
+}
 
-  // ---- adjoint: for every full triple t = (j1, j2, j), with Z_t kept from C,
-  //   P_t = 2 sum_half w Re(conj(U_j) Z_t)        (= B_k when t is idxj triple k)
-  //   Q_t = 2 sum_half w Re(conj(D_j) Z_t),  D = sum_nb dU'_nb . (g_i - g_j)
-  // so that d/dbeta_k [sum_atoms g . F] over this atom's pairs is
-  // Q_t1 + (j+1)/(j1+1) Q_t2 + (j+1)/(j2+1) Q_t3 (compute_dbidrj's three terms,
-  // sna_impl.hpp:330-570, contracted with the loss gradient before the sum
-  // over k instead of after it).
-  if constexpr (MODE == 2) {
-    Cplx<double>* dpart = reinterpret_cast<Cplx<double>*>(zs + S.njobs);  // SNAP_WARPS x nyh
-    Cplx<double>* dsum = dpart + SNAP_WARPS * S.nyh;                      // nyh
-    Cplx<double>* dp = dpart + warp * S.nyh;
-    for (int e = lane; e < S.nyh; e += 32) dp[e] = Cplx<double>{0.0, 0.0};
-    const double gix = A.g[3 * i], giy = A.g[3 * i + 1], giz = A.g[3 * i + 2];
-    Cplx<R>* wd = reinterpret_cast<Cplx<R>*>(work) + warp * (4 * L2);
+template <typename R>
+__global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
+  const SnapDev& S = A.S;
+  extern __shared__ __align__(16) double su_smem[];
+  double* xs = su_smem;                       // nx sums
+  double* tab = su_smem + ((S.nx + 1) & ~1);  // 32 rows
+  const int al = blockIdx.x, lane = threadIdx.x;
+  const int cols = S.cols, n = A.cnt[al];
+  const size_t np = size_t(A.n) * A.cap;
+  const double* pd = A.pd + size_t(al) * A.cap;
+  for (int n0 = 0; n0 < max(n, 1); n0 += 32) {
+    const int m = min(32, n - n0);
+    if (lane < m) {
+      const double* q = pd + n0 + lane;
+      su_row(S, tab + lane * cols, q[PD_AR * np], q[PD_AI * np], q[PD_BR * np], q[PD_BI * np], q[PD_SF * np]);
+    }
     __syncwarp();
-    for (int nb = warp; nb < ninside; nb += SNAP_WARPS) {
-      const R* qr = ndr + nb;
-      const R Rar = qr[ND_AR * A.cap], Rai = qr[ND_AI * A.cap], Rbr = qr[ND_BR * A.cap], Rbi = qr[ND_BI * A.cap];
-      // the pair's reaction force lands on j's owner (newton) or nowhere
-      const int j = in_j[nb];
-      const int jo = j < A.n_local ? j : (A.newton ? A.ghost_owner[j - A.n_local] : -1);
-      const double gjx = jo >= 0 ? A.g[3 * jo] : 0.0, gjy = jo >= 0 ? A.g[3 * jo + 1] : 0.0,
-                   gjz = jo >= 0 ? A.g[3 * jo + 2] : 0.0;
-      const R dv[3] = {R(gix - gjx), R(giy - gjy), R(giz - gjz)};
-      // derivatives of a, b, sfac along dv
-      R tar = 0, tai = 0, tbr = 0, tbi = 0, tu = 0;
+    for (int r0 = 0; r0 < S.nx; r0 += 96) {  // three sums per lane at once
+      int2 s[3];
+      double acc[3];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        tar += qr[(ND_DAR + k) * A.cap] * dv[k];
-        tai += qr[(ND_DAI + k) * A.cap] * dv[k];
-        tbr += qr[(ND_DBR + k) * A.cap] * dv[k];
-        tbi += qr[(ND_DBI + k) * A.cap] * dv[k];
-        tu += qr[(ND_UK + k) * A.cap] * dv[k];
+      for (int h = 0; h < 3; ++h) {
+        const int r = r0 + 32 * h + lane;
+        s[h] = r < S.nx ? __ldg(S.xsum + r) : int2{0, 0};
+        acc[h] = r < S.nx && n0 > 0 ? xs[r] : 0.0;
       }
-      const R Rsfac = qr[ND_SFAC * A.cap], sv = qr[ND_DSFAC * A.cap] * tu;
-      Cplx<R>* P = wd;
-      Cplx<R>* C = wd + L2;
-      Cplx<R>* TP = wd + 2 * L2;
-      Cplx<R>* TC = wd + 3 * L2;
-      if (lane == 0) {
-        P[0] = Cplx<R>{R(1), R(0)};
-        TP[0] = Cplx<R>{R(0), R(0)};
-        dp[0].r += sv;
-      }
-      __syncwarp();
-      auto layer = [&](int jl) {
-        dt_layer<R>(jl, lane, Rar, Rai, Rbr, Rbi, tar, tai, tbr, tbi, P, TP, C, TC);
-        const int nh = (jl + 1) * (jl / 2 + 1), yo = yoff(jl);
-        for (int e = lane; e < nh; e += 32) {  // rescaled: D = sum (sv V + sfac T), times 1/f below
-          dp[yo + e].r += sv * C[e].r + Rsfac * TC[e].r;
-          dp[yo + e].i += sv * C[e].i + Rsfac * TC[e].i;
+      if (r0 + 64 < S.nx) {
+#pragma unroll 2
+        for (int k = 0; k < m; ++k) {
+          const double* t = tab + k * cols;
+#pragma unroll
+          for (int h = 0; h < 3; ++h) acc[h] = fma(t[s[h].x], t[s[h].y], acc[h]);
         }
-        __syncwarp();
-        Cplx<R>* t = P;
-        P = C;
-        C = t;
-        t = TP;
-        TP = TC;
-        TC = t;
-      };
-      if (S.twojmax == 8) {  // layer loop unrolled: constant index arithmetic
+      } else if (r0 + 32 < S.nx) {
+        for (int k = 0; k < m; ++k) {
+          const double* t = tab + k * cols;
 #pragma unroll
-        for (int jl = 1; jl <= 8; ++jl) layer(jl);
+          for (int h = 0; h < 2; ++h) acc[h] = fma(t[s[h].x], t[s[h].y], acc[h]);
+        }
       } else {
-        for (int jl = 1; jl <= S.twojmax; ++jl) layer(jl);
+        for (int k = 0; k < m; ++k) {
+          const double* t = tab + k * cols;
+          acc[0] = fma(t[s[0].x], t[s[0].y], acc[0]);
+        }
       }
+#pragma unroll
+      for (int h = 0; h < 3; ++h)
+        if (r0 + 32 * h + lane < S.nx) xs[r0 + 32 * h + lane] = acc[h];
     }
-    __syncthreads();
-    for (int e = tid; e < S.nyh; e += SNAP_THREADS) {
-      double sr = 0.0, si = 0.0;
-      for (int w = 0; w < SNAP_WARPS; ++w) {
-        sr += dpart[w * S.nyh + e].r;
-        si += dpart[w * S.nyh + e].i;
-      }
-      dsum[e] = Cplx<double>{sr * S.invf[e], si * S.invf[e]};
-    }
-    __syncthreads();
-    const size_t n = size_t(A.n_local);
-    for (int t = tid; t < S.nfull; t += SNAP_THREADS) {
-      const int jt = S.trip[3 * t + 2];
-      double p = 0.0, q = 0.0;
-      for (int jb = S.tjob_off[t]; jb < S.tjob_off[t + 1]; ++jb) {
-        const int code = S.jobs[jb];
-        const int ma = (code >> 4) & 15, mb = code & 15;
-        const double w = hw(jt, ma, mb);
-        if (w == 0.0) continue;
-        const Cplx<double> u = utot[uoff(jt) + ma * (jt + 1) + mb];
-        const Cplx<double> d = dsum[yoff(jt) + mb * (jt + 1) + ma];
-        const double zr = double(zs[jb].r), zi = double(zs[jb].i);
-        p += w * (u.r * zr + u.i * zi);
-        q += w * (d.r * zr + d.i * zi);
-      }
-      A.adj[size_t(t) * n + i] = 2.0 * p;
-      A.adj[size_t(S.nfull + t) * n + i] = 2.0 * q;
-    }
-    if (tid == 0) A.adj[size_t(2 * S.nfull) * n + i] = 1.0;  // atom count column (beta_0)
-    return;
+    __syncwarp();
   }
+  Cplx<R>* U = static_cast<Cplx<R>*>(A.U) + size_t(al) * S.nh;
+  for (int e = lane; e < S.ne; e += 32) su_store<R>(S, e, xs, S.wself, U);
+}
 
-  // ---- D: the pair forces in reverse mode (d_reverse), two neighbours per
-  // warp at a time; the FP64 part (repulsion, scatter to j, the sum for i) is
-  // done afterwards, one thread per neighbour.
-  {
-    const int J = S.twojmax, stride = drev_words(J);
-    Cplx<R>* W = reinterpret_cast<Cplx<R>*>(work) + size_t(warp) * 2 * stride;
-    double* fpair = in_r;  // r_ij is not read after the per-neighbour scalars
-    for (int nb0 = warp; nb0 < ninside; nb0 += 2 * SNAP_WARPS) {
-      const int nb1 = nb0 + SNAP_WARPS;
-      const int nn = nb1 < ninside ? 2 : 1;
-      DRevAB<R> ab[2];
-      for (int n = 0; n < 2; ++n) {
-        const R* qr = ndr + (n < nn ? (n ? nb1 : nb0) : nb0);
-        ab[n] = DRevAB<R>{qr[nrx<kF64>(ND_AR) * A.cap], qr[nrx<kF64>(ND_AI) * A.cap], qr[nrx<kF64>(ND_BR) * A.cap], qr[nrx<kF64>(ND_BI) * A.cap]};
-      }
-      R phi[2];
-      Cplx<R> ga[2], gb[2];
-      if (J == 8) {  // the SNAP-W setting: layer loops unrolled
-        if (nn == 2)
-          d_reverse<R, 2, 8>(J, lane, ab, ytot, W, phi, ga, gb);
-        else
-          d_reverse<R, 1, 8>(J, lane, ab, ytot, W, phi, ga, gb);
-      } else if (nn == 2) {
-        d_reverse<R, 2>(J, lane, ab, ytot, W, phi, ga, gb);
-      } else {
-        d_reverse<R, 1>(J, lane, ab, ytot, W, phi, ga, gb);
-      }
-      for (int n = 0; n < nn; ++n) {
-        const int nb = n ? nb1 : nb0;
-        const R* qr = ndr + nb;
-        const R sf = qr[nrx<kF64>(ND_SFAC) * A.cap], cp = qr[nrx<kF64>(ND_DSFAC) * A.cap] * phi[n];
-        R fk[3];
+// ------------------------------------------------------------------- Z, Y
+// Lanes = atoms of a tile (ta of them; for ta < 32 the 32 / ta lane groups
+// share a record's products), warps = tasks.  A task is one (T, q): it owns
+// Y_j(m, m') at (2m, 2m') = (-q -+ T, -q +- T) for every j, because Z_j at one
+// (m, m') comes from products U_j1(m1, m1') U_j2(m - m1, m' - m1') that do not
+// depend on j: each product is formed once (4 operations) and weighted by both
+// Clebsch-Gordan factors for every j (2 each), where one Z at a time took 6 for
+// each (compute_zi, sna_impl.hpp:197-283); for j1 = j2 the two orders of a pair
+// of elements are one product.  The loops run over product lists, uniform over
+// the lanes.  Y_j = sum cY Z_j stays in registers; cY folds the linear
+// coefficients with the (j+1)/(j1+1), (j+1)/(j2+1) weights of compute_dbidrj's
+// three terms (sna_impl.hpp:330-539).
+template <int NJ>
+__device__ __forceinline__ void z_products(const ZRec& z, const SnapDev& S, const Cplx<double>* __restrict__ U, int str,
+                                           int first, int step, Cplx<double>* Z) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k)
-          fk[k] = cp * qr[nrx<kF64>(ND_UK + k) * A.cap] +
-                  sf * (ga[n].r * qr[nrx<kF64>(ND_DAR + k) * A.cap] - ga[n].i * qr[nrx<kF64>(ND_DAI + k) * A.cap] -
-                        gb[n].r * qr[nrx<kF64>(ND_DBR + k) * A.cap] + gb[n].i * qr[nrx<kF64>(ND_DBI + k) * A.cap]);
-        // summed over the lanes in the contraction type (an FP64 shuffle tree
-        // would cost the mixed form more FP64-pipe time than its FP32 sweeps)
-        const R sx = warp_sum_r(fk[0]), sy = warp_sum_r(fk[1]), sz = warp_sum_r(fk[2]);
-        if (lane == 0) {
-          fpair[3 * nb] = double(sx);
-          fpair[3 * nb + 1] = double(sy);
-          fpair[3 * nb + 2] = double(sz);
+  for (int j = 0; j < NJ; ++j) Z[j] = Cplx<double>{0.0, 0.0};
+  const int2* __restrict__ pl = S.prod + z.p0;
+  const double* __restrict__ c = S.zc + z.c0;
+#pragma unroll 2
+  for (int k = first; k < z.np; k += step) {
+    const int2 p = __ldg(pl + k);
+    const Cplx<double> x = U[p.x * str], y = U[p.y * str];
+    const double pr = fma(x.r, y.r, -x.i * y.i), pi = fma(x.r, y.i, x.i * y.r);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const double w = __ldg(c + k * NJ + j);
+      Z[j].r = fma(w, pr, Z[j].r);
+      Z[j].i = fma(w, pi, Z[j].i);
+    }
+  }
+}
+// FP32: packed f32x2 operations on (re, im), coefficients stored twice
+template <int NJ>
+__device__ __forceinline__ void z_products(const ZRec& z, const SnapDev& S, const Cplx<float>* __restrict__ U, int str,
+                                           int first, int step, Cplx<float>* Z) {
+  constexpr int NC = (NJ + 1) / 2;
+  float2 acc[2 * NC];
+#pragma unroll
+  for (int j = 0; j < 2 * NC; ++j) acc[j] = make_float2(0.f, 0.f);
+  const int2* __restrict__ pl = S.prod + z.p0;
+  const float4* __restrict__ c = reinterpret_cast<const float4*>(S.zc_f + z.cf);
+#pragma unroll 4
+  for (int k = first; k < z.np; k += step) {
+    const int2 p = __ldg(pl + k);
+    const Cplx<float> x = U[p.x * str], y = U[p.y * str];
+    const float2 yy = make_float2(y.r, y.i);
+    const float2 pp = __ffma2_rn(make_float2(x.r, x.r), yy,
+                                 __fmul2_rn(make_float2(x.i, x.i), make_float2(-y.i, y.r)));
+#pragma unroll
+    for (int h = 0; h < NC; ++h) {
+      const float4 w = __ldg(c + k * NC + h);
+      acc[2 * h] = __ffma2_rn(make_float2(w.x, w.y), pp, acc[2 * h]);
+      if (2 * h + 1 < NJ) acc[2 * h + 1] = __ffma2_rn(make_float2(w.z, w.w), pp, acc[2 * h + 1]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) Z[j] = Cplx<float>{acc[j].x, acc[j].y};
+}
+
+template <typename R>
+__device__ __forceinline__ R shfl_xor_r(R v, int o) {
+  return __shfl_xor_sync(FULL_MASK, v, o);
+}
+
+// a record's Z and its part of the task's Y (y[0]: the highest j)
+template <typename R, int NM, int NJ, bool KEEP>
+__device__ __forceinline__ void z_add(const ZRec& z, const SnapDev& S, const Cplx<R>* __restrict__ U, int str,
+                                      const R* __restrict__ cY, int first, int step, Cplx<R>* y, Cplx<double>* zk) {
+  Cplx<R> Z[NJ];
+  z_products<NJ>(z, S, U, str, first, step, Z);
+  R c[NJ];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    c[j] = cY[z.t0 - j];
+    if constexpr (KEEP) {
+      for (int o = 32 / step; o < 32; o <<= 1) {
+        Z[j].r += shfl_xor_r(Z[j].r, o);
+        Z[j].i += shfl_xor_r(Z[j].i, o);
+      }
+      if (first == 0) zk[size_t(z.z0 + j) * 32] = Cplx<double>{double(Z[j].r), double(Z[j].i)};
+    }
+  }
+  // z.d is uniform; one block per value (the marker keeps the compiler from
+  // folding them into an indexed, hence local-memory, y)
+  auto add = [&](auto dc) {
+    constexpr int d = decltype(dc)::value;
+    if constexpr (d + NJ <= NM) {
+      asm volatile("// y + %0" ::"n"(d));
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        y[d + j].r = fma(c[j], Z[j].r, y[d + j].r);
+        y[d + j].i = fma(c[j], Z[j].i, y[d + j].i);
+      }
+    }
+  };
+  if (z.d == 0) add(std::integral_constant<int, 0>{});
+  else if (z.d == 1) add(std::integral_constant<int, 1>{});
+  else if (z.d == 2) add(std::integral_constant<int, 2>{});
+  else if (z.d == 3) add(std::integral_constant<int, 3>{});
+  else if (z.d == 4) add(std::integral_constant<int, 4>{});
+  else if (z.d == 5) add(std::integral_constant<int, 5>{});
+  else if (z.d == 6) add(std::integral_constant<int, 6>{});
+  else add(std::integral_constant<int, 7>{});
+}
+
+// NM: most j of one (m, m') (5 up to twojmax 9, 8 up to 14); FULL: ta = 32
+template <typename R, int NM, bool KEEP, bool FULL>
+__global__ void __launch_bounds__(sizeof(R) == 8 ? 512 : 256) k_snap_y(SnapArgs A) {
+  const SnapDev& S = A.S;
+  extern __shared__ __align__(16) unsigned char sy_smem[];
+  __shared__ int s_next;
+  Cplx<R>* U = reinterpret_cast<Cplx<R>*>(sy_smem);  // [element][atom], rows of ta + 1
+  const int ta = FULL ? 32 : A.ta, str = ta + 1, tile = blockIdx.x / A.nsplit, split = blockIdx.x - tile * A.nsplit;
+  const int lane = threadIdx.x & 31, at = FULL ? lane : lane % ta, sub = FULL ? 0 : lane / ta, nsub = FULL ? 1 : 32 / ta;
+  const int al = tile * ta + at;
+  const bool live = al < A.n;
+  if (threadIdx.x == 0) s_next = 0;
+  // the tile's U, both halves of the grid
+  for (int k = threadIdx.x; k < S.nh * ta; k += blockDim.x) {
+    const int a = k / S.nh, h = k - a * S.nh, ga = tile * ta + a;
+    const Cplx<R> u = ga < A.n ? static_cast<const Cplx<R>*>(A.U)[size_t(ga) * S.nh + h] : Cplx<R>{R(0), R(0)};
+    const int4 f = __ldg(S.hfull + h);
+    U[f.x * str + a] = u;
+    if (f.y != f.x) U[f.y * str + a] = f.z > 0 ? Cplx<R>{u.r, -u.i} : Cplx<R>{-u.r, u.i};
+  }
+  __syncthreads();
+  const int ei = live ? S.map[A.type[A.first + al]] : 0;
+  const R* cY = (sizeof(R) == 8 ? reinterpret_cast<const R*>(S.cY) : reinterpret_cast<const R*>(S.cY_f)) +
+                size_t(ei) * S.nfull;
+  R* Yt = static_cast<R*>(A.Y) + size_t(tile) * 4 * S.ne * ta + at;
+  Cplx<double>* zk = reinterpret_cast<Cplx<double>*>(A.zkeep) + (KEEP ? size_t(al >> 5) * S.nz * 32 + (al & 31) : 0);
+  const Cplx<R>* Ua = U + at;
+  while (true) {
+    int t = 0;
+    if (lane == 0) t = atomicAdd(&s_next, 1);
+    t = __shfl_sync(FULL_MASK, t, 0) * A.nsplit + split;  // tasks longest first
+    if (t >= S.ntask) break;
+    const ZTask K = S.task[t];
+    Cplx<R> y[NM], yp[NM];  // Y of the -T elements (first: +T), of the +T elements
+#pragma unroll
+    for (int k = 0; k < NM; ++k) y[k] = Cplx<R>{R(0), R(0)};
+#pragma unroll 1
+    for (int r = K.rec0; r < K.rec2; ++r) {
+      if (r == K.rec1) {
+#pragma unroll
+        for (int k = 0; k < NM; ++k) {
+          yp[k] = y[k];
+          y[k] = Cplx<R>{R(0), R(0)};
         }
       }
-      __syncwarp();
+      const ZRec z = S.rec[r];
+      switch (z.nj) {  // uniform
+        case 1: z_add<R, NM, 1, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
+        case 2: z_add<R, NM, 2, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
+        case 3: z_add<R, NM, 3, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
+        case 4: z_add<R, NM, 4, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
+        case 5: z_add<R, NM, 5, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
+        default:
+          if constexpr (NM > 5) {
+            if (z.nj == 6) z_add<R, NM, 6, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk);
+            else if (z.nj == 7) z_add<R, NM, 7, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk);
+            else z_add<R, NM, 8, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk);
+          }
+      }
     }
-    __syncthreads();
-    for (int nb = tid; nb < ninside; nb += SNAP_THREADS) {
-      const double Fx = fpair[3 * nb] + nd[ndx<kF64>(ND_FP) * A.cap + nb];
-      const double Fy = fpair[3 * nb + 1] + nd[ndx<kF64>(ND_FP + 1) * A.cap + nb];
-      const double Fz = fpair[3 * nb + 2] + nd[ndx<kF64>(ND_FP + 2) * A.cap + nb];
-      const int j = in_j[nb];
-      atomicAdd(A.f + 3 * j, -Fx);
-      atomicAdd(A.f + 3 * j + 1, -Fy);
-      atomicAdd(A.f + 3 * j + 2, -Fz);
-      fpair[3 * nb] = Fx;
-      fpair[3 * nb + 1] = Fy;
-      fpair[3 * nb + 2] = Fz;
-    }
-    __syncthreads();
-    if (warp == 0) {  // f_i += sum over the neighbours, in a fixed order
+    if (K.rec1 == K.rec2) {  // no -T elements
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        double t = 0.0;
-        for (int nb = lane; nb < ninside; nb += 32) t += fpair[3 * nb + k];
-        t = warp_sum(t);
-        if (lane == 0) atomicAdd(A.f + 3 * i + k, t);
+      for (int k = 0; k < NM; ++k) {
+        yp[k] = y[k];
+        y[k] = Cplx<R>{R(0), R(0)};
+      }
+    }
+    // the lane groups' parts (KEEP: every Z was completed already)
+    for (int o = ta; o < 32 && !KEEP; o <<= 1)
+#pragma unroll
+      for (int k = 0; k < NM; ++k) {
+        yp[k].r += shfl_xor_r(yp[k].r, o);
+        yp[k].i += shfl_xor_r(yp[k].i, o);
+        y[k].r += shfl_xor_r(y[k].r, o);
+        y[k].i += shfl_xor_r(y[k].i, o);
+      }
+    // E = 2N (Y+ + (-1)^T Y-), O = 2N (Y+ - (-1)^T Y-): with a^q and w b^T =
+    // u + i v, twice the real part of conj(U) Y over both signs of T is
+    // u Re(a^q E) + v Im(a^q O) times P_k
+    if (sub == 0) {
+#pragma unroll
+      for (int h = 0; h < NM; ++h)
+        if (h <= K.kmax) {
+          const int k = K.kmax - h;
+          const R N = R(S.ent[K.y0 + k].N), N2 = N + N;
+          R er, ei2, orr, oi;
+          const Cplx<R> p = yp[h], m = y[h];
+          if (K.q == 0) {  // the -T element is the inversion of the +T one
+            er = (K.T ? N2 : N) * p.r;
+            oi = K.T ? N2 * p.i : R(0);
+            ei2 = orr = R(0);
+          } else if (K.T == 0) {
+            er = N2 * p.r;
+            ei2 = N2 * p.i;
+            orr = oi = R(0);
+          } else {
+            const R sg = K.T & 1 ? R(-1) : R(1);
+            er = N2 * fma(sg, m.r, p.r);
+            ei2 = N2 * fma(sg, m.i, p.i);
+            orr = N2 * fma(-sg, m.r, p.r);
+            oi = N2 * fma(-sg, m.i, p.i);
+          }
+          R* o = Yt + size_t(4) * (K.y0 + k) * ta;
+          o[0] = er;
+          o[ta] = ei2;
+          o[2 * ta] = orr;
+          o[3 * ta] = oi;
+        }
+    }
+  }
+}
+
+// ------------------------------------------------------------- pair forces
+// Lanes = pairs, pooled over the CTA's atoms.  Phi = sum_j 2 sum_half w
+// Re(conj(U_j) Y_j) of one neighbour is sum_T u_T Re(Eh_T) + v_T Im(Oh_T) with
+// Eh_T = sum_q a^q sum_k E P_k and Oh_T likewise, and the pair force needs only
+// Phi and its gradient in (a, b):
+//   F_k = dsfac u_k Phi + sfac dPhi/dp dp/dr_k + the r^-14 term,
+// which equals sum_k beta_k dB_k/dr_ij of the reference.  About 1,250
+// operations per neighbour at twojmax 8 (the layered adjoint took 4,100, half
+// its lanes idle).  f_j -= F_ij with FP64 atomics (j may be a ghost;
+// update_force follows) and f_i += sum_j F_ij in a fixed order.
+constexpr int SF_THREADS = 256;
+constexpr int SF_ATOMS = 8;
+
+// NQ: powers of a kept in registers (twojmax + 1 <= NQ)
+template <typename R, int NQ>
+__global__ void __launch_bounds__(SF_THREADS) k_snap_force(SnapArgs A) {
+  const SnapDev& S = A.S;
+  constexpr bool kF64 = sizeof(R) == sizeof(double);
+  extern __shared__ __align__(16) unsigned char sf_smem[];
+  __shared__ int s_off[SF_ATOMS + 1];
+  __shared__ double s_sum[SF_ATOMS][3];
+  const int J = S.twojmax, ny = 4 * S.ne, tid = threadIdx.x;
+  const int apc = A.apc, a0 = blockIdx.x * apc, na = min(apc, A.n - a0);
+  // groups of T on separate warps (small systems): each forms a part of F
+  const int nthr = blockDim.x / A.tsplit, grp = tid / nthr, gt = tid - grp * nthr;
+  R* ys = reinterpret_cast<R*>(sf_smem);                                   // apc x ny
+  double* fs = reinterpret_cast<double*>(sf_smem + ((size_t(apc) * ny * sizeof(R) + 15) & ~size_t(15)));  // blockDim x 3
+  const int ta = A.ta;
+  for (int k = tid; k < ny * na; k += blockDim.x) {
+    const int e = k / na, a = k - e * na, ga = a0 + a;
+    ys[a * ny + e] = static_cast<const R*>(A.Y)[(size_t(ga / ta) * ny + e) * ta + ga % ta];
+  }
+  if (tid == 0) {
+    int o = 0;
+    for (int a = 0; a < na; ++a) {
+      s_off[a] = o;
+      o += A.cnt[a0 + a];
+    }
+    s_off[na] = o;
+  }
+  if (tid < 3 * SF_ATOMS) s_sum[tid / 3][tid % 3] = 0.0;
+  __syncthreads();
+  const int total = s_off[na];
+  const size_t np = size_t(A.n) * A.cap;
+  const R* AB = kF64 ? reinterpret_cast<const R*>(S.AB) : reinterpret_cast<const R*>(S.AB_f);
+  const unsigned mask = A.tsplit > 1 ? unsigned(A.tmask[grp]) : 0xffffffffu;
+  for (int s0 = 0; s0 < total; s0 += nthr) {
+    const int s = s0 + gt;
+    double F[3] = {0.0, 0.0, 0.0};
+    size_t p = 0;
+    if (s < total) {
+      int a = 0;
+      while (s >= s_off[a + 1]) ++a;
+      p = size_t(a0 + a) * A.cap + (s - s_off[a]);
+      const double* qd = A.pd + p;
+      const R* qr = static_cast<const R*>(A.pr) + p;
+      const R ar = qr[PR_AR * np], ai = qr[PR_AI * np], br = qr[PR_BR * np], bi = qr[PR_BI * np];
+      R pq[NQ], rq[NQ];  // a^q
+      pq[0] = R(1);
+      rq[0] = R(0);
+#pragma unroll
+      for (int q = 1; q < NQ; ++q) {
+        pq[q] = fma(pq[q - 1], ar, -rq[q - 1] * ai);
+        rq[q] = fma(pq[q - 1], ai, rq[q - 1] * ar);
+      }
+      const R x = fma(ar, ar, ai * ai) - fma(br, br, bi * bi);
+      R u = R(1), v = R(0), um = R(0), vm = R(0);  // b^T, b^(T-1)
+      R phi = 0, gx = 0, gar = 0, gai = 0, gbr = 0, gbi = 0;
+      const R* Y = ys + a * ny;
+      const R* ab = AB;
+      for (int T = 0; T <= J; ++T) {
+        if (mask >> T & 1) {
+          // sums over q: Re Eh, Im Oh; the same with P'; dEh/da, dOh/da
+          R er = 0, oi = 0, xer = 0, xoi = 0, e1r = 0, e1i = 0, o1r = 0, o1i = 0;
+#pragma unroll
+          for (int q = 0; q < NQ; ++q) {
+            if (q > J - T) break;
+            const int km = (J - T - q) / 2;
+            R g0 = Y[0], g1 = Y[1], g2 = Y[2], g3 = Y[3];  // sum_k E P_k, O P_k
+            R h0 = 0, h1 = 0, h2 = 0, h3 = 0;              // sum_k E P'_k, O P'_k
+            if (km > 0) {
+              R pk = x - ab[0], pm = R(1), dk = R(1), dm = R(0);
+              h0 = Y[4];
+              h1 = Y[5];
+              h2 = Y[6];
+              h3 = Y[7];
+              g0 = fma(h0, pk, g0);
+              g1 = fma(h1, pk, g1);
+              g2 = fma(h2, pk, g2);
+              g3 = fma(h3, pk, g3);
+              for (int k = 2; k <= km; ++k) {
+                const R t = x - ab[2 * (k - 1)], c = ab[2 * (k - 1) + 1];
+                const R pn = fma(t, pk, -c * pm), dn = fma(t, dk, fma(-c, dm, pk));
+                pm = pk;
+                pk = pn;
+                dm = dk;
+                dk = dn;
+                const R* yk = Y + 4 * k;
+                g0 = fma(yk[0], pk, g0);
+                g1 = fma(yk[1], pk, g1);
+                h0 = fma(yk[0], dk, h0);
+                h1 = fma(yk[1], dk, h1);
+                if (T > 0) {
+                  g2 = fma(yk[2], pk, g2);
+                  g3 = fma(yk[3], pk, g3);
+                  h2 = fma(yk[2], dk, h2);
+                  h3 = fma(yk[3], dk, h3);
+                }
+              }
+            }
+            er = fma(pq[q], g0, er);
+            xer = fma(pq[q], h0, xer);
+            if (q > 0) {
+              const R qp = R(q) * pq[q - 1], qr1 = R(q) * rq[q - 1];
+              er = fma(-rq[q], g1, er);
+              xer = fma(-rq[q], h1, xer);
+              e1r = fma(qp, g0, fma(-qr1, g1, e1r));
+              e1i = fma(qp, g1, fma(qr1, g0, e1i));
+              if (T > 0) {
+                oi = fma(rq[q], g2, oi);
+                xoi = fma(rq[q], h2, xoi);
+                o1r = fma(qp, g2, fma(-qr1, g3, o1r));
+                o1i = fma(qp, g3, fma(qr1, g2, o1i));
+              }
+            }
+            if (T > 0) {
+              oi = fma(pq[q], g3, oi);
+              xoi = fma(pq[q], h3, xoi);
+            }
+            Y += 4 * (km + 1);
+            ab += 2 * (km + 1);
+          }
+          phi = fma(u, er, fma(v, oi, phi));
+          gx = fma(u, xer, fma(v, xoi, gx));
+          gar = fma(u, e1r, fma(v, o1i, gar));
+          gai = fma(-u, e1i, fma(v, o1r, gai));
+          if (T > 0) {
+            const R tu = R(T) * um, tv = R(T) * vm;
+            gbr = fma(tu, er, fma(tv, oi, gbr));
+            gbi = fma(tu, oi, fma(-tv, er, gbi));
+          }
+        } else {
+          int sk = 0;
+          for (int q = 0; q <= J - T; ++q) sk += (J - T - q) / 2 + 1;
+          Y += 4 * sk;
+          ab += 2 * sk;
+        }
+        um = u;
+        vm = v;
+        const R un = fma(u, br, -v * bi);
+        v = fma(u, bi, v * br);
+        u = un;
+      }
+      const R gx2 = gx + gx;
+      gar = fma(ar, gx2, gar);
+      gai = fma(ai, gx2, gai);
+      gbr = fma(-br, gx2, gbr);
+      gbi = fma(-bi, gx2, gbi);
+      const R cp = qr[PR_DSF * np] * phi;
+      const R uk[3] = {qr[PR_UX * np], qr[PR_UY * np], qr[PR_UZ * np]};
+      if constexpr (kF64) {
+        const double sf = qd[PD_SF * np];
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          F[d] = fma(cp, uk[d], sf * fma(gar, qr[(PF_DAR + d) * np],
+                                         fma(gai, qr[(PF_DAI + d) * np],
+                                             fma(gbr, qr[(PF_DBR + d) * np], gbi * qr[(PF_DBI + d) * np]))));
+      } else {
+        // along u_k through theta0 and s / r, then the direct terms
+        const R sf = qr[PR_SF * np], c1 = qr[PR_C1 * np], gr = qr[PR_GR * np], r0 = sf * qr[PR_R0 * np];
+        const R rad = fma(sf, fma(c1, gar, gr * fma(-uk[2], gai, fma(uk[1], gbr, -uk[0] * gbi))), cp);
+        F[0] = double(fma(rad, uk[0], -r0 * gbi));
+        F[1] = double(fma(rad, uk[1], r0 * gbr));
+        F[2] = double(fma(rad, uk[2], -r0 * gai));
+      }
+    }
+    if (A.tsplit > 1) {  // the groups' parts, in a fixed order
+      for (int d = 0; d < 3; ++d) fs[3 * tid + d] = F[d];
+      __syncthreads();
+      if (grp == 0)
+        for (int g = 1; g < A.tsplit; ++g)
+          for (int d = 0; d < 3; ++d) F[d] += fs[3 * (g * nthr + gt) + d];
+      __syncthreads();
+    }
+    if (grp == 0) {
+      if (s < total) {
+        const double* qd = A.pd + p;
+        F[0] += qd[PD_FX * np];
+        F[1] += qd[PD_FY * np];
+        F[2] += qd[PD_FZ * np];
+        double* fj = A.f + 3 * size_t(A.pj[p]);
+        for (int d = 0; d < 3; ++d) atomicAdd(fj + d, -F[d]);
+      }
+      for (int d = 0; d < 3; ++d) fs[3 * gt + d] = F[d];
+    }
+    __syncthreads();
+    if (tid < 3 * na) {  // f_i, neighbours in order
+      const int a = tid / 3, d = tid - 3 * a;
+      const int b0 = max(s_off[a] - s0, 0), b1 = min(s_off[a + 1] - s0, nthr);
+      double t = s_sum[a][d];
+      for (int k = b0; k < b1; ++k) t += fs[3 * k + d];
+      s_sum[a][d] = t;
+    }
+    __syncthreads();
+  }
+  if (tid < 3 * na) {
+    const int a = tid / 3, d = tid - 3 * a;
+    atomicAdd(A.f + 3 * size_t(A.first + a0 + a) + d, s_sum[a][d]);
+  }
+}
+
+// ------------------------------------------------------------------ energy
+// beta_0 + (2/3) sum_j sum_half w Re(conj(U) Y) (B is cubic in U, so
+// <U, dB/dU> = 3B) plus 1.25e5 / r^12 per inside pair; one warp per atom.
+static __global__ void __launch_bounds__(128) k_snap_energy(SnapArgs A) {
+  const SnapDev& S = A.S;
+  const int lane = threadIdx.x & 31, al = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (al >= A.n) return;
+  const int ta = A.ta, ny = 4 * S.ne;
+  const double* Y = static_cast<const double*>(A.Y) + size_t(al / ta) * ny * ta + al % ta;
+  const Cplx<double>* U = static_cast<const Cplx<double>*>(A.U) + size_t(al) * S.nh;
+  double acc = 0.0;
+  for (int e = lane; e < S.ne; e += 32) {
+    // U+ + (-1)^T U- = 2N (p u - i r u), U+ - (-1)^T U- = 2N (r v + i p v)
+    const Entry& E = S.ent[e];
+    const int2 h = S.half[e];
+    const double* y = Y + size_t(4) * e * ta;
+    const Cplx<double> u = U[h.x];
+    if (h.y >= 0) {
+      const double sg = E.T & 1 ? -1.0 : 1.0;
+      const Cplx<double> m = U[h.y];
+      acc += 0.5 * E.invN *
+             (fma(y[0], fma(sg, m.r, u.r), y[ta] * fma(sg, m.i, u.i)) +
+              fma(y[2 * ta], fma(-sg, m.r, u.r), y[3 * ta] * fma(-sg, m.i, u.i)));
+    } else if (E.T == 0) {
+      acc += E.invN * fma(y[0], u.r, y[ta] * u.i);
+    } else {
+      acc += E.invN * fma(y[0], u.r, y[3 * ta] * u.i);
+    }
+  }
+  acc *= 0.5;
+  const size_t np = size_t(A.n) * A.cap;
+  const double* ep = A.pd + PD_EP * np + size_t(al) * A.cap;
+  const int n = A.cnt[al];
+  for (int k = lane; k < n; k += 32) acc += 1.5 * ep[k];
+  acc = warp_sum(acc);
+  if (lane == 0) {
+    const int i = A.first + al;
+    A.eatom[i] = S.beta0[S.map[A.type[i]]] + (2.0 / 3.0) * acc;
+  }
+}
+
+// ----------------------------------------------------------------- adjoint
+// For every full triple t = (j1, j2, j), with Z_t as k_snap_y kept it,
+//   P_t = 2 sum_half w Re(conj(U_j) Z_t)        (= B_k when t is idxj triple k)
+//   Q_t = 2 sum_half w Re(conj(D_j) Z_t),  D = sum_nb dU'_nb . (g_i - g_j)
+// so that d/dbeta_k [sum_atoms g . F] over this atom's pairs is
+// Q_t1 + (j+1)/(j1+1) Q_t2 + (j+1)/(j2+1) Q_t3 (compute_dbidrj's three terms,
+// sna_impl.hpp:330-570, contracted with the loss gradient before the sum over
+// k instead of after it).
+//
+// k_snap_dt: D as k_snap_u forms X, from each neighbour's table row and its
+// derivative along g_i - g_j.
+__device__ __forceinline__ void sd_row(const SnapDev& S, double* t, double* dt, double ar, double ai, double br,
+                                       double bi, double w, double tar, double tai, double tbr, double tbi,
+                                       double tw) {
+  const int J = S.twojmax;
+  double* prod = t + 4 * (J + 1);
+  double* dprod = dt + 4 * (J + 1);
+  double p = 1.0, r = 0.0, u = w, v = 0.0, dp = 0.0, dr = 0.0, du = tw, dv = 0.0;
+  for (int q = 0; q <= J; ++q) {
+    t[2 * q] = p;
+    t[2 * q + 1] = r;
+    dt[2 * q] = dp;
+    dt[2 * q + 1] = dr;
+    const int c = 2 * (J + 1) + 2 * q;
+    t[c] = u;
+    t[c + 1] = v;
+    dt[c] = du;
+    dt[c + 1] = dv;
+    const double dpn = fma(dp, ar, fma(-dr, ai, fma(p, tar, -r * tai)));
+    const double drn = fma(dp, ai, fma(dr, ar, fma(p, tai, r * tar)));
+    const double dun = fma(du, br, fma(-dv, bi, fma(u, tbr, -v * tbi)));
+    const double dvn = fma(du, bi, fma(dv, br, fma(u, tbi, v * tbr)));
+    const double pn = fma(p, ar, -r * ai), un = fma(u, br, -v * bi);
+    r = fma(p, ai, r * ar);
+    v = fma(u, bi, v * br);
+    p = pn;
+    u = un;
+    dp = dpn;
+    dr = drn;
+    du = dun;
+    dv = dvn;
+  }
+  const double x = fma(ar, ar, ai * ai) - fma(br, br, bi * bi);
+  const double dx = 2.0 * (fma(ar, tar, ai * tai) - fma(br, tbr, bi * tbi));
+  for (int T = 0; T <= J; ++T) {
+    const int c = 2 * (J + 1) + 2 * T;
+    const double uu = t[c], vv = t[c + 1], duu = dt[c], dvv = dt[c + 1];
+    for (int q = 0; q <= J - T - 2; ++q) {
+      const double2* ab = reinterpret_cast<const double2*>(S.AB) + S.e0[T * (J + 1) + q];
+      const int km = (J - T - q) / 2;
+      double pm = 1.0, pk = x - __ldg(ab).x, dm = 0.0, dk = dx;
+      for (int k = 1; k <= km; ++k) {
+        if (k > 1) {
+          const double2 c = __ldg(ab + k - 1);
+          const double tt = x - c.x;
+          const double pn = fma(tt, pk, -c.y * pm), dn = fma(tt, dk, fma(dx, pk, -c.y * dm));
+          pm = pk;
+          pk = pn;
+          dm = dk;
+          dk = dn;
+        }
+        *prod++ = uu * pk;
+        *dprod++ = fma(duu, pk, uu * dk);
+        if (T > 0) {
+          *prod++ = vv * pk;
+          *dprod++ = fma(dvv, pk, vv * dk);
+        }
       }
     }
   }
+}
+
+static __global__ void __launch_bounds__(32) k_snap_dt(SnapArgs A) {
+  const SnapDev& S = A.S;
+  extern __shared__ __align__(16) double sd_smem[];
+  double* xs = sd_smem;
+  double* tab = sd_smem + ((S.nx + 1) & ~1);
+  const int al = blockIdx.x, lane = threadIdx.x, i = A.first + al;
+  const int cols = S.cols, n = A.cnt[al];
+  const size_t np = size_t(A.n) * A.cap;
+  const double gix = A.g[3 * i], giy = A.g[3 * i + 1], giz = A.g[3 * i + 2];
+  for (int n0 = 0; n0 < max(n, 1); n0 += 32) {
+    const int m = min(32, n - n0);
+    if (lane < m) {
+      const size_t p = size_t(al) * A.cap + n0 + lane;
+      const double* q = A.pd + p;
+      const double* w = static_cast<const double*>(A.pr) + p;
+      // the pair's reaction force lands on j's owner (newton) or nowhere
+      const int j = A.pj[p];
+      const int jo = j < A.n_local ? j : (A.newton ? A.ghost_owner[j - A.n_local] : -1);
+      const double dx = gix - (jo >= 0 ? A.g[3 * jo] : 0.0), dy = giy - (jo >= 0 ? A.g[3 * jo + 1] : 0.0),
+                   dz = giz - (jo >= 0 ? A.g[3 * jo + 2] : 0.0);
+      auto along = [&](int f) { return fma(w[f * np], dx, fma(w[(f + 1) * np], dy, w[(f + 2) * np] * dz)); };
+      double* row = tab + 2 * lane * cols;
+      sd_row(S, row, row + cols, w[PR_AR * np], w[PR_AI * np], w[PR_BR * np], w[PR_BI * np], q[PD_SF * np],
+             along(PF_DAR), along(PF_DAI), along(PF_DBR), along(PF_DBI), w[PR_DSF * np] * along(PR_UX));
+    }
+    __syncwarp();
+    for (int r = lane; r < S.nx; r += 32) {
+      const int2 s = __ldg(S.xsum + r);
+      double acc = n0 > 0 ? xs[r] : 0.0;
+      for (int k = 0; k < m; ++k) {
+        const double* t = tab + 2 * k * cols;
+        const double* d = t + cols;
+        acc = fma(d[s.x], t[s.y], fma(t[s.x], d[s.y], acc));
+      }
+      xs[r] = acc;
+    }
+    __syncwarp();
+  }
+  for (int e = lane; e < S.ne; e += 32) su_store<double>(S, e, xs, 0.0, A.D + size_t(al) * S.nh);
+}
+
+// half-grid elements of U and D, weighted (2, or 1 for the self-inverse ones,
+// which are listed with an equal inversion), atom by atom -> lanes = atoms
+static __global__ void __launch_bounds__(256) k_snap_half(SnapArgs A) {
+  const SnapDev& S = A.S;
+  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int at = int(k & 31), tiles = (A.n + 31) / 32;
+  const long long th = k >> 5;
+  if (th >= (long long)tiles * S.nh) return;
+  const int tile = int(th / S.nh), h = int(th - (long long)tile * S.nh), al = tile * 32 + at;
+  const int4 f = S.hfull[h];
+  const double w = f.x == f.y ? 1.0 : 2.0;
+  for (int d = 0; d < 2; ++d) {
+    const Cplx<double>* src = d ? A.D : static_cast<const Cplx<double>*>(A.U);
+    const Cplx<double> u = al < A.n ? src[size_t(al) * S.nh + h] : Cplx<double>{0.0, 0.0};
+    A.H[((size_t(tile) * 2 + d) * S.nh + h) * 32 + at] = Cplx<double>{w * u.r, w * u.i};
+  }
+}
+
+// lanes = atoms, a warp per triple
+static __global__ void __launch_bounds__(256) k_snap_pq(SnapArgs A) {
+  const SnapDev& S = A.S;
+  const int lane = threadIdx.x & 31, tile = blockIdx.x, t = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (t >= S.nfull) return;
+  const int al = tile * 32 + lane;
+  const Cplx<double>* Z = reinterpret_cast<const Cplx<double>*>(A.zkeep) + size_t(tile) * S.nz * 32 + lane;
+  const Cplx<double>* U = A.H + size_t(tile) * 2 * S.nh * 32 + lane;
+  const Cplx<double>* D = U + size_t(S.nh) * 32;
+  double p = 0.0, q = 0.0;
+  for (int k = S.zt0[t]; k < S.zt0[t + 1]; ++k) {
+    const int2 c = __ldg(S.zt + k);
+    const Cplx<double> z = Z[size_t(c.x) * 32], u = U[size_t(c.y) * 32], d = D[size_t(c.y) * 32];
+    p = fma(u.r, z.r, fma(u.i, z.i, p));
+    q = fma(d.r, z.r, fma(d.i, z.i, q));
+  }
+  if (al < A.n) {
+    const size_t i = size_t(A.first + al), n = size_t(A.n_local);
+    A.adj[size_t(t) * n + i] = p;
+    A.adj[size_t(S.nfull + t) * n + i] = q;
+    if (t == 0) A.adj[size_t(2 * S.nfull) * n + i] = 1.0;  // atom count column (beta_0)
+  }
+}
+
+// ---------------------------------------------------------------- launches
+inline size_t snap_y_smem(const SnapDev& S, int ta, size_t real) { return 2 * real * size_t(S.nuf) * (ta + 1); }
+
+template <typename R, int NM, bool KEEP, bool FULL>
+void launch_y(const SnapArgs& A, cudaStream_t s) {
+  const size_t smem = snap_y_smem(A.S, A.ta, sizeof(R));
+  const int tiles = (A.n + A.ta - 1) / A.ta, threads = sizeof(R) == 8 ? 512 : 256;
+  allow_dyn_smem(k_snap_y<R, NM, KEEP, FULL>);
+  k_snap_y<R, NM, KEEP, FULL><<<tiles * A.nsplit, threads, smem, s>>>(A);
+  EMD_CHECK_LAUNCH();
+}
+template <typename R, int NM>
+void launch_y(const SnapArgs& A, cudaStream_t s) {
+  if constexpr (sizeof(R) == 8)
+    if (A.zkeep) {
+      if (A.ta == 32) launch_y<R, NM, true, true>(A, s);
+      else launch_y<R, NM, true, false>(A, s);
+      return;
+    }
+  if (A.ta == 32) launch_y<R, NM, false, true>(A, s);
+  else launch_y<R, NM, false, false>(A, s);
+}
+
+template <typename R>
+void launch_u(const SnapArgs& A, cudaStream_t s) {
+  const size_t smem = sizeof(double) * (size_t((A.S.nx + 1) & ~1) + 32 * size_t(A.S.cols));
+  allow_dyn_smem(k_snap_u<R>);
+  k_snap_u<R><<<A.n, 32, smem, s>>>(A);
+  EMD_CHECK_LAUNCH();
+}
+
+template <typename R, int NQ>
+void launch_force(const SnapArgs& A, int threads, cudaStream_t s) {
+  const size_t smem = ((size_t(A.apc) * 4 * A.S.ne * sizeof(R) + 15) & ~size_t(15)) + size_t(threads) * 24;
+  allow_dyn_smem(k_snap_force<R, NQ>);
+  k_snap_force<R, NQ><<<(A.n + A.apc - 1) / A.apc, threads, smem, s>>>(A);
+  EMD_CHECK_LAUNCH();
+}
+
+// the kernels of one chunk, up to Y
+template <typename R>
+void launch_pairs(const SnapArgs& A, cudaStream_t s) {
+  const int warps = (A.n + A.rows - 1) / A.rows;
+  k_snap_pairs<R><<<(warps + 1) / 2, 64, 0, s>>>(A);
+  EMD_CHECK_LAUNCH();
 }
 
 }  // namespace snapk

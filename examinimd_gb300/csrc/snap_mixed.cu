@@ -1,16 +1,25 @@
-// The mixed-form SNAP force kernel, k_snap<float, 0> (snap_kernel.cuh).
-// It is compiled apart from snap.cu so that its FP32 contraction and its FP64
-// U recursion may use fused multiply-adds; the FP64 drop-in kernels in
-// snap.cu keep -fmad=false.
+// The mixed form's SNAP kernels (snap_kernel.cuh): pair scalars and U_tot
+// in FP64, Z, Y and the pair forces in FP32.  Compiled apart from snap.cu so
+// that the pair scalars may use fused multiply-adds; the FP64 drop-in keeps
+// -fmad=false.
 #include "snap_kernel.cuh"
 
 namespace emd {
 
-void snap_mixed_launch(const snapk::SnapArgs& A, size_t smem, cudaStream_t s) {
-  auto k = snapk::k_snap<float, 0>;
-  EMD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  k<<<A.n_local, snapk::SNAP_THREADS, smem, s>>>(A);
-  EMD_CHECK_LAUNCH();
+using namespace snapk;
+
+void snap_mixed_pairs(const SnapArgs& A, cudaStream_t s) { launch_pairs<float>(A, s); }
+
+void snap_mixed_u(const SnapArgs& A, cudaStream_t s) { launch_u<float>(A, s); }
+
+void snap_mixed_y(const SnapArgs& A, cudaStream_t s) {
+  if (A.S.twojmax <= 9) launch_y<float, 5>(A, s);
+  else launch_y<float, 8>(A, s);
+}
+
+void snap_mixed_force(const SnapArgs& A, int threads, cudaStream_t s) {
+  if (A.S.twojmax <= 8) launch_force<float, 9>(A, threads, s);
+  else launch_force<float, 15>(A, threads, s);
 }
 
 }  // namespace emd

@@ -1,15 +1,17 @@
 """Floating-point operation count of one SNAP force evaluation, per atom.
 
-The count enumerates the loops of the GB300 kernel (`csrc/snap_kernel.cuh`)
-for a given twojmax and number of inside neighbours, phase by phase, with one
-operation per add, subtract or multiply (a fused multiply-add counts two) and
-one per square root, division or transcendental call.  It counts the
-formulation the kernel runs (the adjoint form with reverse-mode pair forces),
-which needs fewer operations than the reference's
-(compute_ui / compute_zi / compute_duidrj / compute_dbidrj, sna_impl.hpp).
+One operation per add, subtract or multiply (a fused multiply-add counts two)
+and one per square root, division or transcendental call, for a given twojmax
+and number of inside neighbours.
 
-`snap_flops(twojmax, ninside)` returns a dict of per-atom counts by phase and
-by arithmetic type for each precision form:
+`kernel_flops` counts the formulation the GB300 kernels run
+(`csrc/snap_kernel.cuh`): separated Wigner elements, shared products.
+
+`snap_flops` counts the layered formulation (U by the layer recursion, one Z at
+a time, reverse-mode pair forces through the layers), which already needs fewer
+operations than the reference's (compute_ui / compute_zi / compute_duidrj /
+compute_dbidrj, sna_impl.hpp).  It returns a dict of per-atom counts by phase
+and by arithmetic type for each precision form:
 
 - B, the U_tot recursion and its sums, is FP64 in both forms;
 - the per-neighbour scalars are FP64 in both forms;
@@ -83,4 +85,64 @@ def snap_flops(twojmax: int, ninside: float) -> dict:
     }
 
 
-__all__ = ["snap_flops", "z_loop_counts"]
+def _entries(J: int):
+    """(T, q, highest k) of the separated elements conj(a)^q b^T P_k(x)."""
+    for T in range(J + 1):
+        for q in range(J - T + 1):
+            yield T, q, (J - T - q) // 2
+
+
+def product_counts(J: int) -> tuple[int, int, int]:
+    """(products, weighted products, Z values) of the shared-product contraction:
+    each U_j1 U_j2 product of one (m, m') once, weighted for every j; for j1 = j2
+    the two orders of a pair are one product."""
+    products = weighted = zs = 0
+    for T, q, _ in _entries(J):
+        for sign in ((1, -1) if T and q else (1,)):
+            for j1 in range(J + 1):
+                for j2 in range(j1 + 1):
+                    hi = min(J - ((J + j1 + j2) & 1), j1 + j2)
+                    if (j1 + j2 - q - T) & 1 or hi < max(j1 - j2, q + T):
+                        continue
+                    nj = (hi - max(j1 - j2, q + T)) // 2 + 1
+                    M, Mp = (j1 + j2 - q - sign * T) // 2, (j1 + j2 - q + sign * T) // 2
+                    na, nb = min(j1, M) - max(0, M - j2) + 1, min(j1, Mp) - max(0, Mp - j2) + 1
+                    n = na * nb
+                    if j1 == j2:  # pairs and the self-paired one, where there is one
+                        n = (n + (1 if M % 2 == 0 and Mp % 2 == 0 else 0)) // 2
+                    products += n
+                    weighted += n * nj
+                    zs += nj
+    return products, weighted, zs
+
+
+def kernel_flops(twojmax: int, ninside: float) -> dict:
+    """Per-atom operation counts of the kernels' own formulation."""
+    J, n = twojmax, float(ninside)
+    sums = sum((j + 1) ** 2 for j in range(J + 1))
+    # U, per neighbour: powers of a and b (6 each), x, polynomials (4 from k = 2
+    # on), their products with u and v, one multiply-add per real sum
+    poly = sum(1 + 4 * (k - 1) for _, _, k in _entries(J) if k > 0)
+    prods = sum((2 if T else 1) * k for T, _, k in _entries(J))
+    u_stage = n * (12.0 * J + 7 + poly + prods + 2.0 * sums) + 3.0 * sums
+    products, weighted, zs = product_counts(J)
+    y_stage = 6.0 * products + 4.0 * weighted + 4.0 * zs
+    # pair forces, per neighbour: powers, P and P' (9 from k = 2 on), their sums
+    # with E and O (values and derivatives), the sums over q and over T
+    force = 12.0 * J + 7 + 60.0
+    for T, q, k in _entries(J):
+        w = 2 if T else 1
+        force += (1 if k else 0) + 9 * max(0, k - 1) + w * (4 * min(k, 1) + 8 * max(0, k - 1)) + w * (24 if q else 4)
+    force += 22.0 * J
+    scalars, tail = n * 80.0, n * 18.0
+    return {
+        "twojmax": J,
+        "ninside": n,
+        "phases": {"scalars": scalars, "U": u_stage, "Y": y_stage, "force": n * force + tail},
+        "total": scalars + u_stage + y_stage + n * force + tail,
+        "fp64": {"mixed": scalars + u_stage + tail, "fp64": scalars + u_stage + y_stage + n * force + tail},
+        "fp32": {"mixed": y_stage + n * force, "fp64": 0.0},
+    }
+
+
+__all__ = ["snap_flops", "z_loop_counts", "kernel_flops", "product_counts"]
