@@ -27,10 +27,10 @@ struct SnapHost {
   DevBuf<Entry> ent;
   DevBuf<ZTask> task;
   DevBuf<ZRec> rec;
-  DevBuf<int> e0, map, zt0, tmask;
-  DevBuf<int2> xsum, half, zt, prod;
+  DevBuf<int> e0, map, zt0, tmask, eord;
+  DevBuf<int2> xsum, msum, half, zt, prod;
   DevBuf<int4> hfull;
-  DevBuf<double> zc, cY, AB, beta0, wjelem, pr;
+  DevBuf<double> zc, mono, cY, AB, beta0, wjelem, pr;
   DevBuf<float> cY_f, AB_f;
   DevBuf<float2> zc_f;
   // per-chunk work arrays
@@ -98,12 +98,12 @@ double jacobi_B(int al, int be, int k) {
 // The tables of one twojmax (see the structures in snap_kernel.cuh)
 struct SnapTables {
   std::vector<Entry> ent;
-  std::vector<int> e0, zt0, tmask;
-  std::vector<int2> xsum, half, zt, prod;
+  std::vector<int> e0, zt0, tmask, eord;
+  std::vector<int2> xsum, msum, half, zt, prod;
   std::vector<int4> hfull;
   std::vector<ZTask> task;
   std::vector<ZRec> rec;
-  std::vector<double> zc, AB;
+  std::vector<double> zc, AB, mono;
   std::vector<float2> zc_f;
   int nz = 0, nh = 0;
 
@@ -113,10 +113,11 @@ struct SnapTables {
     // entries, real sums and their table columns (k_snap_u: powers of a, of b,
     // then the products in (T, q, k) order)
     e0.assign(size_t(L) * L, -1);
-    int col = 4 * L;
-    for (int T = 0; T <= J; ++T)
+    int col = 4 * L, mcol = 4 * L;
+    for (int T = 0; T <= J; ++T) {
       for (int q = 0; q <= J - T; ++q) {
         e0[size_t(T) * L + q] = int(ent.size());
+        std::vector<double> pk{1.0}, pm;  // P_k and P_{k-1} in powers of x
         for (int k = 0; q + T + 2 * k <= J; ++k) {
           const int j = q + T + 2 * k, ma = (j - q - T) / 2, mb = (j - q + T) / 2;
           Entry E{};
@@ -137,10 +138,22 @@ struct SnapTables {
           E.xo = int(xsum.size());
           const int cu = k == 0 ? 2 * L + 2 * T : col, cv = cu + 1, cp = 2 * q, cr = 2 * q + 1;
           if (k > 0) col += T > 0 ? 2 : 1;
+          const int mu = k == 0 ? cu : mcol + (k - 1) * (T > 0 ? 2 : 1), mv = mu + 1;
           xsum.push_back(int2{cp, cu});
-          if (q > 0) xsum.push_back(int2{cr, cu});
-          if (T > 0) xsum.push_back(int2{cp, cv});
-          if (q > 0 && T > 0) xsum.push_back(int2{cr, cv});
+          msum.push_back(int2{cp, mu});
+          if (q > 0) xsum.push_back(int2{cr, cu}), msum.push_back(int2{cr, mu});
+          if (T > 0) xsum.push_back(int2{cp, cv}), msum.push_back(int2{cp, mv});
+          if (q > 0 && T > 0) xsum.push_back(int2{cr, cv}), msum.push_back(int2{cr, mv});
+          E.mo = int(mono.size());
+          for (double c : pk) mono.push_back(E.N * c);
+          std::vector<double> pn(pk.size() + 1, 0.0);
+          for (size_t l = 0; l < pk.size(); ++l) {
+            pn[l + 1] += pk[l];
+            pn[l] -= E.A * pk[l];
+          }
+          for (size_t l = 0; l < pm.size(); ++l) pn[l] -= E.B * pm[l];
+          pm = pk;
+          pk = pn;
           half.push_back(int2{nh, q > 0 && T > 0 ? nh + 1 : -1});
           nh += q > 0 && T > 0 ? 2 : 1;
           const int sign = T & 1 ? -1 : 1;  // (-1)^(ma + mb)
@@ -149,6 +162,12 @@ struct SnapTables {
           ent.push_back(E);
         }
       }
+      mcol += (T > 0 ? 2 : 1) * ((J - T) / 2);
+    }
+    for (int e = 0; e < int(ent.size()); ++e) eord.push_back(e);
+    std::stable_sort(eord.begin(), eord.end(), [&](int x, int y) {
+      return ent[size_t(x)].j - ent[size_t(x)].q - ent[size_t(x)].T > ent[size_t(y)].j - ent[size_t(y)].q - ent[size_t(y)].T;
+    });
     // Clebsch-Gordan coefficients of every (j1, j2): for each (m1, m2) the
     // allowed j from the highest down
     std::vector<int> cgo(size_t(L) * L), njt(size_t(L) * L), ttop(size_t(L) * L);
@@ -299,9 +318,9 @@ void free_snap(Ctx& c) {
   h->H.release();
   h->hfull.release();
   h->zc_f.release();
-  for (auto* b : {&h->e0, &h->map, &h->zt0, &h->tmask, &h->pj, &h->cnt}) b->release();
-  for (auto* b : {&h->xsum, &h->half, &h->zt, &h->prod}) b->release();
-  for (auto* b : {&h->zc, &h->cY, &h->AB, &h->beta0, &h->wjelem, &h->pr, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk,
+  for (auto* b : {&h->e0, &h->map, &h->zt0, &h->tmask, &h->eord, &h->pj, &h->cnt}) b->release();
+  for (auto* b : {&h->xsum, &h->msum, &h->half, &h->zt, &h->prod}) b->release();
+  for (auto* b : {&h->zc, &h->mono, &h->cY, &h->AB, &h->beta0, &h->wjelem, &h->pr, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk,
                   &h->eatom, &h->adj, &h->adj_sum, &h->adj_g, &h->keep_u, &h->keep_z})
     b->release();
   for (auto* b : {&h->cY_f, &h->AB_f}) b->release();
@@ -624,6 +643,7 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   S.ne = int(tab.ent.size());
   S.nx = int(tab.xsum.size());
   S.cols = su_cols(twojmax);
+  S.mcols = su_mcols(twojmax);
   S.nuf = (twojmax + 1) * (twojmax + 2) * (2 * twojmax + 3) / 6;
   S.ntask = int(tab.task.size());
   S.nz = tab.nz;
@@ -663,6 +683,9 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   upload(c, h->rec, tab.rec);
   upload(c, h->e0, tab.e0);
   upload(c, h->xsum, tab.xsum);
+  upload(c, h->msum, tab.msum);
+  upload(c, h->mono, tab.mono);
+  upload(c, h->eord, tab.eord);
   upload(c, h->half, tab.half);
   upload(c, h->zt0, tab.zt0);
   upload(c, h->zt, tab.zt);
@@ -685,6 +708,9 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   S.rec = h->rec.p;
   S.e0 = h->e0.p;
   S.xsum = h->xsum.p;
+  S.msum = h->msum.p;
+  S.mono = h->mono.p;
+  S.eord = h->eord.p;
   S.half = h->half.p;
   S.zt0 = h->zt0.p;
   S.zt = h->zt.p;

@@ -56,6 +56,7 @@ struct Entry {
   double N, invN;  // the elements' norm and its inverse
   double A, B;     // P_{k+1} = (x - A) P_k - B P_{k-1}
   int xo;          // first of its real sums: p u, [q>0] r u, [T>0] p v, [q>0, T>0] r v
+  int mo;          // its coefficients of x^0 .. x^k, times N (SnapDev::mono)
   int T, q, j;
   int ep, em, mp, mm;  // full-grid elements (ma, mb) and (mb, ma), and their inversions
 };
@@ -73,7 +74,7 @@ struct ZTask {
 
 struct SnapDev {
   int twojmax, ne, nx, nuf;    // entries, real sums, elements of the full grid
-  int cols;                    // columns of a neighbour's table (su_cols)
+  int cols, mcols;             // columns of a neighbour's table (su_cols), of the mixed form's
   int ntask, nfull, nz;        // Z tasks, (j1 >= j2, j) triples, kept Z values per atom
   int ncoeff, ncoeffall, nelem, ntypes;
   double rfac0, rmin0, cutsq, wself;
@@ -81,6 +82,9 @@ struct SnapDev {
   const Entry* ent;
   const int* e0;       // (J + 1) x (J + 1): first entry of (T, q)
   const int2* xsum;    // nx: the two factors of a sum in a neighbour's table (k_snap_u)
+  const int2* msum;    // the same in the mixed form's table
+  const double* mono;  // N P_k in powers of x
+  const int* eord;     // entries, highest k first
   const ZTask* task;
   const ZRec* rec;
   const int2* prod;    // the two U elements of a product
@@ -319,13 +323,21 @@ __global__ void __launch_bounds__(64) k_snap_pairs(SnapArgs A) {
 
 // ---------------------------------------------------------------------- U
 // One warp per atom, 32 neighbours at a time.  Lanes = neighbours: the powers
-// p_q + i r_q = a^q and u_T + i v_T = w b^T, the polynomials, and u P_k, v P_k
-// go to the neighbour's row of a shared table.  Lanes = sums: each of the nx
-// real sums is p or r times u P or v P over the neighbours, one FP64
-// multiply-add per neighbour.  Then the half-grid elements, once per atom, in
-// the contraction's type.  Bound by the FP64 pipe: about 240 instructions for
-// 32 neighbours and nx / 32 for each neighbour (480 per atom at twojmax 8 and
-// 26 neighbours, where the layer recursion and its sums took about 1,700).
+// p_q + i r_q = a^q and u_T + i v_T = w b^T and their products with the
+// polynomials go to the neighbour's row of a shared table.  Lanes = sums: each
+// of the nx real sums is p or r times one of those products over the
+// neighbours, one FP64 multiply-add per neighbour.  Then the half-grid
+// elements, once per atom, in the contraction's type.  Bound by the FP64 pipe.
+//
+// The FP64 form multiplies u and v by P_k(x), for every (T, q): about 240
+// instructions for 32 neighbours, nx / 32 for each neighbour, 530 per atom at
+// twojmax 8 and 26 neighbours.  The mixed form, which rounds U_tot to FP32
+// anyway, sums u x^k and v x^k, the same for every q, and combines the sums
+// into the polynomials' once per atom: the powers' rounding is amplified by the
+// polynomial's coefficients (16 at twojmax 8, 221 at 14: 5e-14), far inside
+// FP32's.
+// The table is half as wide, so that eleven warps share an SM instead of six.
+// Per 128,000 atoms: 4.98 ms with the polynomials in the row, 2.80 with powers.
 inline int su_cols(int J) {  // p, r; u, v; u P_k, v P_k (k >= 1)
   int c = 2 * (J + 1) + 2 * (J + 1);
   for (int T = 0; T <= J; ++T)
@@ -333,7 +345,14 @@ inline int su_cols(int J) {  // p, r; u, v; u P_k, v P_k (k >= 1)
   return c | 1;  // odd: rows start in different banks
 }
 
-// the neighbour's table row: powers, polynomials and products
+inline int su_mcols(int J) {  // p, r; u, v; u x^k, v x^k (1 <= k <= (J - T) / 2)
+  int c = 4 * (J + 1);
+  for (int T = 0; T <= J; ++T) c += (T ? 2 : 1) * ((J - T) / 2);
+  return c | 1;
+}
+
+// the neighbour's table row: powers, polynomials (MONO: powers of x) and products
+template <bool MONO>
 __device__ __forceinline__ void su_row(const SnapDev& S, double* t, double ar, double ai, double br, double bi,
                                        double w) {
   const int J = S.twojmax;
@@ -344,19 +363,39 @@ __device__ __forceinline__ void su_row(const SnapDev& S, double* t, double ar, d
   uT[0] = w;
   uT[1] = 0.0;
   double p = ar, r = ai, u = w * br, v = w * bi;
-  for (int q = 1; q <= J; ++q) {
+#pragma unroll 1
+  for (int q = 1; q < J; ++q) {
     t[2 * q] = p;
     t[2 * q + 1] = r;
     uT[2 * q] = u;
     uT[2 * q + 1] = v;
-    if (q == J) break;
     const double pn = fma(p, ar, -r * ai), un = fma(u, br, -v * bi);
     r = fma(p, ai, r * ar);
     v = fma(u, bi, v * br);
     p = pn;
     u = un;
   }
+  if (J > 0) {
+    t[2 * J] = p;
+    t[2 * J + 1] = r;
+    uT[2 * J] = u;
+    uT[2 * J + 1] = v;
+  }
   const double x = fma(ar, ar, ai * ai) - fma(br, br, bi * bi);
+  if constexpr (MONO) {
+    for (int T = 0; T <= J; ++T) {
+      double uk = uT[2 * T], vk = uT[2 * T + 1];
+      for (int k = 1; k <= (J - T) / 2; ++k) {
+        uk *= x;
+        *prod++ = uk;
+        if (T > 0) {
+          vk *= x;
+          *prod++ = vk;
+        }
+      }
+    }
+    return;
+  }
   for (int T = 0; T <= J; ++T) {
     const double uu = uT[2 * T], vv = uT[2 * T + 1];
     for (int q = 0; q <= J - T - 2; ++q) {
@@ -377,40 +416,60 @@ __device__ __forceinline__ void su_row(const SnapDev& S, double* t, double ar, d
   }
 }
 
-// the half-grid elements of entry e from its real sums: conj(a)^q b^T = (p u +
-// r v) + i (p v - r u); for -T: (-1)^T ((p u - r v) - i (p v + r u)); N scales,
-// the atom's own term is 1 on the diagonal (T = 0)
-template <typename R>
+// the half-grid elements of entry e from its real sums (MONO: sums over the
+// powers of x, one group per k): conj(a)^q b^T = (p u + r v) + i (p v - r u);
+// for -T: (-1)^T ((p u - r v) - i (p v + r u)); N scales, the atom's own term
+// is 1 on the diagonal (T = 0)
+template <typename R, bool MONO>
 __device__ __forceinline__ void su_store(const SnapDev& S, int e, const double* x, double self, Cplx<R>* U) {
   const Entry& E = S.ent[e];
-  x += E.xo;
-  double pu = *x++, ru = 0.0, pv = 0.0, rv = 0.0;
-  if (E.q > 0) ru = *x++;
-  if (E.T > 0) pv = *x++;
-  if (E.q > 0 && E.T > 0) rv = *x;
+  const bool hr = E.q > 0, hv = E.T > 0;
+  double pu, ru = 0.0, pv = 0.0, rv = 0.0;
+  if constexpr (MONO) {
+    const double* m = S.mono + E.mo;
+    const int k = (E.j - E.q - E.T) / 2, g = (hr ? 2 : 1) * (hv ? 2 : 1);
+    x += E.xo - k * g;  // the sums of x^0
+    pu = 0.0;
+    for (int l = 0; l <= k; ++l) {
+      const double c = __ldg(m + l);
+      const double* y = x + l * g;
+      pu = fma(c, *y++, pu);
+      if (hr) ru = fma(c, *y++, ru);
+      if (hv) pv = fma(c, *y++, pv);
+      if (hr && hv) rv = fma(c, *y, rv);
+    }
+  } else {
+    x += E.xo;
+    pu = E.N * *x++;
+    if (hr) ru = E.N * *x++;
+    if (hv) pv = E.N * *x++;
+    if (hr && hv) rv = E.N * *x;
+  }
   const int2 h = S.half[e];
-  U[h.x] = Cplx<R>{R(fma(E.N, pu + rv, E.T == 0 ? self : 0.0)), R(E.N * (pv - ru))};
+  U[h.x] = Cplx<R>{R((pu + rv) + (hv ? 0.0 : self)), R(pv - ru)};
   if (h.y >= 0) {
-    const double sg = E.T & 1 ? -E.N : E.N;
+    const double sg = E.T & 1 ? -1.0 : 1.0;
     U[h.y] = Cplx<R>{R(sg * (pu - rv)), R(-sg * (pv + ru))};
   }
 }
 
 template <typename R>
 __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
+  constexpr bool kMono = sizeof(R) == sizeof(float);
   const SnapDev& S = A.S;
   extern __shared__ __align__(16) double su_smem[];
   double* xs = su_smem;                       // nx sums
   double* tab = su_smem + ((S.nx + 1) & ~1);  // 32 rows
   const int al = blockIdx.x, lane = threadIdx.x;
-  const int cols = S.cols, n = A.cnt[al];
+  const int cols = kMono ? S.mcols : S.cols, n = A.cnt[al];
+  const int2* __restrict__ xsum = kMono ? S.msum : S.xsum;
   const size_t np = size_t(A.n) * A.cap;
   const double* pd = A.pd + size_t(al) * A.cap;
   for (int n0 = 0; n0 < max(n, 1); n0 += 32) {
     const int m = min(32, n - n0);
     if (lane < m) {
       const double* q = pd + n0 + lane;
-      su_row(S, tab + lane * cols, q[PD_AR * np], q[PD_AI * np], q[PD_BR * np], q[PD_BI * np], q[PD_SF * np]);
+      su_row<kMono>(S, tab + lane * cols, q[PD_AR * np], q[PD_AI * np], q[PD_BR * np], q[PD_BI * np], q[PD_SF * np]);
     }
     __syncwarp();
     for (int r0 = 0; r0 < S.nx; r0 += 96) {  // three sums per lane at once
@@ -419,7 +478,7 @@ __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
 #pragma unroll
       for (int h = 0; h < 3; ++h) {
         const int r = r0 + 32 * h + lane;
-        s[h] = r < S.nx ? __ldg(S.xsum + r) : int2{0, 0};
+        s[h] = r < S.nx ? __ldg(xsum + r) : int2{0, 0};
         acc[h] = r < S.nx && n0 > 0 ? xs[r] : 0.0;
       }
       if (r0 + 64 < S.nx) {
@@ -448,7 +507,7 @@ __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
     __syncwarp();
   }
   Cplx<R>* U = static_cast<Cplx<R>*>(A.U) + size_t(al) * S.nh;
-  for (int e = lane; e < S.ne; e += 32) su_store<R>(S, e, xs, S.wself, U);
+  for (int e = lane; e < S.ne; e += 32) su_store<R, kMono>(S, __ldg(S.eord + e), xs, S.wself, U);
 }
 
 // ------------------------------------------------------------------- Z, Y
@@ -1031,7 +1090,7 @@ static __global__ void __launch_bounds__(32) k_snap_dt(SnapArgs A) {
     }
     __syncwarp();
   }
-  for (int e = lane; e < S.ne; e += 32) su_store<double>(S, e, xs, 0.0, A.D + size_t(al) * S.nh);
+  for (int e = lane; e < S.ne; e += 32) su_store<double, false>(S, e, xs, 0.0, A.D + size_t(al) * S.nh);
 }
 
 // half-grid elements of U and D, weighted (2, or 1 for the self-inverse ones,
@@ -1101,7 +1160,7 @@ void launch_y(const SnapArgs& A, cudaStream_t s) {
 
 template <typename R>
 void launch_u(const SnapArgs& A, cudaStream_t s) {
-  const size_t smem = sizeof(double) * (size_t((A.S.nx + 1) & ~1) + 32 * size_t(A.S.cols));
+  const size_t smem = sizeof(double) * (size_t((A.S.nx + 1) & ~1) + 32 * size_t(sizeof(R) == 4 ? A.S.mcols : A.S.cols));
   allow_dyn_smem(k_snap_u<R>);
   k_snap_u<R><<<A.n, 32, smem, s>>>(A);
   EMD_CHECK_LAUNCH();

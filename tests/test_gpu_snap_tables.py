@@ -83,6 +83,22 @@ def test_mixed_form_of_large_twojmax_and_full_tiles():
         assert np.sqrt(np.mean((f[1] - f[0]) ** 2)) <= 1e-5 * np.sqrt(np.mean(f[0] ** 2))
 
 
+@pytest.mark.parametrize("J", [0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10])
+def test_mixed_form_of_every_twojmax(J):
+    """RMS force error of the mixed form; 54 atoms, about 73 neighbours (three 32-lane rounds) or 26."""
+    from examinimd_gb300 import EMD_PREC_MIXED, Context
+    for a in (2.3, 3.1803):
+        st, state = _deck(J, (3, 3, 3), a, seed=J)
+        n = len(state["x"])
+        f = []
+        for prec in (0, EMD_PREC_MIXED):
+            c = Context(0)
+            mdloop.init(c, st, state, precision=prec)
+            f.append(c.get(0, n)["f"])
+            c.close()
+        assert np.sqrt(np.mean((f[1] - f[0]) ** 2)) <= 1e-5 * np.sqrt(np.mean(f[0] ** 2))
+
+
 def test_threads_with_systems_of_different_size():
     """Contexts of different size on several host threads at once: every force
     equals the one computed alone, to the scatter's order of adds."""
