@@ -3,6 +3,7 @@
 // snap_kernel.cuh; the mixed-form instantiation is compiled in snap_mixed.cu.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -20,19 +21,23 @@ namespace {
 
 using namespace snapk;
 
+struct SnapTables;
+
 struct SnapHost {
   SnapDev d;
+  const SnapTables* tab = nullptr;
   int precision = EMD_PREC_FP64;
   // tables
   DevBuf<Entry> ent;
   DevBuf<ZTask> task;
   DevBuf<ZRec> rec;
+  DevBuf<ZGrp> grp;
   DevBuf<int> e0, map, zt0, tmask, eord;
   DevBuf<int2> xsum, msum, half, zt, prod;
   DevBuf<int4> hfull;
   DevBuf<double> zc, mono, cY, AB, beta0, wjelem, pr;
-  DevBuf<float> cY_f, AB_f;
-  DevBuf<float2> zc_f;
+  DevBuf<float> AB_f;
+  DevBuf<uint4> zs;
   // per-chunk work arrays
   DevBuf<double> pd, pr_f, U, Y, zk;
   DevBuf<int> pj, cnt;
@@ -104,7 +109,13 @@ struct SnapTables {
   std::vector<ZTask> task;
   std::vector<ZRec> rec;
   std::vector<double> zc, AB, mono;
-  std::vector<float2> zc_f;
+  std::vector<ZGrp> grp;
+  std::vector<unsigned> words;  // the FP32 stream without its coefficients
+  struct Src {
+    int word, c0, t0, nj;  // of a product: its words, coefficients and highest triple
+  };
+  std::vector<Src> src;
+  std::vector<long long> cost;  // of the tasks
   int nz = 0, nh = 0;
 
   SnapTables(int J, const std::vector<int>& trip) {
@@ -234,20 +245,19 @@ struct SnapTables {
       }
     std::stable_sort(raw.begin(), raw.end(), [](const Raw& x, const Raw& y) { return x.cost > y.cost; });
     std::vector<std::vector<int2>> by_t(static_cast<size_t>(ntrip));
+    // FP32 stream: tasks start on 64 bytes, groups on their products' size
+    auto align = [&](size_t n) { words.resize((words.size() + n - 1) / n * n, 0u); };
     for (Raw& w : raw) {
+      align(16);
+      w.t.s0 = int(words.size());
       w.t.rec0 = int(rec.size());
       for (int s = 0; s < 2; ++s) {
         for (ZRec& z : w.r[s]) {
           const int rp0 = z.p0, rc0 = z.c0;
           z.p0 = int(prod.size());
           z.c0 = int(zc.size());
-          z.cf = int(zc_f.size());
           prod.insert(prod.end(), rp.begin() + rp0, rp.begin() + rp0 + z.np);
           zc.insert(zc.end(), rc.begin() + rc0, rc.begin() + rc0 + z.np * z.nj);
-          for (int k = 0; k < z.np; ++k) {
-            for (int j = 0; j < z.nj; ++j) zc_f.push_back(make_float2(float(rc[rc0 + k * z.nj + j]), float(rc[rc0 + k * z.nj + j])));
-            if (z.nj & 1) zc_f.push_back(make_float2(0.f, 0.f));
-          }
           z.z0 = nz;
           for (int j = 0; j < z.nj; ++j) {  // highest j first: entry kmax - d - j of the task
             const int2 h = half[size_t(w.t.y0 + w.t.kmax - z.d - j)];
@@ -258,8 +268,33 @@ struct SnapTables {
         }
         (s ? w.t.rec2 : w.t.rec1) = int(rec.size());
       }
+      for (int s = 0; s < 2; ++s) {
+        (s ? w.t.grp1 : w.t.grp0) = int(grp.size());
+        std::vector<const ZRec*> rs;
+        for (const ZRec& z : w.r[s]) rs.push_back(&z);
+        std::stable_sort(rs.begin(), rs.end(),
+                         [](const ZRec* x, const ZRec* y) { return x->nj != y->nj ? x->nj > y->nj : x->d < y->d; });
+        for (size_t k = 0; k < rs.size(); ++k) {
+          const ZRec& z = *rs[k];
+          const int nw = zs_words(z.nj);
+          if (k == 0 || rs[k - 1]->nj != z.nj || rs[k - 1]->d != z.d) {
+            align(size_t(nw));
+            grp.push_back(ZGrp{int(words.size()) - w.t.s0, 0, z.nj, z.d});
+          }
+          for (int i = 0; i < z.np; ++i) {
+            const int2 u = prod[size_t(z.p0 + i)];
+            src.push_back(Src{int(words.size()), z.c0 + i * z.nj, z.t0, z.nj});
+            words.push_back(unsigned(u.x) | unsigned(u.y) << 16);
+            words.resize(words.size() + size_t(nw) - 1, 0u);
+          }
+          grp.back().np += z.np;
+        }
+      }
+      w.t.grp2 = int(grp.size());
       task.push_back(w.t);
+      cost.push_back(w.cost);
     }
+    words.resize(((words.size() + 3) & ~size_t(3)) + 3 * ZS_CHUNK, 0u);  // a warp reads up to two chunks ahead
     for (const auto& v : by_t) {
       zt0.push_back(int(zt.size()));
       zt.insert(zt.end(), v.begin(), v.end());
@@ -314,16 +349,17 @@ void free_snap(Ctx& c) {
   h->ent.release();
   h->task.release();
   h->rec.release();
+  h->grp.release();
   h->D.release();
   h->H.release();
   h->hfull.release();
-  h->zc_f.release();
+  h->zs.release();
   for (auto* b : {&h->e0, &h->map, &h->zt0, &h->tmask, &h->eord, &h->pj, &h->cnt}) b->release();
   for (auto* b : {&h->xsum, &h->msum, &h->half, &h->zt, &h->prod}) b->release();
   for (auto* b : {&h->zc, &h->mono, &h->cY, &h->AB, &h->beta0, &h->wjelem, &h->pr, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk,
                   &h->eatom, &h->adj, &h->adj_sum, &h->adj_g, &h->keep_u, &h->keep_z})
     b->release();
-  for (auto* b : {&h->cY_f, &h->AB_f}) b->release();
+  h->AB_f.release();
   delete h;
   c.snap = nullptr;
 }
@@ -332,6 +368,25 @@ template <class T>
 static void upload(Ctx& c, DevBuf<T>& b, const std::vector<T>& v) {
   b.reserve(v.size() + 1, c.stream);
   EMD_CUDA(cudaMemcpyAsync(b.p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, c.stream));
+}
+
+// the FP32 stream of every element: the tables' words with coefficients times cY
+static void upload_stream(Ctx& c, SnapHost* h, const SnapTables& tab, const std::vector<double>& cY) {
+  const SnapDev& S = h->d;
+  const size_t n = tab.words.size();
+  std::vector<unsigned> w(n * size_t(S.nelem));
+  for (int e = 0; e < S.nelem; ++e) {
+    std::copy(tab.words.begin(), tab.words.end(), w.begin() + long(n) * e);
+    const double* ce = &cY[size_t(e) * S.nfull];
+    for (const auto& p : tab.src)
+      for (int j = 0; j < p.nj; ++j) {
+        const float v = float(tab.zc[size_t(p.c0 + j)] * ce[p.t0 - j]);
+        std::memcpy(&w[n * size_t(e) + size_t(p.word + 1 + j)], &v, sizeof v);
+      }
+  }
+  h->zs.reserve(w.size() / 4 + 1, c.stream);
+  EMD_CUDA(cudaMemcpyAsync(h->zs.p, w.data(), w.size() * sizeof(unsigned), cudaMemcpyHostToDevice, c.stream));
+  EMD_CUDA(cudaStreamSynchronize(c.stream));
 }
 
 // Y's coefficients: beta_k folded onto the full triples of compute_dbidrj's
@@ -371,21 +426,39 @@ static int snap_chunk(int n, int cap, bool adjoint_z, const SnapDev& S) {
 // so 32 atoms where the tiles (and their tasks, split over up to four CTAs)
 // fill the 152 SMs, fewer atoms with the rows shared by lane groups (0.89,
 // 0.73, 0.53 of the lanes' work useful at 16, 8, 4) where they would not.
-static int snap_tile_atoms(const SnapDev& S, int n, size_t real, bool keep) {
+static int snap_tile_atoms(const SnapDev& S, int n, bool fp64, bool keep) {
   int ta = 32;
   if (!keep)
     while (ta > 4 && (n + ta - 1) / ta * 4 < 152) ta /= 2;
-  while (ta > 1 && snap_y_smem(S, ta, real) > kMaxDynSmem) ta /= 2;
+  // mixed form: two atoms per lane once the tiles' splits still fill the SMs
+  if (!fp64 && S.twojmax <= 9 && (n + 63) / 64 * 4 >= 2 * 152) ta = 64;
+  while (ta > 1 && snap_y_smem(S, ta, fp64) > kMaxDynSmem) ta /= 2;
   return ta;
 }
-// CTAs that share a tile's tasks: the number (up to four: the longest task is
-// 7% of a tile) that wastes least of the last wave
-static int snap_tile_split(int tiles, int resident) {
+// CTAs that share a tile's tasks (up to four), for the smallest product of waves
+// and time per CTA.  FP64: the SM issues one instruction per 19 cycles, a single
+// warp one per 64.  Mixed: the busiest of the CTA's warps when each takes the
+// next longest task (more CTAs than tasks per warp leave warps idle: two
+// atoms per lane, 128,000 atoms, 2.18 ms with four CTAs a tile, 1.25 with one).
+static int snap_tile_split(const SnapTables& tab, int tiles, bool fp64, int ta) {
+  const int resident = fp64 || ta == 64 ? 1 : 2, warps = sy32_threads(ta == 64 ? 2 : 1) / 32;
   int best = 1;
   double best_cost = 1e300;
   for (int k = 1; k <= 4; ++k) {
+    double cta = 0.0;
+    for (int s = 0; s < k; ++s) {
+      double sum = 0.0, longest = 0.0;
+      std::vector<double> load(size_t(warps), 0.0);
+      for (size_t t = size_t(s); t < tab.cost.size(); t += size_t(k)) {
+        const double c = double(tab.cost[t]);
+        sum += c;
+        longest = std::max(longest, c);
+        *std::min_element(load.begin(), load.end()) += c;
+      }
+      cta = std::max(cta, fp64 ? std::max(19.0 * sum, 64.0 * longest) : *std::max_element(load.begin(), load.end()));
+    }
     const long long ctas = (long long)tiles * k, wave = 152LL * resident;
-    const double cost = double((ctas + wave - 1) / wave) / k + 0.01 * k;
+    const double cost = double((ctas + wave - 1) / wave) * cta;
     if (cost < best_cost) {
       best = k;
       best_cost = cost;
@@ -417,9 +490,9 @@ static SnapArgs snap_args(Ctx& c, SnapHost* h, int first, int n, bool fp64, bool
   A.pr = h->pr_f.p;
   A.pj = h->pj.p;
   A.cnt = h->cnt.p;
-  A.ta = snap_tile_atoms(S, c.N_local, real, keep);
+  A.ta = snap_tile_atoms(S, c.N_local, fp64, keep);
   const int tiles = (n + A.ta - 1) / A.ta;
-  A.nsplit = snap_tile_split(tiles, fp64 ? 1 : 2);
+  A.nsplit = snap_tile_split(*h->tab, tiles, fp64, A.ta);
   h->Y.reserve((size_t(tiles) * 4 * S.ne * A.ta * real + 7) / 8, c.stream);
   A.Y = h->Y.p;
   A.f = c.f.p;
@@ -441,8 +514,8 @@ static void snap_uy(Ctx& c, const SnapArgs& A, bool fp64) {
   }
   TimedLaunch t(c, fp64 ? "snap_y_fp64" : "snap_y_mixed");
   if (!fp64) snap_mixed_y(A, c.stream);
-  else if (A.S.twojmax <= 9) launch_y<double, 5>(A, c.stream);
-  else launch_y<double, 8>(A, c.stream);
+  else if (A.S.twojmax <= 9) launch_y<5>(A, c.stream);
+  else launch_y<8>(A, c.stream);
 }
 
 static void snap_require_list(Ctx& c, const char* what) {
@@ -677,7 +750,7 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
       pr.push_back(rfac0 * MY_PI / (rcut - rmin0));
       pr.push_back(MY_PI / (rcut - rmin0));
     }
-  const std::vector<float> cYf(cY.begin(), cY.end()), ABf(tab.AB.begin(), tab.AB.end());
+  const std::vector<float> ABf(tab.AB.begin(), tab.AB.end());
   upload(c, h->ent, tab.ent);
   upload(c, h->task, tab.task);
   upload(c, h->rec, tab.rec);
@@ -693,11 +766,10 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   upload(c, h->hfull, tab.hfull);
   upload(c, h->prod, tab.prod);
   upload(c, h->zc, tab.zc);
-  upload(c, h->zc_f, tab.zc_f);
+  upload(c, h->grp, tab.grp);
   upload(c, h->AB, tab.AB);
   upload(c, h->AB_f, ABf);
   upload(c, h->cY, cY);
-  upload(c, h->cY_f, cYf);
   upload(c, h->beta0, beta0);
   upload(c, h->pr, pr);
   upload(c, h->wjelem, std::vector<double>(wjelem, wjelem + nelem));
@@ -717,11 +789,14 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   S.hfull = h->hfull.p;
   S.prod = h->prod.p;
   S.zc = h->zc.p;
-  S.zc_f = h->zc_f.p;
+  S.grp = h->grp.p;
+  S.zs_n = int(tab.words.size() / 4);
+  h->tab = &tab;
+  if (precision == EMD_PREC_MIXED) upload_stream(c, h, tab, cY);
+  S.zs = h->zs.p;
   S.AB = h->AB.p;
   S.AB_f = h->AB_f.p;
   S.cY = h->cY.p;
-  S.cY_f = h->cY_f.p;
   S.beta0 = h->beta0.p;
   S.pr = h->pr.p;
   S.wjelem = h->wjelem.p;
@@ -758,9 +833,8 @@ emd_status emd_snap_set_beta(emd_ctx* ctx, const double* beta) {
   require(beta != nullptr, EMD_ERR_ARG, "emd_snap_set_beta: null beta");
   std::vector<double> cY, beta0;
   snap_fold_beta(*h, h->d.nfull, h->d.nelem, h->d.ncoeffall, beta, cY, beta0);
-  std::vector<float> cYf(cY.begin(), cY.end());
   EMD_CUDA(cudaMemcpyAsync(h->cY.p, cY.data(), sizeof(double) * cY.size(), cudaMemcpyHostToDevice, c.stream));
-  EMD_CUDA(cudaMemcpyAsync(h->cY_f.p, cYf.data(), sizeof(float) * cYf.size(), cudaMemcpyHostToDevice, c.stream));
+  if (h->precision == EMD_PREC_MIXED) upload_stream(c, h, *h->tab, cY);
   EMD_CUDA(cudaMemcpyAsync(h->beta0.p, beta0.data(), sizeof(double) * beta0.size(), cudaMemcpyHostToDevice,
                            c.stream));
   EMD_CUDA(cudaStreamSynchronize(c.stream));

@@ -63,13 +63,19 @@ struct Entry {
 
 // The products of one (j1, j2) at one (2m, 2m') = (-q -+ T, -q +- T) of a Z task
 struct ZRec {
-  int p0, np, c0, cf;  // products [p0, p0 + np); first coefficient, in zc and in zc_f
+  int p0, np, c0;      // products [p0, p0 + np), first coefficient
   short nj, d;         // number of j, the highest first; its distance from the task's highest j over 2
   int t0, z0;          // triple of the highest j; first kept Z
 };
 struct ZTask {
   int T, q, rec0, rec1, rec2;  // records of the +T elements [rec0, rec1), of the -T ones [rec1, rec2)
   int y0, kmax;                // first entry, last k
+  int grp0, grp1, grp2, s0;    // FP32: groups, +T and -T; first word of the stream
+};
+// FP32: a task's products of equal nj and d, whatever their (j1, j2)
+struct ZGrp {
+  int w0, np;          // first word (from the task's s0), products
+  short nj, d;
 };
 
 struct SnapDev {
@@ -89,9 +95,12 @@ struct SnapDev {
   const ZRec* rec;
   const int2* prod;    // the two U elements of a product
   const double* zc;    // coefficients, nj per product
-  const float2* zc_f;  // the same, each twice and nj rounded up to an even number
+  // FP32: groups, and per element a stream (zs_n each) of every product's two
+  // U elements (16 bits each) and coefficients times cY, zs_words(nj) words each
+  const ZGrp* grp;
+  const uint4* zs;
+  int zs_n;
   const double* cY;    // nelem x nfull
-  const float* cY_f;
   const double* AB;    // ne x 2
   const float* AB_f;
   const double* beta0;
@@ -542,60 +551,44 @@ __device__ __forceinline__ void z_products(const ZRec& z, const SnapDev& S, cons
     }
   }
 }
-// FP32: packed f32x2 operations on (re, im), coefficients stored twice
-template <int NJ>
-__device__ __forceinline__ void z_products(const ZRec& z, const SnapDev& S, const Cplx<float>* __restrict__ U, int str,
-                                           int first, int step, Cplx<float>* Z) {
-  constexpr int NC = (NJ + 1) / 2;
-  float2 acc[2 * NC];
-#pragma unroll
-  for (int j = 0; j < 2 * NC; ++j) acc[j] = make_float2(0.f, 0.f);
-  const int2* __restrict__ pl = S.prod + z.p0;
-  const float4* __restrict__ c = reinterpret_cast<const float4*>(S.zc_f + z.cf);
-#pragma unroll 4
-  for (int k = first; k < z.np; k += step) {
-    const int2 p = __ldg(pl + k);
-    const Cplx<float> x = U[p.x * str], y = U[p.y * str];
-    const float2 yy = make_float2(y.r, y.i);
-    const float2 pp = __ffma2_rn(make_float2(x.r, x.r), yy,
-                                 __fmul2_rn(make_float2(x.i, x.i), make_float2(-y.i, y.r)));
-#pragma unroll
-    for (int h = 0; h < NC; ++h) {
-      const float4 w = __ldg(c + k * NC + h);
-      acc[2 * h] = __ffma2_rn(make_float2(w.x, w.y), pp, acc[2 * h]);
-      if (2 * h + 1 < NJ) acc[2 * h + 1] = __ffma2_rn(make_float2(w.z, w.w), pp, acc[2 * h + 1]);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < NJ; ++j) Z[j] = Cplx<float>{acc[j].x, acc[j].y};
+
+// f(integral_constant<d>) for the uniform d: one block per value (f's marker
+// keeps the compiler from folding them into an indexed, hence local-memory, y)
+template <typename F>
+__device__ __forceinline__ void at_offset(int d, F&& f) {
+  if (d == 0) f(std::integral_constant<int, 0>{});
+  else if (d == 1) f(std::integral_constant<int, 1>{});
+  else if (d == 2) f(std::integral_constant<int, 2>{});
+  else if (d == 3) f(std::integral_constant<int, 3>{});
+  else if (d == 4) f(std::integral_constant<int, 4>{});
+  else if (d == 5) f(std::integral_constant<int, 5>{});
+  else if (d == 6) f(std::integral_constant<int, 6>{});
+  else f(std::integral_constant<int, 7>{});
 }
 
 template <typename R>
-__device__ __forceinline__ R shfl_xor_r(R v, int o) {
-  return __shfl_xor_sync(FULL_MASK, v, o);
+__device__ __forceinline__ void shfl_add(Cplx<R>& z, int o) {
+  z.r += __shfl_xor_sync(FULL_MASK, z.r, o);
+  z.i += __shfl_xor_sync(FULL_MASK, z.i, o);
 }
 
 // a record's Z and its part of the task's Y (y[0]: the highest j)
-template <typename R, int NM, int NJ, bool KEEP>
-__device__ __forceinline__ void z_add(const ZRec& z, const SnapDev& S, const Cplx<R>* __restrict__ U, int str,
-                                      const R* __restrict__ cY, int first, int step, Cplx<R>* y, Cplx<double>* zk) {
-  Cplx<R> Z[NJ];
+template <int NM, int NJ, bool KEEP>
+__device__ __forceinline__ void z_add(const ZRec& z, const SnapDev& S, const Cplx<double>* __restrict__ U, int str,
+                                      const double* __restrict__ cY, int first, int step, Cplx<double>* y,
+                                      Cplx<double>* zk) {
+  Cplx<double> Z[NJ];
   z_products<NJ>(z, S, U, str, first, step, Z);
-  R c[NJ];
+  double c[NJ];
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
     c[j] = cY[z.t0 - j];
     if constexpr (KEEP) {
-      for (int o = 32 / step; o < 32; o <<= 1) {
-        Z[j].r += shfl_xor_r(Z[j].r, o);
-        Z[j].i += shfl_xor_r(Z[j].i, o);
-      }
-      if (first == 0) zk[size_t(z.z0 + j) * 32] = Cplx<double>{double(Z[j].r), double(Z[j].i)};
+      for (int o = 32 / step; o < 32; o <<= 1) shfl_add(Z[j], o);
+      if (first == 0) zk[size_t(z.z0 + j) * 32] = Z[j];
     }
   }
-  // z.d is uniform; one block per value (the marker keeps the compiler from
-  // folding them into an indexed, hence local-memory, y)
-  auto add = [&](auto dc) {
+  at_offset(z.d, [&](auto dc) {
     constexpr int d = decltype(dc)::value;
     if constexpr (d + NJ <= NM) {
       asm volatile("// y + %0" ::"n"(d));
@@ -605,30 +598,50 @@ __device__ __forceinline__ void z_add(const ZRec& z, const SnapDev& S, const Cpl
         y[d + j].i = fma(c[j], Z[j].i, y[d + j].i);
       }
     }
-  };
-  if (z.d == 0) add(std::integral_constant<int, 0>{});
-  else if (z.d == 1) add(std::integral_constant<int, 1>{});
-  else if (z.d == 2) add(std::integral_constant<int, 2>{});
-  else if (z.d == 3) add(std::integral_constant<int, 3>{});
-  else if (z.d == 4) add(std::integral_constant<int, 4>{});
-  else if (z.d == 5) add(std::integral_constant<int, 5>{});
-  else if (z.d == 6) add(std::integral_constant<int, 6>{});
-  else add(std::integral_constant<int, 7>{});
+  });
 }
 
-// NM: most j of one (m, m') (5 up to twojmax 9, 8 up to 14); FULL: ta = 32
-template <typename R, int NM, bool KEEP, bool FULL>
-__global__ void __launch_bounds__(sizeof(R) == 8 ? 512 : 256) k_snap_y(SnapArgs A) {
+// E = 2N (Y+ + (-1)^T Y-), O = 2N (Y+ - (-1)^T Y-) of a task's entries (p: +T,
+// m: -T, highest j first): with a^q and w b^T = u + i v, twice the real part of
+// conj(U) Y over both signs of T is u Re(a^q E) + v Im(a^q O) times P_k
+template <typename R, int NM>
+__device__ __forceinline__ void y_store(const SnapDev& S, const ZTask& K, const Cplx<R>* yp, const Cplx<R>* ym, R* Yt,
+                                        int ta) {
+#pragma unroll
+  for (int h = 0; h < NM; ++h)
+    if (h <= K.kmax) {
+      const int k = K.kmax - h;
+      const R N = R(S.ent[K.y0 + k].N), N2 = N + N;
+      R er, ei, orr, oi;
+      const Cplx<R> p = yp[h], m = ym[h];
+      if (K.q == 0) {  // the -T element is the inversion of the +T one
+        er = (K.T ? N2 : N) * p.r;
+        oi = K.T ? N2 * p.i : R(0);
+        ei = orr = R(0);
+      } else if (K.T == 0) {
+        er = N2 * p.r;
+        ei = N2 * p.i;
+        orr = oi = R(0);
+      } else {
+        const R sg = K.T & 1 ? R(-1) : R(1);
+        er = N2 * fma(sg, m.r, p.r);
+        ei = N2 * fma(sg, m.i, p.i);
+        orr = N2 * fma(-sg, m.r, p.r);
+        oi = N2 * fma(-sg, m.i, p.i);
+      }
+      R* o = Yt + size_t(4) * (K.y0 + k) * ta;
+      o[0] = er;
+      o[ta] = ei;
+      o[2 * ta] = orr;
+      o[3 * ta] = oi;
+    }
+}
+
+// the tile's U, both halves of the grid, as [element][atom] with rows of ta + 1
+template <typename R>
+__device__ __forceinline__ void y_load_tile(const SnapArgs& A, int tile, int ta, Cplx<R>* U) {
   const SnapDev& S = A.S;
-  extern __shared__ __align__(16) unsigned char sy_smem[];
-  __shared__ int s_next;
-  Cplx<R>* U = reinterpret_cast<Cplx<R>*>(sy_smem);  // [element][atom], rows of ta + 1
-  const int ta = FULL ? 32 : A.ta, str = ta + 1, tile = blockIdx.x / A.nsplit, split = blockIdx.x - tile * A.nsplit;
-  const int lane = threadIdx.x & 31, at = FULL ? lane : lane % ta, sub = FULL ? 0 : lane / ta, nsub = FULL ? 1 : 32 / ta;
-  const int al = tile * ta + at;
-  const bool live = al < A.n;
-  if (threadIdx.x == 0) s_next = 0;
-  // the tile's U, both halves of the grid
+  const int str = ta + 1;
   for (int k = threadIdx.x; k < S.nh * ta; k += blockDim.x) {
     const int a = k / S.nh, h = k - a * S.nh, ga = tile * ta + a;
     const Cplx<R> u = ga < A.n ? static_cast<const Cplx<R>*>(A.U)[size_t(ga) * S.nh + h] : Cplx<R>{R(0), R(0)};
@@ -636,95 +649,238 @@ __global__ void __launch_bounds__(sizeof(R) == 8 ? 512 : 256) k_snap_y(SnapArgs 
     U[f.x * str + a] = u;
     if (f.y != f.x) U[f.y * str + a] = f.z > 0 ? Cplx<R>{u.r, -u.i} : Cplx<R>{-u.r, u.i};
   }
+}
+
+// FP64.  NM: most j of one (m, m') (5 up to twojmax 9, 8 up to 14); FULL: ta = 32
+constexpr int SY_THREADS = 512;
+template <int NM, bool KEEP, bool FULL>
+__global__ void __launch_bounds__(SY_THREADS) k_snap_y(SnapArgs A) {
+  const SnapDev& S = A.S;
+  extern __shared__ __align__(16) unsigned char sy_smem[];
+  __shared__ int s_next;
+  Cplx<double>* U = reinterpret_cast<Cplx<double>*>(sy_smem);
+  const int ta = FULL ? 32 : A.ta, str = ta + 1, tile = blockIdx.x / A.nsplit, split = blockIdx.x - tile * A.nsplit;
+  const int lane = threadIdx.x & 31, at = FULL ? lane : lane % ta, sub = FULL ? 0 : lane / ta, nsub = FULL ? 1 : 32 / ta;
+  const int al = tile * ta + at;
+  if (threadIdx.x == 0) s_next = 0;
+  y_load_tile(A, tile, ta, U);
   __syncthreads();
-  const int ei = live ? S.map[A.type[A.first + al]] : 0;
-  const R* cY = (sizeof(R) == 8 ? reinterpret_cast<const R*>(S.cY) : reinterpret_cast<const R*>(S.cY_f)) +
-                size_t(ei) * S.nfull;
-  R* Yt = static_cast<R*>(A.Y) + size_t(tile) * 4 * S.ne * ta + at;
+  const int ei = al < A.n ? S.map[A.type[A.first + al]] : 0;
+  const double* cY = S.cY + size_t(ei) * S.nfull;
+  double* Yt = static_cast<double*>(A.Y) + size_t(tile) * 4 * S.ne * ta + at;
   Cplx<double>* zk = reinterpret_cast<Cplx<double>*>(A.zkeep) + (KEEP ? size_t(al >> 5) * S.nz * 32 + (al & 31) : 0);
-  const Cplx<R>* Ua = U + at;
+  const Cplx<double>* Ua = U + at;
   while (true) {
     int t = 0;
     if (lane == 0) t = atomicAdd(&s_next, 1);
     t = __shfl_sync(FULL_MASK, t, 0) * A.nsplit + split;  // tasks longest first
     if (t >= S.ntask) break;
     const ZTask K = S.task[t];
-    Cplx<R> y[NM], yp[NM];  // Y of the -T elements (first: +T), of the +T elements
+    Cplx<double> y[NM], yp[NM];  // Y of the -T elements (first: +T), of the +T elements
 #pragma unroll
-    for (int k = 0; k < NM; ++k) y[k] = Cplx<R>{R(0), R(0)};
+    for (int k = 0; k < NM; ++k) y[k] = Cplx<double>{0.0, 0.0};
 #pragma unroll 1
-    for (int r = K.rec0; r < K.rec2; ++r) {
+    for (int r = K.rec0; r <= K.rec2; ++r) {
       if (r == K.rec1) {
 #pragma unroll
         for (int k = 0; k < NM; ++k) {
           yp[k] = y[k];
-          y[k] = Cplx<R>{R(0), R(0)};
+          y[k] = Cplx<double>{0.0, 0.0};
         }
       }
+      if (r == K.rec2) break;
       const ZRec z = S.rec[r];
       switch (z.nj) {  // uniform
-        case 1: z_add<R, NM, 1, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
-        case 2: z_add<R, NM, 2, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
-        case 3: z_add<R, NM, 3, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
-        case 4: z_add<R, NM, 4, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
-        case 5: z_add<R, NM, 5, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
+        case 1: z_add<NM, 1, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
+        case 2: z_add<NM, 2, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
+        case 3: z_add<NM, 3, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
+        case 4: z_add<NM, 4, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
+        case 5: z_add<NM, 5, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
         default:
           if constexpr (NM > 5) {
-            if (z.nj == 6) z_add<R, NM, 6, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk);
-            else if (z.nj == 7) z_add<R, NM, 7, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk);
-            else z_add<R, NM, 8, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk);
+            if (z.nj == 6) z_add<NM, 6, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk);
+            else if (z.nj == 7) z_add<NM, 7, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk);
+            else z_add<NM, 8, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk);
           }
-      }
-    }
-    if (K.rec1 == K.rec2) {  // no -T elements
-#pragma unroll
-      for (int k = 0; k < NM; ++k) {
-        yp[k] = y[k];
-        y[k] = Cplx<R>{R(0), R(0)};
       }
     }
     // the lane groups' parts (KEEP: every Z was completed already)
     for (int o = ta; o < 32 && !KEEP; o <<= 1)
 #pragma unroll
       for (int k = 0; k < NM; ++k) {
-        yp[k].r += shfl_xor_r(yp[k].r, o);
-        yp[k].i += shfl_xor_r(yp[k].i, o);
-        y[k].r += shfl_xor_r(y[k].r, o);
-        y[k].i += shfl_xor_r(y[k].i, o);
+        shfl_add(yp[k], o);
+        shfl_add(y[k], o);
       }
-    // E = 2N (Y+ + (-1)^T Y-), O = 2N (Y+ - (-1)^T Y-): with a^q and w b^T =
-    // u + i v, twice the real part of conj(U) Y over both signs of T is
-    // u Re(a^q E) + v Im(a^q O) times P_k
-    if (sub == 0) {
+    if (sub == 0) y_store<double, NM>(S, K, yp, y, Yt, ta);
+  }
+}
+
+// FP32.  Here the FP64 pipe's slow cadence does not hide the rest, so
+//  - the products of a task with equal nj and d form one group, whatever their
+//    (j1, j2): cY is folded into the coefficients, Y is summed directly and the
+//    255 groups (at twojmax 8) replace 1,285 records;
+//  - the tables (200 KB) do not fit what the tile leaves of L1, so a task's
+//    entries come as one stream through a shared buffer of the warp's own:
+//    while one KB is worked on the next is on its way in registers;
+//  - in large systems a lane takes two atoms (NA), so that every entry and its
+//    addresses serve 64 atoms.
+// Atoms of another element than the stream's are computed and not stored
+// (one launch per element).
+// Per 128,000 atoms: 3.77 ms with records and direct table reads, 2.47 with
+// records streamed, 1.25 as it is.
+__host__ __device__ constexpr int zs_words(int nj) { return nj == 1 ? 2 : (nj <= 3 ? 4 : (nj <= 5 ? 8 : 16)); }
+constexpr int ZS_CHUNK = 256;  // words per buffer
+struct ZStream {
+  const uint4* g;  // the chunk in registers
+  uint4 r0, r1;
+  uint4* buf;
+  int cur;  // chunk in the buffer
+  __device__ __forceinline__ void begin(const uint4* zs, int s0, int lane) {
+    g = zs + s0 / 4 + lane;
+    r0 = __ldg(g);
+    r1 = __ldg(g + 32);
+    cur = -1;
+    next(lane);
+  }
+  __device__ __forceinline__ void next(int lane) {
+    __syncwarp();
+    buf[lane] = r0;
+    buf[lane + 32] = r1;
+    __syncwarp();
+    g += 64;
+    r0 = __ldg(g);
+    r1 = __ldg(g + 32);
+    ++cur;
+  }
+};
+template <int NM, int NJ, int NA>
+__device__ __forceinline__ void zg_add(const ZGrp& G, ZStream& st, const Cplx<float>* __restrict__ U, int str,
+                                       int first, int step, Cplx<float> (*y)[NM]) {
+  constexpr int W = zs_words(NJ);
+  Cplx<float> Z[NA][NJ];
 #pragma unroll
-      for (int h = 0; h < NM; ++h)
-        if (h <= K.kmax) {
-          const int k = K.kmax - h;
-          const R N = R(S.ent[K.y0 + k].N), N2 = N + N;
-          R er, ei2, orr, oi;
-          const Cplx<R> p = yp[h], m = y[h];
-          if (K.q == 0) {  // the -T element is the inversion of the +T one
-            er = (K.T ? N2 : N) * p.r;
-            oi = K.T ? N2 * p.i : R(0);
-            ei2 = orr = R(0);
-          } else if (K.T == 0) {
-            er = N2 * p.r;
-            ei2 = N2 * p.i;
-            orr = oi = R(0);
-          } else {
-            const R sg = K.T & 1 ? R(-1) : R(1);
-            er = N2 * fma(sg, m.r, p.r);
-            ei2 = N2 * fma(sg, m.i, p.i);
-            orr = N2 * fma(-sg, m.r, p.r);
-            oi = N2 * fma(-sg, m.i, p.i);
-          }
-          R* o = Yt + size_t(4) * (K.y0 + k) * ta;
-          o[0] = er;
-          o[ta] = ei2;
-          o[2 * ta] = orr;
-          o[3 * ta] = oi;
+  for (int a = 0; a < NA; ++a)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) Z[a][j] = Cplx<float>{0.f, 0.f};
+  int pos = G.w0, left = G.np;
+  while (left > 0) {
+    if (pos / ZS_CHUNK != st.cur) st.next(threadIdx.x & 31);
+    const int m = min(left, (ZS_CHUNK - pos % ZS_CHUNK) / W);
+    const unsigned* w = reinterpret_cast<const unsigned*>(st.buf) + pos % ZS_CHUNK;
+#pragma unroll 4
+    for (int k = first; k < m; k += step) {
+      unsigned d[W];
+      if constexpr (W == 2) {
+        *reinterpret_cast<uint2*>(d) = *reinterpret_cast<const uint2*>(w + k * W);
+      } else {
+#pragma unroll
+        for (int h = 0; h < (NJ + 4) / 4; ++h)
+          reinterpret_cast<uint4*>(d)[h] = *reinterpret_cast<const uint4*>(w + k * W + 4 * h);
+      }
+      const Cplx<float>* px = U + (d[0] & 0xffffu) * str;
+      const Cplx<float>* py = U + (d[0] >> 16) * str;
+#pragma unroll
+      for (int a = 0; a < NA; ++a) {
+        const Cplx<float> x = px[32 * a], v = py[32 * a];
+        const float pr = fmaf(x.r, v.r, -x.i * v.i), pi = fmaf(x.r, v.i, x.i * v.r);
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const float c = __uint_as_float(d[1 + j]);
+          Z[a][j].r = fmaf(c, pr, Z[a][j].r);
+          Z[a][j].i = fmaf(c, pi, Z[a][j].i);
+        }
+      }
+    }
+    pos += m * W;
+    left -= m;
+  }
+  at_offset(G.d, [&](auto dc) {
+    constexpr int d = decltype(dc)::value;
+    if constexpr (d + NJ <= NM) {
+      asm volatile("// y + %0" ::"n"(d));
+#pragma unroll
+      for (int a = 0; a < NA; ++a)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          y[a][d + j].r += Z[a][j].r;
+          y[a][d + j].i += Z[a][j].i;
         }
     }
+  });
+}
+
+__host__ __device__ constexpr int sy32_threads(int na) { return na == 2 ? 512 : 384; }
+template <int NM, int NA, bool FULL>
+__global__ void __launch_bounds__(sy32_threads(NA), NA == 2 ? 1 : 2) k_snap_y32(SnapArgs A, int elem) {
+  const SnapDev& S = A.S;
+  extern __shared__ __align__(16) unsigned char sy_smem[];
+  __shared__ int s_next;
+  Cplx<float>* U = reinterpret_cast<Cplx<float>*>(sy_smem);
+  const int ta = FULL ? 32 * NA : A.ta, str = ta + 1, tile = blockIdx.x / A.nsplit, split = blockIdx.x - tile * A.nsplit;
+  const int lane = threadIdx.x & 31, at = FULL ? lane : lane % ta, sub = FULL ? 0 : lane / ta, nsub = FULL ? 1 : 32 / ta;
+  if (threadIdx.x == 0) s_next = 0;
+  y_load_tile(A, tile, ta, U);
+  __syncthreads();
+  bool mine[NA];
+#pragma unroll
+  for (int a = 0; a < NA; ++a) {
+    const int al = tile * ta + at + 32 * a;
+    mine[a] = sub == 0 && al < A.n && S.map[A.type[A.first + al]] == elem;
+  }
+  float* Yt = static_cast<float*>(A.Y) + size_t(tile) * 4 * S.ne * ta + at;
+  const Cplx<float>* Ua = U + at;
+  ZStream st;
+  st.buf = reinterpret_cast<uint4*>(sy_smem + ((sizeof(Cplx<float>) * size_t(S.nuf) * str + 15) & ~size_t(15))) +
+           (threadIdx.x >> 5) * (ZS_CHUNK / 4);
+  const uint4* zs = S.zs + size_t(elem) * S.zs_n;
+  while (true) {
+    int t = 0;
+    if (lane == 0) t = atomicAdd(&s_next, 1);
+    t = __shfl_sync(FULL_MASK, t, 0) * A.nsplit + split;  // tasks longest first
+    if (t >= S.ntask) break;
+    const ZTask K = S.task[t];
+    st.begin(zs, K.s0, lane);
+    Cplx<float> y[NA][NM], yp[NA][NM];
+#pragma unroll
+    for (int a = 0; a < NA; ++a)
+#pragma unroll
+      for (int k = 0; k < NM; ++k) y[a][k] = Cplx<float>{0.f, 0.f};
+#pragma unroll 1
+    for (int g = K.grp0; g <= K.grp2; ++g) {
+      if (g == K.grp1) {
+#pragma unroll
+        for (int a = 0; a < NA; ++a)
+#pragma unroll
+          for (int k = 0; k < NM; ++k) {
+            yp[a][k] = y[a][k];
+            y[a][k] = Cplx<float>{0.f, 0.f};
+          }
+      }
+      if (g == K.grp2) break;
+      const ZGrp G = S.grp[g];
+      switch (G.nj) {  // uniform
+        case 1: zg_add<NM, 1, NA>(G, st, Ua, str, sub, nsub, y); break;
+        case 2: zg_add<NM, 2, NA>(G, st, Ua, str, sub, nsub, y); break;
+        case 3: zg_add<NM, 3, NA>(G, st, Ua, str, sub, nsub, y); break;
+        case 4: zg_add<NM, 4, NA>(G, st, Ua, str, sub, nsub, y); break;
+        case 5: zg_add<NM, 5, NA>(G, st, Ua, str, sub, nsub, y); break;
+        default:
+          if constexpr (NM > 5) {
+            if (G.nj == 6) zg_add<NM, 6, NA>(G, st, Ua, str, sub, nsub, y);
+            else if (G.nj == 7) zg_add<NM, 7, NA>(G, st, Ua, str, sub, nsub, y);
+            else zg_add<NM, 8, NA>(G, st, Ua, str, sub, nsub, y);
+          }
+      }
+    }
+    for (int o = ta; o < 32; o <<= 1)  // the lane groups' parts
+#pragma unroll
+      for (int k = 0; k < NM; ++k) {
+        shfl_add(yp[0][k], o);
+        shfl_add(y[0][k], o);
+      }
+#pragma unroll
+    for (int a = 0; a < NA; ++a)
+      if (mine[a]) y_store<float, NM>(S, K, yp[a], y[a], Yt + 32 * a, ta);
   }
 }
 
@@ -1136,26 +1292,36 @@ static __global__ void __launch_bounds__(256) k_snap_pq(SnapArgs A) {
 }
 
 // ---------------------------------------------------------------- launches
-inline size_t snap_y_smem(const SnapDev& S, int ta, size_t real) { return 2 * real * size_t(S.nuf) * (ta + 1); }
+inline size_t snap_y_smem(const SnapDev& S, int ta, bool fp64) {
+  const size_t u = ((fp64 ? 16 : 8) * size_t(S.nuf) * (ta + 1) + 15) & ~size_t(15);
+  return u + (fp64 ? 0 : size_t(sy32_threads(ta == 64 ? 2 : 1)) / 32 * ZS_CHUNK * 4);
+}
 
-template <typename R, int NM, bool KEEP, bool FULL>
+template <int NM, bool KEEP, bool FULL>
 void launch_y(const SnapArgs& A, cudaStream_t s) {
-  const size_t smem = snap_y_smem(A.S, A.ta, sizeof(R));
-  const int tiles = (A.n + A.ta - 1) / A.ta, threads = sizeof(R) == 8 ? 512 : 256;
-  allow_dyn_smem(k_snap_y<R, NM, KEEP, FULL>);
-  k_snap_y<R, NM, KEEP, FULL><<<tiles * A.nsplit, threads, smem, s>>>(A);
+  const int tiles = (A.n + A.ta - 1) / A.ta;
+  allow_dyn_smem(k_snap_y<NM, KEEP, FULL>);
+  k_snap_y<NM, KEEP, FULL><<<tiles * A.nsplit, SY_THREADS, snap_y_smem(A.S, A.ta, true), s>>>(A);
   EMD_CHECK_LAUNCH();
 }
-template <typename R, int NM>
+template <int NM>
 void launch_y(const SnapArgs& A, cudaStream_t s) {
-  if constexpr (sizeof(R) == 8)
-    if (A.zkeep) {
-      if (A.ta == 32) launch_y<R, NM, true, true>(A, s);
-      else launch_y<R, NM, true, false>(A, s);
-      return;
-    }
-  if (A.ta == 32) launch_y<R, NM, false, true>(A, s);
-  else launch_y<R, NM, false, false>(A, s);
+  if (A.zkeep) {
+    if (A.ta == 32) launch_y<NM, true, true>(A, s);
+    else launch_y<NM, true, false>(A, s);
+  } else {
+    if (A.ta == 32) launch_y<NM, false, true>(A, s);
+    else launch_y<NM, false, false>(A, s);
+  }
+}
+template <int NM, int NA, bool FULL>
+void launch_y32(const SnapArgs& A, cudaStream_t s) {
+  const int tiles = (A.n + A.ta - 1) / A.ta;
+  allow_dyn_smem(k_snap_y32<NM, NA, FULL>);
+  for (int e = 0; e < A.S.nelem; ++e) {
+    k_snap_y32<NM, NA, FULL><<<tiles * A.nsplit, sy32_threads(NA), snap_y_smem(A.S, A.ta, false), s>>>(A, e);
+    EMD_CHECK_LAUNCH();
+  }
 }
 
 template <typename R>

@@ -13,8 +13,16 @@ void snap_mixed_pairs(const SnapArgs& A, cudaStream_t s) { launch_pairs<float>(A
 void snap_mixed_u(const SnapArgs& A, cudaStream_t s) { launch_u<float>(A, s); }
 
 void snap_mixed_y(const SnapArgs& A, cudaStream_t s) {
-  if (A.S.twojmax <= 9) launch_y<float, 5>(A, s);
-  else launch_y<float, 8>(A, s);
+  if (A.S.twojmax > 9) {
+    if (A.ta == 32) launch_y32<8, 1, true>(A, s);
+    else launch_y32<8, 1, false>(A, s);
+  } else if (A.ta == 64) {
+    launch_y32<5, 2, true>(A, s);
+  } else if (A.ta == 32) {
+    launch_y32<5, 1, true>(A, s);
+  } else {
+    launch_y32<5, 1, false>(A, s);
+  }
 }
 
 void snap_mixed_force(const SnapArgs& A, int threads, cudaStream_t s) {
