@@ -34,7 +34,7 @@ struct SnapHost {
   DevBuf<ZGrp> grp;
   DevBuf<int> e0, map, zt0, tmask, eord;
   DevBuf<int2> xsum, msum, half, zt, prod;
-  DevBuf<int4> hfull;
+  DevBuf<int4> hfull, ysrc;
   DevBuf<double> zc, mono, cY, AB, beta0, wjelem, pr;
   DevBuf<float> AB_f;
   DevBuf<uint4> zs;
@@ -100,12 +100,17 @@ double jacobi_B(int al, int be, int k) {
   return 4.0 * k * (k + al) * (k + be) * (k + al + be) / (s * s * (s + 1.0) * (s - 1.0));
 }
 
+long long rec_cost(const ZRec& z) { return (long long)z.np * (4 + 2 * z.nj); }  // operations
+constexpr int ZS_PARTS = 48;        // a Z task has at most about this fraction of the work,
+constexpr long long ZS_LEAST = 300; // unless that is less than this
+constexpr int ZS_SPLIT = 16;        // CTAs that may share a tile
+
 // The tables of one twojmax (see the structures in snap_kernel.cuh)
 struct SnapTables {
   std::vector<Entry> ent;
   std::vector<int> e0, zt0, tmask, eord;
   std::vector<int2> xsum, msum, half, zt, prod;
-  std::vector<int4> hfull;
+  std::vector<int4> hfull, ysrc;
   std::vector<ZTask> task;
   std::vector<ZRec> rec;
   std::vector<double> zc, AB, mono;
@@ -115,8 +120,10 @@ struct SnapTables {
     int word, c0, t0, nj;  // of a product: its words, coefficients and highest triple
   };
   std::vector<Src> src;
-  std::vector<long long> cost;  // of the tasks
-  int nz = 0, nh = 0;
+  int nz = 0, nh = 0, ny = 0;
+  // cost of the busiest of k + 1 CTAs that share a tile's tasks: FP64 in cycles,
+  // mixed in instructions of the busiest of 12 or 16 warps
+  double cta64[ZS_SPLIT], cta32[2][ZS_SPLIT];
 
   SnapTables(int J, const std::vector<int>& trip) {
     const int L = J + 1, ntrip = int(trip.size() / 3);
@@ -134,7 +141,6 @@ struct SnapTables {
           Entry E{};
           E.N = std::ldexp(factorial(j) / std::sqrt(factorial(ma) * factorial(j - ma) * factorial(mb) * factorial(j - mb)),
                            -k);
-          E.invN = 1.0 / E.N;
           E.A = jacobi_A(T, q, k);
           E.B = jacobi_B(T, q, k);
           AB.push_back(E.A);
@@ -195,24 +201,26 @@ struct SnapTables {
         for (int t = 0; t < ntrip; ++t)
           if (trip[3 * size_t(t)] == j1 && trip[3 * size_t(t) + 1] == j2 && trip[3 * size_t(t) + 2] == hi) ttop[pr] = t;
       }
-    // Z tasks, longest first
+    // Z tasks, longest first: one (T, q) and sign of T each, in as many parts
+    // as keep a part near 1/ZS_PARTS of the whole
     struct Raw {
       ZTask t;
-      std::vector<ZRec> r[2];
+      std::vector<ZRec> r;
       long long cost;
+      int h0, hs;  // half-grid element of k = 0, elements between two k
     };
     std::vector<int2> rp;    // products and coefficients in record order
     std::vector<double> rc;  // before the tasks are sorted
-    std::vector<Raw> raw;
+    std::vector<Raw> whole, raw;
     for (int T = 0; T <= J; ++T)
-      for (int q = 0; q <= J - T; ++q) {
-        Raw w{};
-        w.t.T = T;
-        w.t.q = q;
-        w.t.y0 = e0[size_t(T) * L + q];
-        w.t.kmax = (J - q - T) / 2;
-        const int top = q + T + 2 * w.t.kmax;
-        for (int s = 0; s < (T > 0 && q > 0 ? 2 : 1); ++s)
+      for (int q = 0; q <= J - T; ++q)
+        for (int s = 0; s < (T > 0 && q > 0 ? 2 : 1); ++s) {
+          Raw w{};
+          w.t.kmax = (J - q - T) / 2;
+          const int top = q + T + 2 * w.t.kmax;
+          const int2 h = half[size_t(e0[size_t(T) * L + q])];
+          w.h0 = s ? h.y : h.x;
+          w.hs = h.y >= 0 ? 2 : 1;
           for (int j1 = 0; j1 <= J; ++j1)
             for (int j2 = 0; j2 <= j1; ++j2) {
               if ((j1 + j2 - q - T) & 1) continue;
@@ -238,11 +246,39 @@ struct SnapTables {
                                  cg[size_t(cgo[pr] + (n1 * (j2 + 1) + n2) * njt[pr] + j)]);
                 }
               z.np = int(rp.size()) - z.p0;
-              w.cost += (long long)z.np * (4 + 2 * z.nj);
-              w.r[s].push_back(z);
+              w.cost += rec_cost(z);
+              w.r.push_back(z);
             }
-        raw.push_back(std::move(w));
+          whole.push_back(std::move(w));
+        }
+    long long total = 0;
+    for (const Raw& w : whole) total += w.cost;
+    const long long most = std::max(ZS_LEAST, total / ZS_PARTS);
+    ysrc.assign(size_t(nh), int4{0, 0, 0, 0});
+    for (const Raw& w : whole) {
+      const long long parts = (w.cost + most - 1) / most;
+      long long done = 0;
+      size_t r = 0;
+      int np = 0;
+      const int y0 = ny;
+      for (long long k = 0; k < parts; ++k) {
+        Raw v{};
+        v.t = w.t;
+        v.t.y0 = ny;
+        v.h0 = w.h0;
+        v.hs = w.hs;
+        while (r < w.r.size() && (v.r.empty() || (done + rec_cost(w.r[r]) / 2) * parts < (k + 1) * w.cost)) {
+          v.cost += rec_cost(w.r[r]);
+          done += rec_cost(w.r[r]);
+          v.r.push_back(w.r[r++]);
+        }
+        if (v.r.empty()) break;
+        ny += w.t.kmax + 1;
+        ++np;
+        raw.push_back(std::move(v));
       }
+      for (int k = 0; k <= w.t.kmax; ++k) ysrc[size_t(w.h0 + k * w.hs)] = int4{y0 + k, w.t.kmax + 1, np, 0};
+    }
     std::stable_sort(raw.begin(), raw.end(), [](const Raw& x, const Raw& y) { return x.cost > y.cost; });
     std::vector<std::vector<int2>> by_t(static_cast<size_t>(ntrip));
     // FP32 stream: tasks start on 64 bytes, groups on their products' size
@@ -251,48 +287,61 @@ struct SnapTables {
       align(16);
       w.t.s0 = int(words.size());
       w.t.rec0 = int(rec.size());
-      for (int s = 0; s < 2; ++s) {
-        for (ZRec& z : w.r[s]) {
-          const int rp0 = z.p0, rc0 = z.c0;
-          z.p0 = int(prod.size());
-          z.c0 = int(zc.size());
-          prod.insert(prod.end(), rp.begin() + rp0, rp.begin() + rp0 + z.np);
-          zc.insert(zc.end(), rc.begin() + rc0, rc.begin() + rc0 + z.np * z.nj);
-          z.z0 = nz;
-          for (int j = 0; j < z.nj; ++j) {  // highest j first: entry kmax - d - j of the task
-            const int2 h = half[size_t(w.t.y0 + w.t.kmax - z.d - j)];
-            by_t[size_t(z.t0 - j)].push_back(int2{nz, s ? h.y : h.x});
-            ++nz;
-          }
-          rec.push_back(z);
+      for (ZRec& z : w.r) {
+        const int rp0 = z.p0, rc0 = z.c0;
+        z.p0 = int(prod.size());
+        z.c0 = int(zc.size());
+        prod.insert(prod.end(), rp.begin() + rp0, rp.begin() + rp0 + z.np);
+        zc.insert(zc.end(), rc.begin() + rc0, rc.begin() + rc0 + z.np * z.nj);
+        z.z0 = nz;
+        for (int j = 0; j < z.nj; ++j) {  // highest j first: k = kmax - d - j
+          by_t[size_t(z.t0 - j)].push_back(int2{nz, w.h0 + (w.t.kmax - z.d - j) * w.hs});
+          ++nz;
         }
-        (s ? w.t.rec2 : w.t.rec1) = int(rec.size());
+        rec.push_back(z);
       }
-      for (int s = 0; s < 2; ++s) {
-        (s ? w.t.grp1 : w.t.grp0) = int(grp.size());
-        std::vector<const ZRec*> rs;
-        for (const ZRec& z : w.r[s]) rs.push_back(&z);
-        std::stable_sort(rs.begin(), rs.end(),
-                         [](const ZRec* x, const ZRec* y) { return x->nj != y->nj ? x->nj > y->nj : x->d < y->d; });
-        for (size_t k = 0; k < rs.size(); ++k) {
-          const ZRec& z = *rs[k];
-          const int nw = zs_words(z.nj);
-          if (k == 0 || rs[k - 1]->nj != z.nj || rs[k - 1]->d != z.d) {
-            align(size_t(nw));
-            grp.push_back(ZGrp{int(words.size()) - w.t.s0, 0, z.nj, z.d});
-          }
-          for (int i = 0; i < z.np; ++i) {
-            const int2 u = prod[size_t(z.p0 + i)];
-            src.push_back(Src{int(words.size()), z.c0 + i * z.nj, z.t0, z.nj});
-            words.push_back(unsigned(u.x) | unsigned(u.y) << 16);
-            words.resize(words.size() + size_t(nw) - 1, 0u);
-          }
-          grp.back().np += z.np;
+      w.t.rec1 = int(rec.size());
+      w.t.grp0 = int(grp.size());
+      std::vector<const ZRec*> rs;
+      for (const ZRec& z : w.r) rs.push_back(&z);
+      std::stable_sort(rs.begin(), rs.end(),
+                       [](const ZRec* x, const ZRec* y) { return x->nj != y->nj ? x->nj > y->nj : x->d < y->d; });
+      for (size_t k = 0; k < rs.size(); ++k) {
+        const ZRec& z = *rs[k];
+        const int nw = zs_words(z.nj);
+        if (k == 0 || rs[k - 1]->nj != z.nj || rs[k - 1]->d != z.d) {
+          align(size_t(nw));
+          grp.push_back(ZGrp{int(words.size()) - w.t.s0, 0, z.nj, z.d});
         }
+        for (int i = 0; i < z.np; ++i) {
+          const int2 u = prod[size_t(z.p0 + i)];
+          src.push_back(Src{int(words.size()), z.c0 + i * z.nj, z.t0, z.nj});
+          words.push_back(unsigned(u.x) | unsigned(u.y) << 16);
+          words.resize(words.size() + size_t(nw) - 1, 0u);
+        }
+        grp.back().np += z.np;
       }
-      w.t.grp2 = int(grp.size());
+      w.t.grp1 = int(grp.size());
       task.push_back(w.t);
-      cost.push_back(w.cost);
+    }
+    // a task's turn in each case: the warp that is free first takes the next
+    for (int k = 1; k <= ZS_SPLIT; ++k) {
+      double c64 = 0.0, c32[2] = {0.0, 0.0};
+      for (int s = 0; s < k; ++s) {
+        double sum = 0.0, longest = 0.0;
+        std::vector<double> load[2] = {std::vector<double>(sy32_threads(1) / 32, 0.0),
+                                       std::vector<double>(sy32_threads(2) / 32, 0.0)};
+        for (size_t t = size_t(s); t < raw.size(); t += size_t(k)) {
+          const double c = double(raw[t].cost);
+          sum += c;
+          longest = std::max(longest, c);
+          for (auto& l : load) *std::min_element(l.begin(), l.end()) += c;
+        }
+        c64 = std::max(c64, std::max(19.0 * sum, 64.0 * longest));
+        for (int v = 0; v < 2; ++v) c32[v] = std::max(c32[v], *std::max_element(load[v].begin(), load[v].end()));
+      }
+      cta64[k - 1] = c64;
+      for (int v = 0; v < 2; ++v) cta32[v][k - 1] = c32[v];
     }
     words.resize(((words.size() + 3) & ~size_t(3)) + 3 * ZS_CHUNK, 0u);  // a warp reads up to two chunks ahead
     for (const auto& v : by_t) {
@@ -353,6 +402,7 @@ void free_snap(Ctx& c) {
   h->D.release();
   h->H.release();
   h->hfull.release();
+  h->ysrc.release();
   h->zs.release();
   for (auto* b : {&h->e0, &h->map, &h->zt0, &h->tmask, &h->eord, &h->pj, &h->cnt}) b->release();
   for (auto* b : {&h->xsum, &h->msum, &h->half, &h->zt, &h->prod}) b->release();
@@ -422,46 +472,40 @@ static int snap_chunk(int n, int cap, bool adjoint_z, const SnapDev& S) {
   return std::min(n, ((n + chunks - 1) / chunks + 31) & ~31);
 }
 
-// Atoms per tile of k_snap_y.  A tile costs the same whatever its lanes hold,
-// so 32 atoms where the tiles (and their tasks, split over up to four CTAs)
-// fill the 152 SMs, fewer atoms with the rows shared by lane groups (0.89,
-// 0.73, 0.53 of the lanes' work useful at 16, 8, 4) where they would not.
-static int snap_tile_atoms(const SnapDev& S, int n, bool fp64, bool keep) {
-  int ta = 32;
-  if (!keep)
-    while (ta > 4 && (n + ta - 1) / ta * 4 < 152) ta /= 2;
-  // mixed form: two atoms per lane once the tiles' splits still fill the SMs
-  if (!fp64 && S.twojmax <= 9 && (n + 63) / 64 * 4 >= 2 * 152) ta = 64;
-  while (ta > 1 && snap_y_smem(S, ta, fp64) > kMaxDynSmem) ta /= 2;
-  return ta;
-}
-// CTAs that share a tile's tasks (up to four), for the smallest product of waves
-// and time per CTA.  FP64: the SM issues one instruction per 19 cycles, a single
-// warp one per 64.  Mixed: the busiest of the CTA's warps when each takes the
-// next longest task (more CTAs than tasks per warp leave warps idle: two
-// atoms per lane, 128,000 atoms, 2.18 ms with four CTAs a tile, 1.25 with one).
-static int snap_tile_split(const SnapTables& tab, int tiles, bool fp64, int ta) {
-  const int resident = fp64 || ta == 64 ? 1 : 2, warps = sy32_threads(ta == 64 ? 2 : 1) / 32;
-  int best = 1;
-  double best_cost = 1e300;
-  for (int k = 1; k <= 4; ++k) {
-    double cta = 0.0;
-    for (int s = 0; s < k; ++s) {
-      double sum = 0.0, longest = 0.0;
-      std::vector<double> load(size_t(warps), 0.0);
-      for (size_t t = size_t(s); t < tab.cost.size(); t += size_t(k)) {
-        const double c = double(tab.cost[t]);
-        sum += c;
-        longest = std::max(longest, c);
-        *std::min_element(load.begin(), load.end()) += c;
-      }
-      cta = std::max(cta, fp64 ? std::max(19.0 * sum, 64.0 * longest) : *std::max_element(load.begin(), load.end()));
+// Atoms per tile of k_snap_y and CTAs that share a tile's tasks: the smallest
+// product of waves over the 152 SMs and time per CTA.  A tile costs the same
+// whatever its lanes hold; with fewer atoms than lanes the lane groups share a
+// record's products (0.89, 0.73, 0.53 of the lanes' work useful at 16, 8, 4
+// atoms).  FP64: the SM issues one instruction per 19 cycles, a single warp one
+// per 64.  Mixed: the busiest of the CTA's warps when each takes the next
+// longest task (more CTAs than tasks per warp leave warps idle).
+struct SnapTiling {
+  int ta, nsplit;
+};
+static SnapTiling snap_tiling(const SnapDev& S, const SnapTables& tab, int n, bool fp64, bool keep) {
+  // mixed form: two atoms per lane once the tiles' splits fill the SMs
+  if (!fp64 && S.twojmax <= 9 && (n + 63) / 64 * 4 >= 2 * 152 && snap_y_smem(S, 64, fp64) <= kMaxDynSmem) {
+    const long long tiles = (n + 63) / 64;
+    SnapTiling best{64, 1};
+    double best_cost = 1e300;
+    for (int k = 1; k <= ZS_SPLIT; ++k) {
+      const double cost = double((tiles * k + 151) / 152) * (tab.cta32[1][k - 1] + 1000.0);
+      if (cost < best_cost) best.nsplit = k, best_cost = cost;
     }
-    const long long ctas = (long long)tiles * k, wave = 152LL * resident;
-    const double cost = double((ctas + wave - 1) / wave) * cta;
-    if (cost < best_cost) {
-      best = k;
-      best_cost = cost;
+    return best;
+  }
+  SnapTiling best{0, 1};
+  double best_cost = 1e300;
+  const double lanes[6] = {0.2, 0.2, 0.236, 0.342, 0.562, 1.0};  // cost of a tile of 1, 2, 4 .. 32 atoms
+  for (int l = 5; l >= 0; --l) {
+    const int ta = 1 << l;
+    if (snap_y_smem(S, ta, fp64) > kMaxDynSmem) continue;
+    if (best.ta != 0 && (keep || ta < 4)) break;
+    const long long tiles = (n + ta - 1) / ta, wave = 152LL * (fp64 ? 1 : 2);
+    for (int k = 1; k <= ZS_SPLIT; ++k) {
+      const double cta = fp64 ? tab.cta64[k - 1] * lanes[l] + 4000.0 : tab.cta32[0][k - 1] * lanes[l] + 1000.0;
+      const double cost = double((tiles * k + wave - 1) / wave) * cta;
+      if (cost < best_cost) best = SnapTiling{ta, k}, best_cost = cost;
     }
   }
   return best;
@@ -490,10 +534,11 @@ static SnapArgs snap_args(Ctx& c, SnapHost* h, int first, int n, bool fp64, bool
   A.pr = h->pr_f.p;
   A.pj = h->pj.p;
   A.cnt = h->cnt.p;
-  A.ta = snap_tile_atoms(S, c.N_local, fp64, keep);
+  const SnapTiling tl = snap_tiling(S, *h->tab, n, fp64, keep);
+  A.ta = tl.ta;
+  A.nsplit = tl.nsplit;
   const int tiles = (n + A.ta - 1) / A.ta;
-  A.nsplit = snap_tile_split(*h->tab, tiles, fp64, A.ta);
-  h->Y.reserve((size_t(tiles) * 4 * S.ne * A.ta * real + 7) / 8, c.stream);
+  h->Y.reserve((size_t(tiles) * 2 * S.ny * A.ta * real + 7) / 8, c.stream);
   A.Y = h->Y.p;
   A.f = c.f.p;
   A.tmask = h->tmask.p;
@@ -721,6 +766,7 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   S.ntask = int(tab.task.size());
   S.nz = tab.nz;
   S.nh = tab.nh;
+  S.ny = tab.ny;
   for (int k = 0; k < S.ncoeff; ++k) {
     const int j1 = idx3[3 * k], j2 = idx3[3 * k + 1], j = idx3[3 * k + 2];
     h->k_t1.push_back(find_full(j1, j2, j));
@@ -764,6 +810,7 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   upload(c, h->zt, tab.zt);
   upload(c, h->tmask, tab.tmask);
   upload(c, h->hfull, tab.hfull);
+  upload(c, h->ysrc, tab.ysrc);
   upload(c, h->prod, tab.prod);
   upload(c, h->zc, tab.zc);
   upload(c, h->grp, tab.grp);
@@ -787,6 +834,7 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   S.zt0 = h->zt0.p;
   S.zt = h->zt.p;
   S.hfull = h->hfull.p;
+  S.ysrc = h->ysrc.p;
   S.prod = h->prod.p;
   S.zc = h->zc.p;
   S.grp = h->grp.p;

@@ -53,7 +53,7 @@ struct Cplx {
 
 // One (T, q, k) entry
 struct Entry {
-  double N, invN;  // the elements' norm and its inverse
+  double N;        // the elements' norm
   double A, B;     // P_{k+1} = (x - A) P_k - B P_{k-1}
   int xo;          // first of its real sums: p u, [q>0] r u, [T>0] p v, [q>0, T>0] r v
   int mo;          // its coefficients of x^0 .. x^k, times N (SnapDev::mono)
@@ -67,10 +67,11 @@ struct ZRec {
   short nj, d;         // number of j, the highest first; its distance from the task's highest j over 2
   int t0, z0;          // triple of the highest j; first kept Z
 };
+// One (T, q), one sign of T, and some of its records
 struct ZTask {
-  int T, q, rec0, rec1, rec2;  // records of the +T elements [rec0, rec1), of the -T ones [rec1, rec2)
-  int y0, kmax;                // first entry, last k
-  int grp0, grp1, grp2, s0;    // FP32: groups, +T and -T; first word of the stream
+  int rec0, rec1;      // records [rec0, rec1)
+  int y0, kmax;        // its part of Y: slots y0 .. y0 + kmax, in the order of k
+  int grp0, grp1, s0;  // FP32: groups [grp0, grp1), first word of the stream
 };
 // FP32: a task's products of equal nj and d, whatever their (j1, j2)
 struct ZGrp {
@@ -114,6 +115,8 @@ struct SnapDev {
   const int4* hfull;   // per half-grid element: its full-grid index, its inversion's, sign
   const int* zt0;
   const int2* zt;
+  int ny;              // slots of Y
+  const int4* ysrc;    // per half-grid element: first slot, slots between parts, parts
 };
 
 // ---- pair fields, one array each of stride `np` (pairs of the chunk)
@@ -137,7 +140,7 @@ struct SnapArgs {
   int* pj;             // n cap
   int* cnt;            // n
   void* U;             // n x nh complex, force type
-  void* Y;             // tiles x (4 ne) x TA, force type
+  void* Y;             // tiles x ny x 2 x TA, force type: parts of the Y of half-grid elements
   int ta, nsplit;      // atoms per tile, CTAs per tile
   double* zkeep;       // tiles x nz x 32 complex, or null
   double* f;
@@ -521,14 +524,20 @@ __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
 
 // ------------------------------------------------------------------- Z, Y
 // Lanes = atoms of a tile (ta of them; for ta < 32 the 32 / ta lane groups
-// share a record's products), warps = tasks.  A task is one (T, q): it owns
+// share a record's products), warps = tasks.  One (T, q) and sign of T owns
 // Y_j(m, m') at (2m, 2m') = (-q -+ T, -q +- T) for every j, because Z_j at one
 // (m, m') comes from products U_j1(m1, m1') U_j2(m - m1, m' - m1') that do not
 // depend on j: each product is formed once (4 operations) and weighted by both
 // Clebsch-Gordan factors for every j (2 each), where one Z at a time took 6 for
 // each (compute_zi, sna_impl.hpp:197-283); for j1 = j2 the two orders of a pair
 // of elements are one product.  The loops run over product lists, uniform over
-// the lanes.  Y_j = sum cY Z_j stays in registers; cY folds the linear
+// the lanes.  The longest lists are cut (SnapTables): each task writes its part
+// of Y, and Y's readers sum the parts in order, so that a CTA's last warps end
+// together and a tile can be shared by many CTAs (a warp alone issues one FP64
+// instruction per 64 cycles, four or more share one per 19; 8,160 atoms, FP64:
+// 2.49 ms with whole (T, q) as tasks, 1.88 with parts of 1/48, 2.15 and 1.95
+// with 1/24 and 1/96; 64 atoms at twojmax 6: 52 -> 22 us).  Y_j = sum cY Z_j stays in
+// registers; cY folds the linear
 // coefficients with the (j+1)/(j1+1), (j+1)/(j2+1) weights of compute_dbidrj's
 // three terms (sna_impl.hpp:330-539).
 template <int NJ>
@@ -601,40 +610,30 @@ __device__ __forceinline__ void z_add(const ZRec& z, const SnapDev& S, const Cpl
   });
 }
 
-// E = 2N (Y+ + (-1)^T Y-), O = 2N (Y+ - (-1)^T Y-) of a task's entries (p: +T,
-// m: -T, highest j first): with a^q and w b^T = u + i v, twice the real part of
-// conj(U) Y over both signs of T is u Re(a^q E) + v Im(a^q O) times P_k
+// a task's part of Y (y[0]: the highest j) to its slots
 template <typename R, int NM>
-__device__ __forceinline__ void y_store(const SnapDev& S, const ZTask& K, const Cplx<R>* yp, const Cplx<R>* ym, R* Yt,
-                                        int ta) {
+__device__ __forceinline__ void y_store(const ZTask& K, const Cplx<R>* y, R* Yt, int ta) {
 #pragma unroll
   for (int h = 0; h < NM; ++h)
     if (h <= K.kmax) {
-      const int k = K.kmax - h;
-      const R N = R(S.ent[K.y0 + k].N), N2 = N + N;
-      R er, ei, orr, oi;
-      const Cplx<R> p = yp[h], m = ym[h];
-      if (K.q == 0) {  // the -T element is the inversion of the +T one
-        er = (K.T ? N2 : N) * p.r;
-        oi = K.T ? N2 * p.i : R(0);
-        ei = orr = R(0);
-      } else if (K.T == 0) {
-        er = N2 * p.r;
-        ei = N2 * p.i;
-        orr = oi = R(0);
-      } else {
-        const R sg = K.T & 1 ? R(-1) : R(1);
-        er = N2 * fma(sg, m.r, p.r);
-        ei = N2 * fma(sg, m.i, p.i);
-        orr = N2 * fma(-sg, m.r, p.r);
-        oi = N2 * fma(-sg, m.i, p.i);
-      }
-      R* o = Yt + size_t(4) * (K.y0 + k) * ta;
-      o[0] = er;
-      o[ta] = ei;
-      o[2 * ta] = orr;
-      o[3 * ta] = oi;
+      R* o = Yt + size_t(2) * (K.y0 + K.kmax - h) * ta;
+      o[0] = y[h].r;
+      o[ta] = y[h].i;
     }
+}
+
+// Y of half-grid element h (y: the atom's column of its tile), parts in order
+template <typename R>
+__device__ __forceinline__ Cplx<R> y_element(const SnapDev& S, int h, const R* y, int ta) {
+  const int4 s = __ldg(S.ysrc + h);
+  const R* p = y + size_t(2) * s.x * ta;
+  Cplx<R> t{p[0], p[ta]};
+  for (int k = 1; k < s.z; ++k) {
+    p += size_t(2) * s.y * ta;
+    t.r += p[0];
+    t.i += p[ta];
+  }
+  return t;
 }
 
 // the tile's U, both halves of the grid, as [element][atom] with rows of ta + 1
@@ -667,7 +666,7 @@ __global__ void __launch_bounds__(SY_THREADS) k_snap_y(SnapArgs A) {
   __syncthreads();
   const int ei = al < A.n ? S.map[A.type[A.first + al]] : 0;
   const double* cY = S.cY + size_t(ei) * S.nfull;
-  double* Yt = static_cast<double*>(A.Y) + size_t(tile) * 4 * S.ne * ta + at;
+  double* Yt = static_cast<double*>(A.Y) + size_t(tile) * 2 * S.ny * ta + at;
   Cplx<double>* zk = reinterpret_cast<Cplx<double>*>(A.zkeep) + (KEEP ? size_t(al >> 5) * S.nz * 32 + (al & 31) : 0);
   const Cplx<double>* Ua = U + at;
   while (true) {
@@ -676,19 +675,11 @@ __global__ void __launch_bounds__(SY_THREADS) k_snap_y(SnapArgs A) {
     t = __shfl_sync(FULL_MASK, t, 0) * A.nsplit + split;  // tasks longest first
     if (t >= S.ntask) break;
     const ZTask K = S.task[t];
-    Cplx<double> y[NM], yp[NM];  // Y of the -T elements (first: +T), of the +T elements
+    Cplx<double> y[NM];
 #pragma unroll
     for (int k = 0; k < NM; ++k) y[k] = Cplx<double>{0.0, 0.0};
 #pragma unroll 1
-    for (int r = K.rec0; r <= K.rec2; ++r) {
-      if (r == K.rec1) {
-#pragma unroll
-        for (int k = 0; k < NM; ++k) {
-          yp[k] = y[k];
-          y[k] = Cplx<double>{0.0, 0.0};
-        }
-      }
-      if (r == K.rec2) break;
+    for (int r = K.rec0; r < K.rec1; ++r) {
       const ZRec z = S.rec[r];
       switch (z.nj) {  // uniform
         case 1: z_add<NM, 1, KEEP>(z, S, Ua, str, cY, sub, nsub, y, zk); break;
@@ -707,11 +698,8 @@ __global__ void __launch_bounds__(SY_THREADS) k_snap_y(SnapArgs A) {
     // the lane groups' parts (KEEP: every Z was completed already)
     for (int o = ta; o < 32 && !KEEP; o <<= 1)
 #pragma unroll
-      for (int k = 0; k < NM; ++k) {
-        shfl_add(yp[k], o);
-        shfl_add(y[k], o);
-      }
-    if (sub == 0) y_store<double, NM>(S, K, yp, y, Yt, ta);
+      for (int k = 0; k < NM; ++k) shfl_add(y[k], o);
+    if (sub == 0) y_store<double, NM>(K, y, Yt, ta);
   }
 }
 
@@ -827,7 +815,7 @@ __global__ void __launch_bounds__(sy32_threads(NA), NA == 2 ? 1 : 2) k_snap_y32(
     const int al = tile * ta + at + 32 * a;
     mine[a] = sub == 0 && al < A.n && S.map[A.type[A.first + al]] == elem;
   }
-  float* Yt = static_cast<float*>(A.Y) + size_t(tile) * 4 * S.ne * ta + at;
+  float* Yt = static_cast<float*>(A.Y) + size_t(tile) * 2 * S.ny * ta + at;
   const Cplx<float>* Ua = U + at;
   ZStream st;
   st.buf = reinterpret_cast<uint4*>(sy_smem + ((sizeof(Cplx<float>) * size_t(S.nuf) * str + 15) & ~size_t(15))) +
@@ -840,23 +828,13 @@ __global__ void __launch_bounds__(sy32_threads(NA), NA == 2 ? 1 : 2) k_snap_y32(
     if (t >= S.ntask) break;
     const ZTask K = S.task[t];
     st.begin(zs, K.s0, lane);
-    Cplx<float> y[NA][NM], yp[NA][NM];
+    Cplx<float> y[NA][NM];
 #pragma unroll
     for (int a = 0; a < NA; ++a)
 #pragma unroll
       for (int k = 0; k < NM; ++k) y[a][k] = Cplx<float>{0.f, 0.f};
 #pragma unroll 1
-    for (int g = K.grp0; g <= K.grp2; ++g) {
-      if (g == K.grp1) {
-#pragma unroll
-        for (int a = 0; a < NA; ++a)
-#pragma unroll
-          for (int k = 0; k < NM; ++k) {
-            yp[a][k] = y[a][k];
-            y[a][k] = Cplx<float>{0.f, 0.f};
-          }
-      }
-      if (g == K.grp2) break;
+    for (int g = K.grp0; g < K.grp1; ++g) {
       const ZGrp G = S.grp[g];
       switch (G.nj) {  // uniform
         case 1: zg_add<NM, 1, NA>(G, st, Ua, str, sub, nsub, y); break;
@@ -874,18 +852,18 @@ __global__ void __launch_bounds__(sy32_threads(NA), NA == 2 ? 1 : 2) k_snap_y32(
     }
     for (int o = ta; o < 32; o <<= 1)  // the lane groups' parts
 #pragma unroll
-      for (int k = 0; k < NM; ++k) {
-        shfl_add(yp[0][k], o);
-        shfl_add(y[0][k], o);
-      }
+      for (int k = 0; k < NM; ++k) shfl_add(y[0][k], o);
 #pragma unroll
     for (int a = 0; a < NA; ++a)
-      if (mine[a]) y_store<float, NM>(S, K, yp[a], y[a], Yt + 32 * a, ta);
+      if (mine[a]) y_store<float, NM>(K, y[a], Yt + 32 * a, ta);
   }
 }
 
 // ------------------------------------------------------------- pair forces
-// Lanes = pairs, pooled over the CTA's atoms.  Phi = sum_j 2 sum_half w
+// Lanes = pairs, pooled over the CTA's atoms.  With a^q and w b^T = u + i v, and
+// E = 2N (Y+ + (-1)^T Y-), O = 2N (Y+ - (-1)^T Y-) of an entry (formed when Y is
+// loaded), twice the real part of conj(U) Y over both signs of T is
+// u Re(a^q E) + v Im(a^q O) times P_k.  So Phi = sum_j 2 sum_half w
 // Re(conj(U_j) Y_j) of one neighbour is sum_T u_T Re(Eh_T) + v_T Im(Oh_T) with
 // Eh_T = sum_q a^q sum_k E P_k and Oh_T likewise, and the pair force needs only
 // Phi and its gradient in (a, b):
@@ -912,9 +890,27 @@ __global__ void __launch_bounds__(SF_THREADS) k_snap_force(SnapArgs A) {
   R* ys = reinterpret_cast<R*>(sf_smem);                                   // apc x ny
   double* fs = reinterpret_cast<double*>(sf_smem + ((size_t(apc) * ny * sizeof(R) + 15) & ~size_t(15)));  // blockDim x 3
   const int ta = A.ta;
-  for (int k = tid; k < ny * na; k += blockDim.x) {
+  for (int k = tid; k < S.ne * na; k += blockDim.x) {
     const int e = k / na, a = k - e * na, ga = a0 + a;
-    ys[a * ny + e] = static_cast<const R*>(A.Y)[(size_t(ga / ta) * ny + e) * ta + ga % ta];
+    const R* Y = static_cast<const R*>(A.Y) + size_t(ga / ta) * 2 * S.ny * ta + ga % ta;
+    const int2 h = __ldg(S.half + e);
+    const R N2 = R(2.0 * S.ent[e].N);
+    const Cplx<R> p = y_element(S, h.x, Y, ta);
+    R* o = ys + a * ny + 4 * e;
+    if (h.y >= 0) {
+      const Cplx<R> m = y_element(S, h.y, Y, ta);
+      const R sg = __ldg(S.hfull + h.x).z > 0 ? R(1) : R(-1);
+      o[0] = N2 * fma(sg, m.r, p.r);
+      o[1] = N2 * fma(sg, m.i, p.i);
+      o[2] = N2 * fma(-sg, m.r, p.r);
+      o[3] = N2 * fma(-sg, m.i, p.i);
+    } else {  // q = 0 (the -T element is the inversion of the +T one), T = 0, or both
+      const int T = S.ent[e].T, q = S.ent[e].q;
+      o[0] = (T + q > 0 ? N2 : R(0.5) * N2) * p.r;
+      o[1] = q > 0 ? N2 * p.i : R(0);
+      o[2] = R(0);
+      o[3] = T > 0 ? N2 * p.i : R(0);
+    }
   }
   if (tid == 0) {
     int o = 0;
@@ -1102,29 +1098,15 @@ static __global__ void __launch_bounds__(128) k_snap_energy(SnapArgs A) {
   const SnapDev& S = A.S;
   const int lane = threadIdx.x & 31, al = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (al >= A.n) return;
-  const int ta = A.ta, ny = 4 * S.ne;
-  const double* Y = static_cast<const double*>(A.Y) + size_t(al / ta) * ny * ta + al % ta;
+  const int ta = A.ta;
+  const double* Y = static_cast<const double*>(A.Y) + size_t(al / ta) * 2 * S.ny * ta + al % ta;
   const Cplx<double>* U = static_cast<const Cplx<double>*>(A.U) + size_t(al) * S.nh;
   double acc = 0.0;
-  for (int e = lane; e < S.ne; e += 32) {
-    // U+ + (-1)^T U- = 2N (p u - i r u), U+ - (-1)^T U- = 2N (r v + i p v)
-    const Entry& E = S.ent[e];
-    const int2 h = S.half[e];
-    const double* y = Y + size_t(4) * e * ta;
-    const Cplx<double> u = U[h.x];
-    if (h.y >= 0) {
-      const double sg = E.T & 1 ? -1.0 : 1.0;
-      const Cplx<double> m = U[h.y];
-      acc += 0.5 * E.invN *
-             (fma(y[0], fma(sg, m.r, u.r), y[ta] * fma(sg, m.i, u.i)) +
-              fma(y[2 * ta], fma(-sg, m.r, u.r), y[3 * ta] * fma(-sg, m.i, u.i)));
-    } else if (E.T == 0) {
-      acc += E.invN * fma(y[0], u.r, y[ta] * u.i);
-    } else {
-      acc += E.invN * fma(y[0], u.r, y[3 * ta] * u.i);
-    }
+  for (int h = lane; h < S.nh; h += 32) {
+    const Cplx<double> y = y_element(S, h, Y, ta), u = U[h];
+    const int4 f = __ldg(S.hfull + h);
+    acc += f.x == f.y ? 0.5 * (y.r * u.r) : fma(y.r, u.r, y.i * u.i);
   }
-  acc *= 0.5;
   const size_t np = size_t(A.n) * A.cap;
   const double* ep = A.pd + PD_EP * np + size_t(al) * A.cap;
   const int n = A.cnt[al];
