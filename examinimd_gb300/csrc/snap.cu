@@ -33,9 +33,10 @@ struct SnapHost {
   DevBuf<ZRec> rec;
   DevBuf<ZGrp> grp;
   DevBuf<int> e0, map, zt0, tmask, eord;
-  DevBuf<int2> xsum, msum, half, zt, prod;
+  DevBuf<int2> xsum, ucol, half, zt, prod;
+  DevBuf<float2> mono;
   DevBuf<int4> hfull, ysrc;
-  DevBuf<double> zc, mono, cY, AB, beta0, wjelem, pr;
+  DevBuf<double> zc, cY, AB, beta0, wjelem, pr;
   DevBuf<float> AB_f;
   DevBuf<uint4> zs;
   // per-chunk work arrays
@@ -109,11 +110,12 @@ constexpr int ZS_SPLIT = 16;        // CTAs that may share a tile
 struct SnapTables {
   std::vector<Entry> ent;
   std::vector<int> e0, zt0, tmask, eord;
-  std::vector<int2> xsum, msum, half, zt, prod;
+  std::vector<int2> xsum, ucol, half, zt, prod;
+  std::vector<float2> mono;
   std::vector<int4> hfull, ysrc;
   std::vector<ZTask> task;
   std::vector<ZRec> rec;
-  std::vector<double> zc, AB, mono;
+  std::vector<double> zc, AB;
   std::vector<ZGrp> grp;
   std::vector<unsigned> words;  // the FP32 stream without its coefficients
   struct Src {
@@ -131,7 +133,7 @@ struct SnapTables {
     // entries, real sums and their table columns (k_snap_u: powers of a, of b,
     // then the products in (T, q, k) order)
     e0.assign(size_t(L) * L, -1);
-    int col = 4 * L, mcol = 4 * L;
+    int col = 4 * L, col32 = L;
     for (int T = 0; T <= J; ++T) {
       for (int q = 0; q <= J - T; ++q) {
         e0[size_t(T) * L + q] = int(ent.size());
@@ -155,14 +157,13 @@ struct SnapTables {
           E.xo = int(xsum.size());
           const int cu = k == 0 ? 2 * L + 2 * T : col, cv = cu + 1, cp = 2 * q, cr = 2 * q + 1;
           if (k > 0) col += T > 0 ? 2 : 1;
-          const int mu = k == 0 ? cu : mcol + (k - 1) * (T > 0 ? 2 : 1), mv = mu + 1;
           xsum.push_back(int2{cp, cu});
-          msum.push_back(int2{cp, mu});
-          if (q > 0) xsum.push_back(int2{cr, cu}), msum.push_back(int2{cr, mu});
-          if (T > 0) xsum.push_back(int2{cp, cv}), msum.push_back(int2{cp, mv});
-          if (q > 0 && T > 0) xsum.push_back(int2{cr, cv}), msum.push_back(int2{cr, mv});
+          if (q > 0) xsum.push_back(int2{cr, cu});
+          if (T > 0) xsum.push_back(int2{cp, cv});
+          if (q > 0 && T > 0) xsum.push_back(int2{cr, cv});
+          ucol.push_back(int2{q, col32 + k});
           E.mo = int(mono.size());
-          for (double c : pk) mono.push_back(E.N * c);
+          for (double c : pk) mono.push_back(float2{float(E.N * c), float(E.N * c - double(float(E.N * c)))});
           std::vector<double> pn(pk.size() + 1, 0.0);
           for (size_t l = 0; l < pk.size(); ++l) {
             pn[l + 1] += pk[l];
@@ -179,7 +180,7 @@ struct SnapTables {
           ent.push_back(E);
         }
       }
-      mcol += (T > 0 ? 2 : 1) * ((J - T) / 2);
+      col32 += (J - T) / 2 + 1;
     }
     for (int e = 0; e < int(ent.size()); ++e) eord.push_back(e);
     std::stable_sort(eord.begin(), eord.end(), [&](int x, int y) {
@@ -405,11 +406,12 @@ void free_snap(Ctx& c) {
   h->ysrc.release();
   h->zs.release();
   for (auto* b : {&h->e0, &h->map, &h->zt0, &h->tmask, &h->eord, &h->pj, &h->cnt}) b->release();
-  for (auto* b : {&h->xsum, &h->msum, &h->half, &h->zt, &h->prod}) b->release();
-  for (auto* b : {&h->zc, &h->mono, &h->cY, &h->AB, &h->beta0, &h->wjelem, &h->pr, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk,
+  for (auto* b : {&h->xsum, &h->ucol, &h->half, &h->zt, &h->prod}) b->release();
+  for (auto* b : {&h->zc, &h->cY, &h->AB, &h->beta0, &h->wjelem, &h->pr, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk,
                   &h->eatom, &h->adj, &h->adj_sum, &h->adj_g, &h->keep_u, &h->keep_z})
     b->release();
   h->AB_f.release();
+  h->mono.release();
   delete h;
   c.snap = nullptr;
 }
@@ -526,7 +528,7 @@ static SnapArgs snap_args(Ctx& c, SnapHost* h, int first, int n, bool fp64, bool
   A.cap = std::max(1, c.neigh_maxrow);
   A.rows = std::min(SP_ROWS, std::max(1, n / (152 * 8)));
   const size_t np = size_t(n) * A.cap;
-  h->pd.reserve(PD_N * np, c.stream);
+  h->pd.reserve((fp64 ? PD_N : PD_N32) * np, c.stream);
   h->pr_f.reserve(fp64 ? PF_N * np : (PR_N * np + 1) / 2, c.stream);
   h->pj.reserve(np, c.stream);
   h->cnt.reserve(size_t(n), c.stream);
@@ -554,7 +556,7 @@ static void snap_uy(Ctx& c, const SnapArgs& A, bool fp64) {
   }
   {
     TimedLaunch t(c, "snap_u");
-    if (fp64) launch_u<double>(A, c.stream);
+    if (fp64) launch_u(A, c.stream);
     else snap_mixed_u(A, c.stream);
   }
   TimedLaunch t(c, fp64 ? "snap_y_fp64" : "snap_y_mixed");
@@ -761,7 +763,7 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   S.ne = int(tab.ent.size());
   S.nx = int(tab.xsum.size());
   S.cols = su_cols(twojmax);
-  S.mcols = su_mcols(twojmax);
+  S.cols32 = su_cols32(twojmax);
   S.nuf = (twojmax + 1) * (twojmax + 2) * (2 * twojmax + 3) / 6;
   S.ntask = int(tab.task.size());
   S.nz = tab.nz;
@@ -802,7 +804,7 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   upload(c, h->rec, tab.rec);
   upload(c, h->e0, tab.e0);
   upload(c, h->xsum, tab.xsum);
-  upload(c, h->msum, tab.msum);
+  upload(c, h->ucol, tab.ucol);
   upload(c, h->mono, tab.mono);
   upload(c, h->eord, tab.eord);
   upload(c, h->half, tab.half);
@@ -827,7 +829,7 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   S.rec = h->rec.p;
   S.e0 = h->e0.p;
   S.xsum = h->xsum.p;
-  S.msum = h->msum.p;
+  S.ucol = h->ucol.p;
   S.mono = h->mono.p;
   S.eord = h->eord.p;
   S.half = h->half.p;

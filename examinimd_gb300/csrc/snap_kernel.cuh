@@ -16,8 +16,8 @@
 // Per force call, over chunks of atoms:
 //   k_snap_pairs  inside list and per-pair scalars (lanes = pairs)
 //   k_snap_u      U_tot = wself + sum over the neighbours of w_j sfac U, from the
-//                 four real products of conj(a)^q and b^T times P_k, FP64 in
-//                 both forms (one warp per atom; lanes = neighbours, then sums)
+//                 four real products of conj(a)^q and b^T times P_k (one warp per
+//                 atom; lanes = neighbours, then sums)
 //   k_snap_y      Z and Y (lanes = atoms, so the Clebsch-Gordan loops are
 //                 uniform and every operand load is coalesced)
 //   k_snap_force  pair forces (lanes = pairs): Phi = Re sum conj(U) Y and its
@@ -26,8 +26,9 @@
 // directional derivative of X) and k_snap_pq.
 //
 // Precision forms: FP64 (the drop-in; snap.cu, -fmad=false) and mixed
-// (snap_mixed.cu), where the pair scalars and X stay FP64 and k_snap_y and the
-// sums of k_snap_force run in FP32, with FP64 force sums.  The recurrences and
+// (snap_mixed.cu), where the pair scalars are FP64, the sums of U_tot are formed
+// from FP32 pairs of 48 bits and rounded to FP32, and k_snap_y and the sums of
+// k_snap_force run in FP32, with FP64 force sums.  The recurrences and
 // contractions use explicit fused multiply-adds in both forms.
 #pragma once
 #include <algorithm>
@@ -81,7 +82,7 @@ struct ZGrp {
 
 struct SnapDev {
   int twojmax, ne, nx, nuf;    // entries, real sums, elements of the full grid
-  int cols, mcols;             // columns of a neighbour's table (su_cols), of the mixed form's
+  int cols, cols32;            // columns of a neighbour's table (su_cols), of the mixed form's (su_cols32)
   int ntask, nfull, nz;        // Z tasks, (j1 >= j2, j) triples, kept Z values per atom
   int ncoeff, ncoeffall, nelem, ntypes;
   double rfac0, rmin0, cutsq, wself;
@@ -89,8 +90,8 @@ struct SnapDev {
   const Entry* ent;
   const int* e0;       // (J + 1) x (J + 1): first entry of (T, q)
   const int2* xsum;    // nx: the two factors of a sum in a neighbour's table (k_snap_u)
-  const int2* msum;    // the same in the mixed form's table
-  const double* mono;  // N P_k in powers of x
+  const int2* ucol;    // ne: the mixed form's two columns of an entry
+  const float2* mono;  // N P_k in powers of x, high and low part
   const int* eord;     // entries, highest k first
   const ZTask* task;
   const ZRec* rec;
@@ -120,11 +121,12 @@ struct SnapDev {
 };
 
 // ---- pair fields, one array each of stride `np` (pairs of the chunk)
-enum { PD_AR, PD_AI, PD_BR, PD_BI, PD_SF, PD_FX, PD_FY, PD_FZ, PD_EP, PD_N };  // FP64
-// force inputs, mixed form (FP32): a, b, sfac, dsfac, u, and the three numbers
-// da/dr and db/dr are made of; FP64 form: a and b as compute_duidrj rounds
+enum { PD_FX, PD_FY, PD_FZ, PD_N32, PD_AR = PD_N32, PD_AI, PD_BR, PD_BI, PD_SF, PD_EP, PD_N };  // FP64 (mixed form: PD_N32)
+// mixed form (FP32): a, b, sfac, dsfac, u, the three numbers da/dr and db/dr are
+// made of, and what the rounding of a, b and sfac left out; FP64 form: a and b as compute_duidrj rounds
 // them, dsfac, u and every derivative in the reference's operations
-enum { PR_AR, PR_AI, PR_BR, PR_BI, PR_DSF, PR_UX, PR_UY, PR_UZ, PR_SF, PR_C1, PR_GR, PR_R0, PR_N };
+enum { PR_AR, PR_AI, PR_BR, PR_BI, PR_DSF, PR_UX, PR_UY, PR_UZ, PR_SF, PR_C1, PR_GR, PR_R0,
+       PR_ARL, PR_AIL, PR_BRL, PR_BIL, PR_SFL, PR_N };
 enum { PF_DAR = PR_SF, PF_DAI = PF_DAR + 3, PF_DBR = PF_DAI + 3, PF_DBI = PF_DBR + 3, PF_N = PF_DBI + 3 };
 
 struct SnapArgs {
@@ -135,7 +137,7 @@ struct SnapArgs {
   int first, n;        // atoms [first, first + n) of this chunk
   int n_local, cap;    // owned atoms; pair slots per atom
   int rows;            // k_snap_pairs: atoms per warp
-  double* pd;          // PD_N x (n cap)
+  double* pd;          // PD_N or PD_N32 x (n cap)
   void* pr;            // PR_N x (n cap), force type (the FP64 form reads a, b and sfac from pd)
   int* pj;             // n cap
   int* cnt;            // n
@@ -242,6 +244,7 @@ __global__ void __launch_bounds__(64) k_snap_pairs(SnapArgs A) {
         q[PD_FY * np] = y * fr;
         q[PD_FZ * np] = z * fr;
         q[PD_EP * np] = in ? 1.25e5 / (r4 * r2) : 0.0;
+        q[PD_SF * np] = sf * wj;
       } else {
         // The same quantities in closed form, once, in FP64.  With s =
         // sin(theta0), c = cos(theta0): z0 = r c / s and r0inv = s / r, so
@@ -265,10 +268,6 @@ __global__ void __launch_bounds__(64) k_snap_pairs(SnapArgs A) {
           }
         }
         const double ar = in ? cs : 1.0, ai = -z * r0inv, br = y * r0inv, bi = -x * r0inv;
-        q[PD_AR * np] = ar;
-        q[PD_AI * np] = ai;
-        q[PD_BR * np] = br;
-        q[PD_BI * np] = bi;
         // the r^-12 repulsion's force stays FP64: its pair terms are of the size
         // of the net force and cancel in the sum over neighbours
         const double ri2 = rinv * rinv, ri4 = ri2 * ri2;
@@ -288,8 +287,13 @@ __global__ void __launch_bounds__(64) k_snap_pairs(SnapArgs A) {
         w[PR_C1 * np] = R(-sn * rscale0);
         w[PR_GR * np] = R(fma(cs, rscale0, -r0inv));
         w[PR_R0 * np] = R(r0inv);
+        auto rest = [](double v) { return R(v - double(R(v))); };
+        w[PR_ARL * np] = rest(ar);
+        w[PR_AIL * np] = rest(ai);
+        w[PR_BRL * np] = rest(br);
+        w[PR_BIL * np] = rest(bi);
+        w[PR_SFL * np] = rest(sf * wj);
       }
-      q[PD_SF * np] = sf * wj;
       A.pj[p] = j;
     }
     __syncwarp();
@@ -339,17 +343,14 @@ __global__ void __launch_bounds__(64) k_snap_pairs(SnapArgs A) {
 // polynomials go to the neighbour's row of a shared table.  Lanes = sums: each
 // of the nx real sums is p or r times one of those products over the
 // neighbours, one FP64 multiply-add per neighbour.  Then the half-grid
-// elements, once per atom, in the contraction's type.  Bound by the FP64 pipe.
+// elements, once per atom.  Bound by the FP64 pipe: about 240 instructions for
+// 32 neighbours' rows, nx / 32 for each neighbour, 530 per atom at twojmax 8 and
+// 26 neighbours.
 //
-// The FP64 form multiplies u and v by P_k(x), for every (T, q): about 240
-// instructions for 32 neighbours, nx / 32 for each neighbour, 530 per atom at
-// twojmax 8 and 26 neighbours.  The mixed form, which rounds U_tot to FP32
-// anyway, sums u x^k and v x^k, the same for every q, and combines the sums
-// into the polynomials' once per atom: the powers' rounding is amplified by the
-// polynomial's coefficients (16 at twojmax 8, 221 at 14: 5e-14), far inside
-// FP32's.
-// The table is half as wide, so that eleven warps share an SM instead of six.
-// Per 128,000 atoms: 4.98 ms with the polynomials in the row, 2.80 with powers.
+// The mixed form, which rounds U_tot to FP32 anyway, takes k_snap_u32
+// (snap_split.cuh): sums over u x^k and v x^k, the same for every q, combined into
+// the polynomials' once per atom.  Per 128,000 atoms: 4.98 ms as the FP64 form
+// does it, 2.80 with powers of x in FP64, 0.95 in FP32 pairs.
 inline int su_cols(int J) {  // p, r; u, v; u P_k, v P_k (k >= 1)
   int c = 2 * (J + 1) + 2 * (J + 1);
   for (int T = 0; T <= J; ++T)
@@ -357,14 +358,14 @@ inline int su_cols(int J) {  // p, r; u, v; u P_k, v P_k (k >= 1)
   return c | 1;  // odd: rows start in different banks
 }
 
-inline int su_mcols(int J) {  // p, r; u, v; u x^k, v x^k (1 <= k <= (J - T) / 2)
-  int c = 4 * (J + 1);
-  for (int T = 0; T <= J; ++T) c += (T ? 2 : 1) * ((J - T) / 2);
-  return c | 1;
+// float4 columns of a neighbour's row: (p, r) of a^q; (u x^k, v x^k) of w b^T
+inline int su_cols32(int J) {
+  int c = J + 1;
+  for (int T = 0; T <= J; ++T) c += (J - T) / 2 + 1;
+  return c | 1;  // odd: eight lanes' rows start in different banks
 }
 
-// the neighbour's table row: powers, polynomials (MONO: powers of x) and products
-template <bool MONO>
+// the neighbour's table row: powers, polynomials and products
 __device__ __forceinline__ void su_row(const SnapDev& S, double* t, double ar, double ai, double br, double bi,
                                        double w) {
   const int J = S.twojmax;
@@ -394,20 +395,6 @@ __device__ __forceinline__ void su_row(const SnapDev& S, double* t, double ar, d
     uT[2 * J + 1] = v;
   }
   const double x = fma(ar, ar, ai * ai) - fma(br, br, bi * bi);
-  if constexpr (MONO) {
-    for (int T = 0; T <= J; ++T) {
-      double uk = uT[2 * T], vk = uT[2 * T + 1];
-      for (int k = 1; k <= (J - T) / 2; ++k) {
-        uk *= x;
-        *prod++ = uk;
-        if (T > 0) {
-          vk *= x;
-          *prod++ = vk;
-        }
-      }
-    }
-    return;
-  }
   for (int T = 0; T <= J; ++T) {
     const double uu = uT[2 * T], vv = uT[2 * T + 1];
     for (int q = 0; q <= J - T - 2; ++q) {
@@ -428,60 +415,40 @@ __device__ __forceinline__ void su_row(const SnapDev& S, double* t, double ar, d
   }
 }
 
-// the half-grid elements of entry e from its real sums (MONO: sums over the
-// powers of x, one group per k): conj(a)^q b^T = (p u + r v) + i (p v - r u);
+// the half-grid elements of entry e from its real sums: conj(a)^q b^T = (p u + r v) + i (p v - r u);
 // for -T: (-1)^T ((p u - r v) - i (p v + r u)); N scales, the atom's own term
 // is 1 on the diagonal (T = 0)
-template <typename R, bool MONO>
-__device__ __forceinline__ void su_store(const SnapDev& S, int e, const double* x, double self, Cplx<R>* U) {
+__device__ __forceinline__ void su_store(const SnapDev& S, int e, const double* x, double self, Cplx<double>* U) {
   const Entry& E = S.ent[e];
   const bool hr = E.q > 0, hv = E.T > 0;
-  double pu, ru = 0.0, pv = 0.0, rv = 0.0;
-  if constexpr (MONO) {
-    const double* m = S.mono + E.mo;
-    const int k = (E.j - E.q - E.T) / 2, g = (hr ? 2 : 1) * (hv ? 2 : 1);
-    x += E.xo - k * g;  // the sums of x^0
-    pu = 0.0;
-    for (int l = 0; l <= k; ++l) {
-      const double c = __ldg(m + l);
-      const double* y = x + l * g;
-      pu = fma(c, *y++, pu);
-      if (hr) ru = fma(c, *y++, ru);
-      if (hv) pv = fma(c, *y++, pv);
-      if (hr && hv) rv = fma(c, *y, rv);
-    }
-  } else {
-    x += E.xo;
-    pu = E.N * *x++;
-    if (hr) ru = E.N * *x++;
-    if (hv) pv = E.N * *x++;
-    if (hr && hv) rv = E.N * *x;
-  }
+  x += E.xo;
+  double pu = E.N * *x++, ru = 0.0, pv = 0.0, rv = 0.0;
+  if (hr) ru = E.N * *x++;
+  if (hv) pv = E.N * *x++;
+  if (hr && hv) rv = E.N * *x;
   const int2 h = S.half[e];
-  U[h.x] = Cplx<R>{R((pu + rv) + (hv ? 0.0 : self)), R(pv - ru)};
+  U[h.x] = Cplx<double>{(pu + rv) + (hv ? 0.0 : self), pv - ru};
   if (h.y >= 0) {
     const double sg = E.T & 1 ? -1.0 : 1.0;
-    U[h.y] = Cplx<R>{R(sg * (pu - rv)), R(-sg * (pv + ru))};
+    U[h.y] = Cplx<double>{sg * (pu - rv), -sg * (pv + ru)};
   }
 }
 
-template <typename R>
-__global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
-  constexpr bool kMono = sizeof(R) == sizeof(float);
+static __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
   const SnapDev& S = A.S;
   extern __shared__ __align__(16) double su_smem[];
   double* xs = su_smem;                       // nx sums
   double* tab = su_smem + ((S.nx + 1) & ~1);  // 32 rows
   const int al = blockIdx.x, lane = threadIdx.x;
-  const int cols = kMono ? S.mcols : S.cols, n = A.cnt[al];
-  const int2* __restrict__ xsum = kMono ? S.msum : S.xsum;
+  const int cols = S.cols, n = A.cnt[al];
+  const int2* __restrict__ xsum = S.xsum;
   const size_t np = size_t(A.n) * A.cap;
   const double* pd = A.pd + size_t(al) * A.cap;
   for (int n0 = 0; n0 < max(n, 1); n0 += 32) {
     const int m = min(32, n - n0);
     if (lane < m) {
       const double* q = pd + n0 + lane;
-      su_row<kMono>(S, tab + lane * cols, q[PD_AR * np], q[PD_AI * np], q[PD_BR * np], q[PD_BI * np], q[PD_SF * np]);
+      su_row(S, tab + lane * cols, q[PD_AR * np], q[PD_AI * np], q[PD_BR * np], q[PD_BI * np], q[PD_SF * np]);
     }
     __syncwarp();
     for (int r0 = 0; r0 < S.nx; r0 += 96) {  // three sums per lane at once
@@ -518,8 +485,8 @@ __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
     }
     __syncwarp();
   }
-  Cplx<R>* U = static_cast<Cplx<R>*>(A.U) + size_t(al) * S.nh;
-  for (int e = lane; e < S.ne; e += 32) su_store<R, kMono>(S, __ldg(S.eord + e), xs, S.wself, U);
+  Cplx<double>* U = static_cast<Cplx<double>*>(A.U) + size_t(al) * S.nh;
+  for (int e = lane; e < S.ne; e += 32) su_store(S, e, xs, S.wself, U);
 }
 
 // ------------------------------------------------------------------- Z, Y
@@ -1228,7 +1195,7 @@ static __global__ void __launch_bounds__(32) k_snap_dt(SnapArgs A) {
     }
     __syncwarp();
   }
-  for (int e = lane; e < S.ne; e += 32) su_store<double, false>(S, e, xs, 0.0, A.D + size_t(al) * S.nh);
+  for (int e = lane; e < S.ne; e += 32) su_store(S, e, xs, 0.0, A.D + size_t(al) * S.nh);
 }
 
 // half-grid elements of U and D, weighted (2, or 1 for the self-inverse ones,
@@ -1306,11 +1273,10 @@ void launch_y32(const SnapArgs& A, cudaStream_t s) {
   }
 }
 
-template <typename R>
-void launch_u(const SnapArgs& A, cudaStream_t s) {
-  const size_t smem = sizeof(double) * (size_t((A.S.nx + 1) & ~1) + 32 * size_t(sizeof(R) == 4 ? A.S.mcols : A.S.cols));
-  allow_dyn_smem(k_snap_u<R>);
-  k_snap_u<R><<<A.n, 32, smem, s>>>(A);
+inline void launch_u(const SnapArgs& A, cudaStream_t s) {
+  const size_t smem = sizeof(double) * (size_t((A.S.nx + 1) & ~1) + 32 * size_t(A.S.cols));
+  allow_dyn_smem(k_snap_u);
+  k_snap_u<<<A.n, 32, smem, s>>>(A);
   EMD_CHECK_LAUNCH();
 }
 

@@ -1,8 +1,9 @@
-// The mixed form's SNAP kernels (snap_kernel.cuh): pair scalars and U_tot
-// in FP64, Z, Y and the pair forces in FP32.  Compiled apart from snap.cu so
+// The mixed form's SNAP kernels (snap_kernel.cuh, snap_split.cuh): pair scalars in
+// FP64, U_tot from FP32 pairs, Z, Y and the pair forces in FP32.  Compiled apart from snap.cu so
 // that the pair scalars may use fused multiply-adds; the FP64 drop-in keeps
 // -fmad=false.
 #include "snap_kernel.cuh"
+#include "snap_split.cuh"
 
 namespace emd {
 
@@ -10,7 +11,7 @@ using namespace snapk;
 
 void snap_mixed_pairs(const SnapArgs& A, cudaStream_t s) { launch_pairs<float>(A, s); }
 
-void snap_mixed_u(const SnapArgs& A, cudaStream_t s) { launch_u<float>(A, s); }
+void snap_mixed_u(const SnapArgs& A, cudaStream_t s) { launch_u32(A, s); }
 
 void snap_mixed_y(const SnapArgs& A, cudaStream_t s) {
   if (A.S.twojmax > 9) {

@@ -1,0 +1,211 @@
+// U_tot of the SNAP mixed form from FP32 pairs (high and low part, 48 bits):
+// the sums of k_snap_u on the FP32 pipe, which issues 76 times as many lane
+// operations as the FP64 one here.  U_tot is rounded to FP32 afterwards, so what
+// counts is what the sums add to that rounding: at most 1e-12 of the neighbours'
+// total weight for 26 neighbours (5e-8 is the rounding; 1 in 2,500 elements comes
+// out one FP32 step from where sums in FP64 round to), times the polynomials'
+// coefficients (16 at twojmax 8).
+#pragma once
+
+namespace emd {
+namespace snapk {
+
+struct F2 {
+  float h, l;
+};
+
+// plain roundings, whatever the compiler may fuse
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float sub_rn(float a, float b) { return __fsub_rn(a, b); }
+
+// h + l renormalised, |h| >= |l| or h = 0
+__device__ __forceinline__ F2 f2_norm(float h, float l) {
+  const float s = add_rn(h, l);
+  return F2{s, sub_rn(l, sub_rn(s, h))};
+}
+
+// 1.5 times a power of two at least four times as large as b: sums below 2 b in
+// magnitude leave it within one binade
+__device__ __forceinline__ float f2_base(float b) {
+  const unsigned e = min(max((__float_as_uint(b) >> 23) & 0xffu, 67u), 250u) + 2u;
+  return __uint_as_float((e << 23) | 0x400000u);
+}
+
+// Sum of products on the grid of a base: s = base + the products rounded to the
+// base's last place one after another, c = what that left out, which is exact
+// (the difference of two neighbouring s and the product less it), plus the
+// cross terms.  Six operations a product.
+struct F2Sum {
+  float s, c;
+  __device__ __forceinline__ void add(F2 a, F2 b) {
+    const float t = fmaf(a.h, b.h, s);
+    const float r = fmaf(a.h, b.h, -sub_rn(t, s));
+    c = fmaf(a.h, b.l, c);
+    c = fmaf(a.l, b.h, c);
+    c = add_rn(c, r);
+    s = t;
+  }
+  __device__ __forceinline__ F2 value(float base) const { return f2_norm(sub_rn(s, base), c); }
+};
+
+__device__ __forceinline__ void su_row32(int J, float4* t, F2 ar, F2 ai, F2 br, F2 bi, F2 w) {
+  const F2 nai{-ai.h, -ai.l}, nbi{-bi.h, -bi.l};
+  const float one = f2_base(1.f), wb = f2_base(fabsf(w.h));
+  F2 x;
+  {
+    F2Sum s{one, 0.f};
+    s.add(ar, ar);
+    s.add(ai, ai);
+    s.add(F2{-br.h, -br.l}, br);
+    s.add(nbi, bi);
+    x = s.value(one);
+  }
+  F2 p{1.f, 0.f}, r{0.f, 0.f}, u = w, v{0.f, 0.f};
+  float4* col = t + J + 1;
+#pragma unroll 1
+  for (int q = 0; q <= J; ++q) {
+    t[q] = float4{p.h, p.l, r.h, r.l};
+    F2 uk = u, vk = v;
+    *col++ = float4{uk.h, uk.l, vk.h, vk.l};
+#pragma unroll 1
+    for (int k = 1; k <= (J - q) / 2; ++k) {
+      F2Sum su{wb, 0.f}, sv{wb, 0.f};
+      su.add(uk, x);
+      sv.add(vk, x);
+      uk = su.value(wb);
+      vk = sv.value(wb);
+      *col++ = float4{uk.h, uk.l, vk.h, vk.l};
+    }
+    F2Sum pn{one, 0.f}, rn{one, 0.f}, un{wb, 0.f}, vn{wb, 0.f};
+    pn.add(p, ar);
+    pn.add(r, nai);
+    rn.add(p, ai);
+    rn.add(r, ar);
+    un.add(u, br);
+    un.add(v, nbi);
+    vn.add(u, bi);
+    vn.add(v, br);
+    p = pn.value(one);
+    r = rn.value(one);
+    u = un.value(wb);
+    v = vn.value(wb);
+  }
+}
+
+// s + c += a b
+__device__ __forceinline__ void f2_dot(F2& s, F2 a, F2 b) {
+  const float h = __fmul_rn(a.h, b.h), e = fmaf(a.h, b.h, -h);
+  const float t = add_rn(s.h, h), y = sub_rn(t, s.h);
+  const float d = add_rn(sub_rn(s.h, sub_rn(t, y)), sub_rn(h, y));
+  s.l = fmaf(a.h, b.l, s.l);
+  s.l = fmaf(a.l, b.h, s.l);
+  s.l = add_rn(s.l, add_rn(d, e));
+  s.h = t;
+}
+// a + b + c, rounded
+__device__ __forceinline__ float f2_sum(F2 a, F2 b, float c) {
+  const float t = add_rn(a.h, b.h), y = sub_rn(t, a.h);
+  const float d = add_rn(sub_rn(a.h, sub_rn(t, y)), sub_rn(b.h, y));
+  const float z = add_rn(t, c), x = sub_rn(z, t);
+  const float f = add_rn(sub_rn(t, sub_rn(z, x)), sub_rn(c, x));
+  return add_rn(z, add_rn(add_rn(f, d), add_rn(a.l, b.l)));
+}
+
+// su_store from the sums over the powers of x (xs: per entry, p u, r u, p v, r v)
+__device__ __forceinline__ void su_store32(const SnapDev& S, int e, const F2Sum* xs, float base, Cplx<float>* U) {
+  const Entry& E = S.ent[e];
+  const int k = (E.j - E.q - E.T) / 2;
+  const float2* m = S.mono + E.mo;
+  F2 s[4];
+#pragma unroll
+  for (int h = 0; h < 4; ++h) s[h] = F2{0.f, 0.f};
+  for (int l = 0; l <= k; ++l) {
+    const float2 cm = __ldg(m + l);
+    const F2Sum* x = xs + 4 * (e - k + l);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) f2_dot(s[h], F2{cm.x, cm.y}, x[h].value(base));
+  }
+  const F2 pu = s[0], ru = s[1], pv = s[2], rv = s[3];
+  const F2 nru{-ru.h, -ru.l}, nrv{-rv.h, -rv.l};
+  const int2 h = S.half[e];
+  U[h.x] = Cplx<float>{f2_sum(pu, rv, E.T > 0 ? 0.f : float(S.wself)), f2_sum(pv, nru, 0.f)};
+  if (h.y >= 0) {
+    const float sg = E.T & 1 ? -1.f : 1.f;
+    U[h.y] = Cplx<float>{sg * f2_sum(pu, nrv, 0.f), -sg * f2_sum(pv, ru, 0.f)};
+  }
+}
+
+// One warp per atom as in k_snap_u.  Lanes = entries: the two columns of an
+// entry give its four sums, for two 16-byte loads.
+static __global__ void __launch_bounds__(32) k_snap_u32(SnapArgs A) {
+  const SnapDev& S = A.S;
+  extern __shared__ __align__(16) unsigned char su_smem32[];
+  F2Sum* xs = reinterpret_cast<F2Sum*>(su_smem32);             // 4 ne sums
+  float4* tab = reinterpret_cast<float4*>(xs + 4 * S.ne);      // 32 rows
+  const int al = blockIdx.x, lane = threadIdx.x, n = A.cnt[al];
+  const size_t np = size_t(A.n) * A.cap;
+  const float* pr = static_cast<const float*>(A.pr) + size_t(al) * A.cap;
+  float weight = 0.f;
+  for (int k = lane; k < n; k += 32) weight += fabsf(pr[PR_SF * np + k]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) weight += __shfl_xor_sync(FULL_MASK, weight, o);
+  const float base = f2_base(1.001f * weight);
+  for (int n0 = 0; n0 < max(n, 1); n0 += 32) {
+    const int m = min(32, n - n0);
+    if (lane < m) {
+      const float* q = pr + n0 + lane;
+      auto get = [&](int h, int l) { return F2{q[h * np], q[l * np]}; };
+      su_row32(S.twojmax, tab + lane * S.cols32, get(PR_AR, PR_ARL), get(PR_AI, PR_AIL), get(PR_BR, PR_BRL),
+               get(PR_BI, PR_BIL), get(PR_SF, PR_SFL));
+    }
+    __syncwarp();
+    for (int e0 = 0; e0 < S.ne; e0 += 96) {  // three entries per lane at once
+      int2 col[3];
+      F2Sum acc[3][4];
+#pragma unroll
+      for (int h = 0; h < 3; ++h) {
+        const int e = e0 + 32 * h + lane;
+        col[h] = e < S.ne ? __ldg(S.ucol + e) : int2{0, 0};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[h][c] = e < S.ne && n0 > 0 ? xs[4 * e + c] : F2Sum{base, 0.f};
+      }
+      auto rows = [&](auto nh) {
+#pragma unroll 2
+        for (int k = 0; k < m; ++k) {
+          const float4* t = tab + k * S.cols32;
+#pragma unroll
+          for (int h = 0; h < decltype(nh)::value; ++h) {
+            const float4 a = t[col[h].x], b = t[col[h].y];
+            acc[h][0].add(F2{a.x, a.y}, F2{b.x, b.y});
+            acc[h][1].add(F2{a.z, a.w}, F2{b.x, b.y});
+            acc[h][2].add(F2{a.x, a.y}, F2{b.z, b.w});
+            acc[h][3].add(F2{a.z, a.w}, F2{b.z, b.w});
+          }
+        }
+      };
+      if (e0 + 64 < S.ne) rows(std::integral_constant<int, 3>{});
+      else if (e0 + 32 < S.ne) rows(std::integral_constant<int, 2>{});
+      else rows(std::integral_constant<int, 1>{});
+#pragma unroll
+      for (int h = 0; h < 3; ++h) {
+        const int e = e0 + 32 * h + lane;
+        if (e < S.ne)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) xs[4 * e + c] = acc[h][c];
+      }
+    }
+    __syncwarp();
+  }
+  Cplx<float>* U = static_cast<Cplx<float>*>(A.U) + size_t(al) * S.nh;
+  for (int e = lane; e < S.ne; e += 32) su_store32(S, __ldg(S.eord + e), xs, base, U);
+}
+
+inline void launch_u32(const SnapArgs& A, cudaStream_t s) {
+  const size_t smem = sizeof(F2Sum) * 4 * size_t(A.S.ne) + 32 * 16 * size_t(A.S.cols32);
+  allow_dyn_smem(k_snap_u32);
+  k_snap_u32<<<A.n, 32, smem, s>>>(A);
+  EMD_CHECK_LAUNCH();
+}
+
+}  // namespace snapk
+}  // namespace emd
