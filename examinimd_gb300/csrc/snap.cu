@@ -143,6 +143,7 @@ struct SnapTables {
           Entry E{};
           E.N = std::ldexp(factorial(j) / std::sqrt(factorial(ma) * factorial(j - ma) * factorial(mb) * factorial(j - mb)),
                            -k);
+          E.Nf = float(E.N);
           E.A = jacobi_A(T, q, k);
           E.B = jacobi_B(T, q, k);
           AB.push_back(E.A);
@@ -615,8 +616,7 @@ static void snap_launch(Ctx& c, bool energy) {
     const int threads = A.tsplit == 4 ? 32 * 4 * std::max(1, std::min(2, A.apc)) : SF_THREADS;
     TimedLaunch t(c, fp64 ? "snap_force_fp64" : "snap_force_mixed");
     if (!fp64) snap_mixed_force(A, threads, c.stream);
-    else if (S.twojmax <= 8) launch_force<double, 9>(A, threads, c.stream);
-    else launch_force<double, 15>(A, threads, c.stream);
+    else launch_force<double>(A, threads, c.stream);
   }
   if (fused) {
     c.snap_pe_fused_valid = true;

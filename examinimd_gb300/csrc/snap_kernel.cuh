@@ -37,6 +37,7 @@
 
 #include "emd_device.cuh"
 #include "emd_internal.h"
+#include "f32_pairs.cuh"
 #include "neigh_rows.cuh"
 
 namespace emd {
@@ -55,6 +56,7 @@ struct Cplx {
 // One (T, q, k) entry
 struct Entry {
   double N;        // the elements' norm
+  float Nf;
   double A, B;     // P_{k+1} = (x - A) P_k - B P_{k-1}
   int xo;          // first of its real sums: p u, [q>0] r u, [T>0] p v, [q>0, T>0] r v
   int mo;          // its coefficients of x^0 .. x^k, times N (SnapDev::mono)
@@ -839,33 +841,89 @@ __global__ void __launch_bounds__(sy32_threads(NA), NA == 2 ? 1 : 2) k_snap_y32(
 // operations per neighbour at twojmax 8 (the layered adjoint took 4,100, half
 // its lanes idle).  f_j -= F_ij with FP64 atomics (j may be a ghost;
 // update_force follows) and f_i += sum_j F_ij in a fixed order.
+//
+// With twojmax a constant (2, 4, 6, 8) every loop is unrolled and the recurrences'
+// constants are operands; other twojmax take the loops.  The mixed form forms the
+// powers of a and b from their 48-bit values and keeps what the sum over T rounds
+// off, 1,000 operations more, half of the FP32 error (rms against the FP64 form, W
+// bcc 2,000 atoms at 0.05 A: 7.5e-6 -> 5.5e-6 eV/A, of which 3.3e-6 are Y's).
+// Bound by instruction issue and the latency of the phases; per 128,000 atoms
+// mixed 0.88 ms as loops, 0.61 unrolled with the extra operations; 8,160 atoms FP64
+// 0.64 and 0.58 (0.50 of FP64 issue).
 constexpr int SF_THREADS = 256;
 constexpr int SF_ATOMS = 8;
 
-// NQ: powers of a kept in registers (twojmax + 1 <= NQ)
-template <typename R, int NQ>
-__global__ void __launch_bounds__(SF_THREADS) k_snap_force(SnapArgs A) {
+// Constants of the recurrences with T + q + 2k < SF_JMAX, in constant memory where
+// an unrolled loop has them as operands (as in SnapDev::AB; k = 0 has no B)
+constexpr int SF_JMAX = 8;
+template <typename R>
+struct JacTable {
+  R a[SF_JMAX][SF_JMAX][SF_JMAX / 2], b[SF_JMAX][SF_JMAX][SF_JMAX / 2];
+  constexpr JacTable() : a{}, b{} {
+    for (int T = 0; T < SF_JMAX; ++T)
+      for (int q = 0; q < SF_JMAX; ++q)
+        for (int k = 0; k < SF_JMAX / 2; ++k) {
+          const double s = 2.0 * k + T + q;
+          a[T][q][k] = R(k == 0 ? (q - T) / (s + 2.0) : double(q * q - T * T) / (s * (s + 2.0)));
+          b[T][q][k] = R(k == 0 ? 0.0 : 4.0 * k * (k + T) * (k + q) * (k + T + q) / (s * s * (s + 1.0) * (s - 1.0)));
+        }
+  }
+};
+static __constant__ JacTable<double> c_jac = JacTable<double>();
+static __constant__ JacTable<float> c_jac32 = JacTable<float>();
+template <typename R>
+__device__ __forceinline__ R jac_a(int T, int q, int k) {
+  if constexpr (sizeof(R) == sizeof(float)) return c_jac32.a[T][q][k];
+  else return c_jac.a[T][q][k];
+}
+template <typename R>
+__device__ __forceinline__ R jac_b(int T, int q, int k) {
+  if constexpr (sizeof(R) == sizeof(float)) return c_jac32.b[T][q][k];
+  else return c_jac.b[T][q][k];
+}
+
+// s + c += t, the sum of T's terms: what the addition rounds off goes to c
+template <typename R>
+struct TSum {
+  R s = 0, c = 0;
+  __device__ __forceinline__ void add(R t) {
+    if constexpr (sizeof(R) == sizeof(float)) {
+      const R z = add_rn(s, t), y = sub_rn(z, s);
+      c = add_rn(c, add_rn(sub_rn(s, sub_rn(z, y)), sub_rn(t, y)));
+      s = z;
+    } else {
+      s += t;
+    }
+  }
+  __device__ __forceinline__ R value() const { return s + c; }
+};
+
+// JC: twojmax (loops unrolled), or -1: any up to 14
+template <typename R, int JC>
+__global__ void __launch_bounds__(SF_THREADS, sizeof(R) == 4 ? 3 : 2) k_snap_force(SnapArgs A) {
   const SnapDev& S = A.S;
   constexpr bool kF64 = sizeof(R) == sizeof(double);
+  static_assert(JC <= SF_JMAX, "recurrence constants");
+  constexpr int NQ = JC >= 0 ? JC + 1 : 15, kUnroll = JC >= 0 ? 16 : 1;
   extern __shared__ __align__(16) unsigned char sf_smem[];
   __shared__ int s_off[SF_ATOMS + 1];
   __shared__ double s_sum[SF_ATOMS][3];
-  const int J = S.twojmax, ny = 4 * S.ne, tid = threadIdx.x;
+  const int J = JC >= 0 ? JC : S.twojmax, ny = 4 * S.ne, tid = threadIdx.x;
   const int apc = A.apc, a0 = blockIdx.x * apc, na = min(apc, A.n - a0);
   // groups of T on separate warps (small systems): each forms a part of F
   const int nthr = blockDim.x / A.tsplit, grp = tid / nthr, gt = tid - grp * nthr;
   R* ys = reinterpret_cast<R*>(sf_smem);                                   // apc x ny
   double* fs = reinterpret_cast<double*>(sf_smem + ((size_t(apc) * ny * sizeof(R) + 15) & ~size_t(15)));  // blockDim x 3
   const int ta = A.ta;
-  for (int k = tid; k < S.ne * na; k += blockDim.x) {
-    const int e = k / na, a = k - e * na, ga = a0 + a;
-    const R* Y = static_cast<const R*>(A.Y) + size_t(ga / ta) * 2 * S.ny * ta + ga % ta;
+  const int la = tid % na, ls = blockDim.x / na, ga = a0 + la;
+  const R* Yt = static_cast<const R*>(A.Y) + size_t(ga / ta) * 2 * S.ny * ta + ga % ta;
+  for (int e = tid / na; tid < ls * na && e < S.ne; e += ls) {
     const int2 h = __ldg(S.half + e);
-    const R N2 = R(2.0 * S.ent[e].N);
-    const Cplx<R> p = y_element(S, h.x, Y, ta);
-    R* o = ys + a * ny + 4 * e;
+    const R N = kF64 ? R(S.ent[e].N) : R(S.ent[e].Nf), N2 = N + N;
+    const Cplx<R> p = y_element(S, h.x, Yt, ta);
+    R* o = ys + la * ny + 4 * e;
     if (h.y >= 0) {
-      const Cplx<R> m = y_element(S, h.y, Y, ta);
+      const Cplx<R> m = y_element(S, h.y, Yt, ta);
       const R sg = __ldg(S.hfull + h.x).z > 0 ? R(1) : R(-1);
       o[0] = N2 * fma(sg, m.r, p.r);
       o[1] = N2 * fma(sg, m.i, p.i);
@@ -873,7 +931,7 @@ __global__ void __launch_bounds__(SF_THREADS) k_snap_force(SnapArgs A) {
       o[3] = N2 * fma(-sg, m.i, p.i);
     } else {  // q = 0 (the -T element is the inversion of the +T one), T = 0, or both
       const int T = S.ent[e].T, q = S.ent[e].q;
-      o[0] = (T + q > 0 ? N2 : R(0.5) * N2) * p.r;
+      o[0] = (T + q > 0 ? N2 : N) * p.r;
       o[1] = q > 0 ? N2 * p.i : R(0);
       o[2] = R(0);
       o[3] = T > 0 ? N2 * p.i : R(0);
@@ -904,47 +962,83 @@ __global__ void __launch_bounds__(SF_THREADS) k_snap_force(SnapArgs A) {
       const double* qd = A.pd + p;
       const R* qr = static_cast<const R*>(A.pr) + p;
       const R ar = qr[PR_AR * np], ai = qr[PR_AI * np], br = qr[PR_BR * np], bi = qr[PR_BI * np];
-      R pq[NQ], rq[NQ];  // a^q
+      // powers of a and b; in the mixed form from the 48-bit a and b and rounded once
+      R pq[NQ], rq[NQ];
       pq[0] = R(1);
       rq[0] = R(0);
+      R x;
+      F2 b0{}, b1{}, nb1{}, u2{}, v2{};
+      const float one = f2_base(1.f);
+      if constexpr (kF64) {
 #pragma unroll
-      for (int q = 1; q < NQ; ++q) {
-        pq[q] = fma(pq[q - 1], ar, -rq[q - 1] * ai);
-        rq[q] = fma(pq[q - 1], ai, rq[q - 1] * ar);
+        for (int q = 1; q < NQ; ++q) {
+          pq[q] = fma(pq[q - 1], ar, -rq[q - 1] * ai);
+          rq[q] = fma(pq[q - 1], ai, rq[q - 1] * ar);
+        }
+        x = fma(ar, ar, ai * ai) - fma(br, br, bi * bi);
+      } else {
+        const F2 c0{ar, qr[PR_ARL * np]}, c1{ai, qr[PR_AIL * np]}, nc1{-c1.h, -c1.l};
+        b0 = F2{br, qr[PR_BRL * np]};
+        b1 = F2{bi, qr[PR_BIL * np]};
+        nb1 = F2{-b1.h, -b1.l};
+        F2Sum sx{one, 0.f};
+        sx.add(c0, c0);
+        sx.add(c1, c1);
+        sx.add(F2{-b0.h, -b0.l}, b0);
+        sx.add(nb1, b1);
+        x = sx.value(one).h;
+        F2 pk{1.f, 0.f}, rk{0.f, 0.f};
+#pragma unroll
+        for (int q = 1; q < NQ; ++q) {
+          if (q == 1) {
+            pk = c0;
+            rk = c1;
+          } else {
+            f2_cmul(pk, rk, c0, c1, nc1, one);
+          }
+          pq[q] = pk.h;
+          rq[q] = rk.h;
+        }
+        u2 = F2{1.f, 0.f};
       }
-      const R x = fma(ar, ar, ai * ai) - fma(br, br, bi * bi);
       R u = R(1), v = R(0), um = R(0), vm = R(0);  // b^T, b^(T-1)
-      R phi = 0, gx = 0, gar = 0, gai = 0, gbr = 0, gbi = 0;
+      TSum<R> phi, gx, gar, gai, gbr, gbi;
       const R* Y = ys + a * ny;
       const R* ab = AB;
+#pragma unroll kUnroll
       for (int T = 0; T <= J; ++T) {
+        const int nT = (J - T + 2) * (J - T + 2) / 4;  // entries of T
         if (mask >> T & 1) {
           // sums over q: Re Eh, Im Oh; the same with P'; dEh/da, dOh/da
           R er = 0, oi = 0, xer = 0, xoi = 0, e1r = 0, e1i = 0, o1r = 0, o1i = 0;
+          int e = 0;
 #pragma unroll
           for (int q = 0; q < NQ; ++q) {
             if (q > J - T) break;
             const int km = (J - T - q) / 2;
-            R g0 = Y[0], g1 = Y[1], g2 = Y[2], g3 = Y[3];  // sum_k E P_k, O P_k
+            const R* y = Y + 4 * e;
+            R g0 = y[0], g1 = y[1], g2 = y[2], g3 = y[3];  // sum_k E P_k, O P_k
             R h0 = 0, h1 = 0, h2 = 0, h3 = 0;              // sum_k E P'_k, O P'_k
             if (km > 0) {
-              R pk = x - ab[0], pm = R(1), dk = R(1), dm = R(0);
-              h0 = Y[4];
-              h1 = Y[5];
-              h2 = Y[6];
-              h3 = Y[7];
+              R pk = x - (JC >= 0 ? jac_a<R>(T, q, 0) : ab[2 * e]), pm = R(1), dk = R(1), dm = R(0);
+              h0 = y[4];
+              h1 = y[5];
+              h2 = y[6];
+              h3 = y[7];
               g0 = fma(h0, pk, g0);
               g1 = fma(h1, pk, g1);
               g2 = fma(h2, pk, g2);
               g3 = fma(h3, pk, g3);
+#pragma unroll kUnroll
               for (int k = 2; k <= km; ++k) {
-                const R t = x - ab[2 * (k - 1)], c = ab[2 * (k - 1) + 1];
+                const R t = x - (JC >= 0 ? jac_a<R>(T, q, k - 1) : ab[2 * (e + k - 1)]);
+                const R c = JC >= 0 ? jac_b<R>(T, q, k - 1) : ab[2 * (e + k - 1) + 1];
                 const R pn = fma(t, pk, -c * pm), dn = fma(t, dk, fma(-c, dm, pk));
                 pm = pk;
                 pk = pn;
                 dm = dk;
                 dk = dn;
-                const R* yk = Y + 4 * k;
+                const R* yk = y + 4 * k;
                 g0 = fma(yk[0], pk, g0);
                 g1 = fma(yk[1], pk, g1);
                 h0 = fma(yk[0], dk, h0);
@@ -976,51 +1070,51 @@ __global__ void __launch_bounds__(SF_THREADS) k_snap_force(SnapArgs A) {
               oi = fma(pq[q], g3, oi);
               xoi = fma(pq[q], h3, xoi);
             }
-            Y += 4 * (km + 1);
-            ab += 2 * (km + 1);
+            e += km + 1;
           }
-          phi = fma(u, er, fma(v, oi, phi));
-          gx = fma(u, xer, fma(v, xoi, gx));
-          gar = fma(u, e1r, fma(v, o1i, gar));
-          gai = fma(-u, e1i, fma(v, o1r, gai));
+          phi.add(fma(u, er, v * oi));
+          gx.add(fma(u, xer, v * xoi));
+          gar.add(fma(u, e1r, v * o1i));
+          gai.add(fma(-u, e1i, v * o1r));
           if (T > 0) {
             const R tu = R(T) * um, tv = R(T) * vm;
-            gbr = fma(tu, er, fma(tv, oi, gbr));
-            gbi = fma(tu, oi, fma(-tv, er, gbi));
+            gbr.add(fma(tu, er, tv * oi));
+            gbi.add(fma(tu, oi, -tv * er));
           }
-        } else {
-          int sk = 0;
-          for (int q = 0; q <= J - T; ++q) sk += (J - T - q) / 2 + 1;
-          Y += 4 * sk;
-          ab += 2 * sk;
         }
+        Y += 4 * nT;
+        ab += 2 * nT;
         um = u;
         vm = v;
-        const R un = fma(u, br, -v * bi);
-        v = fma(u, bi, v * br);
-        u = un;
+        if constexpr (kF64) {
+          const R un = fma(u, br, -v * bi);
+          v = fma(u, bi, v * br);
+          u = un;
+        } else {
+          f2_cmul(u2, v2, b0, b1, nb1, one);
+          u = u2.h;
+          v = v2.h;
+        }
       }
-      const R gx2 = gx + gx;
-      gar = fma(ar, gx2, gar);
-      gai = fma(ai, gx2, gai);
-      gbr = fma(-br, gx2, gbr);
-      gbi = fma(-bi, gx2, gbi);
-      const R cp = qr[PR_DSF * np] * phi;
+      const R gx2 = gx.value() + gx.value();
+      const R ga = fma(ar, gx2, gar.value()), gb = fma(ai, gx2, gai.value());
+      const R gc = fma(-br, gx2, gbr.value()), gd = fma(-bi, gx2, gbi.value());
+      const R cp = qr[PR_DSF * np] * phi.value();
       const R uk[3] = {qr[PR_UX * np], qr[PR_UY * np], qr[PR_UZ * np]};
       if constexpr (kF64) {
         const double sf = qd[PD_SF * np];
 #pragma unroll
         for (int d = 0; d < 3; ++d)
-          F[d] = fma(cp, uk[d], sf * fma(gar, qr[(PF_DAR + d) * np],
-                                         fma(gai, qr[(PF_DAI + d) * np],
-                                             fma(gbr, qr[(PF_DBR + d) * np], gbi * qr[(PF_DBI + d) * np]))));
+          F[d] = fma(cp, uk[d], sf * fma(ga, qr[(PF_DAR + d) * np],
+                                         fma(gb, qr[(PF_DAI + d) * np],
+                                             fma(gc, qr[(PF_DBR + d) * np], gd * qr[(PF_DBI + d) * np]))));
       } else {
         // along u_k through theta0 and s / r, then the direct terms
         const R sf = qr[PR_SF * np], c1 = qr[PR_C1 * np], gr = qr[PR_GR * np], r0 = sf * qr[PR_R0 * np];
-        const R rad = fma(sf, fma(c1, gar, gr * fma(-uk[2], gai, fma(uk[1], gbr, -uk[0] * gbi))), cp);
-        F[0] = double(fma(rad, uk[0], -r0 * gbi));
-        F[1] = double(fma(rad, uk[1], r0 * gbr));
-        F[2] = double(fma(rad, uk[2], -r0 * gai));
+        const R rad = fma(sf, fma(c1, ga, gr * fma(-uk[2], gb, fma(uk[1], gc, -uk[0] * gd))), cp);
+        F[0] = double(fma(rad, uk[0], -r0 * gd));
+        F[1] = double(fma(rad, uk[1], r0 * gc));
+        F[2] = double(fma(rad, uk[2], -r0 * gb));
       }
     }
     if (A.tsplit > 1) {  // the groups' parts, in a fixed order
@@ -1043,12 +1137,15 @@ __global__ void __launch_bounds__(SF_THREADS) k_snap_force(SnapArgs A) {
       for (int d = 0; d < 3; ++d) fs[3 * gt + d] = F[d];
     }
     __syncthreads();
-    if (tid < 3 * na) {  // f_i, neighbours in order
-      const int a = tid / 3, d = tid - 3 * a;
+    // f_i: four lanes take every fourth neighbour
+    if (tid < 32 * ((12 * na + 31) / 32)) {
+      const int a = min(tid / 12, na - 1), d = tid % 12 / 4, l = tid & 3;
       const int b0 = max(s_off[a] - s0, 0), b1 = min(s_off[a + 1] - s0, nthr);
-      double t = s_sum[a][d];
-      for (int k = b0; k < b1; ++k) t += fs[3 * k + d];
-      s_sum[a][d] = t;
+      double t = 0.0;
+      for (int k = b0 + l; k < b1; k += 4) t += fs[3 * k + d];
+      t += __shfl_xor_sync(FULL_MASK, t, 1);
+      t += __shfl_xor_sync(FULL_MASK, t, 2);
+      if (l == 0 && tid < 12 * na) s_sum[a][d] += t;
     }
     __syncthreads();
   }
@@ -1280,12 +1377,22 @@ inline void launch_u(const SnapArgs& A, cudaStream_t s) {
   EMD_CHECK_LAUNCH();
 }
 
-template <typename R, int NQ>
-void launch_force(const SnapArgs& A, int threads, cudaStream_t s) {
+template <typename R, int JC>
+void launch_force_j(const SnapArgs& A, int threads, cudaStream_t s) {
   const size_t smem = ((size_t(A.apc) * 4 * A.S.ne * sizeof(R) + 15) & ~size_t(15)) + size_t(threads) * 24;
-  allow_dyn_smem(k_snap_force<R, NQ>);
-  k_snap_force<R, NQ><<<(A.n + A.apc - 1) / A.apc, threads, smem, s>>>(A);
+  allow_dyn_smem(k_snap_force<R, JC>);
+  k_snap_force<R, JC><<<(A.n + A.apc - 1) / A.apc, threads, smem, s>>>(A);
   EMD_CHECK_LAUNCH();
+}
+template <typename R>
+void launch_force(const SnapArgs& A, int threads, cudaStream_t s) {
+  switch (A.S.twojmax) {
+    case 2: return launch_force_j<R, 2>(A, threads, s);
+    case 4: return launch_force_j<R, 4>(A, threads, s);
+    case 6: return launch_force_j<R, 6>(A, threads, s);
+    case 8: return launch_force_j<R, 8>(A, threads, s);
+    default: return launch_force_j<R, -1>(A, threads, s);
+  }
 }
 
 // the kernels of one chunk, up to Y

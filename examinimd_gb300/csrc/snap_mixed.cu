@@ -26,9 +26,6 @@ void snap_mixed_y(const SnapArgs& A, cudaStream_t s) {
   }
 }
 
-void snap_mixed_force(const SnapArgs& A, int threads, cudaStream_t s) {
-  if (A.S.twojmax <= 8) launch_force<float, 9>(A, threads, s);
-  else launch_force<float, 15>(A, threads, s);
-}
+void snap_mixed_force(const SnapArgs& A, int threads, cudaStream_t s) { launch_force<float>(A, threads, s); }
 
 }  // namespace emd
