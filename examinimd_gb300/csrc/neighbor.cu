@@ -1,18 +1,7 @@
 // NeighborCSR / Neighbor2D on the device (neighbor_csr.h:176-435,
 // neighbor_2d.h:175-331).
 //
-// One warp per interior bin.  The warp stages the particles of its 27-bin
-// stencil in the reference order (bx_j slowest, bz_j fastest; inside a bin
-// in permutation order) into shared memory as FP32 positions relative to the
-// centre of ITS bin (exact bin-relative FP32 coordinates come from the
-// binning pass), so a candidate test is three FP32 subtractions and an FP32
-// r^2.  Only when r^2 lies within 4e-5 relative of the cutoff is the pair
-// re-tested with the FP64 positions, so every accept / reject equals the FP64
-// test `rsq <= neigh_cut^2` of the reference.  Each lane owns one centre atom
-// of the bin and walks the staged candidates in order (one broadcast
-// shared-memory read per candidate for the whole warp), appending the
-// accepted ones, so row i lists its neighbours in exactly the order the
-// serial reference appends them.
+// One warp per interior bin (rows_of_bin, neigh_bin.cuh).
 //
 // One pass writes rows column-major in 16-byte granules (neigh_rows.cuh:
 // the LayoutLeft of the reference's Neighbor2D view on a GPU, four entries
@@ -27,45 +16,24 @@
 
 #include "emd_device.cuh"
 #include "emd_internal.h"
-#include "neigh_rows.cuh"
+#include "neigh_bin.cuh"
 
 namespace emd {
 namespace {
 
 constexpr int NB_WARPS = 4;     // warps per CTA, one interior bin each (independent)
 constexpr int NB_THREADS = 32 * NB_WARPS;
-constexpr int NB_CAP = 256;     // staged candidates per chunk and warp
 constexpr int NB_SLOTS = 64;  // spread slots for the longest-row reduction
 static_assert(1 + NB_SLOTS <= kHostInts, "read-back of the row-length slots exceeds the pinned scratch");
 
 struct NeighArgs {
-  const double4_32a* x4;
-  const float4* xl;  // FP32 position relative to the particle's bin centre
+  RowArgs r;
   const int* bincount;
   const int* binoffsets;
-  const int* permute;
-  int nbx, nby, nbz, nhalo;
-  float wx, wy, wz;  // bin widths
-  int n_local;
-  double cutsq;
-  float cut_lo, cut_hi;  // FP32 decision band
-  int half, newton, packed;
-  int* num_neighs;
-  int* rows;  // column-major, leading dimension `stride`, capacity K
-  int stride, K;
+  int nbx, nhalo;
   int* flags;  // [0] overflow, [1] longest row
   int ibins;   // interior bins
 };
-
-// Exact FP64 re-test of a pair whose FP32 r^2 fell inside the guard band.
-// Kept out of line: inlined, the compiler predicates it into the candidate
-// loop and every batch of 32 candidates then issues its FP64 instructions
-// (64 cycles each on this part) whether or not a lane needs them.
-__device__ __noinline__ bool retest_fp64(const double4_32a* __restrict__ x4, int i, int j, double cutsq) {
-  const double4_32a pi = x4[i], pj = x4[j];
-  const double ddx = pi.x - pj.x, ddy = pi.y - pj.y, ddz = pi.z - pj.z;
-  return (ddx * ddx + ddy * ddy + ddz * ddz) <= cutsq;
-}
 
 // FP32 offsets of the binned particles from their bin centres, exactly as
 // the binning writes them (k_bin_index), for a list built again from the
@@ -82,200 +50,26 @@ __global__ void __launch_bounds__(256) k_xl_from_bins(const double4_32a* __restr
                       __int_as_float(int(p.w)));
 }
 
-// monotone integer key of a double (exact ordering, integer pipe)
-__device__ __forceinline__ long long okey(double v) {
-  const long long b = __double_as_longlong(v);
-  return b >= 0 ? b : (b ^ 0x7fffffffffffffffLL);
-}
-
-// The half list's order rule (neighbor_csr.h:287-291): j "above" i when
-// (x_j, y_j, z_j) > (x_i, y_i, z_i) lexicographically, from the FP64
-// positions.  Out of line for the same reason as retest_fp64.
-__device__ __noinline__ bool above_fp64(const double4_32a* __restrict__ x4, long long kx, long long ky,
-                                        long long kz, int j) {
-  const double4_32a xj = x4[j];
-  const long long jx = okey(xj.x), jy = okey(xj.y), jz = okey(xj.z);
-  return (jx > kx) || ((jx == kx) && ((jy > ky) || ((jy == ky) && (jz > kz))));
-}
-
 template <bool HALF, bool PACKED>
 __global__ void __launch_bounds__(NB_THREADS) k_neigh_bin(NeighArgs a) {
   // each warp of the CTA builds the rows of its own bin with its own staging
   // arrays; the warps never wait for each other (more resident warps than one
   // warp per CTA allows, at the same shared memory per warp)
-  __shared__ float4 cand_w[NB_WARPS][NB_CAP];
-  __shared__ int pre_w[NB_WARPS][28];
-  __shared__ int boff_w[NB_WARPS][27];
+  __shared__ __align__(16) RowStage st[NB_WARPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int bin = blockIdx.x * NB_WARPS + warp;
   if (bin >= a.ibins) return;
-  float4* cand = cand_w[warp];
-  int* pre = pre_w[warp];
-  int* boff = boff_w[warp];
-  // interior bin of this warp
-  const int ix = a.nbx - 2 * a.nhalo, iy = a.nby - 2 * a.nhalo, iz = a.nbz - 2 * a.nhalo;
-  (void)ix;
-  const int bx = bin / (iy * iz) + a.nhalo;
-  const int by = (bin / iz) % iy + a.nhalo;
-  const int bz = bin % iz + a.nhalo;
-  const int bc = (bx * a.nby + by) * a.nbz + bz;
-  int cntb = 0, offb = 0;
-  if (lane < 27) {
-    const int dbx = lane / 9 - 1, dby = (lane / 3) % 3 - 1, dbz = lane % 3 - 1;
-    const int b = ((bx + dbx) * a.nby + (by + dby)) * a.nbz + (bz + dbz);
-    cntb = a.bincount[b];
-    offb = a.binoffsets[b];
-  }
-  // inclusive scan of the 27 stencil counts over the lanes
-  int inc = cntb;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(FULL_MASK, inc, o);
-    if (lane >= o) inc += v;
-  }
-  if (lane < 27) {
-    pre[lane + 1] = inc;
-    boff[lane] = offb;
-  }
-  if (lane == 0) pre[0] = 0;
-  __syncwarp();
-  const int M = pre[27];
-  const int nc = a.bincount[bc], oc = a.binoffsets[bc];
-  int mx = 0;
-  // Candidates farther than the cutoff from every centre atom of the chunk
-  // are dropped while staging, once per warp: the FP32 r^2 of a centre atom
-  // to a candidate is at least the candidate's squared FP32 distance to the
-  // bounding box of the chunk's centre atoms (rounding is monotone), and a
-  // dropped candidate's exceeds cut_hi by a 1e-5 margin, so no lane would
-  // accept the pair or re-test it in FP64.  Rows keep their order.
-  const float prune_sq = a.cut_hi * 1.00001f;
-  // half lists: the FP32 x offset of a candidate from a centre atom has the
-  // sign of the FP64 x difference once it exceeds the FP32 rounding of the
-  // two offsets and the bin shift (below 2^-24 (3 w + 2 drift) in all); only
-  // x ties within that bound need the FP64 order keys
-  const float otol = 1e-6f * (1.0f + 4.0f * fmaxf(a.wx, fmaxf(a.wy, a.wz)));
-  const unsigned lt = (1u << lane) - 1u;
-  for (int a0 = 0; a0 < nc; a0 += 32) {
-    // this lane's centre atom
-    const int bi = a0 + lane;
-    const int i = bi < nc ? a.permute[oc + bi] : -1;
-    const bool own = i >= 0 && i < a.n_local;  // ghosts own no row
-    float4 xi = make_float4(0.f, 0.f, 0.f, 0.f);
-    long long kx = 0, ky = 0, kz = 0;
-    // i's own entry: the centre bin's code (1, 1, 1) when packed
-    const int self = PACKED ? int((unsigned(i) << 6) | 0x15u) : i;
-    if (own) {
-      xi = a.xl[i];
-      if (HALF) {
-        const double4_32a xd = a.x4[i];
-        kx = okey(xd.x);
-        ky = okey(xd.y);
-        kz = okey(xd.z);
-      }
-    }
-    // bounding box of the chunk's centre atoms that own rows
-    float lox = own ? xi.x : 3.0e38f, loy = own ? xi.y : 3.0e38f, loz = own ? xi.z : 3.0e38f;
-    float hix = own ? xi.x : -3.0e38f, hiy = own ? xi.y : -3.0e38f, hiz = own ? xi.z : -3.0e38f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lox = fminf(lox, __shfl_xor_sync(FULL_MASK, lox, o));
-      loy = fminf(loy, __shfl_xor_sync(FULL_MASK, loy, o));
-      loz = fminf(loz, __shfl_xor_sync(FULL_MASK, loz, o));
-      hix = fmaxf(hix, __shfl_xor_sync(FULL_MASK, hix, o));
-      hiy = fmaxf(hiy, __shfl_xor_sync(FULL_MASK, hiy, o));
-      hiz = fmaxf(hiz, __shfl_xor_sync(FULL_MASK, hiz, o));
-    }
-    int cnt = 0;
-    // next slot of the row: +1 inside a 4-entry granule, then on to the
-    // row's next granule (4 stride - 3 ints further)
-    int* rp = a.rows + quad_index(own ? i : 0, 0, a.stride);
-    const int jump = 4 * a.stride - 3;
-    for (int base = 0; base < M; base += NB_CAP) {
-      const int mc = min(NB_CAP, M - base);
-      int m = 0;  // candidates kept
-      __syncwarp();
-      for (int t0 = 0; t0 < mc; t0 += 32) {
-        const int t = t0 + lane;
-        bool keep = false;
-        float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (t < mc) {
-          const int g = base + t;
-          int s = 0;  // stencil bin of candidate g: binary search of the prefix
-#pragma unroll
-          for (int h = 16; h >= 1; h >>= 1)
-            if (s + h <= 27 && pre[s + h] <= g) s += h;
-          const int j = a.permute[boff[s] + (g - pre[s])];
-          const float4 p = a.xl[j];
-          const float sx = float(s / 9 - 1) * a.wx, sy = float((s / 3) % 3 - 1) * a.wy, sz = float(s % 3 - 1) * a.wz;
-          const int code = ((s / 9) << 4) | (((s / 3) % 3) << 2) | (s % 3);
-          const int w = PACKED ? ((j << 6) | code) : j;
-          c = make_float4(p.x + sx, p.y + sy, p.z + sz, __int_as_float(w));
-          const float bx = fmaxf(fmaxf(lox - c.x, c.x - hix), 0.f), by = fmaxf(fmaxf(loy - c.y, c.y - hiy), 0.f),
-                      bz = fmaxf(fmaxf(loz - c.z, c.z - hiz), 0.f);
-          // the lanes' r^2 expression, so monotone rounding bounds it below
-          keep = __fmaf_rn(bz, bz, __fadd_rn(__fmul_rn(bx, bx), __fmul_rn(by, by))) <= prune_sq;
-        }
-        const unsigned bal = __ballot_sync(FULL_MASK, keep);
-        if (keep) cand[m + __popc(bal & lt)] = c;
-        m += __popc(bal);
-      }
-      const int m4 = (m + 3) & ~3;
-      __syncwarp();
-      // pad to a multiple of four with copies of the first candidate moved far
-      // outside the cutoff (a valid particle, never accepted)
-      if (lane < m4 - m) cand[m + lane] = make_float4(1.0e4f, 1.0e4f, 1.0e4f, cand[0].w);
-      __syncwarp();
-      if (own) {
-        for (int k = 0; k < m4; k += 4) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float4 c = cand[k + u];
-            const int w = __float_as_int(c.w);
-            // FP32 r^2 with packed (x, y) and a fused z term (this file is
-            // compiled without contraction for the FP64 re-test; the FP32
-            // value only has to be within the guard band)
-            const float2 dxy = __ffma2_rn(make_float2(c.x, c.y), make_float2(-1.f, -1.f), make_float2(xi.x, xi.y));
-            const float dz = __fsub_rn(xi.z, c.z);
-            const float2 sq = __fmul2_rn(dxy, dxy);
-            const float rsq = __fmaf_rn(dz, dz, __fadd_rn(sq.x, sq.y));
-            bool in = rsq < a.cut_lo;
-            const bool decided = in || rsq > a.cut_hi;
-            bool take;
-            if (HALF) {
-              // neighbor_csr.h:287-291: skip unless j is "above" i
-              // lexicographically, or j is a ghost with newton off
-              const int j = PACKED ? (w >> 6) : w;
-              bool skip = false;
-              if ((j == i) || (j < a.n_local || a.newton)) {
-                const float gx = __fsub_rn(c.x, xi.x);
-                skip = fabsf(gx) > otol ? !(gx > 0.f) : !above_fp64(a.x4, kx, ky, kz, j);
-              }
-              if (!skip && !decided) in = retest_fp64(a.x4, i, j, a.cutsq);
-              take = !skip && in;
-            } else {
-              if (!decided) in = retest_fp64(a.x4, i, PACKED ? (w >> 6) : w, a.cutsq);
-              take = in && (w != self);
-            }
-            if (take) {
-              if (cnt < a.K) *rp = w;
-              rp += (cnt & 3) == 3 ? jump : 1;
-              ++cnt;
-            }
-          }
-        }
-      }
-    }
-    if (own) {
-      a.num_neighs[i] = cnt;
-      mx = max(mx, cnt);
-    }
-  }
+  const int iy = a.r.nby - 2 * a.nhalo, iz = a.r.nbz - 2 * a.nhalo;
+  const int mx = rows_of_bin<HALF, PACKED>(a.r, st[warp], bin / (iy * iz) + a.nhalo, (bin / iz) % iy + a.nhalo,
+                                           bin % iz + a.nhalo, [&](int b, int& off) {
+                                             off = a.binoffsets[b];
+                                             return a.bincount[b];
+                                           });
   // overflow flag and longest row: one atomic per warp into one of 64 slots
   // (a single shared address would serialise millions of atomics in L2)
-  mx = __reduce_max_sync(FULL_MASK, mx);
   if (lane == 0) {
     if (mx > 0) atomicMax(&a.flags[1 + (bin & (NB_SLOTS - 1))], mx);
-    if (mx > a.K) a.flags[0] = 1;
+    if (mx > a.r.K) a.flags[0] = 1;
   }
 }
 
@@ -350,27 +144,26 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
     c.xl_bin_valid = true;
   }
   NeighArgs a;
-  a.x4 = c.x4.p;
-  a.xl = c.xl_bin.p;
+  a.r.x4 = c.x4.p;
+  a.r.xl = c.xl_bin.p;
   a.bincount = c.bincount.p;
   a.binoffsets = c.binoffsets.p;
-  a.permute = c.permute.p;
+  a.r.permute = c.permute.p;
   a.nbx = c.nbin[0];
-  a.nby = c.nbin[1];
-  a.nbz = c.nbin[2];
+  a.r.nby = c.nbin[1];
+  a.r.nbz = c.nbin[2];
   a.nhalo = c.nhalo;
-  a.wx = float((c.bmax[0] - c.bmin[0]) / c.nbin[0]);
-  a.wy = float((c.bmax[1] - c.bmin[1]) / c.nbin[1]);
-  a.wz = float((c.bmax[2] - c.bmin[2]) / c.nbin[2]);
-  a.n_local = n;
-  a.cutsq = c.neigh_cut * c.neigh_cut;
-  a.cut_lo = float(a.cutsq * (1.0 - 4e-5));
-  a.cut_hi = float(a.cutsq * (1.0 + 4e-5));
-  a.half = c.half_neigh;
-  a.newton = c.comm_newton;
-  a.packed = packed;
-  a.num_neighs = c.num_neighs.p;
-  a.stride = n + 1;
+  a.r.wx = float((c.bmax[0] - c.bmin[0]) / c.nbin[0]);
+  a.r.wy = float((c.bmax[1] - c.bmin[1]) / c.nbin[1]);
+  a.r.wz = float((c.bmax[2] - c.bmin[2]) / c.nbin[2]);
+  a.r.n_local = n;
+  a.r.cutsq = c.neigh_cut * c.neigh_cut;
+  const double band = row_band(std::max({double(a.r.wx), double(a.r.wy), double(a.r.wz)}), c.neigh_cut);
+  a.r.cut_lo = float(a.r.cutsq * (1.0 - band));
+  a.r.cut_hi = float(a.r.cutsq * (1.0 + band));
+  a.r.newton = c.comm_newton;
+  a.r.num_neighs = c.num_neighs.p;
+  a.r.stride = n + 1;
   a.flags = c.resize_flag.p;
   const int ibins = (c.nbin[0] - 2 * c.nhalo) * (c.nbin[1] - 2 * c.nhalo) * (c.nbin[2] - 2 * c.nhalo);
   a.ibins = ibins;
@@ -379,8 +172,8 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
   DevBuf<int>& rows = two_d ? c.neighs : c.neigh_rows2d;
   while (true) {
     rows.reserve(size_t(n + 1) * size_t((K + 3) & ~3) + 4, c.stream);
-    a.rows = rows.p;
-    a.K = K;
+    a.r.rows = rows.p;
+    a.r.K = K;
     EMD_CUDA(cudaMemsetAsync(c.resize_flag.p, 0, (1 + NB_SLOTS) * sizeof(int), c.stream));
     if (n > 0) {
       {
@@ -390,7 +183,7 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
       }
       if (ibins > 0) {
         TimedLaunch t(c, "neigh_build");
-        auto k = a.half ? (packed ? k_neigh_bin<true, true> : k_neigh_bin<true, false>)
+        auto k = c.half_neigh ? (packed ? k_neigh_bin<true, true> : k_neigh_bin<true, false>)
                         : (packed ? k_neigh_bin<false, true> : k_neigh_bin<false, false>);
         k<<<(ibins + NB_WARPS - 1) / NB_WARPS, NB_THREADS, 0, c.stream>>>(a);
         EMD_CHECK_LAUNCH();
