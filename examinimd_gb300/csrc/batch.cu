@@ -19,11 +19,15 @@
 // captures a run's launches (`steps_per_launch` steps each) in a CUDA graph.
 //
 // A second, phased form keeps the per-system rebuild (wrap, halo, binning)
-// on one CTA per system.  It runs every other phase (NVE, neighbour rows,
-// halo refresh, force) as one launch over 128-atom chunks of all systems,
-// so one large system no longer sets the time of a step.  All of a run's
-// launches again go into one CUDA graph.  Both forms do the same per-atom
-// arithmetic in the same order.
+// on one CTA per system and runs the rest over chunks of all systems, so one
+// large system no longer sets the time of a step.  A step is two launches: halo
+// refresh (or, on a rebuild step, the rebuild and the neighbour rows, a warp
+// per bin), then force, final half kick and the next step's half kick and drift
+// in one kernel that writes the new positions to a second set of buffers, since
+// other atoms still read the old ones.  All of a run's launches again go into one
+// CUDA graph.  Both forms do the same per-atom arithmetic in the same order.
+// 1,360,000 atoms in 256 systems, ms per 20 steps: 9.7 with a launch per phase and
+// rows an atom per thread, 6.7 as it is.
 //
 // emd_batch_tune picks the form, the CTA size and the steps per launch by
 // timing the candidates on the ensemble itself.
@@ -43,6 +47,7 @@
 #include "emd_device.cuh"
 #include "emd_internal.h"
 #include "lj_pair.cuh"
+#include "neigh_bin.cuh"
 #include "neigh_rows.cuh"
 
 namespace emd {
@@ -70,6 +75,10 @@ struct BArgs {
   int* owner;      // per particle slot: ghost -> owned particle (system-local)
   int* img;        // per particle slot: 2 bits per dimension, shift + 1
   int* binof;      // per particle slot: system-local bin
+  ushort4* binc;   // per particle slot: its bin's coordinates and img
+  const double* mid;  // k - 0.5: centre of bin k in bin widths
+  double4_32a* xn;    // phased form: the next step's x and xl
+  float4* xln;
   int* perm;       // per particle slot: particles sorted by bin (system-local indices)
   int* binstart;   // per bin slot: first position in perm
   int* num;        // per particle slot (owned): row length
@@ -83,7 +92,6 @@ struct BArgs {
   LJParamsF P;
   int every;
   int step0, nsteps;   // steps step0+1 .. step0+nsteps
-  int mode;            // k_batch: 0 timesteps, 1 initial build + force, 2 wrap / halo / binning only
 };
 
 // inclusive scan within a warp
@@ -121,11 +129,9 @@ __device__ __forceinline__ void bin_coords(const BSys& S, int b, int& bx, int& b
   bz = b % nz;
 }
 
-__device__ __forceinline__ float4 rel_to_bin(const BSys& S, const double4_32a& p, int b) {
-  int bx, by, bz;
-  bin_coords(S, b, bx, by, bz);
-  return make_float4(float(p.x - (bx - 0.5) * S.w[0]), float(p.y - (by - 0.5) * S.w[1]),
-                     float(p.z - (bz - 0.5) * S.w[2]), 0.f);
+__device__ __forceinline__ float4 rel_to_bin(const BArgs& A, const BSys& S, const double4_32a& p, ushort4 b) {
+  return make_float4(float(fma(-A.mid[b.x], S.w[0], p.x)), float(fma(-A.mid[b.y], S.w[1], p.y)),
+                     float(fma(-A.mid[b.z], S.w[2], p.z)), 0.f);
 }
 
 // exact FP64 neighbour test of a candidate inside the FP32 band (out of line:
@@ -186,6 +192,51 @@ __device__ void build_row(const BArgs& A, const BSys& S, int i) {
   if (cnt > A.K) latch_status(A.status, ST_NEIGH);
 }
 
+// floor(x / w), the division only where FP32 leaves it open: one CTA bins a whole
+// system, and three FP64 divisions a particle took most of the rebuild
+__device__ __noinline__ int bin_fp64(double x, double w) { return int(floor(x / w)); }
+__device__ __forceinline__ int bin_of(double x, double w, float winv) {
+  const float t = f32_bits(x) * winv;  // within 2.5e-7 |t|
+  const float b = floorf(t), r = t - b, e = 4e-7f * (fabsf(t) + 1.f);
+  return r < e || r > 1.f - e ? bin_fp64(x, w) : int(b);
+}
+
+// a double's order as an integer's (the integer pipe compares 8 times as fast here)
+__device__ __forceinline__ long long order_key(double v) {
+  const long long b = __double_as_longlong(v);
+  return b >= 0 ? b : (b ^ 0x7fffffffffffffffLL);
+}
+
+// a bin's positions of the permutation into ascending index, by one warp
+__device__ __forceinline__ void sort_bin(int* perm, int n, int lane) {
+  if (n <= 64) {
+    const int v0 = lane < n ? perm[lane] : 0x7fffffff, v1 = lane + 32 < n ? perm[lane + 32] : 0x7fffffff;
+    int r0 = 0, r1 = 0;  // particles before v0, v1
+    for (int k = 0; k < min(n, 32); ++k) {
+      const int u = __shfl_sync(FULL_MASK, v0, k);
+      r0 += u < v0;
+      r1 += u < v1;
+    }
+    for (int k = 32; k < n; ++k) {
+      const int u = __shfl_sync(FULL_MASK, v1, k - 32);
+      r0 += u < v0;
+      r1 += u < v1;
+    }
+    if (lane < n) perm[r0] = v0;
+    if (lane + 32 < n) perm[r1] = v1;
+  } else if (lane == 0) {
+    for (int k = 1; k < n; ++k) {
+      const int v = perm[k];
+      int m = k - 1;
+      while (m >= 0 && perm[m] > v) {
+        perm[m + 1] = perm[m];
+        --m;
+      }
+      perm[m + 1] = v;
+    }
+  }
+}
+
 __device__ void rebuild(const BArgs& A, const BSys& S, int* sh, int* hist) {
   const int tid = threadIdx.x, T = blockDim.x;
   double4_32a* x = A.x + S.base;
@@ -193,6 +244,7 @@ __device__ void rebuild(const BArgs& A, const BSys& S, int* sh, int* hist) {
   int* owner = A.owner + S.base;
   int* img = A.img + S.base;
   int* binof = A.binof + S.base;
+  ushort4* binc = A.binc + S.base;
   int* perm = A.perm + S.base;
   int* bstart = A.binstart + S.bin_base;
   const int n = S.n;
@@ -201,8 +253,9 @@ __device__ void rebuild(const BArgs& A, const BSys& S, int* sh, int* hist) {
     double4_32a p = x[i];
     double* c = &p.x;
     for (int d = 0; d < 3; ++d) {
-      if (c[d] >= S.L[d]) c[d] -= S.L[d];
-      else if (c[d] < 0.0) c[d] += S.L[d];
+      const long long key = order_key(c[d]);
+      if (key >= order_key(S.L[d])) c[d] -= S.L[d];
+      else if (key < -1) c[d] += S.L[d];  // -1: minus zero
     }
     x[i] = p;
     owner[i] = i;
@@ -215,15 +268,15 @@ __device__ void rebuild(const BArgs& A, const BSys& S, int* sh, int* hist) {
   bool over = false;
   for (int d = 0; d < 3; ++d) {
     const int cur = n + ng;
+    const long long klo = order_key(A.cut_nb), khi = order_key(S.L[d] - A.cut_nb);
     for (int c0 = 0; c0 < cur; c0 += T) {
       const int c = c0 + tid;
       bool lo = false, hi = false;
-      double xd = 0.0;
       if (c < cur) {
         const double4_32a p = x[c];
-        xd = d == 0 ? p.x : (d == 1 ? p.y : p.z);
-        lo = xd < A.cut_nb;
-        hi = xd >= S.L[d] - A.cut_nb;
+        const long long key = order_key(d == 0 ? p.x : (d == 1 ? p.y : p.z));
+        lo = key < klo;
+        hi = key >= khi;
       }
       int tot;
       const int pos = block_excl(int(lo) + int(hi), sh, tot);
@@ -257,13 +310,19 @@ __device__ void rebuild(const BArgs& A, const BSys& S, int* sh, int* hist) {
   const int nbt = (S.nb[0] + 2) * (S.nb[1] + 2) * (S.nb[2] + 2);
   for (int b = tid; b < nbt; b += T) hist[b] = 0;
   __syncthreads();
+  const float wi[3] = {float(1.0 / S.w[0]), float(1.0 / S.w[1]), float(1.0 / S.w[2])};
   for (int p = tid; p < np; p += T) {
     const double4_32a q = x[p];
-    const int bx = min(max(int(floor(q.x / S.w[0])) + 1, 0), S.nb[0] + 1);
-    const int by = min(max(int(floor(q.y / S.w[1])) + 1, 0), S.nb[1] + 1);
-    const int bz = min(max(int(floor(q.z / S.w[2])) + 1, 0), S.nb[2] + 1);
+    // owned atoms stay in the interior bins, also one that rounds onto the upper face
+    const int o = p < n ? 1 : 0;
+    const int bx = min(max(bin_of(q.x, S.w[0], wi[0]) + 1, o), S.nb[0] + 1 - o);
+    const int by = min(max(bin_of(q.y, S.w[1], wi[1]) + 1, o), S.nb[1] + 1 - o);
+    const int bz = min(max(bin_of(q.z, S.w[2], wi[2]) + 1, o), S.nb[2] + 1 - o);
     const int b = (bx * (S.nb[1] + 2) + by) * (S.nb[2] + 2) + bz;
     binof[p] = b;
+    const ushort4 c = make_ushort4(bx, by, bz, img[p]);
+    binc[p] = c;
+    xl[p] = rel_to_bin(A, S, q, c);
     atomicAdd(&hist[b], 1);
   }
   __syncthreads();
@@ -284,22 +343,10 @@ __device__ void rebuild(const BArgs& A, const BSys& S, int* sh, int* hist) {
   __syncthreads();
   for (int p = tid; p < np; p += T) perm[atomicAdd(&hist[binof[p]], 1)] = p;
   __syncthreads();
-  for (int b = tid; b < nbt; b += T) {  // insertion sort: bins hold a few dozen particles
-    const int s0 = bstart[b], s1 = bstart[b + 1];
-    for (int k = s0 + 1; k < s1; ++k) {
-      const int v = perm[k];
-      int m = k - 1;
-      while (m >= s0 && perm[m] > v) {
-        perm[m + 1] = perm[m];
-        --m;
-      }
-      perm[m + 1] = v;
-    }
-  }
-  for (int p = tid; p < np; p += T) xl[p] = rel_to_bin(S, x[p], binof[p]);
+  for (int b = tid >> 5; b < nbt; b += T >> 5) sort_bin(perm + bstart[b], bstart[b + 1] - bstart[b], tid & 31);
   __syncthreads();
   // full neighbour list, one owned atom per thread
-  if (A.mode != 2)
+  if (A.nsteps > 0)
     for (int i = tid; i < n; i += T) build_row(A, S, i);
   __syncthreads();
 }
@@ -307,22 +354,22 @@ __device__ void rebuild(const BArgs& A, const BSys& S, int* sh, int* hist) {
 __device__ __forceinline__ void halo_ghost(const BArgs& A, const BSys& S, int g) {
   double4_32a* x = A.x + S.base;
   double4_32a p = x[A.owner[S.base + g]];
-  const int im = A.img[S.base + g];
-  p.x += ((im & 3) - 1) * S.L[0];
-  p.y += (((im >> 2) & 3) - 1) * S.L[1];
-  p.z += (((im >> 4) & 3) - 1) * S.L[2];
+  const ushort4 b = A.binc[S.base + g];
+  auto shift = [](int code, double L) { return code == 1 ? 0.0 : (code == 2 ? L : -L); };
+  p.x += shift(b.w & 3, S.L[0]);
+  p.y += shift((b.w >> 2) & 3, S.L[1]);
+  p.z += shift((b.w >> 4) & 3, S.L[2]);
   x[g] = p;
-  A.xl[S.base + g] = rel_to_bin(S, p, A.binof[S.base + g]);
+  A.xl[S.base + g] = rel_to_bin(A, S, p, b);
 }
 
 __device__ void halo_refresh(const BArgs& A, const BSys& S, int ng) {
   for (int g = S.n + threadIdx.x; g < S.n + ng; g += blockDim.x) halo_ghost(A, S, g);
 }
 
-__device__ __forceinline__ void force_atom(const BArgs& A, const BSys& S, int i) {
+__device__ __forceinline__ double3 force_of(const BArgs& A, const BSys& S, int i) {
   const float4* xl = A.xl + S.base;
   const int4* rows4 = reinterpret_cast<const int4*>(A.rows + S.row_base);
-  double* f = A.f + 3 * size_t(S.base);
   PairCtx C;
   C.xi = xl[i];
   C.i = i;
@@ -343,9 +390,16 @@ __device__ __forceinline__ void force_atom(const BArgs& A, const BSys& S, int i)
     t.w = self;
     lj_quad<true>(C, t, xl, A.P, acc);
   }
-  f[3 * i] = double(acc.sxy.x) - double(acc.cxy.x);
-  f[3 * i + 1] = double(acc.sxy.y) - double(acc.cxy.y);
-  f[3 * i + 2] = double(acc.sz) - double(acc.cz);
+  return make_double3(double(acc.sxy.x) - double(acc.cxy.x), double(acc.sxy.y) - double(acc.cxy.y),
+                      double(acc.sz) - double(acc.cz));
+}
+
+__device__ __forceinline__ void force_atom(const BArgs& A, const BSys& S, int i) {
+  const double3 t = force_of(A, S, i);
+  double* f = A.f + 3 * size_t(S.base);
+  f[3 * i] = t.x;
+  f[3 * i + 1] = t.y;
+  f[3 * i + 2] = t.z;
 }
 
 __device__ void force(const BArgs& A, const BSys& S) {
@@ -368,7 +422,7 @@ __device__ __forceinline__ void nve_initial_atom(const BArgs& A, const BSys& S, 
   p.y = fma(A.dt, vy, p.y);
   p.z = fma(A.dt, vz, p.z);
   x[i] = p;
-  A.xl[S.base + i] = rel_to_bin(S, p, A.binof[S.base + i]);
+  A.xl[S.base + i] = rel_to_bin(A, S, p, A.binc[S.base + i]);
 }
 
 // IntegratorNVE::final_integrate
@@ -380,16 +434,14 @@ __device__ __forceinline__ void nve_final_atom(const BArgs& A, const BSys& S, in
   v[3 * i + 2] = fma(A.dtf, f[3 * i + 2], v[3 * i + 2]);
 }
 
-// Persistent form: one CTA advances one system.  mode 1: initial build +
-// force; mode 2: wrap, halo and binning only (the phased form's rebuild);
-// mode 0: nsteps timesteps.
+// One CTA per system: nsteps timesteps (the persistent form), or with nsteps = 0
+// wrap, halo and binning only (the phased form's rebuild).
 __global__ void __launch_bounds__(BATCH_MAX_THREADS) k_batch(BArgs A) {
   extern __shared__ int hist[];
   __shared__ int sh[33];
   const BSys S = A.sys[blockIdx.x];
-  if (A.mode != 0) {
+  if (A.nsteps == 0) {
     rebuild(A, S, sh, hist);
-    if (A.mode == 1) force(A, S);
     return;
   }
   int ng = A.nghost[blockIdx.x];
@@ -411,29 +463,91 @@ __global__ void __launch_bounds__(BATCH_MAX_THREADS) k_batch(BArgs A) {
   }
 }
 
-// Phased form: one launch per phase over every system, 128-atom chunks of
-// one system per CTA (chunk table: system, first atom; ghosts relative to
-// the first ghost slot).
+// Phased form: 128-atom chunks of one system per CTA (chunk table: system,
+// first atom; ghosts relative to the first ghost slot), bins for the rows.
 constexpr int BP_THREADS = 128;
 struct BChunk {
   int sys, first;
 };
-enum { BP_NVE_INITIAL = 0, BP_NEIGH = 1, BP_FORCE = 2, BP_NVE_FINAL = 3, BP_HALO = 4 };
+enum { BP_NVE_INITIAL, BP_HALO, BP_FORCE, BP_STEP, BP_LAST };
 
-__global__ void __launch_bounds__(BP_THREADS) k_batch_phase(BArgs A, const BChunk* __restrict__ chunks, int phase) {
+template <int PHASE>
+__global__ void __launch_bounds__(BP_THREADS) k_batch_phase(BArgs A, const BChunk* __restrict__ chunks) {
   const BChunk ch = chunks[blockIdx.x];
   const BSys& S = A.sys[ch.sys];
   const int k = ch.first + threadIdx.x;
-  if (phase == BP_HALO) {
+  if (PHASE == BP_HALO) {
     const int ng = min(A.nghost[ch.sys], S.cap - S.n);
     if (k < ng) halo_ghost(A, S, S.n + k);
     return;
   }
   if (k >= S.n) return;
-  if (phase == BP_NVE_INITIAL) nve_initial_atom(A, S, k);
-  else if (phase == BP_NEIGH) build_row(A, S, k);
-  else if (phase == BP_FORCE) force_atom(A, S, k);
-  else nve_final_atom(A, S, k);
+  if (PHASE == BP_NVE_INITIAL) {
+    nve_initial_atom(A, S, k);
+    return;
+  }
+  if (PHASE == BP_FORCE) {
+    force_atom(A, S, k);
+    return;
+  }
+  // force and final half kick; BP_STEP: also the next step's half kick and drift
+  const double3 f = force_of(A, S, k);
+  double* v = A.v + 3 * size_t(S.base + k);
+  double vx = fma(A.dtf, f.x, v[0]), vy = fma(A.dtf, f.y, v[1]), vz = fma(A.dtf, f.z, v[2]);
+  if (PHASE == BP_STEP) {
+    vx = fma(A.dtf, f.x, vx);
+    vy = fma(A.dtf, f.y, vy);
+    vz = fma(A.dtf, f.z, vz);
+    double4_32a p = A.x[S.base + k];
+    p.x = fma(A.dt, vx, p.x);
+    p.y = fma(A.dt, vy, p.y);
+    p.z = fma(A.dt, vz, p.z);
+    A.xn[S.base + k] = p;
+    A.xln[S.base + k] = rel_to_bin(A, S, p, A.binc[S.base + k]);
+  } else {
+    double* fo = A.f + 3 * size_t(S.base + k);
+    fo[0] = f.x;
+    fo[1] = f.y;
+    fo[2] = f.z;
+  }
+  v[0] = vx;
+  v[1] = vy;
+  v[2] = vz;
+}
+
+// neighbour rows, one warp per interior bin
+constexpr int BR_WARPS = 4;
+__global__ void __launch_bounds__(32 * BR_WARPS) k_batch_rows(BArgs A, const BChunk* __restrict__ chunks) {
+  __shared__ __align__(16) RowStage st[BR_WARPS];
+  const BChunk ch = chunks[blockIdx.x];
+  const BSys& S = A.sys[ch.sys];
+  const int warp = threadIdx.x >> 5, bin = ch.first + warp;
+  if (bin >= S.nb[0] * S.nb[1] * S.nb[2]) return;
+  RowArgs r;
+  r.x4 = A.x + S.base;
+  r.xl = A.xl + S.base;
+  r.permute = A.perm + S.base;
+  r.nby = S.nb[1] + 2;
+  r.nbz = S.nb[2] + 2;
+  r.wx = float(S.w[0]);
+  r.wy = float(S.w[1]);
+  r.wz = float(S.w[2]);
+  r.n_local = S.n;
+  r.newton = 0;
+  r.cutsq = A.cutsq_nb;
+  r.cut_lo = A.nb_lo;
+  r.cut_hi = A.nb_hi;
+  r.num_neighs = A.num + S.base;
+  r.rows = A.rows + S.row_base;
+  r.stride = S.n;
+  r.K = A.K;
+  const int* bstart = A.binstart + S.bin_base;
+  const int mx = rows_of_bin<false, true>(r, st[warp], bin / (S.nb[1] * S.nb[2]) + 1, (bin / S.nb[2]) % S.nb[1] + 1,
+                                          bin % S.nb[2] + 1, [&](int b, int& off) {
+                                            off = bstart[b];
+                                            return bstart[b + 1] - off;
+                                          });
+  if (mx > A.K && (threadIdx.x & 31) == 0) latch_status(A.status, ST_NEIGH);
 }
 
 // per system: sum m v^2 over owned atoms and the shifted LJ energy (FP64,
@@ -488,9 +602,10 @@ struct emd_batch {
   std::vector<long long> in_off;  // caller's atom offsets
   std::vector<BSys> sys;        // device order
   BSys* d_sys = nullptr;
-  DevBuf<double4_32a> x;
-  DevBuf<float4> xl;
-  DevBuf<double> v, f, thermo;
+  DevBuf<double4_32a> x, x2;  // a.x is one of the two
+  DevBuf<float4> xl, xl2;
+  DevBuf<double> v, f, thermo, mid;
+  DevBuf<ushort4> binc;
   DevBuf<int> owner, img, binof, perm, binstart, num, rows, nghost;
   BArgs a{};
   double mass = 1.0, lj1 = 0, lj2 = 0, cutsq = 0;
@@ -498,11 +613,12 @@ struct emd_batch {
   size_t smem = 0;
   long long steps_done = 0;
   size_t slots = 0;  // particle slots over all systems (owned + ghost capacity)
-  // phased form: chunk tables of the owned atoms and of the ghost capacity
+  // phased form: chunk tables of the owned atoms, of the ghost capacity and of the bins
   bool phased = false;
   BChunk* d_chunks = nullptr;
   BChunk* d_gchunks = nullptr;
-  int n_chunks = 0, n_gchunks = 0;
+  BChunk* d_bchunks = nullptr;
+  int n_chunks = 0, n_gchunks = 0, n_bchunks = 0;
 };
 
 namespace {
@@ -531,34 +647,40 @@ void batch_check(emd_batch* b) {
   if (st) throw Error(EMD_ERR_BOUNDS, "batch: device status " + std::to_string(st));
 }
 
-// persistent launch: nsteps timesteps, or (nsteps == 0) the initial build and force
-void batch_launch(emd_batch* b, int step0, int nsteps, int threads, int mode = -1) {
+// nsteps timesteps, or (nsteps == 0) wrap, halo and binning
+void batch_launch(emd_batch* b, int step0, int nsteps, int threads) {
   BArgs a = b->a;
   a.step0 = step0;
   a.nsteps = nsteps;
-  a.mode = mode >= 0 ? mode : (nsteps == 0 ? 1 : 0);
   k_batch<<<b->nsys, threads, b->smem, b->stream>>>(a);
   EMD_CHECK_LAUNCH();
 }
 
-void batch_phase(emd_batch* b, int phase) {
-  const bool ghosts = phase == BP_HALO;
-  k_batch_phase<<<ghosts ? b->n_gchunks : b->n_chunks, BP_THREADS, 0, b->stream>>>(
-      b->a, ghosts ? b->d_gchunks : b->d_chunks, phase);
+template <int PHASE>
+void batch_phase(emd_batch* b) {
+  const bool ghosts = PHASE == BP_HALO;
+  k_batch_phase<PHASE><<<ghosts ? b->n_gchunks : b->n_chunks, BP_THREADS, 0, b->stream>>>(
+      b->a, ghosts ? b->d_gchunks : b->d_chunks);
   EMD_CHECK_LAUNCH();
 }
 
-// one timestep of the phased form
-void batch_phased_step(emd_batch* b, long long step, int threads) {
-  batch_phase(b, BP_NVE_INITIAL);
+void batch_rebuild(emd_batch* b, int threads) {
+  batch_launch(b, 0, 0, threads);
+  k_batch_rows<<<b->n_bchunks, 32 * BR_WARPS, 0, b->stream>>>(b->a, b->d_bchunks);
+  EMD_CHECK_LAUNCH();
+}
+
+// one timestep of the phased form; the drift to the next one is part of it
+void batch_phased_step(emd_batch* b, long long step, int threads, bool last) {
   if (step % b->a.every == 0) {
-    batch_launch(b, 0, 0, threads, 2);  // per system: wrap, halo, binning
-    batch_phase(b, BP_NEIGH);
+    batch_rebuild(b, threads);
   } else {
-    batch_phase(b, BP_HALO);
+    batch_phase<BP_HALO>(b);
   }
-  batch_phase(b, BP_FORCE);
-  batch_phase(b, BP_NVE_FINAL);
+  if (last) return batch_phase<BP_LAST>(b);
+  batch_phase<BP_STEP>(b);
+  std::swap(b->a.x, b->a.xn);
+  std::swap(b->a.xl, b->a.xln);
 }
 
 // runs nsteps in one CUDA graph: ceil(nsteps / spl) persistent launches, or
@@ -566,10 +688,18 @@ void batch_phased_step(emd_batch* b, long long step, int threads) {
 void batch_run(emd_batch* b, int nsteps, int threads, int spl, bool phased) {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  const BArgs before = b->a;
+  if (phased) {
+    b->x2.reserve(b->slots, b->stream);
+    b->xl2.reserve(b->slots, b->stream);
+    b->a.xn = b->a.x == b->x.p ? b->x2.p : b->x.p;
+    b->a.xln = b->a.xl == b->xl.p ? b->xl2.p : b->xl.p;
+  }
   EMD_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   try {
     if (phased) {
-      for (int s = 1; s <= nsteps; ++s) batch_phased_step(b, b->steps_done + s, threads);
+      batch_phase<BP_NVE_INITIAL>(b);
+      for (int s = 1; s <= nsteps; ++s) batch_phased_step(b, b->steps_done + s, threads, s == nsteps);
     } else {
       for (int s = 0; s < nsteps; s += spl)
         batch_launch(b, int(b->steps_done + s), std::min(spl, nsteps - s), threads);
@@ -577,6 +707,7 @@ void batch_run(emd_batch* b, int nsteps, int threads, int spl, bool phased) {
   } catch (...) {
     cudaStreamEndCapture(b->stream, &graph);
     if (graph) cudaGraphDestroy(graph);
+    b->a = before;
     throw;
   }
   EMD_CUDA(cudaStreamEndCapture(b->stream, &graph));
@@ -584,6 +715,7 @@ void batch_run(emd_batch* b, int nsteps, int threads, int spl, bool phased) {
   if (e == cudaSuccess) e = cudaGraphLaunch(exec, b->stream);
   if (exec) cudaGraphExecDestroy(exec);
   cudaGraphDestroy(graph);
+  if (e != cudaSuccess) b->a = before;
   EMD_CUDA(e);
   b->steps_done += nsteps;
 }
@@ -629,7 +761,8 @@ emd_status emd_batch_create(emd_batch** out, int device, int nsys, const int* na
   std::iota(b->order.begin(), b->order.end(), 0);
   std::stable_sort(b->order.begin(), b->order.end(), [&](int p, int q) { return natoms[p] > natoms[q]; });
   long long slot = 0, bins = 0, rows = 0;
-  int max_bins = 0;
+  int max_bins = 0, max_dim = 0;
+  double max_w = 0.0;
   for (int s = 0; s < nsys; ++s) {
     const int k = b->order[size_t(s)];
     BSys S{};
@@ -639,6 +772,8 @@ emd_status emd_batch_create(emd_batch** out, int device, int nsys, const int* na
       require(S.L[d] > 2.0 * cut_nb, EMD_ERR_ARG, "emd_batch_create: every box edge must exceed 2 (cut + skin)");
       S.nb[d] = std::max(1, int(std::floor(S.L[d] / cut_nb)));
       S.w[d] = S.L[d] / S.nb[d];
+      max_dim = std::max(max_dim, S.nb[d] + 2);
+      max_w = std::max(max_w, S.w[d]);
       vol *= S.L[d];
       outer *= S.L[d] + 2.0 * cut_nb;
     }
@@ -668,6 +803,7 @@ emd_status emd_batch_create(emd_batch** out, int device, int nsys, const int* na
   b->owner.reserve(ns, b->stream);
   b->img.reserve(ns, b->stream);
   b->binof.reserve(ns, b->stream);
+  b->binc.reserve(ns, b->stream);
   b->perm.reserve(ns, b->stream);
   b->num.reserve(ns, b->stream);
   b->binstart.reserve(size_t(bins), b->stream);
@@ -677,14 +813,23 @@ emd_status emd_batch_create(emd_batch** out, int device, int nsys, const int* na
   EMD_CUDA(device_malloc(reinterpret_cast<void**>(&b->d_sys), sizeof(BSys) * size_t(nsys)));
   EMD_CUDA(cudaMemcpyAsync(b->d_sys, b->sys.data(), sizeof(BSys) * size_t(nsys), cudaMemcpyHostToDevice, b->stream));
   {
-    std::vector<BChunk> ch, gch;
+    std::vector<double> mid;
+    for (int k = 0; k < max_dim; ++k) mid.push_back(k - 0.5);
+    b->mid.reserve(mid.size(), b->stream);
+    EMD_CUDA(cudaMemcpyAsync(b->mid.p, mid.data(), sizeof(double) * mid.size(), cudaMemcpyHostToDevice, b->stream));
+    std::vector<BChunk> ch, gch, bch;
     for (int s = 0; s < nsys; ++s) {
       const BSys& S = b->sys[size_t(s)];
       for (int f0 = 0; f0 < S.n; f0 += BP_THREADS) ch.push_back(BChunk{s, f0});
       for (int f0 = 0; f0 < S.cap - S.n; f0 += BP_THREADS) gch.push_back(BChunk{s, f0});
+      for (int f0 = 0; f0 < S.nb[0] * S.nb[1] * S.nb[2]; f0 += BR_WARPS) bch.push_back(BChunk{s, f0});
     }
     b->n_chunks = int(ch.size());
     b->n_gchunks = int(gch.size());
+    b->n_bchunks = int(bch.size());
+    EMD_CUDA(device_malloc(reinterpret_cast<void**>(&b->d_bchunks), sizeof(BChunk) * bch.size()));
+    EMD_CUDA(cudaMemcpyAsync(b->d_bchunks, bch.data(), sizeof(BChunk) * bch.size(), cudaMemcpyHostToDevice,
+                             b->stream));
     EMD_CUDA(device_malloc(reinterpret_cast<void**>(&b->d_chunks), sizeof(BChunk) * ch.size()));
     EMD_CUDA(device_malloc(reinterpret_cast<void**>(&b->d_gchunks), sizeof(BChunk) * gch.size()));
     EMD_CUDA(cudaMemcpyAsync(b->d_chunks, ch.data(), sizeof(BChunk) * ch.size(), cudaMemcpyHostToDevice, b->stream));
@@ -718,6 +863,8 @@ emd_status emd_batch_create(emd_batch** out, int device, int nsys, const int* na
   a.owner = b->owner.p;
   a.img = b->img.p;
   a.binof = b->binof.p;
+  a.binc = b->binc.p;
+  a.mid = b->mid.p;
   a.perm = b->perm.p;
   a.binstart = b->binstart.p;
   a.num = b->num.p;
@@ -729,8 +876,9 @@ emd_status emd_batch_create(emd_batch** out, int device, int nsys, const int* na
   a.dtf = 0.5 * dt / mass;
   a.cut_nb = cut_nb;
   a.cutsq_nb = cut_nb * cut_nb;
-  a.nb_lo = float(a.cutsq_nb * (1.0 - 4e-5));
-  a.nb_hi = float(a.cutsq_nb * (1.0 + 4e-5));
+  const double band = row_band(max_w, cut_nb);
+  a.nb_lo = float(a.cutsq_nb * (1.0 - band));
+  a.nb_hi = float(a.cutsq_nb * (1.0 + band));
   b->lj1 = 48.0 * eps * std::pow(sigma, 12.0);
   b->lj2 = 24.0 * eps * std::pow(sigma, 6.0);
   b->cutsq = cut * cut;
@@ -740,7 +888,8 @@ emd_status emd_batch_create(emd_batch** out, int device, int nsys, const int* na
   cudaDeviceProp prop{};
   EMD_CUDA(cudaGetDeviceProperties(&prop, device));
   b->threads = 512;
-  batch_launch(b, 0, 0, b->threads);
+  batch_rebuild(b, b->threads);
+  batch_phase<BP_FORCE>(b);
   batch_check(b);
   *out = b;
   return EMD_OK;
@@ -763,12 +912,17 @@ void emd_batch_destroy(emd_batch* b) {
   for (auto* p : {&b->owner, &b->img, &b->binof, &b->perm, &b->binstart, &b->num, &b->rows, &b->nghost}) p->release();
   b->x.release();
   b->xl.release();
+  b->x2.release();
+  b->xl2.release();
+  b->mid.release();
+  b->binc.release();
   b->v.release();
   b->f.release();
   b->thermo.release();
   if (b->d_sys) cudaFree(b->d_sys);
   if (b->d_chunks) cudaFree(b->d_chunks);
   if (b->d_gchunks) cudaFree(b->d_gchunks);
+  if (b->d_bchunks) cudaFree(b->d_bchunks);
   if (b->d_status) cudaFree(b->d_status);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
@@ -806,7 +960,7 @@ emd_status emd_batch_tune(emd_batch* b, int trial_steps, int* threads_out, int* 
   x0.reserve(ns, b->stream);
   v0.reserve(3 * ns, b->stream);
   f0.reserve(3 * ns, b->stream);
-  EMD_CUDA(cudaMemcpyAsync(x0.p, b->x.p, sizeof(double4_32a) * ns, cudaMemcpyDeviceToDevice, b->stream));
+  EMD_CUDA(cudaMemcpyAsync(x0.p, b->a.x, sizeof(double4_32a) * ns, cudaMemcpyDeviceToDevice, b->stream));
   EMD_CUDA(cudaMemcpyAsync(v0.p, b->v.p, sizeof(double) * 3 * ns, cudaMemcpyDeviceToDevice, b->stream));
   EMD_CUDA(cudaMemcpyAsync(f0.p, b->f.p, sizeof(double) * 3 * ns, cudaMemcpyDeviceToDevice, b->stream));
   const long long saved_steps = b->steps_done;
@@ -822,11 +976,12 @@ emd_status emd_batch_tune(emd_batch* b, int trial_steps, int* threads_out, int* 
     for (int spl : {0, every, 5 * every, trial_steps}) {
       if (spl > trial_steps) continue;
       // state of the trial's start (a rebuild step boundary)
-      EMD_CUDA(cudaMemcpyAsync(b->x.p, x0.p, sizeof(double4_32a) * ns, cudaMemcpyDeviceToDevice, b->stream));
+      EMD_CUDA(cudaMemcpyAsync(b->a.x, x0.p, sizeof(double4_32a) * ns, cudaMemcpyDeviceToDevice, b->stream));
       EMD_CUDA(cudaMemcpyAsync(b->v.p, v0.p, sizeof(double) * 3 * ns, cudaMemcpyDeviceToDevice, b->stream));
       EMD_CUDA(cudaMemcpyAsync(b->f.p, f0.p, sizeof(double) * 3 * ns, cudaMemcpyDeviceToDevice, b->stream));
       b->steps_done = saved_steps;
-      batch_launch(b, 0, 0, threads);  // rebuild from the restored positions
+      batch_rebuild(b, threads);  // from the restored positions
+      batch_phase<BP_FORCE>(b);
       EMD_CUDA(cudaEventRecord(e0, b->stream));
       batch_run(b, trial_steps, threads, std::max(spl, 1), spl == 0);
       EMD_CUDA(cudaEventRecord(e1, b->stream));
@@ -841,11 +996,12 @@ emd_status emd_batch_tune(emd_batch* b, int trial_steps, int* threads_out, int* 
       }
     }
   }
-  EMD_CUDA(cudaMemcpyAsync(b->x.p, x0.p, sizeof(double4_32a) * ns, cudaMemcpyDeviceToDevice, b->stream));
+  EMD_CUDA(cudaMemcpyAsync(b->a.x, x0.p, sizeof(double4_32a) * ns, cudaMemcpyDeviceToDevice, b->stream));
   EMD_CUDA(cudaMemcpyAsync(b->v.p, v0.p, sizeof(double) * 3 * ns, cudaMemcpyDeviceToDevice, b->stream));
   EMD_CUDA(cudaMemcpyAsync(b->f.p, f0.p, sizeof(double) * 3 * ns, cudaMemcpyDeviceToDevice, b->stream));
   b->steps_done = saved_steps;
-  batch_launch(b, 0, 0, bt);
+  batch_rebuild(b, bt);
+  batch_phase<BP_FORCE>(b);
   batch_check(b);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -865,7 +1021,7 @@ emd_status emd_batch_get(emd_batch* b, double* x, double* v, double* f) {
   const size_t ns = b->slots;
   std::vector<double4_32a> hx(x ? ns : 0);
   std::vector<double> hv(v ? 3 * ns : 0), hf(f ? 3 * ns : 0);
-  if (x) EMD_CUDA(cudaMemcpyAsync(hx.data(), b->x.p, sizeof(double4_32a) * ns, cudaMemcpyDeviceToHost, b->stream));
+  if (x) EMD_CUDA(cudaMemcpyAsync(hx.data(), b->a.x, sizeof(double4_32a) * ns, cudaMemcpyDeviceToHost, b->stream));
   if (v) EMD_CUDA(cudaMemcpyAsync(hv.data(), b->v.p, sizeof(double) * 3 * ns, cudaMemcpyDeviceToHost, b->stream));
   if (f) EMD_CUDA(cudaMemcpyAsync(hf.data(), b->f.p, sizeof(double) * 3 * ns, cudaMemcpyDeviceToHost, b->stream));
   EMD_CUDA(cudaStreamSynchronize(b->stream));

@@ -1,0 +1,47 @@
+"""The batch's phased form (rows by bin masks, force and integration in one kernel,
+two sets of position buffers) against its persistent form (rows and force an atom
+per thread, in place), which does the same arithmetic: equal bits.  GPU.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+A = (4.0 / 0.8442) ** (1.0 / 3.0)
+BASIS = np.array([(0, 0, 0), (0.5, 0.5, 0), (0.5, 0, 0.5), (0, 0.5, 0.5)])
+
+
+def _system(cells, rng):
+    g = np.stack(np.meshgrid(*[np.arange(k) for k in cells], indexing="ij"), -1).reshape(-1, 3)
+    x = ((g[:, None, :] + BASIS[None]) * A).reshape(-1, 3)
+    box = A * np.asarray(cells, float)
+    x = np.mod(x + 0.05 * rng.standard_normal(x.shape), box)
+    # atoms on the faces: bins of the first and the last layer, wraps either way
+    x[0] = 0.0
+    x[1, 2] = np.nextafter(box[2], 0.0)
+    x[2, 1] = np.nextafter(box[1], 0.0)
+    x[3, 0] = 0.0
+    v = 1.2 * rng.standard_normal(x.shape)
+    return x, v, box
+
+
+@pytest.mark.parametrize("systems", [[(4, 4, 4)], [(4, 5, 9), (5, 4, 4), (11, 6, 4)], [(14, 13, 12), (4, 4, 4)]])
+@pytest.mark.parametrize("runs", [(41,), (1, 2, 17, 20, 5)])
+def test_phased_equals_persistent(systems, runs):
+    from examinimd_gb300 import Batch
+    rng = np.random.default_rng(11)
+    parts = [_system(c, rng) for c in systems]
+    ns = [len(p[0]) for p in parts]
+    boxes = np.array([p[2] for p in parts])
+    x, v = np.concatenate([p[0] for p in parts]), np.concatenate([p[1] for p in parts])
+    out = []
+    for threads, spl in ((256, 7), (512, 0)):
+        b = Batch(ns, boxes, x, v, dt=0.0005)
+        b.set_shape(threads, spl)
+        for k in runs:
+            b.run(k)
+        out.append([*b.get(), *b.thermo()])
+        b.close()
+    assert np.all(np.isfinite(out[0][0]))
+    for p, q in zip(*out):
+        np.testing.assert_array_equal(p, q)
