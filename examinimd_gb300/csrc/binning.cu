@@ -4,8 +4,8 @@
 // flattened with x slowest (the decode of binning_kksort.cpp:61-63).  The
 // permutation is a stable counting sort: each bin lists its particles in
 // ascending index, which is what a serial BinSort produces.  Four kernels:
-// bin + histogram, scan, scatter through per-bin cursors, and a per-bin
-// rank pass that restores ascending order inside each bin.  With sort=true
+// bin + histogram (whose counts number a bin's members), scan, scatter, and a
+// per-bin rank pass that restores ascending order inside each bin.  With sort=true
 // a gather reorders x, v, f, type, id, q of the binned range.
 #include <algorithm>
 
@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(256) k_bin_index(const double4_32a* __restrict
                                                    int nby, int nbz, double minx, double miny, double minz,
                                                    double mulx, double muly, double mulz,
                                                    const double* __restrict__ ctab, int* __restrict__ binof,
-                                                   int* __restrict__ bincount, float4* __restrict__ xl,
+                                                   int* __restrict__ slot, int* __restrict__ bincount, float4* __restrict__ xl,
                                                    unsigned* status) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
@@ -49,20 +49,18 @@ __global__ void __launch_bounds__(256) k_bin_index(const double4_32a* __restrict
   }
   const int b = (ix * nby + iy) * nbz + iz;
   binof[r] = b;
-  atomicAdd(&bincount[b], 1);
+  slot[r] = atomicAdd(&bincount[b], 1);
   // FP32 position relative to the bin centre, for the neighbour candidate tests
   xl[first + r] = make_float4(float(p.x - ctab[ix]), float(p.y - ctab[nbx + iy]), float(p.z - ctab[nbx + nby + iz]),
                               __int_as_float(int(p.w)));
 }
 
 __global__ void __launch_bounds__(256) k_bin_scatter(const int* __restrict__ binof, int n,
-                                                     const int* __restrict__ binoffsets, int* __restrict__ cursor,
-                                                     int* __restrict__ perm_tmp) {
+                                                     const int* __restrict__ binoffsets,
+                                                     const int* __restrict__ slot, int* __restrict__ perm_tmp) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
-  const int b = binof[r];
-  const int slot = atomicAdd(&cursor[b], 1);
-  perm_tmp[binoffsets[b] + slot] = r;
+  perm_tmp[binoffsets[binof[r]] + slot[r]] = r;
 }
 
 // One warp per bin: each member's rank = number of members with a smaller
@@ -104,6 +102,27 @@ __global__ void __launch_bounds__(256) k_sort_gather(const int* __restrict__ per
   oid[r] = id[s];
 }
 
+// the sorted fields back in place, in one launch
+__global__ void __launch_bounds__(256) k_sort_copy(int n, const double4_32a* __restrict__ x4,
+                                                   const double* __restrict__ d, const int* __restrict__ t,
+                                                   double4_32a* __restrict__ ox4, double* __restrict__ ov,
+                                                   double* __restrict__ of, double* __restrict__ oq,
+                                                   int* __restrict__ otype, int* __restrict__ oid) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  ox4[r] = x4[r];
+  const size_t m = size_t(n);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const size_t e = r + k * m;
+    ov[e] = d[e];
+    of[e] = d[3 * m + e];
+  }
+  oq[r] = d[6 * m + r];
+  otype[r] = t[r];
+  oid[r] = t[m + r];
+}
+
 }  // namespace
 }  // namespace emd
 
@@ -141,27 +160,30 @@ emd_status emd_binning_create(emd_ctx* ctx, double dx_in, double dy_in, double d
   const int nbins = int(nbins_ll);
   c.bincount.reserve(size_t(nbins) + 1, c.stream);
   c.binoffsets.reserve(size_t(nbins) + 1, c.stream);
-  c.bin_cursor.reserve(size_t(nbins) + 1, c.stream);
   c.binof.reserve(size_t(n) + 1, c.stream);
   c.permute.reserve(size_t(n) + 1, c.stream);
   c.perm_tmp.reserve(size_t(n) + 1, c.stream);
+  c.bin_slot.reserve(size_t(n) + 1, c.stream);
   EMD_CUDA(cudaMemsetAsync(c.bincount.p, 0, sizeof(int) * nbins, c.stream));
-  EMD_CUDA(cudaMemsetAsync(c.bin_cursor.p, 0, sizeof(int) * nbins, c.stream));
   c.xl_bin.reserve(size_t(first + n) + 1, c.stream, true);
   const int ntab = nb[0] + nb[1] + nb[2];
-  c.bin_ctab.reserve(size_t(ntab), c.stream);
-  {
+  // a box binned as before keeps its table
+  const double key[9] = {double(nb[0]), double(nb[1]), double(nb[2]), c.bmin[0], c.bmin[1],
+                         c.bmin[2],     c.bmax[0],     c.bmax[1],     c.bmax[2]};
+  if (size_t(ntab) > c.bin_ctab.cap || !std::equal(key, key + 9, c.bin_ctab_key)) {
+    c.bin_ctab.reserve(size_t(ntab), c.stream);
     TimedLaunch t(c, "bin_ctab");
     k_bin_ctab<<<blocks_for(ntab, 256), 256, 0, c.stream>>>(
         nb[0], nb[1], nb[2], c.bmin[0], c.bmin[1], c.bmin[2], (c.bmax[0] - c.bmin[0]) / nb[0],
         (c.bmax[1] - c.bmin[1]) / nb[1], (c.bmax[2] - c.bmin[2]) / nb[2], c.bin_ctab.p);
     EMD_CHECK_LAUNCH();
+    std::copy(key, key + 9, c.bin_ctab_key);
   }
   if (n > 0) {
     TimedLaunch t(c, "bin_index");
     k_bin_index<<<blocks_for(n, 256), 256, 0, c.stream>>>(c.x4.p, first, n, nb[0], nb[1], nb[2], c.bmin[0],
                                                           c.bmin[1], c.bmin[2], c.bmul[0], c.bmul[1], c.bmul[2],
-                                                          c.bin_ctab.p, c.binof.p, c.bincount.p, c.xl_bin.p,
+                                                          c.bin_ctab.p, c.binof.p, c.bin_slot.p, c.bincount.p, c.xl_bin.p,
                                                           c.d_status);
     EMD_CHECK_LAUNCH();
   }
@@ -171,7 +193,7 @@ emd_status emd_binning_create(emd_ctx* ctx, double dx_in, double dy_in, double d
   if (n > 0) {
     {
       TimedLaunch t(c, "bin_scatter");
-      k_bin_scatter<<<blocks_for(n, 256), 256, 0, c.stream>>>(c.binof.p, n, c.binoffsets.p, c.bin_cursor.p,
+      k_bin_scatter<<<blocks_for(n, 256), 256, 0, c.stream>>>(c.binof.p, n, c.binoffsets.p, c.bin_slot.p,
                                                               c.perm_tmp.p);
       EMD_CHECK_LAUNCH();
     }
@@ -185,7 +207,7 @@ emd_status emd_binning_create(emd_ctx* ctx, double dx_in, double dy_in, double d
   if (sort && n > 0) {
     c.x_version++;
     // BinSort::sort of x, v, f, type, id, q over the binned range: one
-    // fused gather kernel into staging buffers, then copies back
+    // fused gather kernel into staging buffers, then one copy back
     materialize_zero(c, true, false);
     c.xl_ok = 0;
     const int* perm = c.permute.p;
@@ -200,15 +222,13 @@ emd_status emd_binning_create(emd_ctx* ctx, double dx_in, double dy_in, double d
           c.stage_d.p + 6 * size_t(n), c.stage_i.p, c.stage_i.p + n);
       EMD_CHECK_LAUNCH();
     }
-    EMD_CUDA(cudaMemcpyAsync(c.x4.p + first, c.stage_x4.p, sizeof(double4_32a) * n, cudaMemcpyDeviceToDevice, c.stream));
-    EMD_CUDA(cudaMemcpyAsync(c.v.p + 3 * size_t(first), c.stage_d.p, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice,
-                             c.stream));
-    EMD_CUDA(cudaMemcpyAsync(c.f.p + 3 * size_t(first), c.stage_d.p + 3 * size_t(n), sizeof(double) * 3 * n,
-                             cudaMemcpyDeviceToDevice, c.stream));
-    EMD_CUDA(cudaMemcpyAsync(c.q.p + first, c.stage_d.p + 6 * size_t(n), sizeof(double) * n, cudaMemcpyDeviceToDevice,
-                             c.stream));
-    EMD_CUDA(cudaMemcpyAsync(c.type.p + first, c.stage_i.p, sizeof(int) * n, cudaMemcpyDeviceToDevice, c.stream));
-    EMD_CUDA(cudaMemcpyAsync(c.id.p + first, c.stage_i.p + n, sizeof(int) * n, cudaMemcpyDeviceToDevice, c.stream));
+    {
+      TimedLaunch t(c, "bin_sort_copy");
+      k_sort_copy<<<blocks_for(n, 256), 256, 0, c.stream>>>(n, c.stage_x4.p, c.stage_d.p, c.stage_i.p, c.x4.p + first,
+                                                            c.v.p + 3 * size_t(first), c.f.p + 3 * size_t(first),
+                                                            c.q.p + first, c.type.p + first, c.id.p + first);
+      EMD_CHECK_LAUNCH();
+    }
     c.neigh_ready = false;
     // the bin indices, FP32 offsets and permutation of this binning refer to
     // the order before the sort: no neighbour list is built from it

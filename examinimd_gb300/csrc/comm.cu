@@ -1,9 +1,10 @@
 // CommSerial on the device (comm_serial.h:95-213, comm_serial.cpp:47-127):
-// periodic wrap, six-phase ghost creation with stable (flag + scan)
+// periodic wrap, six-phase ghost creation with stable (count + place)
 // compaction so ghosts land at exactly the indices the serial reference
 // gives them, one-launch ghost position refresh, and the phase-ordered
 // reverse force accumulation.  -fmad=false (pure add/sub anyway).
 #include <algorithm>
+#include <cstring>
 
 #include "emd_device.cuh"
 #include "emd_internal.h"
@@ -29,46 +30,153 @@ __global__ void k_exchange(double4_32a* __restrict__ x4, int n, double lx, doubl
 
 __device__ __forceinline__ double comp(const double4_32a& p, int d) { return d == 0 ? p.x : (d == 1 ? p.y : p.z); }
 
-// TagHaloSelf selection predicate (comm_serial.h:112-181) for both phases
-// of one dimension: flag[i] for the upper face (x >= hi - depth), flag[n + i]
-// for the lower face (x <= lo + depth).  The odd phase's candidates are the
-// even phase's (comm_serial.cpp:68 leaves out only the ghosts the even phase
-// made), so one exclusive scan over the 2n flags ranks the upper face's
-// ghosts first and the lower face's after them, the reference's append order.
-__global__ void k_halo_flag2(const double4_32a* __restrict__ x4, int n, int dim, double bound_hi, double bound_lo,
-                             int* __restrict__ flag) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double c = comp(x4[i], dim);
-  flag[i] = c >= bound_hi ? 1 : 0;
-  flag[n + i] = c <= bound_lo ? 1 : 0;
+// TagHaloSelf (comm_serial.h:112-181) for both phases of one dimension: the
+// upper face's particles (x >= hi - depth, imaged at x - L) in index order, then
+// the lower face's (x <= lo + depth).  The odd phase's candidates are the even
+// phase's (comm_serial.cpp:68 leaves out only the ghosts the even phase made).
+// k_halo_count counts them per tile of the candidates, its last block to finish
+// scans the tiles; k_halo_place finds each particle's rank and writes its image.
+// The number of candidates and the room left are read on the device, so the three
+// dimensions run without a read-back in between: seven operations and one wait
+// (nine launches or copies and a wait per dimension took 150 us in a small system).
+constexpr int HALO_THREADS = 256, HALO_PER = 4, HALO_TILE = HALO_THREADS * HALO_PER;
+struct HaloState {
+  int base[4];     // ghosts before dimension d; after the last
+  int upper[3];    // ghosts of the upper face
+  int overflow;    // particles needed when they were more than the capacity
+  unsigned done[3];  // blocks of k_halo_count that finished
+};
+static_assert(sizeof(HaloState) <= kHostInts * sizeof(int), "read back through the pinned scratch");
+
+// a tile's flags: bit k and 16 + k of the thread's candidate 4 tid + k, upper and lower
+__device__ __forceinline__ int halo_flags(const double4_32a* __restrict__ x4, int first, int n, int dim, double hi,
+                                          double lo) {
+  int m = 0;
+#pragma unroll
+  for (int k = 0; k < HALO_PER; ++k)
+    if (first + k < n) {
+      const double c = comp(x4[first + k], dim);
+      m |= (c >= hi ? 1 << k : 0) | (c <= lo ? 0x10000 << k : 0);
+    }
+  return m;
+}
+__device__ __forceinline__ int halo_counts(int m) { return __popc(m & 0xffff) | __popc(m >> 16) << 16; }
+
+// exclusive block scan (256 threads) and total of an int that holds two 16-bit counts
+__device__ __forceinline__ int halo_scan(int v, int& total) {
+  __shared__ int sh[HALO_THREADS / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(FULL_MASK, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) sh[w] = x;
+  __syncthreads();
+  int off = 0;
+  total = 0;
+#pragma unroll
+  for (int k = 0; k < HALO_THREADS / 32; ++k) {
+    off += k < w ? sh[k] : 0;
+    total += sh[k];
+  }
+  __syncthreads();
+  return off + x - v;
 }
 
-// Appends the flagged particles as shifted copies at dest_base + rank.
-__global__ void k_halo_scatter(double4_32a* __restrict__ x4, double* __restrict__ v, double* __restrict__ q,
-                               int* __restrict__ id, int* __restrict__ type, const int* __restrict__ flag,
-                               const int* __restrict__ rank, int n, int dim, double shift, int dest_base,
-                               int n_local, int* __restrict__ pack, int* __restrict__ owner, int* __restrict__ img,
-                               int img_bit) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !flag[i]) return;
-  const int k = rank[i];
-  const int dst = dest_base + k;
-  double4_32a p = x4[i];
-  if (dim == 0) p.x += shift;
-  else if (dim == 1) p.y += shift;
-  else p.z += shift;
-  x4[dst] = p;
-  v[3 * dst] = v[3 * i];
-  v[3 * dst + 1] = v[3 * i + 1];
-  v[3 * dst + 2] = v[3 * i + 2];
-  q[dst] = q[i];
-  id[dst] = id[i];
-  type[dst] = type[i];
-  pack[k] = i;
-  const int g = dst - n_local;
-  owner[g] = i < n_local ? i : owner[i - n_local];
-  img[g] = (i < n_local ? 0 : img[i - n_local]) | img_bit;
+// tiles: (upper, lower) counts, then ranks of each tile's first
+__global__ void __launch_bounds__(HALO_THREADS) k_halo_count(const double4_32a* __restrict__ x4, int n_local,
+                                                             int capacity, int dim, double hi, double lo,
+                                                             HaloState* st, int2* __restrict__ tiles) {
+  __shared__ bool s_last;
+  __shared__ int s_run[2];
+  const int n = n_local + st->base[dim], nt = (n + HALO_TILE - 1) / HALO_TILE;
+  if (blockIdx.x < nt && !st->overflow) {
+    int total;
+    const int m = halo_flags(x4, blockIdx.x * HALO_TILE + threadIdx.x * HALO_PER, n, dim, hi, lo);
+    halo_scan(halo_counts(m), total);
+    if (threadIdx.x == 0) tiles[blockIdx.x] = int2{total & 0xffff, total >> 16};
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(&st->done[dim], 1u) == gridDim.x - 1;
+    s_run[0] = s_run[1] = 0;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (st->overflow) return;
+  for (int t0 = 0; t0 < nt; t0 += HALO_THREADS) {
+    const int t = t0 + threadIdx.x;
+    const int2 c = t < nt ? __ldcg(tiles + t) : int2{0, 0};
+    // a tile's counts reach 1,024: two scans
+    int tu, tl;
+    const int u = halo_scan(c.x, tu), l = halo_scan(c.y, tl);
+    const int ru = s_run[0], rl = s_run[1];
+    if (t < nt) tiles[t] = int2{ru + u, rl + l};
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_run[0] = ru + tu;
+      s_run[1] = rl + tl;
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    const long long need = (long long)n + s_run[0] + s_run[1];
+    st->upper[dim] = s_run[0];
+    st->base[dim + 1] = st->base[dim] + s_run[0] + s_run[1];
+    if (need > capacity) st->overflow = int(min(need, 0x7fffffffLL));
+  }
+}
+
+__global__ void __launch_bounds__(HALO_THREADS) k_halo_place(double4_32a* __restrict__ x4, double* __restrict__ v,
+                                                             double* __restrict__ q, int* __restrict__ id,
+                                                             int* __restrict__ type, int n_local, int dim, double hi,
+                                                             double lo, double L, const HaloState* __restrict__ st,
+                                                             const int2* __restrict__ tiles, int* __restrict__ pack,
+                                                             int* __restrict__ owner, int* __restrict__ img) {
+  const int base = st->base[dim], n = n_local + base;
+  if (blockIdx.x * HALO_TILE >= n || st->overflow) return;
+  const int first = blockIdx.x * HALO_TILE + threadIdx.x * HALO_PER;
+  const int m = halo_flags(x4, first, n, dim, hi, lo);
+  int total;
+  const int before = halo_scan(halo_counts(m), total);
+  // the tile's images in order, so that every thread copies one at a time
+  __shared__ unsigned short list[2 * HALO_TILE];
+  const int nu = total & 0xffff, nl = total >> 16;
+  int u = before & 0xffff, l = nu + (before >> 16);
+#pragma unroll
+  for (int k = 0; k < HALO_PER; ++k) {
+    if (m >> k & 1) list[u++] = (unsigned short)(threadIdx.x * HALO_PER + k);
+    if (m >> (16 + k) & 1) list[l++] = (unsigned short)(threadIdx.x * HALO_PER + k);
+  }
+  __syncthreads();
+  const int2 tile = tiles[blockIdx.x];
+  for (int e = threadIdx.x; e < nu + nl; e += HALO_THREADS) {
+    const bool lower = e >= nu;
+    const int i = blockIdx.x * HALO_TILE + list[e];
+    const int g = lower ? base + st->upper[dim] + tile.y + e - nu : base + tile.x + e, dst = n_local + g;
+    const double shift = lower ? L : -L;
+    double4_32a p = x4[i];
+    const double v0 = v[3 * size_t(i)], v1 = v[3 * size_t(i) + 1], v2 = v[3 * size_t(i) + 2], qi = q[i];
+    const int idi = id[i], ti = type[i];
+    const int own = i < n_local ? i : owner[i - n_local], im = i < n_local ? 0 : img[i - n_local];
+    if (dim == 0) p.x += shift;
+    else if (dim == 1) p.y += shift;
+    else p.z += shift;
+    x4[dst] = p;
+    v[3 * size_t(dst)] = v0;
+    v[3 * size_t(dst) + 1] = v1;
+    v[3 * size_t(dst) + 2] = v2;
+    q[dst] = qi;
+    id[dst] = idi;
+    type[dst] = ti;
+    pack[g] = i;
+    owner[g] = own;
+    img[g] = im | 1 << (2 * dim + (lower ? 1 : 0));
+  }
 }
 
 // TagHaloUpdateSelf for all six phases at once: every ghost is its owner
@@ -107,17 +215,40 @@ __global__ void k_halo_force(double* __restrict__ f, const int* __restrict__ pac
   f[3 * i + 2] += f[3 * g + 2];
 }
 
+// The six phases of a small halo in order, one block (a launch per phase costs
+// more than its additions): 9,000 ghosts 36 -> @@ us.
+constexpr int HALO_FORCE_MAX = 16384;
+struct HaloPhases {
+  int pack[6], count[6], ghost[6];
+};
+__global__ void __launch_bounds__(1024) k_halo_force_all(double* __restrict__ f, const int* __restrict__ pack,
+                                                         HaloPhases P) {
+  for (int phase = 5; phase >= 0; --phase) {
+    for (int k = threadIdx.x; k < P.count[phase]; k += blockDim.x) {
+      const int i = pack[P.pack[phase] + k], g = P.ghost[phase] + k;
+      f[3 * i] += f[3 * g];
+      f[3 * i + 1] += f[3 * g + 1];
+      f[3 * i + 2] += f[3 * g + 2];
+    }
+    __syncthreads();
+  }
+}
+
 }  // namespace
 
-static void grow_particles(Ctx& c, int need) {
-  if (need <= c.N_max) return;
-  const size_t n = size_t(need) + 1;
+static void reserve_particles(Ctx& c, size_t need) {
+  const size_t n = need + 1;
   c.x4.reserve(n, c.stream, true);
   c.v.reserve(3 * n, c.stream, true);
   c.f.reserve(3 * n, c.stream, true);
   c.q.reserve(n, c.stream, true);
   c.type.reserve(n, c.stream, true);
   c.id.reserve(n, c.stream, true);
+}
+
+static void grow_particles(Ctx& c, int need) {
+  if (need <= c.N_max) return;
+  reserve_particles(c, size_t(need));
   // new force rows are cleared by the per-step deep_copy(f, 0) (emd_zero_forces)
   c.N_max = need;
 }
@@ -154,54 +285,57 @@ emd_status emd_comm_exchange_halo(emd_ctx* ctx, int* n_ghost_out) {
     require(c.comm_depth < c.domain[d], EMD_ERR_ARG,
             "emd_comm_exchange_halo: comm_depth must be smaller than the box (one periodic image per face)");
   const int N_local = c.N_local;
-  int N_ghost = 0;
-  int pack_total = 0;
   c.neigh_ready = false;
   c.xl_ok &= ~2;
-  for (int dim = 0; dim < 3; ++dim) {
-    // phases 2 dim (upper face, image at x - L) and 2 dim + 1 (lower face,
-    // image at x + L) over the same candidates, with one count read-back
-    const double bound_hi = c.sub_hi[dim] - c.comm_depth, bound_lo = c.sub_lo[dim] + c.comm_depth;
-    const int nparticles = N_local + N_ghost;
-    const size_t n2 = 2 * size_t(nparticles);
-    c.flags.reserve(n2 + 1, c.stream);
-    c.flags_scan.reserve(n2 + 2, c.stream);
-    if (nparticles > 0) {
-      TimedLaunch t(c, "comm_halo_flag");
-      k_halo_flag2<<<blocks_for(nparticles, 256), 256, 0, c.stream>>>(c.x4.p, nparticles, dim, bound_hi, bound_lo,
-                                                                      c.flags.p);
+  c.halo_state.reserve(sizeof(HaloState), c.stream);
+  HaloState* st = reinterpret_cast<HaloState*>(c.halo_state.p);
+  HaloState h{};
+  while (N_local > 0) {
+    // room for particles; the reference grows System and the pack list, then
+    // redoes the phase
+    const size_t room = std::min({c.x4.cap, c.v.cap / 3, c.f.cap / 3, c.q.cap, c.type.cap, c.id.cap}) - 1;
+    const int capacity = int(std::min<size_t>(room, 0x7ffffffe));
+    const size_t ghosts = size_t(std::max(0, capacity - N_local)) + 1;
+    const int blocks = (capacity + HALO_TILE - 1) / HALO_TILE;
+    c.pack.reserve(ghosts, c.stream);
+    c.ghost_owner.reserve(ghosts, c.stream);
+    c.ghost_img.reserve(ghosts, c.stream);
+    c.halo_tiles.reserve(size_t(blocks) + 1, c.stream);
+    EMD_CUDA(cudaMemsetAsync(st, 0, sizeof(HaloState), c.stream));
+    for (int dim = 0; dim < 3; ++dim) {
+      const double hi = c.sub_hi[dim] - c.comm_depth, lo = c.sub_lo[dim] + c.comm_depth;
+      {
+        TimedLaunch t(c, "comm_halo_count");
+        k_halo_count<<<blocks, HALO_THREADS, 0, c.stream>>>(c.x4.p, N_local, capacity, dim, hi, lo, st,
+                                                            c.halo_tiles.p);
+        EMD_CHECK_LAUNCH();
+      }
+      TimedLaunch t(c, "comm_halo_place");
+      k_halo_place<<<blocks, HALO_THREADS, 0, c.stream>>>(c.x4.p, c.v.p, c.q.p, c.id.p, c.type.p, N_local, dim, hi, lo,
+                                                          c.domain[dim], st, c.halo_tiles.p, c.pack.p,
+                                                          c.ghost_owner.p, c.ghost_img.p);
       EMD_CHECK_LAUNCH();
     }
-    require(n2 < 0x7fffffffULL, EMD_ERR_OVERFLOW_GHOST, "emd_comm_exchange_halo: more than 2^30 particles");
-    exclusive_scan_int(c, c.flags.p, c.flags_scan.p, int(n2), c.flags_scan.p + n2);
-    EMD_CUDA(cudaMemcpyAsync(c.h_int, c.flags_scan.p + nparticles, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    EMD_CUDA(cudaMemcpyAsync(c.h_int + 1, c.flags_scan.p + n2, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    EMD_CUDA(cudaMemcpyAsync(c.h_int, st, sizeof(HaloState), cudaMemcpyDeviceToHost, c.stream));
     EMD_CUDA(cudaStreamSynchronize(c.stream));
-    const int count_hi = nparticles > 0 ? c.h_int[0] : 0;
-    const int count = nparticles > 0 ? c.h_int[1] : 0;
-    // capacity (the reference grows System and the pack list, then redoes the phase)
-    const long long need = (long long)N_local + N_ghost + count;
-    require(need < 0x7fffffffLL, EMD_ERR_OVERFLOW_GHOST, "emd_comm_exchange_halo: more than 2^31 particles");
-    grow_particles(c, int(need));
-    c.pack.reserve(size_t(pack_total) + count + 1, c.stream, true);
-    c.ghost_owner.reserve(size_t(N_ghost) + count + 1, c.stream, true);
-    c.ghost_img.reserve(size_t(N_ghost) + count + 1, c.stream, true);
-    for (int side = 0; side < 2 && count > 0; ++side) {
-      if ((side == 0 ? count_hi : count - count_hi) == 0) continue;
-      TimedLaunch t(c, "comm_halo_scatter");
-      const size_t off = side == 0 ? 0 : size_t(nparticles);
-      k_halo_scatter<<<blocks_for(nparticles, 256), 256, 0, c.stream>>>(
-          c.x4.p, c.v.p, c.q.p, c.id.p, c.type.p, c.flags.p + off, c.flags_scan.p + off, nparticles, dim,
-          side == 0 ? -c.domain[dim] : c.domain[dim], N_local + N_ghost, N_local, c.pack.p + pack_total,
-          c.ghost_owner.p, c.ghost_img.p, 1 << (2 * dim + side));
-      EMD_CHECK_LAUNCH();
-    }
-    c.num_ghost[2 * dim] = count_hi;
-    c.num_ghost[2 * dim + 1] = count - count_hi;
-    c.ghost_offsets[2 * dim] = N_local + N_ghost;
-    c.ghost_offsets[2 * dim + 1] = N_local + N_ghost + count_hi;
-    pack_total += count;
-    N_ghost += count;
+    std::memcpy(&h, c.h_int, sizeof h);
+    require((long long)N_local + std::max(h.base[1], h.base[2]) < (1LL << 30), EMD_ERR_OVERFLOW_GHOST,
+            "emd_comm_exchange_halo: more than 2^30 particles");
+    require(h.overflow < 0x7fffffff, EMD_ERR_OVERFLOW_GHOST, "emd_comm_exchange_halo: more than 2^31 particles");
+    if (!h.overflow) break;
+    // at least what is known to be needed, and what a uniform density needs
+    double part = 1.0;
+    for (int d = 0; d < 3; ++d)
+      part *= 1.0 + 2.0 * c.comm_depth / c.domain[d];
+    reserve_particles(c, size_t(std::min(double(0x7ffffffe), std::max(double(h.overflow), N_local * part))));
+  }
+  const int N_ghost = h.base[3];
+  grow_particles(c, N_local + N_ghost);
+  for (int dim = 0; dim < 3; ++dim) {
+    c.num_ghost[2 * dim] = h.upper[dim];
+    c.num_ghost[2 * dim + 1] = h.base[dim + 1] - h.base[dim] - h.upper[dim];
+    c.ghost_offsets[2 * dim] = N_local + h.base[dim];
+    c.ghost_offsets[2 * dim + 1] = N_local + h.base[dim] + h.upper[dim];
   }
   c.N_ghost = N_ghost;
   if (n_ghost_out) *n_ghost_out = N_ghost;
@@ -231,6 +365,18 @@ emd_status emd_comm_update_force(emd_ctx* ctx) {
   }
   materialize_kick(c);  // owned forces are about to change
   materialize_zero(c, true, true);
+  if (acc > 0 && acc <= HALO_FORCE_MAX) {
+    HaloPhases P;
+    for (int p = 0; p < 6; ++p) {
+      P.pack[p] = pack_off[p];
+      P.count[p] = c.num_ghost[p];
+      P.ghost[p] = c.ghost_offsets[p];
+    }
+    TimedLaunch t(c, "comm_update_force");
+    k_halo_force_all<<<1, 1024, 0, c.stream>>>(c.f.p, c.pack.p, P);
+    EMD_CHECK_LAUNCH();
+    return EMD_OK;
+  }
   for (int phase = 5; phase >= 0; --phase) {
     const int count = c.num_ghost[phase];
     if (count == 0) continue;

@@ -69,9 +69,11 @@ __device__ __forceinline__ int warp_incl_scan(int v) {
   return v;
 }
 
-// Exclusive scan of one tile per block; block totals to sums[blockIdx.x].
+// Exclusive scan of one tile per block; block totals to sums[blockIdx.x] (and a
+// zero after them, whose exclusive scan is the total), the total of a single tile
+// to *total.
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(const int* __restrict__ in, int* __restrict__ out,
-                                                              int n, int* __restrict__ sums) {
+                                                              int n, int* __restrict__ sums, int* total) {
   __shared__ int warp_tot[SCAN_THREADS / 32];
   const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_PER_THREAD;
   int vals[SCAN_PER_THREAD];
@@ -99,16 +101,20 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(const int* __restri
     if (idx < n) out[idx] = run;
     run += vals[k];
   }
-  if (threadIdx.x == SCAN_THREADS - 1 && sums) sums[blockIdx.x] = run;
+  if (threadIdx.x == SCAN_THREADS - 1) {
+    if (gridDim.x > 1) {
+      sums[blockIdx.x] = run;
+      if (blockIdx.x == 0) sums[gridDim.x] = 0;
+    } else if (total) {
+      *total = run;
+    }
+  }
 }
 
-__global__ void k_scan_add(int* __restrict__ out, int n, const int* __restrict__ offs) {
+__global__ void k_scan_add(int* __restrict__ out, int n, const int* __restrict__ offs, int tiles, int* total) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] += offs[i / SCAN_TILE];
-}
-
-__global__ void k_scan_total(const int* __restrict__ in, const int* __restrict__ scanned, int n, int* total) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *total = n > 0 ? scanned[n - 1] + in[n - 1] : 0;
+  if (i == 0 && total) *total = offs[tiles];
 }
 
 // Deterministic FP64 sum: fixed grid, fixed per-thread partition.
@@ -131,20 +137,20 @@ __global__ void __launch_bounds__(SUM_THREADS) k_sum_final(const double* __restr
 }
 }  // namespace
 
-static void scan_rec(Ctx& c, const int* in, int* out, int n, int level) {
+static void scan_rec(Ctx& c, const int* in, int* out, int n, int level, int* total) {
   const int tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
   require(level < (int)c.scan_levels.size(), EMD_ERR_ARG, "scan: too many levels");
   DevBuf<int>& sums = c.scan_levels[level];
   sums.reserve(size_t(tiles) + 1, c.stream);
   {
     TimedLaunch t(c, "scan_tiles");
-    k_scan_tiles<<<tiles, SCAN_THREADS, 0, c.stream>>>(in, out, n, sums.p);
+    k_scan_tiles<<<tiles, SCAN_THREADS, 0, c.stream>>>(in, out, n, sums.p, total);
     EMD_CHECK_LAUNCH();
   }
   if (tiles > 1) {
-    scan_rec(c, sums.p, sums.p, tiles, level + 1);
+    scan_rec(c, sums.p, sums.p, tiles + 1, level + 1, nullptr);
     TimedLaunch t(c, "scan_add");
-    k_scan_add<<<blocks_for(n, 256), 256, 0, c.stream>>>(out, n, sums.p);
+    k_scan_add<<<blocks_for(n, 256), 256, 0, c.stream>>>(out, n, sums.p, tiles, total);
     EMD_CHECK_LAUNCH();
   }
 }
@@ -156,16 +162,7 @@ void exclusive_scan_int(Ctx& c, const int* d_in, int* d_out, int n, int* d_total
   }
   // levels are sized once so references into the vector stay valid
   if (c.scan_levels.size() < 6) c.scan_levels.resize(6);
-  // The total needs the last input, which an in-place scan overwrites.
-  c.scan_aux.reserve(2, c.stream);
-  if (d_total)
-    EMD_CUDA(cudaMemcpyAsync(c.scan_aux.p, d_in + n - 1, sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
-  scan_rec(c, d_in, d_out, n, 0);
-  if (d_total) {
-    TimedLaunch t(c, "scan_total");
-    k_scan_total<<<1, 32, 0, c.stream>>>(c.scan_aux.p, d_out + n - 1, 1, d_total);
-    EMD_CHECK_LAUNCH();
-  }
+  scan_rec(c, d_in, d_out, n, 0, d_total);
 }
 
 double device_sum(Ctx& c, const double* d_vals, int n) {
@@ -342,8 +339,8 @@ void emd_destroy(emd_ctx* ctx) {
   for (auto* b : {&c.v, &c.f, &c.q, &c.mass_d, &c.stage_d, &c.stage_dl, &c.lj_params, &c.red, &c.red2, &c.dtfm_d,
                   &c.lj_intensity, &c.lj_pe_part})
     b->release();
-  for (auto* b : {&c.type, &c.id, &c.stage_i, &c.pack, &c.ghost_owner, &c.ghost_img, &c.flags, &c.flags_scan,
-                  &c.bincount, &c.binoffsets, &c.permute, &c.binof, &c.bin_cursor, &c.perm_tmp, &c.num_neighs,
+  for (auto* b : {&c.type, &c.id, &c.stage_i, &c.pack, &c.ghost_owner, &c.ghost_img, 
+                  &c.bincount, &c.binoffsets, &c.permute, &c.binof, &c.bin_slot, &c.perm_tmp, &c.num_neighs,
                   &c.neigh_offsets, &c.neighs, &c.resize_flag, &c.abin})
     b->release();
   for (auto& b : c.stage_up) b.release();
@@ -358,7 +355,8 @@ void emd_destroy(emd_ctx* ctx) {
   c.neigh_rows2d.release();
   c.lj_params_f.release();
   for (auto& b : c.scan_levels) b.release();
-  c.scan_aux.release();
+  c.halo_state.release();
+  c.halo_tiles.release();
   for (auto& kv : c.timer.slots)
     for (auto& p : kv.second.pending) {
       cudaEventDestroy(p.a);

@@ -155,13 +155,14 @@ struct Ctx {
   DevBuf<int> pack;         // concatenated per-phase source indices
   DevBuf<int> ghost_owner;  // owned atom each ghost images (for the one-launch halo update)
   DevBuf<int> ghost_img;    // 6 bits: shift sign per dimension
-  DevBuf<int> flags, flags_scan;
+  DevBuf<unsigned char> halo_state;
+  DevBuf<int2> halo_tiles;
 
   // ---- Binning
   int nbin[3] = {0, 0, 0}, nhalo = 0;
   double bmin[3] = {0, 0, 0}, bmax[3] = {0, 0, 0}, bmul[3] = {0, 0, 0};
   int bin_first = 0, bin_count_n = 0;
-  DevBuf<int> bincount, binoffsets, permute, binof, bin_cursor, perm_tmp;
+  DevBuf<int> bincount, binoffsets, permute, binof, bin_slot, perm_tmp;
   bool binning_ready = false;
 
   // ---- Neighbor
@@ -220,6 +221,7 @@ struct Ctx {
   DevBuf<int> bin_c3;
   DevBuf<double> ctr_tab;
   int ctr_nb[3] = {0, 0, 0};
+  double bin_ctab_key[9] = {};  // the geometry bin_ctab was formed for
   DevBuf<double> bin_ctab;      // bin centre coordinate per bin and dimension (nbx | nby | nbz)
   long long neigh_builds = 0;
   int xl_ok = 0;  // xl == FP32(x - bin centre) holds for owned (1) / ghost (2) rows
@@ -238,7 +240,6 @@ struct Ctx {
 
   // ---- scan scratch
   std::vector<DevBuf<int>> scan_levels;
-  DevBuf<int> scan_aux;
 
   LaunchTimer timer;
   double* h_scalar = nullptr;  // pinned scratch for read-backs

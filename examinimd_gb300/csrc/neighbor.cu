@@ -24,7 +24,7 @@ namespace {
 constexpr int NB_WARPS = 4;     // warps per CTA, one interior bin each (independent)
 constexpr int NB_THREADS = 32 * NB_WARPS;
 constexpr int NB_SLOTS = 64;  // spread slots for the longest-row reduction
-static_assert(1 + NB_SLOTS <= kHostInts, "read-back of the row-length slots exceeds the pinned scratch");
+static_assert(2 + NB_SLOTS <= kHostInts, "read-back of the row-length slots exceeds the pinned scratch");
 
 struct NeighArgs {
   RowArgs r;
@@ -75,9 +75,10 @@ __global__ void __launch_bounds__(NB_THREADS) k_neigh_bin(NeighArgs a) {
 
 // owned atoms outside every interior bin get an empty row (the reference
 // never visits them)
-__global__ void k_zero_rows(int* num, int n) {
+__global__ void k_zero_rows(int* num, int n, int* flags) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) num[i] = 0;
+  if (i < 1 + NB_SLOTS) flags[i] = 0;
 }
 
 // column-major rows -> CSR rows at offs[i]
@@ -170,17 +171,20 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
   const bool two_d = c.neigh_kind == EMD_NEIGH_2D;
   int& K = two_d ? c.maxneighs : c.neigh_scratch_k;
   DevBuf<int>& rows = two_d ? c.neighs : c.neigh_rows2d;
+  // the total sizes the compacted CSR list; column-major rows (2D, packed)
+  // need it only when the caller asks, so it is read later on demand there
+  const bool need_total = (!two_d && !packed) || total_out;
   while (true) {
     rows.reserve(size_t(n + 1) * size_t((K + 3) & ~3) + 4, c.stream);
     a.r.rows = rows.p;
     a.r.K = K;
-    EMD_CUDA(cudaMemsetAsync(c.resize_flag.p, 0, (1 + NB_SLOTS) * sizeof(int), c.stream));
+    {
+      TimedLaunch t(c, "neigh_zero_rows");
+      k_zero_rows<<<blocks_for(std::max(n, 1 + NB_SLOTS), 256), 256, 0, c.stream>>>(c.num_neighs.p, n,
+                                                                                  c.resize_flag.p);
+      EMD_CHECK_LAUNCH();
+    }
     if (n > 0) {
-      {
-        TimedLaunch t(c, "neigh_zero_rows");
-        k_zero_rows<<<blocks_for(n, 256), 256, 0, c.stream>>>(c.num_neighs.p, n);
-        EMD_CHECK_LAUNCH();
-      }
       if (ibins > 0) {
         TimedLaunch t(c, "neigh_build");
         auto k = c.half_neigh ? (packed ? k_neigh_bin<true, true> : k_neigh_bin<true, false>)
@@ -189,8 +193,13 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
         EMD_CHECK_LAUNCH();
       }
     }
+    // the scan before the flags are known (a regrow does it again): one wait for both
+    exclusive_scan_int(c, c.num_neighs.p, c.neigh_offsets.p, n, c.neigh_offsets.p + n);
     EMD_CUDA(cudaMemcpyAsync(c.h_int, c.resize_flag.p, (1 + NB_SLOTS) * sizeof(int), cudaMemcpyDeviceToHost,
                              c.stream));
+    if (need_total)
+      EMD_CUDA(cudaMemcpyAsync(c.h_int + 1 + NB_SLOTS, c.neigh_offsets.p + n, sizeof(int), cudaMemcpyDeviceToHost,
+                               c.stream));
     EMD_CUDA(cudaStreamSynchronize(c.stream));
     int longest = 0;
     for (int k = 1; k <= NB_SLOTS; ++k) longest = std::max(longest, c.h_int[k]);
@@ -200,15 +209,7 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
     // neighbor_2d.h:325-327: grow to 1.2x the longest row and redo
     K = int(c.h_int[1] * 1.2);
   }
-  exclusive_scan_int(c, c.num_neighs.p, c.neigh_offsets.p, n, c.neigh_offsets.p + n);
-  // the total sizes the compacted CSR list; column-major rows (2D, packed)
-  // need it only when the caller asks, so it is read later on demand there
-  long long total = -1;
-  if ((!two_d && !packed) || total_out) {
-    EMD_CUDA(cudaMemcpyAsync(c.h_int, c.neigh_offsets.p + n, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    EMD_CUDA(cudaStreamSynchronize(c.stream));
-    total = n > 0 ? c.h_int[0] : 0;
-  }
+  const long long total = !need_total ? -1 : (n > 0 ? c.h_int[1 + NB_SLOTS] : 0);
   if (!two_d && !packed) {
     // NeighListCSR (neighbor_csr.h:81-124): rows contiguous at row_map(i)
     c.neighs.reserve(size_t(total) + 1, c.stream);
