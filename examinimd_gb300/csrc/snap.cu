@@ -34,7 +34,7 @@ struct SnapHost {
   DevBuf<ZGrp> grp;
   DevBuf<int> e0, map, zt0, tmask, eord;
   DevBuf<int2> xsum, ucol, half, zt, prod;
-  DevBuf<float2> mono;
+  DevBuf<float2> mono, pr32, wj32;
   DevBuf<int4> hfull, ysrc;
   DevBuf<double> zc, cY, AB, beta0, wjelem, pr;
   DevBuf<float> AB_f;
@@ -412,7 +412,7 @@ void free_snap(Ctx& c) {
                   &h->eatom, &h->adj, &h->adj_sum, &h->adj_g, &h->keep_u, &h->keep_z})
     b->release();
   h->AB_f.release();
-  h->mono.release();
+  for (auto* b : {&h->mono, &h->pr32, &h->wj32}) b->release();
   delete h;
   c.snap = nullptr;
 }
@@ -821,6 +821,13 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   upload(c, h->cY, cY);
   upload(c, h->beta0, beta0);
   upload(c, h->pr, pr);
+  auto pair32 = [](double v) { return float2{float(v), float(v - double(float(v)))}; };
+  std::vector<float2> pr32, wj32;
+  for (double v : pr) pr32.push_back(pair32(v));
+  for (int e = 0; e < nelem; ++e) wj32.push_back(pair32(wjelem[e]));
+  S.nrmin32 = pair32(-rmin0);
+  upload(c, h->pr32, pr32);
+  upload(c, h->wj32, wj32);
   upload(c, h->wjelem, std::vector<double>(wjelem, wjelem + nelem));
   upload(c, h->map, std::vector<int>(map, map + ntypes));
   EMD_CUDA(cudaStreamSynchronize(c.stream));
@@ -849,6 +856,8 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   S.cY = h->cY.p;
   S.beta0 = h->beta0.p;
   S.pr = h->pr.p;
+  S.pr32 = h->pr32.p;
+  S.wj32 = h->wj32.p;
   S.wjelem = h->wjelem.p;
   S.map = h->map.p;
   EMD_API_END
