@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(64) k_snap_pairs(SnapArgs A) {
 // The mixed form, which rounds U_tot to FP32 anyway, takes k_snap_u32
 // (snap_split.cuh): sums over u x^k and v x^k, the same for every q, combined into
 // the polynomials' once per atom.  Per 128,000 atoms: 4.98 ms as the FP64 form
-// does it, 2.80 with powers of x in FP64, 0.95 in FP32 pairs.
+// does it, 2.80 with powers of x in FP64, 0.87 in FP32 pairs.
 inline int su_cols(int J) {  // p, r; u, v; u P_k, v P_k (k >= 1)
   int c = 2 * (J + 1) + 2 * (J + 1);
   for (int T = 0; T <= J; ++T)
@@ -692,7 +692,7 @@ __global__ void __launch_bounds__(SY_THREADS) k_snap_y(SnapArgs A) {
 // Atoms of another element than the stream's are computed and not stored
 // (one launch per element).
 // Per 128,000 atoms: 3.77 ms with records and direct table reads, 2.47 with
-// records streamed, 1.25 as it is.
+// records streamed, 1.28 as it is with 16 warps, 1.23 with 24.
 __host__ __device__ constexpr int zs_words(int nj) { return nj == 1 ? 2 : (nj <= 3 ? 4 : (nj <= 5 ? 8 : 16)); }
 constexpr int ZS_CHUNK = 256;  // words per buffer
 struct ZStream {
@@ -774,7 +774,7 @@ __device__ __forceinline__ void zg_add(const ZGrp& G, ZStream& st, const Cplx<fl
   });
 }
 
-__host__ __device__ constexpr int sy32_threads(int na) { return na == 2 ? 512 : 384; }
+__host__ __device__ constexpr int sy32_threads(int na) { return na == 2 ? 768 : 384; }
 template <int NM, int NA, bool FULL>
 __global__ void __launch_bounds__(sy32_threads(NA), NA == 2 ? 1 : 2) k_snap_y32(SnapArgs A, int elem) {
   const SnapDev& S = A.S;

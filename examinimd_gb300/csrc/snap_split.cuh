@@ -9,27 +9,33 @@
 namespace emd {
 namespace snapk {
 
-__device__ __forceinline__ void su_row32(int J, float4* t, F2 ar, F2 ai, F2 br, F2 bi, F2 w) {
-  const F2 nai{-ai.h, -ai.l}, nbi{-bi.h, -bi.l};
-  const float one = f2_base(1.f), wb = f2_base(fabsf(w.h));
-  F2 x;
-  {
-    F2Sum s{one, 0.f};
-    s.add(ar, ar);
-    s.add(ai, ai);
-    s.add(F2{-br.h, -br.l}, br);
-    s.add(nbi, bi);
-    x = s.value(one);
-  }
-  F2 p{1.f, 0.f}, r{0.f, 0.f}, u = w, v{0.f, 0.f};
-  float4* col = t + J + 1;
+// a row's powers of a; its powers of b times those of x
+__device__ __forceinline__ void su_row_a(int J, float4* t, F2 ar, F2 ai) {
+  const F2 nai{-ai.h, -ai.l};
+  const float one = f2_base(1.f);
+  F2 p{1.f, 0.f}, r{0.f, 0.f};
 #pragma unroll 1
   for (int q = 0; q <= J; ++q) {
     t[q] = float4{p.h, p.l, r.h, r.l};
+    f2_cmul(p, r, ar, ai, nai, one);
+  }
+}
+__device__ __forceinline__ void su_row_b(int J, float4* col, F2 ar, F2 ai, F2 br, F2 bi, F2 w) {
+  const F2 nbi{-bi.h, -bi.l};
+  const float one = f2_base(1.f), wb = f2_base(fabsf(w.h));
+  F2Sum sx{one, 0.f};
+  sx.add(ar, ar);
+  sx.add(ai, ai);
+  sx.add(F2{-br.h, -br.l}, br);
+  sx.add(nbi, bi);
+  const F2 x = sx.value(one);
+  F2 u = w, v{0.f, 0.f};
+#pragma unroll 1
+  for (int T = 0; T <= J; ++T) {
     F2 uk = u, vk = v;
     *col++ = float4{uk.h, uk.l, vk.h, vk.l};
 #pragma unroll 1
-    for (int k = 1; k <= (J - q) / 2; ++k) {
+    for (int k = 1; k <= (J - T) / 2; ++k) {
       F2Sum su{wb, 0.f}, sv{wb, 0.f};
       su.add(uk, x);
       sv.add(vk, x);
@@ -37,7 +43,6 @@ __device__ __forceinline__ void su_row32(int J, float4* t, F2 ar, F2 ai, F2 br, 
       vk = sv.value(wb);
       *col++ = float4{uk.h, uk.l, vk.h, vk.l};
     }
-    f2_cmul(p, r, ar, ai, nai, one);
     f2_cmul(u, v, br, bi, nbi, wb);
   }
 }
@@ -66,13 +71,16 @@ __device__ __forceinline__ void su_store32(const SnapDev& S, int e, const F2Sum*
   }
 }
 
-// One warp per atom as in k_snap_u.  Lanes = entries: the two columns of an
-// entry give its four sums, for two 16-byte loads.
+// One warp per atom as in k_snap_u, 16 neighbours at a time: 16 lanes form the
+// powers of a and 16 those of b (a table of 32 rows, each by one lane, left ten
+// warps on an SM, 0.92 ms per 128,000 atoms; 0.87 so).  Then lanes = entries: the two
+// columns of an entry give its four sums, for two 16-byte loads.
+constexpr int SU_ROWS = 16;
 static __global__ void __launch_bounds__(32) k_snap_u32(SnapArgs A) {
   const SnapDev& S = A.S;
   extern __shared__ __align__(16) unsigned char su_smem32[];
   F2Sum* xs = reinterpret_cast<F2Sum*>(su_smem32);             // 4 ne sums
-  float4* tab = reinterpret_cast<float4*>(xs + 4 * S.ne);      // 32 rows
+  float4* tab = reinterpret_cast<float4*>(xs + 4 * S.ne);      // SU_ROWS rows
   const int al = blockIdx.x, lane = threadIdx.x, n = A.cnt[al];
   const size_t np = size_t(A.n) * A.cap;
   const float* pr = static_cast<const float*>(A.pr) + size_t(al) * A.cap;
@@ -81,13 +89,15 @@ static __global__ void __launch_bounds__(32) k_snap_u32(SnapArgs A) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) weight += __shfl_xor_sync(FULL_MASK, weight, o);
   const float base = f2_base(1.001f * weight);
-  for (int n0 = 0; n0 < max(n, 1); n0 += 32) {
-    const int m = min(32, n - n0);
-    if (lane < m) {
-      const float* q = pr + n0 + lane;
+  for (int n0 = 0; n0 < max(n, 1); n0 += SU_ROWS) {
+    const int m = min(SU_ROWS, n - n0), nb = lane & (SU_ROWS - 1);
+    if (nb < m) {
+      const float* q = pr + n0 + nb;
       auto get = [&](int h, int l) { return F2{q[h * np], q[l * np]}; };
-      su_row32(S.twojmax, tab + lane * S.cols32, get(PR_AR, PR_ARL), get(PR_AI, PR_AIL), get(PR_BR, PR_BRL),
-               get(PR_BI, PR_BIL), get(PR_SF, PR_SFL));
+      const F2 ar = get(PR_AR, PR_ARL), ai = get(PR_AI, PR_AIL);
+      float4* t = tab + nb * S.cols32;
+      if (lane < SU_ROWS) su_row_a(S.twojmax, t, ar, ai);
+      else su_row_b(S.twojmax, t + S.twojmax + 1, ar, ai, get(PR_BR, PR_BRL), get(PR_BI, PR_BIL), get(PR_SF, PR_SFL));
     }
     __syncwarp();
     for (int e0 = 0; e0 < S.ne; e0 += 96) {  // three entries per lane at once
@@ -132,7 +142,7 @@ static __global__ void __launch_bounds__(32) k_snap_u32(SnapArgs A) {
 }
 
 inline void launch_u32(const SnapArgs& A, cudaStream_t s) {
-  const size_t smem = sizeof(F2Sum) * 4 * size_t(A.S.ne) + 32 * 16 * size_t(A.S.cols32);
+  const size_t smem = sizeof(F2Sum) * 4 * size_t(A.S.ne) + SU_ROWS * 16 * size_t(A.S.cols32);
   allow_dyn_smem(k_snap_u32);
   k_snap_u32<<<A.n, 32, smem, s>>>(A);
   EMD_CHECK_LAUNCH();
