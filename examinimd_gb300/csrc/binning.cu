@@ -27,32 +27,40 @@ __global__ void k_bin_ctab(int nbx, int nby, int nbz, double minx, double miny, 
   else if (t < nbx + nby + nbz) tab[t] = minz + (t - nbx - nby + 0.5) * wz;
 }
 
-__global__ void __launch_bounds__(256) k_bin_index(const double4_32a* __restrict__ x4, int first, int n, int nbx,
-                                                   int nby, int nbz, double minx, double miny, double minz,
-                                                   double mulx, double muly, double mulz,
-                                                   const double* __restrict__ ctab, int* __restrict__ binof,
-                                                   int* __restrict__ slot, int* __restrict__ bincount, float4* __restrict__ xl,
-                                                   unsigned* status) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  const double4_32a p = x4[first + r];
-  int ix = int((p.x - minx) * mulx);
-  int iy = int((p.y - miny) * muly);
-  int iz = int((p.z - minz) * mulz);
-  if (ix < 0 || ix >= nbx || iy < 0 || iy >= nby || iz < 0 || iz >= nbz) {
+struct BinGrid {
+  int nbx, nby, nbz;
+  double minx, miny, minz, mulx, muly, mulz;
+  const double* ctab;
+};
+
+// bin of a particle, and its FP32 position relative to the bin's centre, for the
+// neighbour candidate tests
+__device__ __forceinline__ int bin_particle(const BinGrid& G, const double4_32a& p, float4* xl, unsigned* status) {
+  int ix = int((p.x - G.minx) * G.mulx);
+  int iy = int((p.y - G.miny) * G.muly);
+  int iz = int((p.z - G.minz) * G.mulz);
+  if (ix < 0 || ix >= G.nbx || iy < 0 || iy >= G.nby || iz < 0 || iz >= G.nbz) {
     // outside the binned box: the reference would index out of bounds; keep
     // the particle in the nearest bin and report it
     latch_status(status, ST_BOUNDS);
-    ix = min(max(ix, 0), nbx - 1);
-    iy = min(max(iy, 0), nby - 1);
-    iz = min(max(iz, 0), nbz - 1);
+    ix = min(max(ix, 0), G.nbx - 1);
+    iy = min(max(iy, 0), G.nby - 1);
+    iz = min(max(iz, 0), G.nbz - 1);
   }
-  const int b = (ix * nby + iy) * nbz + iz;
+  *xl = make_float4(float(p.x - G.ctab[ix]), float(p.y - G.ctab[G.nbx + iy]),
+                    float(p.z - G.ctab[G.nbx + G.nby + iz]), __int_as_float(int(p.w)));
+  return (ix * G.nby + iy) * G.nbz + iz;
+}
+
+__global__ void __launch_bounds__(256) k_bin_index(BinGrid G, const double4_32a* __restrict__ x4, int first, int n,
+                                                   int* __restrict__ binof, int* __restrict__ slot,
+                                                   int* __restrict__ bincount, float4* __restrict__ xl,
+                                                   unsigned* status) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  const int b = bin_particle(G, x4[first + r], xl + first + r, status);
   binof[r] = b;
   slot[r] = atomicAdd(&bincount[b], 1);
-  // FP32 position relative to the bin centre, for the neighbour candidate tests
-  xl[first + r] = make_float4(float(p.x - ctab[ix]), float(p.y - ctab[nbx + iy]), float(p.z - ctab[nbx + nby + iz]),
-                              __int_as_float(int(p.w)));
 }
 
 __global__ void __launch_bounds__(256) k_bin_scatter(const int* __restrict__ binof, int n,
@@ -78,6 +86,68 @@ __global__ void __launch_bounds__(256) k_bin_rank(const int* __restrict__ bincou
     int rank = 0;
     for (int k = 0; k < n; ++k) rank += perm_tmp[off + k] < val ? 1 : 0;
     permute[off + rank] = val;
+  }
+}
+
+// The whole binning of a small system by one CTA: its passes take less than the
+// launches (64 atoms: five operations, 27 us, 9 in one; 864 atoms, then with their
+// 2,200 ghosts: 28 and 19).
+constexpr int BIN_SMALL = 4096, BIN_SMALL_BINS = 2048, BIN_SMALL_THREADS = 1024;
+__global__ void __launch_bounds__(BIN_SMALL_THREADS) k_bin_small(BinGrid G, const double4_32a* __restrict__ x4,
+                                                                 int first, int n, int* __restrict__ binof,
+                                                                 int* __restrict__ bincount,
+                                                                 int* __restrict__ binoffsets, int* perm_tmp,
+                                                                 int* __restrict__ permute,
+                                                                 float4* __restrict__ xl, unsigned* status) {
+  constexpr int PER = BIN_SMALL / BIN_SMALL_THREADS;
+  __shared__ int cnt[BIN_SMALL_BINS], off[BIN_SMALL_BINS];
+  __shared__ int wsum[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nbins = G.nbx * G.nby * G.nbz;
+  cnt[tid] = cnt[tid + BIN_SMALL_THREADS] = 0;
+  __syncthreads();
+  int bin[PER], slot[PER];
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int r = tid + k * BIN_SMALL_THREADS;
+    if (r >= n) continue;
+    bin[k] = bin_particle(G, x4[first + r], xl + first + r, status);
+    binof[r] = bin[k];
+    slot[k] = atomicAdd(&cnt[bin[k]], 1);
+  }
+  __syncthreads();
+  const int c0 = cnt[2 * tid], c1 = cnt[2 * tid + 1];
+  int x = c0 + c1;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(FULL_MASK, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) wsum[warp] = x;
+  __syncthreads();
+  int base = x - c0 - c1;
+  for (int k = 0; k < warp; ++k) base += wsum[k];
+  off[2 * tid] = base;
+  off[2 * tid + 1] = base + c0;
+  __syncthreads();
+  for (int b = tid; b < nbins; b += BIN_SMALL_THREADS) {
+    bincount[b] = cnt[b];
+    binoffsets[b] = off[b];
+  }
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int r = tid + k * BIN_SMALL_THREADS;
+    if (r < n) perm_tmp[off[bin[k]] + slot[k]] = r;
+  }
+  __syncthreads();
+  // each particle's rank in its bin: members with a smaller index
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int r = tid + k * BIN_SMALL_THREADS;
+    if (r >= n) continue;
+    const int o = off[bin[k]], m = cnt[bin[k]];
+    int rank = 0;
+    for (int e = 0; e < m; ++e) rank += perm_tmp[o + e] < r ? 1 : 0;
+    permute[o + rank] = r;
   }
 }
 
@@ -164,7 +234,6 @@ emd_status emd_binning_create(emd_ctx* ctx, double dx_in, double dy_in, double d
   c.permute.reserve(size_t(n) + 1, c.stream);
   c.perm_tmp.reserve(size_t(n) + 1, c.stream);
   c.bin_slot.reserve(size_t(n) + 1, c.stream);
-  EMD_CUDA(cudaMemsetAsync(c.bincount.p, 0, sizeof(int) * nbins, c.stream));
   c.xl_bin.reserve(size_t(first + n) + 1, c.stream, true);
   const int ntab = nb[0] + nb[1] + nb[2];
   // a box binned as before keeps its table
@@ -179,25 +248,30 @@ emd_status emd_binning_create(emd_ctx* ctx, double dx_in, double dy_in, double d
     EMD_CHECK_LAUNCH();
     std::copy(key, key + 9, c.bin_ctab_key);
   }
-  if (n > 0) {
-    TimedLaunch t(c, "bin_index");
-    k_bin_index<<<blocks_for(n, 256), 256, 0, c.stream>>>(c.x4.p, first, n, nb[0], nb[1], nb[2], c.bmin[0],
-                                                          c.bmin[1], c.bmin[2], c.bmul[0], c.bmul[1], c.bmul[2],
-                                                          c.bin_ctab.p, c.binof.p, c.bin_slot.p, c.bincount.p, c.xl_bin.p,
-                                                          c.d_status);
-    EMD_CHECK_LAUNCH();
-  }
+  const BinGrid G{nb[0], nb[1], nb[2], c.bmin[0], c.bmin[1], c.bmin[2], c.bmul[0], c.bmul[1], c.bmul[2], c.bin_ctab.p};
   c.xl_bin_valid = true;
   c.bin_sorted = false;
-  exclusive_scan_int(c, c.bincount.p, c.binoffsets.p, nbins, nullptr);
-  if (n > 0) {
-    {
-      TimedLaunch t(c, "bin_scatter");
-      k_bin_scatter<<<blocks_for(n, 256), 256, 0, c.stream>>>(c.binof.p, n, c.binoffsets.p, c.bin_slot.p,
-                                                              c.perm_tmp.p);
+  if (n > 0 && n <= BIN_SMALL && nbins <= BIN_SMALL_BINS) {
+    TimedLaunch t(c, "bin_small");
+    k_bin_small<<<1, BIN_SMALL_THREADS, 0, c.stream>>>(G, c.x4.p, first, n, c.binof.p, c.bincount.p, c.binoffsets.p,
+                                                       c.perm_tmp.p, c.permute.p, c.xl_bin.p, c.d_status);
+    EMD_CHECK_LAUNCH();
+  } else {
+    EMD_CUDA(cudaMemsetAsync(c.bincount.p, 0, sizeof(int) * nbins, c.stream));
+    if (n > 0) {
+      TimedLaunch t(c, "bin_index");
+      k_bin_index<<<blocks_for(n, 256), 256, 0, c.stream>>>(G, c.x4.p, first, n, c.binof.p, c.bin_slot.p,
+                                                            c.bincount.p, c.xl_bin.p, c.d_status);
       EMD_CHECK_LAUNCH();
     }
-    {
+    exclusive_scan_int(c, c.bincount.p, c.binoffsets.p, nbins, nullptr);
+    if (n > 0) {
+      {
+        TimedLaunch t(c, "bin_scatter");
+        k_bin_scatter<<<blocks_for(n, 256), 256, 0, c.stream>>>(c.binof.p, n, c.binoffsets.p, c.bin_slot.p,
+                                                                c.perm_tmp.p);
+        EMD_CHECK_LAUNCH();
+      }
       TimedLaunch t(c, "bin_rank");
       k_bin_rank<<<blocks_for((long long)nbins * 32, 256), 256, 0, c.stream>>>(c.bincount.p, c.binoffsets.p, nbins,
                                                                                c.perm_tmp.p, c.permute.p);
