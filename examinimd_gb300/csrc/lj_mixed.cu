@@ -112,41 +112,7 @@ __global__ void __launch_bounds__(256) k_nve_final_mixed(double* __restrict__ v,
   v[3 * i + 2] = fma(dtfm, f[3 * i + 2], v[3 * i + 2]);
 }
 
-// One thread per owned atom; four list entries per coalesced int4 load, the
-// next granule prefetched while the current four pairs are evaluated.
-// a granule of the neighbour list: read once, so it bypasses L1 and leaves
-// the L1 lines to the gathered neighbour positions
-__device__ __forceinline__ int4 ld_list(const int4* p) {
-  int4 r;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
-  return r;
-}
-
-// One row: four entries per coalesced int4 load, the next granule
-// prefetched while the current four pairs are evaluated; `quad` evaluates a
-// granule.  Unused slots of the last granule become padding: i itself with
-// the code k = (3, 3, 3), far outside the cutoff, so they add nothing.
-template <typename Quad>
-__device__ __forceinline__ void lj_row(int i, const int4* __restrict__ q, int cnt, int stride, Quad&& quad) {
-  const int nfull = cnt >> 2;
-  int4 e = nfull > 0 ? ld_list(q) : make_int4(0, 0, 0, 0);
-  for (int kq = 0; kq < nfull; ++kq) {
-    const int4 en = (kq + 1 < nfull) ? ld_list(q + (size_t)(kq + 1) * stride) : e;
-    quad(e);
-    e = en;
-  }
-  const int rem = cnt & 3;
-  if (rem) {
-    int4 t = ld_list(q + (size_t)nfull * stride);
-    const int self = (i << 6) | 0x3f;
-    if (rem < 2) t.y = self;
-    if (rem < 3) t.z = self;
-    t.w = self;
-    quad(t);
-  }
-}
-
+// One thread per owned atom (lj_row)
 template <bool SINGLE, bool ZERO>
 __global__ void __launch_bounds__(128) k_lj_full_mixed(const float4* __restrict__ xl,
                                                        const double4_32a* __restrict__ x4, double* __restrict__ f,

@@ -349,5 +349,44 @@ __device__ __forceinline__ void lj_energy_quad(const PairCtx& C, const int4& e, 
   energy_pair2(C, P, E, e.z, e.w, x2, x3, ea);
 }
 
+// A granule of the neighbour list: read once, so it bypasses L1 and leaves
+// the L1 lines to the gathered neighbour positions.  NC: the list was written by
+// another launch (the non-coherent path may be taken).
+template <bool NC = true>
+__device__ __forceinline__ int4 ld_list(const int4* p) {
+  int4 r;
+  if (NC)
+    asm volatile("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  else
+    asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+  return r;
+}
+
+// One row: four entries per coalesced int4 load, the next granule
+// prefetched while the current four pairs are evaluated; `quad` evaluates a
+// granule.  Unused slots of the last granule become padding: i itself with
+// the code k = (3, 3, 3), far outside the cutoff, so they add nothing.
+template <bool NC = true, typename Quad>
+__device__ __forceinline__ void lj_row(int i, const int4* __restrict__ q, int cnt, int stride, Quad&& quad) {
+  const int nfull = cnt >> 2;
+  int4 e = nfull > 0 ? ld_list<NC>(q) : make_int4(0, 0, 0, 0);
+  for (int kq = 0; kq < nfull; ++kq) {
+    const int4 en = (kq + 1 < nfull) ? ld_list<NC>(q + (size_t)(kq + 1) * stride) : e;
+    quad(e);
+    e = en;
+  }
+  const int rem = cnt & 3;
+  if (rem) {
+    int4 t = ld_list<NC>(q + (size_t)nfull * stride);
+    const int self = (i << 6) | 0x3f;
+    if (rem < 2) t.y = self;
+    if (rem < 3) t.z = self;
+    t.w = self;
+    quad(t);
+  }
+}
+
 }  // namespace
 }  // namespace emd
