@@ -33,10 +33,10 @@ struct SnapHost {
   DevBuf<ZRec> rec;
   DevBuf<ZGrp> grp;
   DevBuf<int> e0, map, zt0, tmask, eord;
-  DevBuf<int2> xsum, ucol, half, zt, prod;
+  DevBuf<int2> xsum, msum, ucol, half, zt, prod;
   DevBuf<float2> mono, pr32, wj32;
   DevBuf<int4> hfull, ysrc;
-  DevBuf<double> zc, cY, AB, beta0, wjelem, pr;
+  DevBuf<double> zc, monod, cY, AB, beta0, wjelem, pr;
   DevBuf<float> AB_f;
   DevBuf<uint4> zs;
   // per-chunk work arrays
@@ -110,12 +110,12 @@ constexpr int ZS_SPLIT = 16;        // CTAs that may share a tile
 struct SnapTables {
   std::vector<Entry> ent;
   std::vector<int> e0, zt0, tmask, eord;
-  std::vector<int2> xsum, ucol, half, zt, prod;
+  std::vector<int2> xsum, msum, ucol, half, zt, prod;
   std::vector<float2> mono;
   std::vector<int4> hfull, ysrc;
   std::vector<ZTask> task;
   std::vector<ZRec> rec;
-  std::vector<double> zc, AB;
+  std::vector<double> zc, AB, monod;
   std::vector<ZGrp> grp;
   std::vector<unsigned> words;  // the FP32 stream without its coefficients
   struct Src {
@@ -158,13 +158,14 @@ struct SnapTables {
           E.xo = int(xsum.size());
           const int cu = k == 0 ? 2 * L + 2 * T : col, cv = cu + 1, cp = 2 * q, cr = 2 * q + 1;
           if (k > 0) col += T > 0 ? 2 : 1;
-          xsum.push_back(int2{cp, cu});
-          if (q > 0) xsum.push_back(int2{cr, cu});
-          if (T > 0) xsum.push_back(int2{cp, cv});
-          if (q > 0 && T > 0) xsum.push_back(int2{cr, cv});
+          const int mu = 2 * (col32 + k), mv = mu + 1;
+          xsum.push_back(int2{cp, cu}), msum.push_back(int2{cp, mu});
+          if (q > 0) xsum.push_back(int2{cr, cu}), msum.push_back(int2{cr, mu});
+          if (T > 0) xsum.push_back(int2{cp, cv}), msum.push_back(int2{cp, mv});
+          if (q > 0 && T > 0) xsum.push_back(int2{cr, cv}), msum.push_back(int2{cr, mv});
           ucol.push_back(int2{q, col32 + k});
           E.mo = int(mono.size());
-          for (double c : pk) mono.push_back(float2{float(E.N * c), float(E.N * c - double(float(E.N * c)))});
+          for (double c : pk) monod.push_back(E.N * c), mono.push_back(float2{float(E.N * c), float(E.N * c - double(float(E.N * c)))});
           std::vector<double> pn(pk.size() + 1, 0.0);
           for (size_t l = 0; l < pk.size(); ++l) {
             pn[l + 1] += pk[l];
@@ -407,8 +408,8 @@ void free_snap(Ctx& c) {
   h->ysrc.release();
   h->zs.release();
   for (auto* b : {&h->e0, &h->map, &h->zt0, &h->tmask, &h->eord, &h->pj, &h->cnt}) b->release();
-  for (auto* b : {&h->xsum, &h->ucol, &h->half, &h->zt, &h->prod}) b->release();
-  for (auto* b : {&h->zc, &h->cY, &h->AB, &h->beta0, &h->wjelem, &h->pr, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk,
+  for (auto* b : {&h->xsum, &h->msum, &h->ucol, &h->half, &h->zt, &h->prod}) b->release();
+  for (auto* b : {&h->zc, &h->monod, &h->cY, &h->AB, &h->beta0, &h->wjelem, &h->pr, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk,
                   &h->eatom, &h->adj, &h->adj_sum, &h->adj_g, &h->keep_u, &h->keep_z})
     b->release();
   h->AB_f.release();
@@ -674,7 +675,7 @@ static void snap_adjoint(Ctx& c, const double* dL_dF, double dL_dE, double* grad
       A.adj = h->adj.p;
       {
         TimedLaunch t(c, "snap_dt");
-        const size_t smem = sizeof(double) * (size_t((S.nx + 1) & ~1) + 64 * size_t(S.cols));
+        const size_t smem = sizeof(double) * (size_t((S.nx + 1) & ~1) + 64 * size_t(sd_cols(S.cols32)));
         require(smem <= kMaxDynSmem, EMD_ERR_ARG, "SNAP adjoint: twojmax too large for shared memory");
         allow_dyn_smem(k_snap_dt);
         k_snap_dt<<<A.n, 32, smem, c.stream>>>(A);
@@ -805,6 +806,8 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   upload(c, h->e0, tab.e0);
   upload(c, h->xsum, tab.xsum);
   upload(c, h->ucol, tab.ucol);
+  upload(c, h->msum, tab.msum);
+  upload(c, h->monod, tab.monod);
   upload(c, h->mono, tab.mono);
   upload(c, h->eord, tab.eord);
   upload(c, h->half, tab.half);
@@ -837,6 +840,8 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   S.e0 = h->e0.p;
   S.xsum = h->xsum.p;
   S.ucol = h->ucol.p;
+  S.msum = h->msum.p;
+  S.monod = h->monod.p;
   S.mono = h->mono.p;
   S.eord = h->eord.p;
   S.half = h->half.p;

@@ -93,7 +93,9 @@ struct SnapDev {
   const int* e0;       // (J + 1) x (J + 1): first entry of (T, q)
   const int2* xsum;    // nx: the two factors of a sum in a neighbour's table (k_snap_u)
   const int2* ucol;    // ne: the mixed form's two columns of an entry
+  const int2* msum;    // nx: the two factors of a sum over powers of x (k_snap_dt)
   const float2* mono;  // N P_k in powers of x, high and low part
+  const double* monod; // the same in FP64
   const int* eord;     // entries, highest k first
   const ZTask* task;
   const ZRec* rec;
@@ -375,6 +377,9 @@ inline int su_cols32(int J) {
   return c | 1;  // odd: eight lanes' rows start in different banks
 }
 
+// doubles of a row of k_snap_dt's tables
+__host__ __device__ inline int sd_cols(int cols32) { return (2 * cols32) | 1; }
+
 // the neighbour's table row: powers, polynomials and products
 __device__ __forceinline__ void su_row(const SnapDev& S, double* t, double ar, double ai, double br, double bi,
                                        double w) {
@@ -428,20 +433,20 @@ __device__ __forceinline__ void su_row(const SnapDev& S, double* t, double ar, d
 // the half-grid elements of entry e from its real sums: conj(a)^q b^T = (p u + r v) + i (p v - r u);
 // for -T: (-1)^T ((p u - r v) - i (p v + r u)); N scales, the atom's own term
 // is 1 on the diagonal (T = 0)
-__device__ __forceinline__ void su_store(const SnapDev& S, int e, const double* x, double self, Cplx<double>* U) {
+__device__ __forceinline__ void su_elements(const SnapDev& S, int e, const double* x, double N, double self,
+                                            Cplx<double>* U) {
   const Entry& E = S.ent[e];
   const bool hr = E.q > 0, hv = E.T > 0;
-  x += E.xo;
-  double pu = E.N * *x++, ru = 0.0, pv = 0.0, rv = 0.0;
-  if (hr) ru = E.N * *x++;
-  if (hv) pv = E.N * *x++;
-  if (hr && hv) rv = E.N * *x;
+  const double pu = N * *x++, ru = hr ? N * *x++ : 0.0, pv = hv ? N * *x++ : 0.0, rv = hr && hv ? N * *x : 0.0;
   const int2 h = S.half[e];
   U[h.x] = Cplx<double>{(pu + rv) + (hv ? 0.0 : self), pv - ru};
   if (h.y >= 0) {
     const double sg = E.T & 1 ? -1.0 : 1.0;
     U[h.y] = Cplx<double>{sg * (pu - rv), -sg * (pv + ru)};
   }
+}
+__device__ __forceinline__ void su_store(const SnapDev& S, int e, const double* x, double self, Cplx<double>* U) {
+  su_elements(S, e, x + S.ent[e].xo, S.ent[e].N, self, U);
 }
 
 static __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
@@ -1201,24 +1206,36 @@ static __global__ void __launch_bounds__(128) k_snap_energy(SnapArgs A) {
 // k instead of after it).
 //
 // k_snap_dt: D as k_snap_u forms X, from each neighbour's table row and its
-// derivative along g_i - g_j.
+// derivative along g_i - g_j.  The rows hold u x^k and v x^k, the same for every q
+// (columns as k_snap_u32's), and the sums are combined into the polynomials' once
+// per atom: 310 FP64 instructions for 32 neighbours' rows where the products with
+// every P_k took 720, and half the table (10,360 atoms in 28 calls: 2.76 -> 1.59 ms).
 __device__ __forceinline__ void sd_row(const SnapDev& S, double* t, double* dt, double ar, double ai, double br,
                                        double bi, double w, double tar, double tai, double tbr, double tbi,
                                        double tw) {
   const int J = S.twojmax;
-  double* prod = t + 4 * (J + 1);
-  double* dprod = dt + 4 * (J + 1);
+  double *col = t + 2 * (J + 1), *dcol = dt + 2 * (J + 1);
+  const double x = fma(ar, ar, ai * ai) - fma(br, br, bi * bi);
+  const double dx = 2.0 * (fma(ar, tar, ai * tai) - fma(br, tbr, bi * tbi));
   double p = 1.0, r = 0.0, u = w, v = 0.0, dp = 0.0, dr = 0.0, du = tw, dv = 0.0;
+#pragma unroll 1
   for (int q = 0; q <= J; ++q) {
     t[2 * q] = p;
     t[2 * q + 1] = r;
     dt[2 * q] = dp;
     dt[2 * q + 1] = dr;
-    const int c = 2 * (J + 1) + 2 * q;
-    t[c] = u;
-    t[c + 1] = v;
-    dt[c] = du;
-    dt[c + 1] = dv;
+    double uk = u, vk = v, duk = du, dvk = dv;
+#pragma unroll 1
+    for (int k = 0; k <= (J - q) / 2; ++k) {
+      *col++ = uk;
+      *col++ = vk;
+      *dcol++ = duk;
+      *dcol++ = dvk;
+      duk = fma(duk, x, uk * dx);
+      dvk = fma(dvk, x, vk * dx);
+      uk *= x;
+      vk *= x;
+    }
     const double dpn = fma(dp, ar, fma(-dr, ai, fma(p, tar, -r * tai)));
     const double drn = fma(dp, ai, fma(dr, ar, fma(p, tai, r * tar)));
     const double dun = fma(du, br, fma(-dv, bi, fma(u, tbr, -v * tbi)));
@@ -1233,33 +1250,17 @@ __device__ __forceinline__ void sd_row(const SnapDev& S, double* t, double* dt, 
     du = dun;
     dv = dvn;
   }
-  const double x = fma(ar, ar, ai * ai) - fma(br, br, bi * bi);
-  const double dx = 2.0 * (fma(ar, tar, ai * tai) - fma(br, tbr, bi * tbi));
-  for (int T = 0; T <= J; ++T) {
-    const int c = 2 * (J + 1) + 2 * T;
-    const double uu = t[c], vv = t[c + 1], duu = dt[c], dvv = dt[c + 1];
-    for (int q = 0; q <= J - T - 2; ++q) {
-      const double2* ab = reinterpret_cast<const double2*>(S.AB) + S.e0[T * (J + 1) + q];
-      const int km = (J - T - q) / 2;
-      double pm = 1.0, pk = x - __ldg(ab).x, dm = 0.0, dk = dx;
-      for (int k = 1; k <= km; ++k) {
-        if (k > 1) {
-          const double2 c = __ldg(ab + k - 1);
-          const double tt = x - c.x;
-          const double pn = fma(tt, pk, -c.y * pm), dn = fma(tt, dk, fma(dx, pk, -c.y * dm));
-          pm = pk;
-          pk = pn;
-          dm = dk;
-          dk = dn;
-        }
-        *prod++ = uu * pk;
-        *dprod++ = fma(duu, pk, uu * dk);
-        if (T > 0) {
-          *prod++ = vv * pk;
-          *dprod++ = fma(dvv, pk, vv * dk);
-        }
-      }
-    }
+}
+
+// su_store's sums of entry e from those over the powers of x, one group per k
+__device__ __forceinline__ void sd_combine(const SnapDev& S, int e, const double* xs, double* x) {
+  const Entry& E = S.ent[e];
+  const double* m = S.monod + E.mo;
+  const int k = (E.j - E.q - E.T) / 2, g = (E.q > 0 ? 2 : 1) * (E.T > 0 ? 2 : 1);
+  for (int h = 0; h < g; ++h) {
+    double s = 0.0;
+    for (int l = 0; l <= k; ++l) s = fma(__ldg(m + l), xs[E.xo + (l - k) * g + h], s);
+    x[h] = s;
   }
 }
 
@@ -1269,7 +1270,7 @@ static __global__ void __launch_bounds__(32) k_snap_dt(SnapArgs A) {
   double* xs = sd_smem;
   double* tab = sd_smem + ((S.nx + 1) & ~1);
   const int al = blockIdx.x, lane = threadIdx.x, i = A.first + al;
-  const int cols = S.cols, n = A.cnt[al];
+  const int cols = sd_cols(S.cols32), n = A.cnt[al];
   const size_t np = size_t(A.n) * A.cap;
   const double gix = A.g[3 * i], giy = A.g[3 * i + 1], giz = A.g[3 * i + 2];
   for (int n0 = 0; n0 < max(n, 1); n0 += 32) {
@@ -1290,7 +1291,7 @@ static __global__ void __launch_bounds__(32) k_snap_dt(SnapArgs A) {
     }
     __syncwarp();
     for (int r = lane; r < S.nx; r += 32) {
-      const int2 s = __ldg(S.xsum + r);
+      const int2 s = __ldg(S.msum + r);
       double acc = n0 > 0 ? xs[r] : 0.0;
       for (int k = 0; k < m; ++k) {
         const double* t = tab + 2 * k * cols;
@@ -1301,7 +1302,12 @@ static __global__ void __launch_bounds__(32) k_snap_dt(SnapArgs A) {
     }
     __syncwarp();
   }
-  for (int e = lane; e < S.ne; e += 32) su_store(S, e, xs, 0.0, A.D + size_t(al) * S.nh);
+  for (int e = lane; e < S.ne; e += 32) {
+    double x[4];
+    const int ee = __ldg(S.eord + e);
+    sd_combine(S, ee, xs, x);
+    su_elements(S, ee, x, 1.0, 0.0, A.D + size_t(al) * S.nh);
+  }
 }
 
 // half-grid elements of U and D, weighted (2, or 1 for the self-inverse ones,
