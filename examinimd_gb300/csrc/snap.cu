@@ -33,7 +33,7 @@ struct SnapHost {
   DevBuf<ZRec> rec;
   DevBuf<ZGrp> grp;
   DevBuf<int> e0, map, zt0, tmask, eord;
-  DevBuf<int2> xsum, msum, ucol, half, zt, prod;
+  DevBuf<int2> xsum, ucol, half, zt, prod;
   DevBuf<float2> mono, pr32, wj32;
   DevBuf<int4> hfull, ysrc;
   DevBuf<double> zc, monod, cY, AB, beta0, wjelem, pr;
@@ -110,7 +110,7 @@ constexpr int ZS_SPLIT = 16;        // CTAs that may share a tile
 struct SnapTables {
   std::vector<Entry> ent;
   std::vector<int> e0, zt0, tmask, eord;
-  std::vector<int2> xsum, msum, ucol, half, zt, prod;
+  std::vector<int2> xsum, ucol, half, zt, prod;
   std::vector<float2> mono;
   std::vector<int4> hfull, ysrc;
   std::vector<ZTask> task;
@@ -130,10 +130,10 @@ struct SnapTables {
   SnapTables(int J, const std::vector<int>& trip) {
     const int L = J + 1, ntrip = int(trip.size() / 3);
     auto uidx = [](int j, int ma, int mb) { return j * (j + 1) * (2 * j + 1) / 6 + ma * (j + 1) + mb; };
-    // entries, real sums and their table columns (k_snap_u: powers of a, of b,
-    // then the products in (T, q, k) order)
+    // entries, real sums and their columns (powers of a, then those of b times
+    // those of x in (T, k) order)
     e0.assign(size_t(L) * L, -1);
-    int col = 4 * L, col32 = L;
+    int col = L;
     for (int T = 0; T <= J; ++T) {
       for (int q = 0; q <= J - T; ++q) {
         e0[size_t(T) * L + q] = int(ent.size());
@@ -156,14 +156,12 @@ struct SnapTables {
           E.mp = uidx(j, j - ma, j - mb);
           E.mm = uidx(j, j - mb, j - ma);
           E.xo = int(xsum.size());
-          const int cu = k == 0 ? 2 * L + 2 * T : col, cv = cu + 1, cp = 2 * q, cr = 2 * q + 1;
-          if (k > 0) col += T > 0 ? 2 : 1;
-          const int mu = 2 * (col32 + k), mv = mu + 1;
-          xsum.push_back(int2{cp, cu}), msum.push_back(int2{cp, mu});
-          if (q > 0) xsum.push_back(int2{cr, cu}), msum.push_back(int2{cr, mu});
-          if (T > 0) xsum.push_back(int2{cp, cv}), msum.push_back(int2{cp, mv});
-          if (q > 0 && T > 0) xsum.push_back(int2{cr, cv}), msum.push_back(int2{cr, mv});
-          ucol.push_back(int2{q, col32 + k});
+          const int cp = 2 * q, cr = 2 * q + 1, cu = 2 * (col + k), cv = cu + 1;
+          xsum.push_back(int2{cp, cu});
+          if (q > 0) xsum.push_back(int2{cr, cu});
+          if (T > 0) xsum.push_back(int2{cp, cv});
+          if (q > 0 && T > 0) xsum.push_back(int2{cr, cv});
+          ucol.push_back(int2{q, col + k});
           E.mo = int(mono.size());
           for (double c : pk) monod.push_back(E.N * c), mono.push_back(float2{float(E.N * c), float(E.N * c - double(float(E.N * c)))});
           std::vector<double> pn(pk.size() + 1, 0.0);
@@ -182,7 +180,7 @@ struct SnapTables {
           ent.push_back(E);
         }
       }
-      col32 += (J - T) / 2 + 1;
+      col += (J - T) / 2 + 1;
     }
     for (int e = 0; e < int(ent.size()); ++e) eord.push_back(e);
     std::stable_sort(eord.begin(), eord.end(), [&](int x, int y) {
@@ -408,7 +406,7 @@ void free_snap(Ctx& c) {
   h->ysrc.release();
   h->zs.release();
   for (auto* b : {&h->e0, &h->map, &h->zt0, &h->tmask, &h->eord, &h->pj, &h->cnt}) b->release();
-  for (auto* b : {&h->xsum, &h->msum, &h->ucol, &h->half, &h->zt, &h->prod}) b->release();
+  for (auto* b : {&h->xsum, &h->ucol, &h->half, &h->zt, &h->prod}) b->release();
   for (auto* b : {&h->zc, &h->monod, &h->cY, &h->AB, &h->beta0, &h->wjelem, &h->pr, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk,
                   &h->eatom, &h->adj, &h->adj_sum, &h->adj_g, &h->keep_u, &h->keep_z})
     b->release();
@@ -675,7 +673,7 @@ static void snap_adjoint(Ctx& c, const double* dL_dF, double dL_dE, double* grad
       A.adj = h->adj.p;
       {
         TimedLaunch t(c, "snap_dt");
-        const size_t smem = sizeof(double) * (size_t((S.nx + 1) & ~1) + 64 * size_t(sd_cols(S.cols32)));
+        const size_t smem = sizeof(double) * (size_t((S.nx + 1) & ~1) + 64 * size_t(su_stride(S.cols)));
         require(smem <= kMaxDynSmem, EMD_ERR_ARG, "SNAP adjoint: twojmax too large for shared memory");
         allow_dyn_smem(k_snap_dt);
         k_snap_dt<<<A.n, 32, smem, c.stream>>>(A);
@@ -764,7 +762,6 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   S.ne = int(tab.ent.size());
   S.nx = int(tab.xsum.size());
   S.cols = su_cols(twojmax);
-  S.cols32 = su_cols32(twojmax);
   S.nuf = (twojmax + 1) * (twojmax + 2) * (2 * twojmax + 3) / 6;
   S.ntask = int(tab.task.size());
   S.nz = tab.nz;
@@ -806,7 +803,6 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   upload(c, h->e0, tab.e0);
   upload(c, h->xsum, tab.xsum);
   upload(c, h->ucol, tab.ucol);
-  upload(c, h->msum, tab.msum);
   upload(c, h->monod, tab.monod);
   upload(c, h->mono, tab.mono);
   upload(c, h->eord, tab.eord);
@@ -840,7 +836,6 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   S.e0 = h->e0.p;
   S.xsum = h->xsum.p;
   S.ucol = h->ucol.p;
-  S.msum = h->msum.p;
   S.monod = h->monod.p;
   S.mono = h->mono.p;
   S.eord = h->eord.p;

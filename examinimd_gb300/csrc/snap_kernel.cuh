@@ -16,8 +16,8 @@
 // Per force call, over chunks of atoms:
 //   k_snap_pairs  inside list and per-pair scalars (lanes = pairs)
 //   k_snap_u      U_tot = wself + sum over the neighbours of w_j sfac U, from the
-//                 four real products of conj(a)^q and b^T times P_k (one warp per
-//                 atom; lanes = neighbours, then sums)
+//                 four real products of conj(a)^q and b^T times powers of x (one warp
+//                 per atom; lanes = neighbours, then sums)
 //   k_snap_y      Z and Y (lanes = atoms, so the Clebsch-Gordan loops are
 //                 uniform and every operand load is coalesced)
 //   k_snap_force  pair forces (lanes = pairs): Phi = Re sum conj(U) Y and its
@@ -84,16 +84,15 @@ struct ZGrp {
 
 struct SnapDev {
   int twojmax, ne, nx, nuf;    // entries, real sums, elements of the full grid
-  int cols, cols32;            // columns of a neighbour's table (su_cols), of the mixed form's (su_cols32)
+  int cols;                    // pairs of columns of a neighbour's table (su_cols)
   int ntask, nfull, nz;        // Z tasks, (j1 >= j2, j) triples, kept Z values per atom
   int ncoeff, ncoeffall, nelem, ntypes;
   double rfac0, rmin0, cutsq, wself;
   int switchflag;
   const Entry* ent;
   const int* e0;       // (J + 1) x (J + 1): first entry of (T, q)
-  const int2* xsum;    // nx: the two factors of a sum in a neighbour's table (k_snap_u)
+  const int2* xsum;    // nx: the two factors of a sum in a neighbour's row (k_snap_u, k_snap_dt)
   const int2* ucol;    // ne: the mixed form's two columns of an entry
-  const int2* msum;    // nx: the two factors of a sum over powers of x (k_snap_dt)
   const float2* mono;  // N P_k in powers of x, high and low part
   const double* monod; // the same in FP64
   const int* eord;     // entries, highest k first
@@ -351,102 +350,77 @@ __global__ void __launch_bounds__(64) k_snap_pairs(SnapArgs A) {
 
 // ---------------------------------------------------------------------- U
 // One warp per atom, 32 neighbours at a time.  Lanes = neighbours: the powers
-// p_q + i r_q = a^q and u_T + i v_T = w b^T and their products with the
-// polynomials go to the neighbour's row of a shared table.  Lanes = sums: each
-// of the nx real sums is p or r times one of those products over the
-// neighbours, one FP64 multiply-add per neighbour.  Then the half-grid
-// elements, once per atom.  Bound by the FP64 pipe: about 240 instructions for
-// 32 neighbours' rows, nx / 32 for each neighbour, 530 per atom at twojmax 8 and
-// 26 neighbours.
+// p_q + i r_q = a^q and u_T + i v_T = w b^T, the latter times the powers of x (the
+// same for every q), go to the neighbour's row of a shared table.  Lanes = sums:
+// each of the nx real sums is p or r times a power's u or v over the neighbours, one
+// FP64 multiply-add per neighbour.  Then, once per atom, the sums over powers are
+// combined into the polynomials' and those into the half-grid elements.  The powers'
+// rounding is amplified by the polynomials' coefficients (16 at twojmax 8, 221 at
+// 14); the forces' error against long double is what it was with P_k in the row
+// (4e-15 of the RMS force).  Bound by the FP64 pipe: about 100 instructions for 32
+// neighbours' rows (240 with P_k), nx / 32 for each neighbour; the table, half as
+// wide, lets eleven warps share an SM instead of six (8,160 atoms: 0.33 -> 0.21 ms).
 //
 // The mixed form, which rounds U_tot to FP32 anyway, takes k_snap_u32
-// (snap_split.cuh): sums over u x^k and v x^k, the same for every q, combined into
-// the polynomials' once per atom.  Per 128,000 atoms: 4.98 ms as the FP64 form
-// does it, 2.80 with powers of x in FP64, 0.87 in FP32 pairs.
-inline int su_cols(int J) {  // p, r; u, v; u P_k, v P_k (k >= 1)
-  int c = 2 * (J + 1) + 2 * (J + 1);
-  for (int T = 0; T <= J; ++T)
-    for (int q = 0; q <= J - T; ++q) c += (T ? 2 : 1) * ((J - T - q) / 2);
-  return c | 1;  // odd: rows start in different banks
-}
-
-// float4 columns of a neighbour's row: (p, r) of a^q; (u x^k, v x^k) of w b^T
-inline int su_cols32(int J) {
+// (snap_split.cuh): per 128,000 atoms 2.80 ms in FP64, 0.87 in FP32 pairs.
+// pairs of columns of a neighbour's row: (p, r) of a^q; (u x^k, v x^k) of w b^T
+inline int su_cols(int J) {
   int c = J + 1;
   for (int T = 0; T <= J; ++T) c += (J - T) / 2 + 1;
   return c | 1;  // odd: eight lanes' rows start in different banks
 }
 
-// doubles of a row of k_snap_dt's tables
-__host__ __device__ inline int sd_cols(int cols32) { return (2 * cols32) | 1; }
+// doubles of an FP64 row (odd: rows start in different banks)
+__host__ __device__ inline int su_stride(int cols) { return (2 * cols) | 1; }
 
-// the neighbour's table row: powers, polynomials and products
-__device__ __forceinline__ void su_row(const SnapDev& S, double* t, double ar, double ai, double br, double bi,
-                                       double w) {
-  const int J = S.twojmax;
-  double* uT = t + 2 * (J + 1);  // u_T, v_T
-  double* prod = t + 4 * (J + 1);
-  t[0] = 1.0;
-  t[1] = 0.0;
-  uT[0] = w;
-  uT[1] = 0.0;
-  double p = ar, r = ai, u = w * br, v = w * bi;
+// the neighbour's table row: powers of a, those of b times those of x
+__device__ __forceinline__ void su_row(int J, double* t, double ar, double ai, double br, double bi, double w) {
+  double* col = t + 2 * (J + 1);
+  const double x = fma(ar, ar, ai * ai) - fma(br, br, bi * bi);
+  double p = 1.0, r = 0.0, u = w, v = 0.0;
 #pragma unroll 1
-  for (int q = 1; q < J; ++q) {
+  for (int q = 0; q <= J; ++q) {
     t[2 * q] = p;
     t[2 * q + 1] = r;
-    uT[2 * q] = u;
-    uT[2 * q + 1] = v;
+    double uk = u, vk = v;
+#pragma unroll 1
+    for (int k = 0; k <= (J - q) / 2; ++k) {
+      *col++ = uk;
+      *col++ = vk;
+      uk *= x;
+      vk *= x;
+    }
     const double pn = fma(p, ar, -r * ai), un = fma(u, br, -v * bi);
     r = fma(p, ai, r * ar);
     v = fma(u, bi, v * br);
     p = pn;
     u = un;
   }
-  if (J > 0) {
-    t[2 * J] = p;
-    t[2 * J + 1] = r;
-    uT[2 * J] = u;
-    uT[2 * J + 1] = v;
-  }
-  const double x = fma(ar, ar, ai * ai) - fma(br, br, bi * bi);
-  for (int T = 0; T <= J; ++T) {
-    const double uu = uT[2 * T], vv = uT[2 * T + 1];
-    for (int q = 0; q <= J - T - 2; ++q) {
-      const double2* ab = reinterpret_cast<const double2*>(S.AB) + S.e0[T * (J + 1) + q];
-      const int km = (J - T - q) / 2;
-      double pm = 1.0, pk = x - __ldg(ab).x;
-      *prod++ = uu * pk;
-      if (T > 0) *prod++ = vv * pk;
-      for (int k = 2; k <= km; ++k) {
-        const double2 c = __ldg(ab + k - 1);
-        const double pn = fma(x - c.x, pk, -c.y * pm);
-        pm = pk;
-        pk = pn;
-        *prod++ = uu * pk;
-        if (T > 0) *prod++ = vv * pk;
-      }
-    }
-  }
 }
 
-// the half-grid elements of entry e from its real sums: conj(a)^q b^T = (p u + r v) + i (p v - r u);
-// for -T: (-1)^T ((p u - r v) - i (p v + r u)); N scales, the atom's own term
-// is 1 on the diagonal (T = 0)
-__device__ __forceinline__ void su_elements(const SnapDev& S, int e, const double* x, double N, double self,
-                                            Cplx<double>* U) {
+// the half-grid elements of entry e from its sums over the powers of x (one group
+// per k): conj(a)^q b^T = (p u + r v) + i (p v - r u); for -T: (-1)^T ((p u - r v)
+// - i (p v + r u)); the coefficients hold N, the atom's own term is 1 on the
+// diagonal (T = 0)
+__device__ __forceinline__ void su_store(const SnapDev& S, int e, const double* xs, double self, Cplx<double>* U) {
   const Entry& E = S.ent[e];
   const bool hr = E.q > 0, hv = E.T > 0;
-  const double pu = N * *x++, ru = hr ? N * *x++ : 0.0, pv = hv ? N * *x++ : 0.0, rv = hr && hv ? N * *x : 0.0;
+  const int k = (E.j - E.q - E.T) / 2, g = (hr ? 2 : 1) * (hv ? 2 : 1);
+  const double *m = S.monod + E.mo, *x = xs + E.xo - k * g;
+  double pu = 0.0, ru = 0.0, pv = 0.0, rv = 0.0;
+  for (int l = 0; l <= k; ++l, x += g) {
+    const double c = __ldg(m + l);
+    pu = fma(c, x[0], pu);
+    if (hr) ru = fma(c, x[1], ru);
+    if (hv) pv = fma(c, x[hr ? 2 : 1], pv);
+    if (hr && hv) rv = fma(c, x[3], rv);
+  }
   const int2 h = S.half[e];
   U[h.x] = Cplx<double>{(pu + rv) + (hv ? 0.0 : self), pv - ru};
   if (h.y >= 0) {
     const double sg = E.T & 1 ? -1.0 : 1.0;
     U[h.y] = Cplx<double>{sg * (pu - rv), -sg * (pv + ru)};
   }
-}
-__device__ __forceinline__ void su_store(const SnapDev& S, int e, const double* x, double self, Cplx<double>* U) {
-  su_elements(S, e, x + S.ent[e].xo, S.ent[e].N, self, U);
 }
 
 static __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
@@ -455,7 +429,7 @@ static __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
   double* xs = su_smem;                       // nx sums
   double* tab = su_smem + ((S.nx + 1) & ~1);  // 32 rows
   const int al = blockIdx.x, lane = threadIdx.x;
-  const int cols = S.cols, n = A.cnt[al];
+  const int cols = su_stride(S.cols), n = A.cnt[al];
   const int2* __restrict__ xsum = S.xsum;
   const size_t np = size_t(A.n) * A.cap;
   const double* pd = A.pd + size_t(al) * A.cap;
@@ -463,7 +437,7 @@ static __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
     const int m = min(32, n - n0);
     if (lane < m) {
       const double* q = pd + n0 + lane;
-      su_row(S, tab + lane * cols, q[PD_AR * np], q[PD_AI * np], q[PD_BR * np], q[PD_BI * np], q[PD_SF * np]);
+      su_row(S.twojmax, tab + lane * cols, q[PD_AR * np], q[PD_AI * np], q[PD_BR * np], q[PD_BI * np], q[PD_SF * np]);
     }
     __syncwarp();
     for (int r0 = 0; r0 < S.nx; r0 += 96) {  // three sums per lane at once
@@ -501,7 +475,7 @@ static __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
     __syncwarp();
   }
   Cplx<double>* U = static_cast<Cplx<double>*>(A.U) + size_t(al) * S.nh;
-  for (int e = lane; e < S.ne; e += 32) su_store(S, e, xs, S.wself, U);
+  for (int e = lane; e < S.ne; e += 32) su_store(S, __ldg(S.eord + e), xs, S.wself, U);
 }
 
 // ------------------------------------------------------------------- Z, Y
@@ -1252,25 +1226,13 @@ __device__ __forceinline__ void sd_row(const SnapDev& S, double* t, double* dt, 
   }
 }
 
-// su_store's sums of entry e from those over the powers of x, one group per k
-__device__ __forceinline__ void sd_combine(const SnapDev& S, int e, const double* xs, double* x) {
-  const Entry& E = S.ent[e];
-  const double* m = S.monod + E.mo;
-  const int k = (E.j - E.q - E.T) / 2, g = (E.q > 0 ? 2 : 1) * (E.T > 0 ? 2 : 1);
-  for (int h = 0; h < g; ++h) {
-    double s = 0.0;
-    for (int l = 0; l <= k; ++l) s = fma(__ldg(m + l), xs[E.xo + (l - k) * g + h], s);
-    x[h] = s;
-  }
-}
-
 static __global__ void __launch_bounds__(32) k_snap_dt(SnapArgs A) {
   const SnapDev& S = A.S;
   extern __shared__ __align__(16) double sd_smem[];
   double* xs = sd_smem;
   double* tab = sd_smem + ((S.nx + 1) & ~1);
   const int al = blockIdx.x, lane = threadIdx.x, i = A.first + al;
-  const int cols = sd_cols(S.cols32), n = A.cnt[al];
+  const int cols = su_stride(S.cols), n = A.cnt[al];
   const size_t np = size_t(A.n) * A.cap;
   const double gix = A.g[3 * i], giy = A.g[3 * i + 1], giz = A.g[3 * i + 2];
   for (int n0 = 0; n0 < max(n, 1); n0 += 32) {
@@ -1291,7 +1253,7 @@ static __global__ void __launch_bounds__(32) k_snap_dt(SnapArgs A) {
     }
     __syncwarp();
     for (int r = lane; r < S.nx; r += 32) {
-      const int2 s = __ldg(S.msum + r);
+      const int2 s = __ldg(S.xsum + r);
       double acc = n0 > 0 ? xs[r] : 0.0;
       for (int k = 0; k < m; ++k) {
         const double* t = tab + 2 * k * cols;
@@ -1302,12 +1264,7 @@ static __global__ void __launch_bounds__(32) k_snap_dt(SnapArgs A) {
     }
     __syncwarp();
   }
-  for (int e = lane; e < S.ne; e += 32) {
-    double x[4];
-    const int ee = __ldg(S.eord + e);
-    sd_combine(S, ee, xs, x);
-    su_elements(S, ee, x, 1.0, 0.0, A.D + size_t(al) * S.nh);
-  }
+  for (int e = lane; e < S.ne; e += 32) su_store(S, __ldg(S.eord + e), xs, 0.0, A.D + size_t(al) * S.nh);
 }
 
 // half-grid elements of U and D, weighted (2, or 1 for the self-inverse ones,
@@ -1386,7 +1343,7 @@ void launch_y32(const SnapArgs& A, cudaStream_t s) {
 }
 
 inline void launch_u(const SnapArgs& A, cudaStream_t s) {
-  const size_t smem = sizeof(double) * (size_t((A.S.nx + 1) & ~1) + 32 * size_t(A.S.cols));
+  const size_t smem = sizeof(double) * (size_t((A.S.nx + 1) & ~1) + 32 * size_t(su_stride(A.S.cols)));
   allow_dyn_smem(k_snap_u);
   k_snap_u<<<A.n, 32, smem, s>>>(A);
   EMD_CHECK_LAUNCH();

@@ -95,7 +95,7 @@ static __global__ void __launch_bounds__(32) k_snap_u32(SnapArgs A) {
       const float* q = pr + n0 + nb;
       auto get = [&](int h, int l) { return F2{q[h * np], q[l * np]}; };
       const F2 ar = get(PR_AR, PR_ARL), ai = get(PR_AI, PR_AIL);
-      float4* t = tab + nb * S.cols32;
+      float4* t = tab + nb * S.cols;
       if (lane < SU_ROWS) su_row_a(S.twojmax, t, ar, ai);
       else su_row_b(S.twojmax, t + S.twojmax + 1, ar, ai, get(PR_BR, PR_BRL), get(PR_BI, PR_BIL), get(PR_SF, PR_SFL));
     }
@@ -113,7 +113,7 @@ static __global__ void __launch_bounds__(32) k_snap_u32(SnapArgs A) {
       auto rows = [&](auto nh) {
 #pragma unroll 2
         for (int k = 0; k < m; ++k) {
-          const float4* t = tab + k * S.cols32;
+          const float4* t = tab + k * S.cols;
 #pragma unroll
           for (int h = 0; h < decltype(nh)::value; ++h) {
             const float4 a = t[col[h].x], b = t[col[h].y];
@@ -142,7 +142,7 @@ static __global__ void __launch_bounds__(32) k_snap_u32(SnapArgs A) {
 }
 
 inline void launch_u32(const SnapArgs& A, cudaStream_t s) {
-  const size_t smem = sizeof(F2Sum) * 4 * size_t(A.S.ne) + SU_ROWS * 16 * size_t(A.S.cols32);
+  const size_t smem = sizeof(F2Sum) * 4 * size_t(A.S.ne) + SU_ROWS * 16 * size_t(A.S.cols);
   allow_dyn_smem(k_snap_u32);
   k_snap_u32<<<A.n, 32, smem, s>>>(A);
   EMD_CHECK_LAUNCH();
