@@ -120,16 +120,12 @@ def kernel_flops(twojmax: int, ninside: float) -> dict:
     """Per-atom operation counts of the kernels' own formulation."""
     J, n = twojmax, float(ninside)
     sums = sum((j + 1) ** 2 for j in range(J + 1))
-    # U, per neighbour: powers of a and b (6 each), x, one multiply-add per real
-    # sum, and the products with u and v: of the polynomials (4 operations from
-    # k = 2 on) in the FP64 form; of the powers of x in the mixed form, whose
-    # sums are combined once per atom
-    poly = sum(1 + 4 * (k - 1) for _, _, k in _entries(J) if k > 0)
-    prods = sum((2 if T else 1) * k for T, _, k in _entries(J))
+    # U, per neighbour: powers of a and b (6 each), x, their products with the
+    # powers of x, one multiply-add per real sum; the sums are combined into the
+    # polynomials' once per atom
     powers = sum((2 if T else 1) * ((J - T) // 2) for T in range(J + 1))
     combine = sum((2 if T else 1) * (2 if q else 1) * (k + 1) * (k + 2) for T, q, k in _entries(J))
-    u_base = n * (12.0 * J + 7 + 2.0 * sums) + 3.0 * sums
-    u_stage = {"fp64": u_base + n * (poly + prods), "mixed": u_base + n * powers + combine}
+    u_stage = n * (12.0 * J + 7 + 2.0 * sums + powers) + 3.0 * sums + combine
     products, weighted, zs = product_counts(J)
     y_stage = 6.0 * products + 4.0 * weighted + 4.0 * zs
     # pair forces, per neighbour: powers, P and P' (9 from k = 2 on), their sums
@@ -139,15 +135,17 @@ def kernel_flops(twojmax: int, ninside: float) -> dict:
         w = 2 if T else 1
         force += (1 if k else 0) + 9 * max(0, k - 1) + w * (4 * min(k, 1) + 8 * max(0, k - 1)) + w * (24 if q else 4)
     force += 22.0 * J
-    scalars, tail = n * 80.0, n * 18.0
+    # the mixed form's FP64: r^2, the r^-14 term and the force sums; its scalars and
+    # U sums run in FP32 pairs, each operation counted once although a product
+    # takes six
+    scalars, tail = n * 80.0, n * 26.0
     return {
         "twojmax": J,
         "ninside": n,
-        "phases": {"scalars": scalars, "U": u_stage["fp64"], "Y": y_stage, "force": n * force + tail},
-        "total": scalars + u_stage["fp64"] + y_stage + n * force + tail,
-        "fp64": {"mixed": scalars + u_stage["mixed"] + tail,
-                 "fp64": scalars + u_stage["fp64"] + y_stage + n * force + tail},
-        "fp32": {"mixed": y_stage + n * force, "fp64": 0.0},
+        "phases": {"scalars": scalars, "U": u_stage, "Y": y_stage, "force": n * force + tail},
+        "total": scalars + u_stage + y_stage + n * force + tail,
+        "fp64": {"mixed": tail, "fp64": scalars + u_stage + y_stage + n * force + tail},
+        "fp32": {"mixed": scalars + u_stage + y_stage + n * force, "fp64": 0.0},
     }
 
 
