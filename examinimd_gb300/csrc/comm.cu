@@ -3,6 +3,8 @@
 // compaction so ghosts land at exactly the indices the serial reference
 // gives them, one-launch ghost position refresh, and the phase-ordered
 // reverse force accumulation.  -fmad=false (pure add/sub anyway).
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstring>
 
@@ -278,22 +280,31 @@ __global__ void k_halo_force(double* __restrict__ f, const int* __restrict__ pac
   f[3 * i + 2] += f[3 * g + 2];
 }
 
-// The six phases of a small halo in order, one block (a launch per phase costs
-// more than its additions): 7,000 ghosts 36 -> 20 us, 400 ghosts 36 -> 10 us.
-constexpr int HALO_FORCE_MAX = 16384;
+// The six phases in order by one CTA, or one cluster of eight, which goes past L1
+// because a phase reads what another CTA wrote (a launch per phase costs more than
+// its additions up to here): 400 ghosts 36 -> 10 us, 7,000 36 -> 20 (the cluster
+// takes as long), 48,000 39 -> 26.
+constexpr int HALO_FORCE_MAX = 200000, HALO_FORCE_ONE = 8192, HALO_FORCE_CTAS = 8, HALO_FORCE_THREADS = 1024;
 struct HaloPhases {
   int pack[6], count[6], ghost[6];
 };
-__global__ void __launch_bounds__(1024) k_halo_force_all(double* __restrict__ f, const int* __restrict__ pack,
-                                                         HaloPhases P) {
+template <bool CLUSTER>
+__global__ void __launch_bounds__(HALO_FORCE_THREADS)
+    k_halo_force_all(double* __restrict__ f, const int* __restrict__ pack, HaloPhases P) {
   for (int phase = 5; phase >= 0; --phase) {
-    for (int k = threadIdx.x; k < P.count[phase]; k += blockDim.x) {
+    for (int k = blockIdx.x * HALO_FORCE_THREADS + threadIdx.x; k < P.count[phase];
+         k += gridDim.x * HALO_FORCE_THREADS) {
       const int i = pack[P.pack[phase] + k], g = P.ghost[phase] + k;
-      f[3 * i] += f[3 * g];
-      f[3 * i + 1] += f[3 * g + 1];
-      f[3 * i + 2] += f[3 * g + 2];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        double *fi = f + 3 * size_t(i) + d, *fg = f + 3 * size_t(g) + d;
+        if (CLUSTER) __stcg(fi, __ldcg(fi) + __ldcg(fg));
+        else *fi += *fg;
+      }
     }
-    __syncthreads();
+    if (phase == 0) break;
+    if (CLUSTER) cooperative_groups::this_cluster().sync();
+    else __syncthreads();
   }
 }
 
@@ -401,7 +412,14 @@ emd_status emd_comm_exchange_halo(emd_ctx* ctx, int* n_ghost_out) {
     double part = 1.0;
     for (int d = 0; d < 3; ++d)
       part *= 1.0 + 2.0 * c.comm_depth / c.domain[d];
-    reserve_particles(c, size_t(std::min(double(0x7ffffffe), std::max(double(h.overflow), N_local * part))));
+    const size_t known = size_t(h.overflow);
+    const size_t guess = size_t(std::min(double(0x7ffffffe), std::max(double(known), N_local * part)));
+    try {
+      reserve_particles(c, guess);
+    } catch (const Error& e) {
+      if (e.code != EMD_ERR_NOMEM || guess == known) throw;
+      reserve_particles(c, known);
+    }
   }
   const int N_ghost = h.base[3];
   grow_particles(c, N_local + N_ghost);
@@ -447,8 +465,22 @@ emd_status emd_comm_update_force(emd_ctx* ctx) {
       P.ghost[p] = c.ghost_offsets[p];
     }
     TimedLaunch t(c, "comm_update_force");
-    k_halo_force_all<<<1, 1024, 0, c.stream>>>(c.f.p, c.pack.p, P);
-    EMD_CHECK_LAUNCH();
+    if (acc <= HALO_FORCE_ONE) {
+      k_halo_force_all<false><<<1, HALO_FORCE_THREADS, 0, c.stream>>>(c.f.p, c.pack.p, P);
+      EMD_CHECK_LAUNCH();
+      return EMD_OK;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(HALO_FORCE_CTAS);
+    cfg.blockDim = dim3(HALO_FORCE_THREADS);
+    cfg.stream = c.stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = HALO_FORCE_CTAS;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    EMD_CUDA(cudaLaunchKernelEx(&cfg, k_halo_force_all<true>, c.f.p, static_cast<const int*>(c.pack.p), P));
     return EMD_OK;
   }
   for (int phase = 5; phase >= 0; --phase) {

@@ -1,7 +1,7 @@
 """Halo, binning and reverse forces at the sizes where their kernels change, against
 the CPU oracle: one CTA (up to 1,024 owned, 4,096 binned particles) and tiles of
-1,024 (the last block scans 256 of them at a time), one launch for up to 16,384
-ghosts' forces and one per phase.  GPU.
+1,024 (the last block scans 256 of them at a time), one CTA for up to 8,192
+ghosts' forces and a cluster beyond.  GPU.
 """
 import numpy as np
 import pytest
@@ -51,7 +51,7 @@ def test_halo_and_binning_match_the_oracle(n, box):
         np.testing.assert_array_equal(p, q)
 
 
-@pytest.mark.parametrize("n,box", [(700, 9.0), (9000, 25.0), (40000, 38.0)])
+@pytest.mark.parametrize("n,box", [(700, 9.0), (9000, 25.0), (20000, 30.0), (40000, 38.0)])
 def test_reverse_forces(n, box):
     """Half list with newton: ghosts' forces return to their owners; the sums are
     in another order than the oracle's, a few hundred terms rounded to 2^-53 each."""
