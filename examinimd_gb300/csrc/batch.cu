@@ -27,7 +27,7 @@
 // other atoms still read the old ones.  All of a run's launches again go into one
 // CUDA graph.  Both forms do the same per-atom arithmetic in the same order.
 // 1,360,000 atoms in 256 systems, ms per 20 steps: 9.7 with a launch per phase and
-// rows an atom per thread, 6.1 as it is.
+// rows an atom per thread, 5.9 as it is.
 //
 // emd_batch_tune picks the form, the CTA size and the steps per launch by
 // timing the candidates on the ensemble itself.
@@ -91,6 +91,7 @@ struct BArgs {
   double cut_nb, cutsq_nb;
   float nb_lo, nb_hi;  // FP32 decision band of the neighbour test
   LJParamsF P;
+  int n_chunks;  // of owned atoms, in front of the ghosts' chunks
   int every;
   int step0, nsteps;   // steps step0+1 .. step0+nsteps
 };
@@ -268,36 +269,34 @@ __device__ void rebuild(const BArgs& A, const BSys& S, int* sh, int* hist) {
   int ng = 0;
   bool over = false;
   for (int d = 0; d < 3; ++d) {
-    const int cur = n + ng;
+    const int cur = min(n + ng, S.cap);
     const long long klo = order_key(A.cut_nb), khi = order_key(S.L[d] - A.cut_nb);
-    for (int c0 = 0; c0 < cur; c0 += T) {
-      const int c = c0 + tid;
-      bool lo = false, hi = false;
-      if (c < cur) {
-        const double4_32a p = x[c];
-        const long long key = order_key(d == 0 ? p.x : (d == 1 ? p.y : p.z));
-        lo = key < klo;
-        hi = key >= khi;
-      }
-      int tot;
-      const int pos = block_excl(int(lo) + int(hi), sh, tot);
-      if (lo || hi) {
-        const double4_32a p = x[c];
-        const int own = owner[c], im = img[c];
-        for (int s = 0; s < 2; ++s) {
-          if (s == 0 ? !lo : !hi) continue;
-          const int g = n + ng + pos + (s == 1 && lo ? 1 : 0);
-          if (g >= S.cap) {
-            over = true;
-            continue;
-          }
-          double4_32a q = p;
-          double* qc = &q.x;
-          qc[d] += s == 0 ? S.L[d] : -S.L[d];
-          x[g] = q;
-          owner[g] = own;
-          img[g] = (im & ~(3 << (2 * d))) | ((s == 0 ? 2 : 0) << (2 * d));
+    // four candidates a thread and scan: a scan's barriers cost more than its sweep
+    for (int c0 = 0; c0 < cur; c0 += 4 * T) {
+      const int c1 = c0 + 4 * tid;
+      int faces = 0;  // bits 2 k and 2 k + 1: candidate c1 + k at the lower, the upper face
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (c1 + k < cur) {
+          const long long key = order_key((&x[c1 + k].x)[d]);
+          faces |= (key < klo ? 1 << (2 * k) : 0) | (key >= khi ? 2 << (2 * k) : 0);
         }
+      int tot;
+      int g = n + ng + block_excl(__popc(faces), sh, tot);
+      while (faces) {
+        const int bit = __ffs(faces) - 1, c = c1 + (bit >> 1), s = bit & 1;
+        faces &= faces - 1;
+        if (g >= S.cap) {
+          over = true;
+          break;
+        }
+        double4_32a q = x[c];
+        double* qc = &q.x;
+        qc[d] += s == 0 ? S.L[d] : -S.L[d];
+        x[g] = q;
+        owner[g] = owner[c];
+        img[g] = (img[c] & ~(3 << (2 * d))) | ((s == 0 ? 2 : 0) << (2 * d));
+        ++g;
       }
       ng += tot;
     }
@@ -323,7 +322,7 @@ __device__ void rebuild(const BArgs& A, const BSys& S, int* sh, int* hist) {
     binof[p] = b;
     const ushort4 c = make_ushort4(bx, by, bz, img[p]);
     binc[p] = c;
-    xl[p] = rel_to_bin(A, S, q, c);
+    if (A.nsteps > 0) xl[p] = rel_to_bin(A, S, q, c);  // phased form: BP_REL, on all SMs
     atomicAdd(&hist[b], 1);
   }
   __syncthreads();
@@ -356,10 +355,14 @@ __device__ __forceinline__ void halo_ghost(const BArgs& A, const BSys& S, int g)
   double4_32a* x = A.x + S.base;
   double4_32a p = x[A.owner[S.base + g]];
   const ushort4 b = A.binc[S.base + g];
-  auto shift = [](int code, double L) { return code == 1 ? 0.0 : (code == 2 ? L : -L); };
-  p.x += shift(b.w & 3, S.L[0]);
-  p.y += shift((b.w >> 2) & 3, S.L[1]);
-  p.z += shift((b.w >> 4) & 3, S.L[2]);
+  // most ghosts are images in one dimension, and neighbours in the same one: no FP64
+  // addition for the others
+  auto shift = [](double& v, int code, double L) {
+    if (code != 1) v += code == 2 ? L : -L;
+  };
+  shift(p.x, b.w & 3, S.L[0]);
+  shift(p.y, (b.w >> 2) & 3, S.L[1]);
+  shift(p.z, (b.w >> 4) & 3, S.L[2]);
   x[g] = p;
   A.xl[S.base + g] = rel_to_bin(A, S, p, b);
 }
@@ -460,13 +463,19 @@ constexpr int BP_THREADS = 128;
 struct BChunk {
   int sys, first;
 };
-enum { BP_NVE_INITIAL, BP_HALO, BP_FORCE, BP_STEP, BP_LAST };
+enum { BP_NVE_INITIAL, BP_HALO, BP_REL, BP_FORCE, BP_STEP, BP_LAST };
 
 template <int PHASE>
 __global__ void __launch_bounds__(BP_THREADS) k_batch_phase(BArgs A, const BChunk* __restrict__ chunks) {
   const BChunk ch = chunks[blockIdx.x];
   const BSys& S = A.sys[ch.sys];
   const int k = ch.first + threadIdx.x;
+  if (PHASE == BP_REL) {  // owned atoms' chunks, then ghosts'
+    const int p = blockIdx.x < A.n_chunks ? k : S.n + k;
+    if (p < (blockIdx.x < A.n_chunks ? S.n : S.n + min(A.nghost[ch.sys], S.cap - S.n)))
+      A.xl[S.base + p] = rel_to_bin(A, S, A.x[S.base + p], A.binc[S.base + p]);
+    return;
+  }
   if (PHASE == BP_HALO) {
     const int ng = min(A.nghost[ch.sys], S.cap - S.n);
     if (k < ng) halo_ghost(A, S, S.n + k);
@@ -619,8 +628,7 @@ struct emd_batch {
   size_t slots = 0;  // particle slots over all systems (owned + ghost capacity)
   // phased form: chunk tables of the owned atoms, of the ghost capacity and of the bins
   bool phased = false;
-  BChunk* d_chunks = nullptr;
-  BChunk* d_gchunks = nullptr;
+  BChunk* d_chunks = nullptr;  // the ghosts' behind the owned atoms'
   BChunk* d_bchunks = nullptr;
   int n_chunks = 0, n_gchunks = 0, n_bchunks = 0;
 };
@@ -663,13 +671,14 @@ void batch_launch(emd_batch* b, int step0, int nsteps, int threads) {
 template <int PHASE>
 void batch_phase(emd_batch* b) {
   const bool ghosts = PHASE == BP_HALO;
-  k_batch_phase<PHASE><<<ghosts ? b->n_gchunks : b->n_chunks, BP_THREADS, 0, b->stream>>>(
-      b->a, ghosts ? b->d_gchunks : b->d_chunks);
+  const int blocks = PHASE == BP_REL ? b->n_chunks + b->n_gchunks : (ghosts ? b->n_gchunks : b->n_chunks);
+  k_batch_phase<PHASE><<<blocks, BP_THREADS, 0, b->stream>>>(b->a, b->d_chunks + (ghosts ? b->n_chunks : 0));
   EMD_CHECK_LAUNCH();
 }
 
 void batch_rebuild(emd_batch* b, int threads) {
   batch_launch(b, 0, 0, threads);
+  batch_phase<BP_REL>(b);
   k_batch_rows<<<b->n_bchunks, 32 * BR_WARPS, 0, b->stream>>>(b->a, b->d_bchunks);
   EMD_CHECK_LAUNCH();
 }
@@ -835,11 +844,9 @@ emd_status emd_batch_create(emd_batch** out, int device, int nsys, const int* na
     EMD_CUDA(device_malloc(reinterpret_cast<void**>(&b->d_bchunks), sizeof(BChunk) * bch.size()));
     EMD_CUDA(cudaMemcpyAsync(b->d_bchunks, bch.data(), sizeof(BChunk) * bch.size(), cudaMemcpyHostToDevice,
                              b->stream));
+    ch.insert(ch.end(), gch.begin(), gch.end());
     EMD_CUDA(device_malloc(reinterpret_cast<void**>(&b->d_chunks), sizeof(BChunk) * ch.size()));
-    EMD_CUDA(device_malloc(reinterpret_cast<void**>(&b->d_gchunks), sizeof(BChunk) * gch.size()));
     EMD_CUDA(cudaMemcpyAsync(b->d_chunks, ch.data(), sizeof(BChunk) * ch.size(), cudaMemcpyHostToDevice, b->stream));
-    EMD_CUDA(cudaMemcpyAsync(b->d_gchunks, gch.data(), sizeof(BChunk) * gch.size(), cudaMemcpyHostToDevice,
-                             b->stream));
     EMD_CUDA(cudaStreamSynchronize(b->stream));
   }
   // positions / velocities into the device slots (owned atoms keep the caller's order)
@@ -889,6 +896,7 @@ emd_status emd_batch_create(emd_batch** out, int device, int nsys, const int* na
   b->cutsq = cut * cut;
   a.P = LJParamsF{nullptr, nullptr, nullptr, nullptr, 1, float(b->lj1), float(b->lj2), float(b->cutsq), b->cutsq};
   a.every = every;
+  a.n_chunks = b->n_chunks;
   // initial halo, binning, list and forces
   cudaDeviceProp prop{};
   EMD_CUDA(cudaGetDeviceProperties(&prop, device));
@@ -927,7 +935,6 @@ void emd_batch_destroy(emd_batch* b) {
   b->thermo.release();
   if (b->d_sys) cudaFree(b->d_sys);
   if (b->d_chunks) cudaFree(b->d_chunks);
-  if (b->d_gchunks) cudaFree(b->d_gchunks);
   if (b->d_bchunks) cudaFree(b->d_bchunks);
   if (b->d_status) cudaFree(b->d_status);
   if (b->stream) cudaStreamDestroy(b->stream);
