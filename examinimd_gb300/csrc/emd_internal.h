@@ -180,7 +180,6 @@ struct Ctx {
   int neigh_packed = 0;     // entries are (j << 5) | stencil code
   int neigh_maxrow = 0;     // longest row of the current list
   int neigh_scratch_k = 16; // capacity of the column-major rows behind a CSR list
-  bool neigh_layout_2d = false;  // force kernels read column-major rows
   DevBuf<int> neigh_rows2d;      // column-major rows behind a CSR list
   DevBuf<float4> xl_bin;         // FP32 position relative to the bin centre (last binning)
   bool xl_bin_valid = false;     // xl_bin holds the last binning's offsets (not handed to the mixed force)
@@ -288,6 +287,8 @@ void device_sum_launch(Ctx& c, const double* d_vals, int n, double* scratch);
 unsigned read_status(Ctx& c, bool clear);
 // applies a pending deep_copy(f, 0) to owned and/or ghost rows (after any
 // pending final half kick, which still needs the forces)
+// the current list, column-major (neigh_rows.cuh)
+inline const int* neigh_rows(const Ctx& c) { return c.neigh_kind == EMD_NEIGH_2D ? c.neighs.p : c.neigh_rows2d.p; }
 void materialize_zero(Ctx& c, bool locals, bool ghosts);
 // applies a pending final half kick (integrate.cu)
 void materialize_kick(Ctx& c);

@@ -51,12 +51,12 @@ int lj_tile_rows(int n, bool half) {
 // the sum depends on the atom count only and its scratch is bounded
 constexpr int LJE_BLOCKS = 152 * 6;
 
-template <int MODE, bool TWO_D, bool UNI, bool IDIAL = false, bool ZERO = false>
+template <int MODE, bool UNI, bool IDIAL = false, bool ZERO = false>
 void launch_lj_fp64(LJTile T, cudaStream_t s) {
   T.rows = lj_tile_rows(T.n, T.half);
   T.cap = ljt_cap(T.rows, T.half);
   const size_t smem = LJT_WARPS * ljt_warp_bytes(T.cap, T.half, UNI);
-  auto k = k_lj_fp64<MODE, TWO_D, UNI, IDIAL, ZERO>;
+  auto k = k_lj_fp64<MODE, UNI, IDIAL, ZERO>;
   allow_dyn_smem(k);
   const int tiles = (T.n + T.rows - 1) / T.rows;
   const int grid = MODE == LJ_ENERGY ? LJE_BLOCKS : (tiles + LJT_WARPS - 1) / LJT_WARPS;
@@ -65,14 +65,9 @@ void launch_lj_fp64(LJTile T, cudaStream_t s) {
 }
 
 template <int MODE, bool IDIAL = false, bool ZERO = false>
-void launch_lj_fp64(const LJTile& T, bool two_d, bool uniform, cudaStream_t s) {
-  if (two_d) {
-    if (uniform) launch_lj_fp64<MODE, true, true, IDIAL, ZERO>(T, s);
-    else launch_lj_fp64<MODE, true, false, IDIAL, ZERO>(T, s);
-  } else {
-    if (uniform) launch_lj_fp64<MODE, false, true, IDIAL, ZERO>(T, s);
-    else launch_lj_fp64<MODE, false, false, IDIAL, ZERO>(T, s);
-  }
+void launch_lj_fp64(const LJTile& T, bool uniform, cudaStream_t s) {
+  if (uniform) launch_lj_fp64<MODE, true, IDIAL, ZERO>(T, s);
+  else launch_lj_fp64<MODE, false, IDIAL, ZERO>(T, s);
 }
 
 }  // namespace
@@ -91,7 +86,6 @@ double lj_mixed_energy(Ctx& c);
 //   eps d/deps   of e and fpair: e and fpair themselves
 //   sigma d/dsigma: lj1 -> 12 lj1, lj2 -> 6 lj2.
 // Block partial sums of the four values, in a fixed order.
-template <bool TWO_D>
 __global__ void __launch_bounds__(256) k_lj_adjoint(const double4_32a* __restrict__ x4, ListView L, double lj1,
                                                     double lj2, double cutsq, int n, int packed,
                                                     const double* __restrict__ g, int nblk,
@@ -103,7 +97,7 @@ __global__ void __launch_bounds__(256) k_lj_adjoint(const double4_32a* __restric
     const double4_32a xi = x4[i];
     const double gx = g[3 * i], gy = g[3 * i + 1], gz = g[3 * i + 2];
     const double r2c = 1.0 / cutsq, r6c = r2c * r2c * r2c;
-    const Row<TWO_D> row(L, i);
+    const Row row(L, i);
     for (int jj = 0; jj < row.n; ++jj) {
       const int j = entry_j(row[jj], packed);
       const double4_32a xj = x4[j];
@@ -127,12 +121,9 @@ __global__ void __launch_bounds__(256) k_lj_adjoint(const double4_32a* __restric
 
 ListView list_view(Ctx& c) {
   ListView L;
-  // CSR rows live in neighs; column-major rows in neighs (Neighbor2D) or in
-  // the scratch rows behind a packed CSR list
-  L.entries = (c.neigh_layout_2d && c.neigh_kind != EMD_NEIGH_2D) ? c.neigh_rows2d.p : c.neighs.p;
-  L.offsets = c.neigh_offsets.p;
+  L.entries = neigh_rows(c);
   L.num_neighs = c.num_neighs.p;
-  L.stride = c.neigh_layout_2d ? c.neigh_stride : 0;
+  L.stride = c.neigh_stride;
   return L;
 }
 
@@ -155,7 +146,7 @@ static LJTile lj_tile(Ctx& c) {
 static void launch_lj_energy(Ctx& c, double* part) {
   LJTile T = lj_tile(c);
   T.part = part;
-  launch_lj_fp64<LJ_ENERGY>(T, c.neigh_layout_2d, c.lj_uniform, c.stream);
+  launch_lj_fp64<LJ_ENERGY>(T, c.lj_uniform, c.stream);
 }
 
 // ---- scratch of emd_lj_energy_noalloc
@@ -296,24 +287,23 @@ emd_status emd_lj_compute(emd_ctx* ctx) {
   }
   require(!c.neigh_packed, EMD_ERR_STATE, "emd_lj_compute: list was built for the mixed form");
   const LJTile T = lj_tile(c);
-  const bool two_d = c.neigh_layout_2d;
   const bool uniform = c.lj_uniform && (!c.lj_idial || c.lj_ntypes == 1);
   if (c.lj_half) materialize_zero(c, true, true);
   const bool zero = c.f_zero_pending & 1;
   TimedLaunch t(c, c.lj_half ? "lj_half_fp64" : "lj_full_fp64");
   if (!c.lj_half) {
     if (c.lj_idial) {
-      if (zero) launch_lj_fp64<LJ_FULL, true, true>(T, two_d, uniform, c.stream);
-      else launch_lj_fp64<LJ_FULL, true, false>(T, two_d, uniform, c.stream);
+      if (zero) launch_lj_fp64<LJ_FULL, true, true>(T, uniform, c.stream);
+      else launch_lj_fp64<LJ_FULL, true, false>(T, uniform, c.stream);
     } else {
-      if (zero) launch_lj_fp64<LJ_FULL, false, true>(T, two_d, uniform, c.stream);
-      else launch_lj_fp64<LJ_FULL, false, false>(T, two_d, uniform, c.stream);
+      if (zero) launch_lj_fp64<LJ_FULL, false, true>(T, uniform, c.stream);
+      else launch_lj_fp64<LJ_FULL, false, false>(T, uniform, c.stream);
     }
     c.f_zero_pending &= ~1;
   } else if (c.lj_idial) {
-    launch_lj_fp64<LJ_HALF, true>(T, two_d, uniform, c.stream);
+    launch_lj_fp64<LJ_HALF, true>(T, uniform, c.stream);
   } else {
-    launch_lj_fp64<LJ_HALF, false>(T, two_d, uniform, c.stream);
+    launch_lj_fp64<LJ_HALF, false>(T, uniform, c.stream);
   }
   EMD_API_END
 }
@@ -378,12 +368,7 @@ emd_status emd_lj_adjoint(emd_ctx* ctx, const double* dL_dF, double dL_dE, doubl
     {
       TimedLaunch t(c, "lj_adjoint");
       const ListView L = list_view(c);
-      if (c.neigh_layout_2d)
-        k_lj_adjoint<true><<<grid, 256, 0, c.stream>>>(c.x4.p, L, lj1, lj2, cutsq, n, c.neigh_packed, g.p, grid,
-                                                       c.red2.p);
-      else
-        k_lj_adjoint<false><<<grid, 256, 0, c.stream>>>(c.x4.p, L, lj1, lj2, cutsq, n, c.neigh_packed, g.p, grid,
-                                                        c.red2.p);
+      k_lj_adjoint<<<grid, 256, 0, c.stream>>>(c.x4.p, L, lj1, lj2, cutsq, n, c.neigh_packed, g.p, grid, c.red2.p);
       EMD_CHECK_LAUNCH();
     }
     for (int k = 0; k < 4; ++k) s[k] = device_sum(c, c.red2.p + size_t(k) * grid, grid);

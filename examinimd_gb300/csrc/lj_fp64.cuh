@@ -112,7 +112,7 @@ struct LJTile {
 };
 
 // UNI: one parameter set for every type pair
-template <int MODE, bool TWO_D, bool UNI, bool IDIAL, bool ZERO>
+template <int MODE, bool UNI, bool IDIAL, bool ZERO>
 __global__ void __launch_bounds__(LJT_THREADS) k_lj_fp64(LJTile T) {
   extern __shared__ __align__(16) unsigned char ljt_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(LJT_THREADS) k_lj_fp64(LJTile T) {
     size_t off_l = 0;
     double4_32a xl = make_double4_32a(0.0, 0.0, 0.0, 0.0);
     if (lane < nrow) {
-      const Row<TWO_D> row(T.L, i0 + lane);
+      const Row row(T.L, i0 + lane);
       len_l = row.n;
       off_l = size_t(row.p - T.L.entries);
       xl = T.x4[i0 + lane];
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(LJT_THREADS) k_lj_fp64(LJTile T) {
         const int k = kr + 32 * h + lane;
         e[h] = -1;
         if (ar < nrow && k < len) {
-          e[h] = TWO_D ? __ldg(p + ((size_t(k >> 2) * T.L.stride) << 2) + (k & 3)) : __ldg(p + k);
+          e[h] = __ldg(p + ((size_t(k >> 2) * T.L.stride) << 2) + (k & 3));
           if (T.packed) e[h] >>= 6;
         }
       }

@@ -7,8 +7,9 @@
 // the LayoutLeft of the reference's Neighbor2D view on a GPU, four entries
 // per granule) with capacity K; the host grows K like
 // Neighbor2D's regrow loop (x1.2) when a row overflows.
-// NeighborCSR rows are then compacted behind an exclusive scan of the
-// counts.  Rows built for the mixed-precision force carry packed entries
+// NeighborCSR rows are compacted behind an exclusive scan of the counts when
+// they are read (emd_neigh_get): the force kernels take column-major rows as fast
+// (905,728 atoms: 2.66 ms either way), and compacting them took 0.54 ms a build.  Rows built for the mixed-precision force carry packed entries
 // (j << 6) | (kx << 4) | (ky << 2) | kz with k = (bin_j - bin_i) + 1 per
 // dimension, which the force kernel uses to difference FP32 bin-relative
 // coordinates; the FP64 drop-in stores plain j.
@@ -24,7 +25,7 @@ namespace {
 constexpr int NB_WARPS = 4;     // warps per CTA, one interior bin each (independent)
 constexpr int NB_THREADS = 32 * NB_WARPS;
 constexpr int NB_SLOTS = 64;  // spread slots for the longest-row reduction
-static_assert(2 + NB_SLOTS <= kHostInts, "read-back of the row-length slots exceeds the pinned scratch");
+static_assert(1 + NB_SLOTS <= kHostInts, "read-back of the row-length slots exceeds the pinned scratch");
 
 struct NeighArgs {
   RowArgs r;
@@ -102,6 +103,18 @@ __global__ void k_unpack(int* __restrict__ e, long long n) {
 
 using namespace emd;
 
+// row starts (NeighListCSR::row_map) and number of entries of the current list
+static long long neigh_total(Ctx& c) {
+  if (c.neigh_total >= 0) return c.neigh_total;
+  const int n = c.neigh_rows;
+  c.neigh_offsets.reserve(size_t(n) + 2, c.stream);
+  exclusive_scan_int(c, c.num_neighs.p, c.neigh_offsets.p, n, c.neigh_offsets.p + n);
+  EMD_CUDA(cudaMemcpyAsync(c.h_int, c.neigh_offsets.p + n, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  EMD_CUDA(cudaStreamSynchronize(c.stream));
+  c.neigh_total = n > 0 ? c.h_int[0] : 0;
+  return c.neigh_total;
+}
+
 extern "C" {
 
 emd_status emd_neigh_init(emd_ctx* ctx, int kind, double neigh_cut, int comm_newton) {
@@ -131,7 +144,6 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
   require(!packed || (long long)(c.N_local + c.N_ghost) < (1LL << 25), EMD_ERR_ARG,
           "emd_neigh_create: packed rows need fewer than 2^25 particles");
   c.num_neighs.reserve(size_t(n) + 1, c.stream);
-  c.neigh_offsets.reserve(size_t(n) + 2, c.stream);
   c.resize_flag.reserve(1 + NB_SLOTS, c.stream);
   if (!c.xl_bin_valid) {  // a second build from one binning in the mixed form
     const int n_all = c.N_local + c.N_ghost;
@@ -171,9 +183,8 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
   const bool two_d = c.neigh_kind == EMD_NEIGH_2D;
   int& K = two_d ? c.maxneighs : c.neigh_scratch_k;
   DevBuf<int>& rows = two_d ? c.neighs : c.neigh_rows2d;
-  // the total sizes the compacted CSR list; column-major rows (2D, packed)
-  // need it only when the caller asks, so it is read later on demand there
-  const bool need_total = (!two_d && !packed) || total_out;
+  // row starts and total are read when asked for (emd_neigh_get): the force
+  // kernels take the column-major rows of either kind of list as they are
   while (true) {
     rows.reserve(size_t(n + 1) * size_t((K + 3) & ~3) + 4, c.stream);
     a.r.rows = rows.p;
@@ -193,13 +204,8 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
         EMD_CHECK_LAUNCH();
       }
     }
-    // the scan before the flags are known (a regrow does it again): one wait for both
-    exclusive_scan_int(c, c.num_neighs.p, c.neigh_offsets.p, n, c.neigh_offsets.p + n);
     EMD_CUDA(cudaMemcpyAsync(c.h_int, c.resize_flag.p, (1 + NB_SLOTS) * sizeof(int), cudaMemcpyDeviceToHost,
                              c.stream));
-    if (need_total)
-      EMD_CUDA(cudaMemcpyAsync(c.h_int + 1 + NB_SLOTS, c.neigh_offsets.p + n, sizeof(int), cudaMemcpyDeviceToHost,
-                               c.stream));
     EMD_CUDA(cudaStreamSynchronize(c.stream));
     int longest = 0;
     for (int k = 1; k <= NB_SLOTS; ++k) longest = std::max(longest, c.h_int[k]);
@@ -209,17 +215,6 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
     // neighbor_2d.h:325-327: grow to 1.2x the longest row and redo
     K = int(c.h_int[1] * 1.2);
   }
-  const long long total = !need_total ? -1 : (n > 0 ? c.h_int[1 + NB_SLOTS] : 0);
-  if (!two_d && !packed) {
-    // NeighListCSR (neighbor_csr.h:81-124): rows contiguous at row_map(i)
-    c.neighs.reserve(size_t(total) + 1, c.stream);
-    if (n > 0) {
-      TimedLaunch t(c, "neigh_rows_to_csr");
-      k_rows_to_csr<<<blocks_for(n, 256), 256, 0, c.stream>>>(c.neigh_rows2d.p, n + 1, c.num_neighs.p,
-                                                                c.neigh_offsets.p, n, c.neighs.p);
-      EMD_CHECK_LAUNCH();
-    }
-  }
   if (packed) {
     const int n_all = c.N_local + c.N_ghost;
     c.abin.reserve(size_t(n_all) + 1, c.stream);
@@ -227,14 +222,12 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
   }
   c.neigh_stride = n + 1;
   c.neigh_rows = n;
-  c.neigh_total = total;
+  c.neigh_total = -1;
   c.neigh_ready = true;
   c.neigh_packed = packed;
   c.neigh_builds++;
   if (packed) lj_mixed_after_build(c);
-  // the force kernels read CSR (plain rows) or column-major rows
-  c.neigh_layout_2d = two_d || packed;
-  if (total_out) *total_out = total;
+  if (total_out) *total_out = neigh_total(c);
   EMD_API_END
 }
 
@@ -242,24 +235,15 @@ emd_status emd_neigh_get(emd_ctx* ctx, int* num_neighs, int* entries) {
   EMD_API_BEGIN
   require(c.neigh_ready, EMD_ERR_STATE, "emd_neigh_get: no neighbour list");
   const int n = c.neigh_rows;
-  if (c.neigh_total < 0) {  // not read at build time
-    EMD_CUDA(cudaMemcpyAsync(c.h_int, c.neigh_offsets.p + n, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    EMD_CUDA(cudaStreamSynchronize(c.stream));
-    c.neigh_total = n > 0 ? c.h_int[0] : 0;
-  }
+  neigh_total(c);
   if (num_neighs && n > 0)
     EMD_CUDA(cudaMemcpyAsync(num_neighs, c.num_neighs.p, sizeof(int) * n, cudaMemcpyDeviceToHost, c.stream));
   if (entries && c.neigh_total > 0) {
     DevBuf<int> tmp;
     tmp.reserve(size_t(c.neigh_total), c.stream);
-    if (!c.neigh_layout_2d) {
-      EMD_CUDA(cudaMemcpyAsync(tmp.p, c.neighs.p, sizeof(int) * c.neigh_total, cudaMemcpyDeviceToDevice, c.stream));
-    } else {
-      const int* src = c.neigh_kind == EMD_NEIGH_2D ? c.neighs.p : c.neigh_rows2d.p;
-      k_rows_to_csr<<<blocks_for(n, 256), 256, 0, c.stream>>>(src, c.neigh_stride, c.num_neighs.p,
-                                                              c.neigh_offsets.p, n, tmp.p);
-      EMD_CHECK_LAUNCH();
-    }
+    k_rows_to_csr<<<blocks_for(n, 256), 256, 0, c.stream>>>(neigh_rows(c), c.neigh_stride, c.num_neighs.p,
+                                                            c.neigh_offsets.p, n, tmp.p);
+    EMD_CHECK_LAUNCH();
     if (c.neigh_packed) {
       k_unpack<<<blocks_for(c.neigh_total, 256), 256, 0, c.stream>>>(tmp.p, c.neigh_total);
       EMD_CHECK_LAUNCH();

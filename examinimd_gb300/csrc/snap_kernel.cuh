@@ -316,16 +316,14 @@ __global__ void __launch_bounds__(64) k_snap_pairs(SnapArgs A) {
     const double4_32a xi = A.x4[i];
     const float xf = f32_bits(xi.x), yf = f32_bits(xi.y), zf = f32_bits(xi.z);
     const float thr = f32_cut_threshold(cutsq_f, xf, yf, zf);
-    const Row<false> rowc(A.L, i);
-    const Row<true> row2(A.L, i);
-    const bool two_d = A.L.stride != 0;
+    const Row row(A.L, i);
     int m = 0;  // pairs of this atom
-    for (int k0 = 0; k0 < rowc.n; k0 += 32) {
+    for (int k0 = 0; k0 < row.n; k0 += 32) {
       const int k = k0 + lane;
       bool keep = false;
       int j = 0;
-      if (k < rowc.n) {
-        j = two_d ? row2[k] : rowc[k];
+      if (k < row.n) {
+        j = row[k];
         const double4_32a p = A.x4[j];
         const float fx = xf - f32_bits(p.x), fy = yf - f32_bits(p.y), fz = zf - f32_bits(p.z);
         keep = !(fmaf(fz, fz, fmaf(fy, fy, fx * fx)) > thr);
