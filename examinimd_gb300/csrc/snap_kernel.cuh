@@ -834,8 +834,8 @@ __global__ void __launch_bounds__(sy32_threads(NA), NA == 2 ? 1 : 2) k_snap_y32(
 // off, 1,000 operations more, half of the FP32 error (rms against the FP64 form, W
 // bcc 2,000 atoms at 0.05 A: 7.5e-6 -> 5.5e-6 eV/A, of which 3.3e-6 are Y's).
 // Bound by instruction issue and the latency of the phases; per 128,000 atoms
-// mixed 0.88 ms as loops, 0.61 unrolled with the extra operations; 8,160 atoms FP64
-// 0.64 and 0.58 (0.50 of FP64 issue).
+// mixed 0.88 ms as loops, 0.50 unrolled with the extra operations; 8,160 atoms FP64
+// 0.64 and 0.55 (0.50 of FP64 issue).
 constexpr int SF_THREADS = 256;
 constexpr int SF_ATOMS = 8;
 
@@ -882,6 +882,15 @@ struct TSum {
     }
   }
   __device__ __forceinline__ R value() const { return s + c; }
+};
+
+// T as a constant and as a variable (the compiler does not unroll so long a loop)
+template <int T>
+struct FixedT {
+  static constexpr int value = T;
+};
+struct AnyT {
+  int value;
 };
 
 // JC: twojmax (loops unrolled), or -1: any up to 14
@@ -991,8 +1000,8 @@ __global__ void __launch_bounds__(SF_THREADS, sizeof(R) == 4 ? 3 : 2) k_snap_for
       TSum<R> phi, gx, gar, gai, gbr, gbi;
       const R* Y = ys + a * ny;
       const R* ab = AB;
-#pragma unroll kUnroll
-      for (int T = 0; T <= J; ++T) {
+      auto one_T = [&](auto t) __attribute__((always_inline)) {
+        const int T = t.value;
         const int nT = (J - T + 2) * (J - T + 2) / 4;  // entries of T
         if (mask >> T & 1) {
           // sums over q: Re Eh, Im Oh; the same with P'; dEh/da, dOh/da
@@ -1081,6 +1090,14 @@ __global__ void __launch_bounds__(SF_THREADS, sizeof(R) == 4 ? 3 : 2) k_snap_for
           u = u2.h;
           v = v2.h;
         }
+      };
+      if constexpr (JC >= 0) {
+        [&]<int... T>(std::integer_sequence<int, T...>) {
+          (one_T(FixedT<T>{}), ...);
+        }(std::make_integer_sequence<int, JC + 1>{});
+      } else {
+#pragma unroll 1
+        for (int T = 0; T <= J; ++T) one_T(AnyT{T});
       }
       const R gx2 = gx.value() + gx.value();
       const R ga = fma(ar, gx2, gar.value()), gb = fma(ai, gx2, gai.value());
