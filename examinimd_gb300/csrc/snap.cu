@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -24,20 +25,12 @@ using namespace snapk;
 struct SnapTables;
 
 struct SnapHost {
-  SnapDev d;
+  SnapDev d{};
+  const int* tmask = nullptr;  // k_snap_force: groups of T
   const SnapTables* tab = nullptr;
   int precision = EMD_PREC_FP64;
-  // tables
-  DevBuf<Entry> ent;
-  DevBuf<ZTask> task;
-  DevBuf<ZRec> rec;
-  DevBuf<ZGrp> grp;
-  DevBuf<int> e0, map, zt0, tmask, eord;
-  DevBuf<int2> xsum, ucol, half, zt, prod;
-  DevBuf<float2> mono, pr32, wj32;
-  DevBuf<int4> hfull, ysrc;
-  DevBuf<double> zc, monod, cY, AB, beta0, wjelem, pr;
-  DevBuf<float> AB_f;
+  DevBuf<unsigned char> tables;  // every constant table, one allocation and copy
+  DevBuf<double> cY, beta0;
   DevBuf<uint4> zs;
   // per-chunk work arrays
   DevBuf<double> pd, pr_f, U, Y, zk;
@@ -396,22 +389,14 @@ __global__ void __launch_bounds__(256) k_adj_reduce(const double* __restrict__ a
 void free_snap(Ctx& c) {
   if (!c.snap) return;
   SnapHost* h = static_cast<SnapHost*>(c.snap);
-  h->ent.release();
-  h->task.release();
-  h->rec.release();
-  h->grp.release();
+  h->tables.release();
+  h->zs.release();
   h->D.release();
   h->H.release();
-  h->hfull.release();
-  h->ysrc.release();
-  h->zs.release();
-  for (auto* b : {&h->e0, &h->map, &h->zt0, &h->tmask, &h->eord, &h->pj, &h->cnt}) b->release();
-  for (auto* b : {&h->xsum, &h->ucol, &h->half, &h->zt, &h->prod}) b->release();
-  for (auto* b : {&h->zc, &h->monod, &h->cY, &h->AB, &h->beta0, &h->wjelem, &h->pr, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk,
-                  &h->eatom, &h->adj, &h->adj_sum, &h->adj_g, &h->keep_u, &h->keep_z})
+  for (auto* b : {&h->pj, &h->cnt}) b->release();
+  for (auto* b : {&h->cY, &h->beta0, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk, &h->eatom, &h->adj, &h->adj_sum, &h->adj_g,
+                  &h->keep_u, &h->keep_z})
     b->release();
-  h->AB_f.release();
-  for (auto* b : {&h->mono, &h->pr32, &h->wj32}) b->release();
   delete h;
   c.snap = nullptr;
 }
@@ -543,7 +528,7 @@ static SnapArgs snap_args(Ctx& c, SnapHost* h, int first, int n, bool fp64, bool
   h->Y.reserve((size_t(tiles) * 2 * S.ny * A.ta * real + 7) / 8, c.stream);
   A.Y = h->Y.p;
   A.f = c.f.p;
-  A.tmask = h->tmask.p;
+  A.tmask = h->tmask;
   return A;
 }
 
@@ -797,69 +782,54 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
       pr.push_back(MY_PI / (rcut - rmin0));
     }
   const std::vector<float> ABf(tab.AB.begin(), tab.AB.end());
-  upload(c, h->ent, tab.ent);
-  upload(c, h->task, tab.task);
-  upload(c, h->rec, tab.rec);
-  upload(c, h->e0, tab.e0);
-  upload(c, h->xsum, tab.xsum);
-  upload(c, h->ucol, tab.ucol);
-  upload(c, h->monod, tab.monod);
-  upload(c, h->mono, tab.mono);
-  upload(c, h->eord, tab.eord);
-  upload(c, h->half, tab.half);
-  upload(c, h->zt0, tab.zt0);
-  upload(c, h->zt, tab.zt);
-  upload(c, h->tmask, tab.tmask);
-  upload(c, h->hfull, tab.hfull);
-  upload(c, h->ysrc, tab.ysrc);
-  upload(c, h->prod, tab.prod);
-  upload(c, h->zc, tab.zc);
-  upload(c, h->grp, tab.grp);
-  upload(c, h->AB, tab.AB);
-  upload(c, h->AB_f, ABf);
-  upload(c, h->cY, cY);
-  upload(c, h->beta0, beta0);
-  upload(c, h->pr, pr);
   auto pair32 = [](double v) { return float2{float(v), float(v - double(float(v)))}; };
   std::vector<float2> pr32, wj32;
   for (double v : pr) pr32.push_back(pair32(v));
   for (int e = 0; e < nelem; ++e) wj32.push_back(pair32(wjelem[e]));
   S.nrmin32 = pair32(-rmin0);
-  upload(c, h->pr32, pr32);
-  upload(c, h->wj32, wj32);
-  upload(c, h->wjelem, std::vector<double>(wjelem, wjelem + nelem));
-  upload(c, h->map, std::vector<int>(map, map + ntypes));
+  std::vector<unsigned char> bytes;
+  std::vector<std::function<void(unsigned char*)>> place;
+  auto put = [&](auto& field, const auto& v) {
+    const size_t at = (bytes.size() + 255) & ~size_t(255), n = v.size() * sizeof(v[0]);
+    bytes.resize(at + n + 16);
+    if (n) std::memcpy(&bytes[at], v.data(), n);
+    place.push_back([&field, at](unsigned char* p) { field = reinterpret_cast<std::decay_t<decltype(field)>>(p + at); });
+  };
+  put(S.ent, tab.ent);
+  put(S.task, tab.task);
+  put(S.rec, tab.rec);
+  put(S.xsum, tab.xsum);
+  put(S.ucol, tab.ucol);
+  put(S.monod, tab.monod);
+  put(S.mono, tab.mono);
+  put(S.eord, tab.eord);
+  put(S.half, tab.half);
+  put(S.zt0, tab.zt0);
+  put(S.zt, tab.zt);
+  put(h->tmask, tab.tmask);
+  put(S.hfull, tab.hfull);
+  put(S.ysrc, tab.ysrc);
+  put(S.prod, tab.prod);
+  put(S.zc, tab.zc);
+  put(S.grp, tab.grp);
+  put(S.AB, tab.AB);
+  put(S.AB_f, ABf);
+  put(S.pr, pr);
+  put(S.pr32, pr32);
+  put(S.wj32, wj32);
+  put(S.wjelem, std::vector<double>(wjelem, wjelem + nelem));
+  put(S.map, std::vector<int>(map, map + ntypes));
+  upload(c, h->tables, bytes);
+  for (auto& f : place) f(h->tables.p);
+  upload(c, h->cY, cY);
+  upload(c, h->beta0, beta0);
   EMD_CUDA(cudaStreamSynchronize(c.stream));
-  S.ent = h->ent.p;
-  S.task = h->task.p;
-  S.rec = h->rec.p;
-  S.e0 = h->e0.p;
-  S.xsum = h->xsum.p;
-  S.ucol = h->ucol.p;
-  S.monod = h->monod.p;
-  S.mono = h->mono.p;
-  S.eord = h->eord.p;
-  S.half = h->half.p;
-  S.zt0 = h->zt0.p;
-  S.zt = h->zt.p;
-  S.hfull = h->hfull.p;
-  S.ysrc = h->ysrc.p;
-  S.prod = h->prod.p;
-  S.zc = h->zc.p;
-  S.grp = h->grp.p;
+  S.cY = h->cY.p;
+  S.beta0 = h->beta0.p;
   S.zs_n = int(tab.words.size() / 4);
   h->tab = &tab;
   if (precision == EMD_PREC_MIXED) upload_stream(c, h, tab, cY);
   S.zs = h->zs.p;
-  S.AB = h->AB.p;
-  S.AB_f = h->AB_f.p;
-  S.cY = h->cY.p;
-  S.beta0 = h->beta0.p;
-  S.pr = h->pr.p;
-  S.pr32 = h->pr32.p;
-  S.wj32 = h->wj32.p;
-  S.wjelem = h->wjelem.p;
-  S.map = h->map.p;
   EMD_API_END
 }
 

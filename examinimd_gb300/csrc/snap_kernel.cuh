@@ -90,7 +90,6 @@ struct SnapDev {
   double rfac0, rmin0, cutsq, wself;
   int switchflag;
   const Entry* ent;
-  const int* e0;       // (J + 1) x (J + 1): first entry of (T, q)
   const int2* xsum;    // nx: the two factors of a sum in a neighbour's row (k_snap_u, k_snap_dt)
   const int2* ucol;    // ne: the mixed form's two columns of an entry
   const float2* mono;  // N P_k in powers of x, high and low part
