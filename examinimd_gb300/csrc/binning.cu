@@ -8,6 +8,7 @@
 // per-bin rank pass that restores ascending order inside each bin.  With sort=true
 // a gather reorders x, v, f, type, id, q of the binned range.
 #include <algorithm>
+#include <cmath>
 
 #include "emd_device.cuh"
 #include "emd_internal.h"
@@ -31,14 +32,26 @@ struct BinGrid {
   int nbx, nby, nbz;
   double minx, miny, minz, mulx, muly, mulz;
   const double* ctab;
+  float min32[3], mul32[3], off32[3];  // off32: 2 |min| mul + 2
 };
+
+// int((x - min) mul) as the reference rounds it (binning_kksort.cpp:61-63), in FP64 only
+// where FP32 leaves it open: t is within 3e-7 (|t| + 2 |min| mul) of the FP64 value, so
+// away from integers by more than three times that both truncate alike.  Nine FP64
+// instructions a particle less (4.4 million: 0.127 -> 0.066 ms).
+__device__ __noinline__ int bin_fp64(double x, double min, double mul) { return int((x - min) * mul); }
+__device__ __forceinline__ int bin_of(const BinGrid& G, int d, double x, double min, double mul) {
+  const float t = (f32_bits(x) - G.min32[d]) * G.mul32[d];
+  const float b = floorf(t), r = t - b, e = 1e-6f * (t + G.off32[d]);
+  return t > e && t < 1e6f && r > e && r < 1.f - e ? int(b) : bin_fp64(x, min, mul);
+}
 
 // bin of a particle, and its FP32 position relative to the bin's centre, for the
 // neighbour candidate tests
 __device__ __forceinline__ int bin_particle(const BinGrid& G, const double4_32a& p, float4* xl, unsigned* status) {
-  int ix = int((p.x - G.minx) * G.mulx);
-  int iy = int((p.y - G.miny) * G.muly);
-  int iz = int((p.z - G.minz) * G.mulz);
+  int ix = bin_of(G, 0, p.x, G.minx, G.mulx);
+  int iy = bin_of(G, 1, p.y, G.miny, G.muly);
+  int iz = bin_of(G, 2, p.z, G.minz, G.mulz);
   if (ix < 0 || ix >= G.nbx || iy < 0 || iy >= G.nby || iz < 0 || iz >= G.nbz) {
     // outside the binned box: the reference would index out of bounds; keep
     // the particle in the nearest bin and report it
@@ -48,7 +61,7 @@ __device__ __forceinline__ int bin_particle(const BinGrid& G, const double4_32a&
     iz = min(max(iz, 0), G.nbz - 1);
   }
   *xl = make_float4(float(p.x - G.ctab[ix]), float(p.y - G.ctab[G.nbx + iy]),
-                    float(p.z - G.ctab[G.nbx + G.nby + iz]), __int_as_float(int(p.w)));
+                    float(p.z - G.ctab[G.nbx + G.nby + iz]), __int_as_float(int(f32_bits(p.w))));
   return (ix * G.nby + iy) * G.nbz + iz;
 }
 
@@ -248,7 +261,12 @@ emd_status emd_binning_create(emd_ctx* ctx, double dx_in, double dy_in, double d
     EMD_CHECK_LAUNCH();
     std::copy(key, key + 9, c.bin_ctab_key);
   }
-  const BinGrid G{nb[0], nb[1], nb[2], c.bmin[0], c.bmin[1], c.bmin[2], c.bmul[0], c.bmul[1], c.bmul[2], c.bin_ctab.p};
+  BinGrid G{nb[0], nb[1], nb[2], c.bmin[0], c.bmin[1], c.bmin[2], c.bmul[0], c.bmul[1], c.bmul[2], c.bin_ctab.p, {}, {}, {}};
+  for (int d = 0; d < 3; ++d) {
+    G.min32[d] = float(c.bmin[d]);
+    G.mul32[d] = float(c.bmul[d]);
+    G.off32[d] = float(2.0 * std::fabs(c.bmin[d]) * c.bmul[d] + 2.0);
+  }
   c.xl_bin_valid = true;
   c.bin_sorted = false;
   if (n > 0 && n <= BIN_SMALL && nbins <= BIN_SMALL_BINS) {
