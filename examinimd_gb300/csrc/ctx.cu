@@ -135,6 +135,22 @@ __global__ void __launch_bounds__(SUM_THREADS) k_sum_final(const double* __restr
   double t = block_sum(acc, sh);
   if (threadIdx.x == 0) *out = t;
 }
+// Both stages of a short sum (per-CTA partials) in one launch: the same tree, so the
+// same bits, as k_sum_partial and k_sum_final (912 values: 12 -> 8 us).
+constexpr int SUM_SHORT = 2048;
+__global__ void __launch_bounds__(SUM_THREADS) k_sum_short(const double* __restrict__ v, int n, double* out) {
+  __shared__ double sh[SUM_THREADS / 32];
+  __shared__ double part[SUM_SHORT / SUM_THREADS];
+  const int blocks = (n + SUM_THREADS - 1) / SUM_THREADS;
+  for (int b = 0; b < blocks; ++b) {
+    const int i = b * SUM_THREADS + int(threadIdx.x);
+    const double t = block_sum(i < n ? 0.0 + v[i] : 0.0, sh);
+    if (threadIdx.x == 0) part[b] = t;
+  }
+  __syncthreads();
+  const double t = block_sum(int(threadIdx.x) < blocks ? 0.0 + part[threadIdx.x] : 0.0, sh);
+  if (threadIdx.x == 0) *out = t;
+}
 }  // namespace
 
 static void scan_rec(Ctx& c, const int* in, int* out, int n, int level, int* total) {
@@ -167,12 +183,16 @@ void exclusive_scan_int(Ctx& c, const int* d_in, int* d_out, int n, int* d_total
 
 double device_sum(Ctx& c, const double* d_vals, int n) {
   c.red.reserve(SUM_BLOCKS + 2, c.stream);
-  {
-    TimedLaunch t(c, "sum_partial");
-    k_sum_partial<<<SUM_BLOCKS, SUM_THREADS, 0, c.stream>>>(d_vals, n, c.red.p);
+  if (n <= SUM_SHORT) {
+    TimedLaunch t(c, "sum_short");
+    k_sum_short<<<1, SUM_THREADS, 0, c.stream>>>(d_vals, n, c.red.p + SUM_BLOCKS);
     EMD_CHECK_LAUNCH();
-  }
-  {
+  } else {
+    {
+      TimedLaunch t(c, "sum_partial");
+      k_sum_partial<<<SUM_BLOCKS, SUM_THREADS, 0, c.stream>>>(d_vals, n, c.red.p);
+      EMD_CHECK_LAUNCH();
+    }
     TimedLaunch t(c, "sum_final");
     k_sum_final<<<1, SUM_THREADS, 0, c.stream>>>(c.red.p, SUM_BLOCKS, c.red.p + SUM_BLOCKS);
     EMD_CHECK_LAUNCH();
