@@ -19,6 +19,12 @@ __device__ __forceinline__ F2 f2_norm(float h, float l) {
   return F2{s, sub_rn(l, sub_rn(s, h))};
 }
 
+// a + b and what its rounding leaves off (Knuth's two-sum)
+__device__ __forceinline__ F2 f2_two_sum(float a, float b) {
+  const float t = add_rn(a, b), y = sub_rn(t, a);
+  return F2{t, add_rn(sub_rn(a, sub_rn(t, y)), sub_rn(b, y))};
+}
+
 // 1.5 times a power of two at least four times as large as b: sums below 2 b in
 // magnitude leave it within one binade
 __device__ __forceinline__ float f2_base(float b) {

@@ -883,6 +883,12 @@ struct TSum {
   __device__ __forceinline__ R value() const { return s + c; }
 };
 
+// one T's sums over q: Re Eh, Im Oh; the same with P'; dEh/da, dOh/da
+template <typename R>
+struct QSum {
+  R er = 0, oi = 0, xer = 0, xoi = 0, e1r = 0, e1i = 0, o1r = 0, o1i = 0;
+};
+
 // T as a constant and as a variable (the compiler does not unroll so long a loop)
 template <int T>
 struct FixedT {
@@ -1003,13 +1009,13 @@ __global__ void __launch_bounds__(SF_THREADS, sizeof(R) == 4 ? 3 : 2) k_snap_for
         const int T = t.value;
         const int nT = (J - T + 2) * (J - T + 2) / 4;  // entries of T
         if (mask >> T & 1) {
-          // sums over q: Re Eh, Im Oh; the same with P'; dEh/da, dOh/da
-          R er = 0, oi = 0, xer = 0, xoi = 0, e1r = 0, e1i = 0, o1r = 0, o1i = 0;
+          QSum<R> qs[kF64 ? 1 : 2];  // mixed form: of even and of odd q
           int e = 0;
 #pragma unroll
           for (int q = 0; q < NQ; ++q) {
             if (q > J - T) break;
             const int km = (J - T - q) / 2;
+            QSum<R>& Q = qs[kF64 ? 0 : q & 1];
             const R* y = Y + 4 * e;
             R g0 = y[0], g1 = y[1], g2 = y[2], g3 = y[3];  // sum_k E P_k, O P_k
             R h0 = 0, h1 = 0, h2 = 0, h3 = 0;              // sum_k E P'_k, O P'_k
@@ -1045,27 +1051,30 @@ __global__ void __launch_bounds__(SF_THREADS, sizeof(R) == 4 ? 3 : 2) k_snap_for
                 }
               }
             }
-            er = fma(pq[q], g0, er);
-            xer = fma(pq[q], h0, xer);
+            Q.er = fma(pq[q], g0, Q.er);
+            Q.xer = fma(pq[q], h0, Q.xer);
             if (q > 0) {
               const R qp = R(q) * pq[q - 1], qr1 = R(q) * rq[q - 1];
-              er = fma(-rq[q], g1, er);
-              xer = fma(-rq[q], h1, xer);
-              e1r = fma(qp, g0, fma(-qr1, g1, e1r));
-              e1i = fma(qp, g1, fma(qr1, g0, e1i));
+              Q.er = fma(-rq[q], g1, Q.er);
+              Q.xer = fma(-rq[q], h1, Q.xer);
+              Q.e1r = fma(qp, g0, fma(-qr1, g1, Q.e1r));
+              Q.e1i = fma(qp, g1, fma(qr1, g0, Q.e1i));
               if (T > 0) {
-                oi = fma(rq[q], g2, oi);
-                xoi = fma(rq[q], h2, xoi);
-                o1r = fma(qp, g2, fma(-qr1, g3, o1r));
-                o1i = fma(qp, g3, fma(qr1, g2, o1i));
+                Q.oi = fma(rq[q], g2, Q.oi);
+                Q.xoi = fma(rq[q], h2, Q.xoi);
+                Q.o1r = fma(qp, g2, fma(-qr1, g3, Q.o1r));
+                Q.o1i = fma(qp, g3, fma(qr1, g2, Q.o1i));
               }
             }
             if (T > 0) {
-              oi = fma(pq[q], g3, oi);
-              xoi = fma(pq[q], h3, xoi);
+              Q.oi = fma(pq[q], g3, Q.oi);
+              Q.xoi = fma(pq[q], h3, Q.xoi);
             }
             e += km + 1;
           }
+          auto both = [&](auto f) { return kF64 ? qs[0].*f : qs[0].*f + qs[kF64 ? 0 : 1].*f; };
+          const R er = both(&QSum<R>::er), oi = both(&QSum<R>::oi), xer = both(&QSum<R>::xer), xoi = both(&QSum<R>::xoi);
+          const R e1r = both(&QSum<R>::e1r), e1i = both(&QSum<R>::e1i), o1r = both(&QSum<R>::o1r), o1i = both(&QSum<R>::o1i);
           phi.add(fma(u, er, v * oi));
           gx.add(fma(u, xer, v * xoi));
           gar.add(fma(u, e1r, v * o1i));
@@ -1099,8 +1108,21 @@ __global__ void __launch_bounds__(SF_THREADS, sizeof(R) == 4 ? 3 : 2) k_snap_for
         for (int T = 0; T <= J; ++T) one_T(AnyT{T});
       }
       const R gx2 = gx.value() + gx.value();
-      const R ga = fma(ar, gx2, gar.value()), gb = fma(ai, gx2, gai.value());
-      const R gc = fma(-br, gx2, gbr.value()), gd = fma(-bi, gx2, gbi.value());
+      R ga = fma(ar, gx2, gar.value()), gb = fma(ai, gx2, gai.value());
+      R gc = fma(-br, gx2, gbr.value()), gd = fma(-bi, gx2, gbi.value());
+      if constexpr (!kF64) {
+        // |a|^2 + |b|^2 = 1, so the gradient's part along (a, b), which is the larger
+        // one (a degree j times Phi), drops out of the force below; rounded with it, it
+        // left a third of the error.  Taken off before the last roundings: ga = ar (gx2
+        // - rho) + gar, gc = -br (gx2 + rho) + gbr
+        const R rho = fma(ar, ga, fma(ai, gb, fma(br, gc, bi * gd)));
+        const F2 wa = f2_two_sum(gx.s + gx.s, -rho), wb = f2_two_sum(-gx.s - gx.s, -rho);
+        const R la = wa.l + (gx.c + gx.c), lb = wb.l - (gx.c + gx.c);
+        ga = fma(ar, wa.h, gar.s) + fma(ar, la, gar.c);
+        gb = fma(ai, wa.h, gai.s) + fma(ai, la, gai.c);
+        gc = fma(br, wb.h, gbr.s) + fma(br, lb, gbr.c);
+        gd = fma(bi, wb.h, gbi.s) + fma(bi, lb, gbi.c);
+      }
       const R cp = qr[PR_DSF * np] * phi.value();
       const R uk[3] = {qr[PR_UX * np], qr[PR_UY * np], qr[PR_UZ * np]};
       if constexpr (kF64) {

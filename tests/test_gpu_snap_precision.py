@@ -1,0 +1,37 @@
+"""Precision of the SNAP forms (GPU).
+
+Mixed forces against the FP64 form's on jittered lattices of 128 (26 neighbours) and
+54 (about 73) atoms.  The bounds, RMS error over RMS force of six systems each, are
+the errors of a form whose U recursion and pair scalars are FP64 throughout and
+whose Z, Y and pair forces are FP32: the mixed form's FP32 pairs are to be no worse.
+"""
+import numpy as np
+import pytest
+
+from tests import mdloop
+from tests.test_gpu_snap_tables import _deck
+
+pytestmark = pytest.mark.gpu
+
+
+def _forces(st, state, precision):
+    from examinimd_gb300 import Context
+    c = Context(0)
+    mdloop.init(c, st, state, precision=precision)
+    f = mdloop.by_id(c.get(0, len(state["x"])))["f"]
+    c.close()
+    return f
+
+
+@pytest.mark.parametrize("J,cells,a,bound", [
+    (4, (4, 4, 4), 3.1803, 3.35e-7), (6, (4, 4, 4), 3.1803, 3.76e-7), (7, (4, 4, 4), 3.1803, 3.97e-7),
+    (8, (4, 4, 4), 3.1803, 3.09e-7), (9, (4, 4, 4), 3.1803, 2.99e-7), (4, (3, 3, 3), 2.3, 1.70e-8),
+    (6, (3, 3, 3), 2.3, 5.13e-8), (8, (3, 3, 3), 2.3, 8.20e-8), (9, (3, 3, 3), 2.3, 7.31e-8)])
+def test_mixed_forces_are_as_good_as_with_fp64_recursions(J, cells, a, bound):
+    from examinimd_gb300 import EMD_PREC_MIXED
+    err = []
+    for seed in range(6):
+        deck = _deck(J, cells, a, seed=100 * J + seed)
+        ref, got = _forces(*deck, 0), _forces(*deck, EMD_PREC_MIXED)
+        err.append(np.mean((got - ref) ** 2) / np.mean(ref ** 2))
+    assert np.sqrt(np.mean(err)) <= bound
