@@ -42,30 +42,6 @@ struct LJParams {
   double cutsq_max;
 };
 
-__device__ __forceinline__ double f64_of_normal(float f) {  // exact for a normal f > 0
-  const unsigned b = __float_as_uint(f);
-  return __hiloint2double(int((b >> 3) + 0x38000000u), int(b << 29));
-}
-
-// IEEE 1 / d.  For d within [2^-96, 2^96] whose significand is not all ones: an
-// FP32 reciprocal (2^-21 off), one cubic step in FP64 and Markstein's final
-// correction y + y (1 - d y), which returns the correctly rounded reciprocal
-// for every other significand (P. Markstein, IBM J. Res. Dev. 34 (1990) 111):
-// five FP64 instructions.  Everything else takes the divide, out of line.
-__device__ __noinline__ double recip_div(double d) { return 1.0 / d; }
-__device__ __forceinline__ double recip_rn(double d) {
-  const unsigned hi = __double2hiint(d);
-  const bool plain = hi - 0x39f00000u < 0x0c000000u &&
-                     !((hi & 0xfffffu) == 0xfffffu && unsigned(__double2loint(d)) == 0xffffffffu);
-  if (!plain) return recip_div(d);
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f32_bits(d)));
-  const double r0 = f64_of_normal(r);
-  const double e = __fma_rn(-d, r0, 1.0);
-  const double y = __fma_rn(r0, __fma_rn(e, e, e), r0);
-  return __fma_rn(y, __fma_rn(-d, y, 1.0), y);
-}
-
 // pair force over r: the plain LJ term, or (IDIAL) ForceLJIDialNeigh's
 // repeated evaluation, each repeat adding 1/intensity of the term
 // (force_lj_idial_neigh_impl.h:137-149)

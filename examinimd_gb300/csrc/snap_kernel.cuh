@@ -295,11 +295,11 @@ __global__ void __launch_bounds__(64) k_snap_pairs(SnapArgs A) {
         put(PR_C1, -1, neg(f2_mul(sn, scale)));
         put(PR_GR, -1, f2_add(f2_mul(cs, scale), neg(r0)));
         put(PR_R0, -1, r0);
-        // the r^-12 repulsion's force stays FP64: its pair terms are of the size
-        // of the net force and cancel in the sum over neighbours
-        const double rinv = in ? double(rv.h) + double(rv.l) : 0.0;
-        const double ri2 = rinv * rinv, ri4 = ri2 * ri2;
-        const double fr = -1.5e6 * (ri4 * ri4 * ri4 * ri2);
+        // the r^-12 repulsion's force is FP64 from the FP64 r^2: its pair terms are of
+        // the size of the net force and cancel in the sum over neighbours (from the 48
+        // bits of 1 / r, r^-14 was off by 1e-13 of them)
+        const double r2 = rsq * rsq, r4 = r2 * r2;
+        const double fr = in ? -1.5e6 * recip_rn(r4 * r2 * rsq) : 0.0;
         q[PD_FX * np] = x * fr;
         q[PD_FY * np] = y * fr;
         q[PD_FZ * np] = z * fr;

@@ -35,3 +35,23 @@ def test_mixed_forces_are_as_good_as_with_fp64_recursions(J, cells, a, bound):
         ref, got = _forces(*deck, 0), _forces(*deck, EMD_PREC_MIXED)
         err.append(np.mean((got - ref) ** 2) / np.mean(ref ** 2))
     assert np.sqrt(np.mean(err)) <= bound
+
+
+@pytest.mark.parametrize("cells,a", [((4, 4, 4), 3.1803), ((3, 3, 3), 2.3)])
+def test_mixed_repulsion_is_fp64(cells, a):
+    """With zero coefficients only the r^-14 repulsion is left.  A pair's force takes
+    ten FP64 roundings in either form and an atom adds up to 2 n of them, n neighbours'
+    own and reactions, in another order."""
+    from examinimd_gb300 import EMD_PREC_MIXED
+    st, state = _deck(4, cells, a, seed=3)
+    st.elements[0]["beta"] = list(np.zeros(len(st.elements[0]["beta"])))
+    ref, got = _forces(st, state, 0), _forces(st, state, EMD_PREC_MIXED)
+    L, x = np.asarray(st.domain), state["x"]
+    shifts = np.stack(np.meshgrid(*[(-1, 0, 1)] * 3, indexing="ij"), -1).reshape(-1, 3) * L
+    d = x[None, :, None, :] - x[:, None, None, :] + shifts
+    r = np.linalg.norm(d, axis=-1).reshape(len(x), -1)
+    near = (r > 0) & (r < st.cut)
+    pair = np.where(near, 1.5e6 * np.where(near, r, 1.0) ** -13, 0.0).sum(axis=1)  # sum of |f_ij| of each atom
+    n = near.sum(axis=1)
+    tol = 2.0 ** -53 * (20 + 2 * n) * 2 * pair
+    assert np.all(np.abs(got - ref).max(axis=1) <= tol)
