@@ -103,7 +103,7 @@ constexpr int ZS_SPLIT = 16;        // CTAs that may share a tile
 struct SnapTables {
   std::vector<Entry> ent;
   std::vector<int> e0, zt0, tmask, eord;
-  std::vector<int2> xsum, ucol, half, zt, prod;
+  std::vector<int2> xsum, psum, ucol, half, zt, prod;
   std::vector<float2> mono;
   std::vector<int4> hfull, ysrc;
   std::vector<ZTask> task;
@@ -124,9 +124,10 @@ struct SnapTables {
     const int L = J + 1, ntrip = int(trip.size() / 3);
     auto uidx = [](int j, int ma, int mb) { return j * (j + 1) * (2 * j + 1) / 6 + ma * (j + 1) + mb; };
     // entries, real sums and their columns (powers of a, then those of b times
-    // those of x in (T, k) order)
+    // those of x in (T, k) order; psum: powers of a, of b, then those of b times
+    // P_k, k > 0, in (T, q, k) order)
     e0.assign(size_t(L) * L, -1);
-    int col = L;
+    int col = L, pcol = 4 * L;
     for (int T = 0; T <= J; ++T) {
       for (int q = 0; q <= J - T; ++q) {
         e0[size_t(T) * L + q] = int(ent.size());
@@ -150,10 +151,12 @@ struct SnapTables {
           E.mm = uidx(j, j - mb, j - ma);
           E.xo = int(xsum.size());
           const int cp = 2 * q, cr = 2 * q + 1, cu = 2 * (col + k), cv = cu + 1;
-          xsum.push_back(int2{cp, cu});
-          if (q > 0) xsum.push_back(int2{cr, cu});
-          if (T > 0) xsum.push_back(int2{cp, cv});
-          if (q > 0 && T > 0) xsum.push_back(int2{cr, cv});
+          const int pu = k == 0 ? 2 * L + 2 * T : pcol, pv = pu + 1;
+          if (k > 0) pcol += T > 0 ? 2 : 1;
+          xsum.push_back(int2{cp, cu}), psum.push_back(int2{cp, pu});
+          if (q > 0) xsum.push_back(int2{cr, cu}), psum.push_back(int2{cr, pu});
+          if (T > 0) xsum.push_back(int2{cp, cv}), psum.push_back(int2{cp, pv});
+          if (q > 0 && T > 0) xsum.push_back(int2{cr, cv}), psum.push_back(int2{cr, pv});
           ucol.push_back(int2{q, col + k});
           E.mo = int(mono.size());
           for (double c : pk) monod.push_back(E.N * c), mono.push_back(float2{float(E.N * c), float(E.N * c - double(float(E.N * c)))});
@@ -798,7 +801,9 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   put(S.ent, tab.ent);
   put(S.task, tab.task);
   put(S.rec, tab.rec);
+  put(S.e0, tab.e0);
   put(S.xsum, tab.xsum);
+  put(S.psum, tab.psum);
   put(S.ucol, tab.ucol);
   put(S.monod, tab.monod);
   put(S.mono, tab.mono);

@@ -90,7 +90,9 @@ struct SnapDev {
   double rfac0, rmin0, cutsq, wself;
   int switchflag;
   const Entry* ent;
+  const int* e0;       // (J + 1) x (J + 1): first entry of (T, q)
   const int2* xsum;    // nx: the two factors of a sum in a neighbour's row (k_snap_u, k_snap_dt)
+  const int2* psum;    // the same where the row holds P_k (k_snap_u above SU_POWERS)
   const int2* ucol;    // ne: the mixed form's two columns of an entry
   const float2* mono;  // N P_k in powers of x, high and low part
   const double* monod; // the same in FP64
@@ -358,6 +360,12 @@ __global__ void __launch_bounds__(64) k_snap_pairs(SnapArgs A) {
 // neighbours' rows (240 with P_k), nx / 32 for each neighbour; the table, half as
 // wide, lets eleven warps share an SM instead of six (8,160 atoms: 0.33 -> 0.21 ms).
 //
+// Above twojmax 9 (SU_POWERS) the row holds u P_k and v P_k, so that nothing is
+// amplified: forces of 54 and 128 atoms, RMS error against long double relative to the
+// layer recursion's, 1.13 / 1.03 with powers and 1.06 / 1.02 with P_k at twojmax 10, 1.08
+// and 1.01 at 11 (1.07 and 1.06, 1.08 and 1.05 at 8 and 9, where powers are kept); the
+// bispectrum's own error 2.6e-15 and 1.0e-15 at 12.
+//
 // The mixed form, which rounds U_tot to FP32 anyway, takes k_snap_u32
 // (snap_split.cuh): per 128,000 atoms 2.80 ms in FP64, 0.87 in FP32 pairs.
 // pairs of columns of a neighbour's row: (p, r) of a^q; (u x^k, v x^k) of w b^T
@@ -369,6 +377,55 @@ inline int su_cols(int J) {
 
 // doubles of an FP64 row (odd: rows start in different banks)
 __host__ __device__ inline int su_stride(int cols) { return (2 * cols) | 1; }
+
+constexpr int SU_POWERS = 9;
+
+// columns of a row with P_k: p, r; u, v; u P_k, v P_k (k > 0)
+__host__ __device__ inline int su_pcols(int J) {
+  int c = 4 * (J + 1);
+  for (int T = 0; T <= J; ++T)
+    for (int q = 0; q <= J - T; ++q) c += (T ? 2 : 1) * ((J - T - q) / 2);
+  return c | 1;
+}
+
+// that row
+__device__ __forceinline__ void su_row_p(const SnapDev& S, double* t, double ar, double ai, double br, double bi,
+                                         double w) {
+  const int J = S.twojmax;
+  double *uT = t + 2 * (J + 1), *prod = t + 4 * (J + 1);
+  double p = 1.0, r = 0.0, u = w, v = 0.0;
+#pragma unroll 1
+  for (int q = 0; q <= J; ++q) {
+    t[2 * q] = p;
+    t[2 * q + 1] = r;
+    uT[2 * q] = u;
+    uT[2 * q + 1] = v;
+    const double pn = fma(p, ar, -r * ai), un = fma(u, br, -v * bi);
+    r = fma(p, ai, r * ar);
+    v = fma(u, bi, v * br);
+    p = pn;
+    u = un;
+  }
+  const double x = fma(ar, ar, ai * ai) - fma(br, br, bi * bi);
+  for (int T = 0; T <= J; ++T) {
+    const double uu = uT[2 * T], vv = uT[2 * T + 1];
+    for (int q = 0; q <= J - T - 2; ++q) {
+      const double2* ab = reinterpret_cast<const double2*>(S.AB) + __ldg(S.e0 + T * (J + 1) + q);
+      const int km = (J - T - q) / 2;
+      double pm = 1.0, pk = x - __ldg(ab).x;
+      *prod++ = uu * pk;
+      if (T > 0) *prod++ = vv * pk;
+      for (int k = 2; k <= km; ++k) {
+        const double2 c = __ldg(ab + k - 1);
+        const double pn = fma(x - c.x, pk, -c.y * pm);
+        pm = pk;
+        pk = pn;
+        *prod++ = uu * pk;
+        if (T > 0) *prod++ = vv * pk;
+      }
+    }
+  }
+}
 
 // the neighbour's table row: powers of a, those of b times those of x
 __device__ __forceinline__ void su_row(int J, double* t, double ar, double ai, double br, double bi, double w) {
@@ -398,15 +455,16 @@ __device__ __forceinline__ void su_row(int J, double* t, double ar, double ai, d
 // the half-grid elements of entry e from its sums over the powers of x (one group
 // per k): conj(a)^q b^T = (p u + r v) + i (p v - r u); for -T: (-1)^T ((p u - r v)
 // - i (p v + r u)); the coefficients hold N, the atom's own term is 1 on the
-// diagonal (T = 0)
+// diagonal (T = 0).  POLY: from the sums over P_k
+template <bool POLY>
 __device__ __forceinline__ void su_store(const SnapDev& S, int e, const double* xs, double self, Cplx<double>* U) {
   const Entry& E = S.ent[e];
   const bool hr = E.q > 0, hv = E.T > 0;
-  const int k = (E.j - E.q - E.T) / 2, g = (hr ? 2 : 1) * (hv ? 2 : 1);
+  const int k = POLY ? 0 : (E.j - E.q - E.T) / 2, g = (hr ? 2 : 1) * (hv ? 2 : 1);
   const double *m = S.monod + E.mo, *x = xs + E.xo - k * g;
   double pu = 0.0, ru = 0.0, pv = 0.0, rv = 0.0;
   for (int l = 0; l <= k; ++l, x += g) {
-    const double c = __ldg(m + l);
+    const double c = POLY ? E.N : __ldg(m + l);
     pu = fma(c, x[0], pu);
     if (hr) ru = fma(c, x[1], ru);
     if (hv) pv = fma(c, x[hr ? 2 : 1], pv);
@@ -420,21 +478,24 @@ __device__ __forceinline__ void su_store(const SnapDev& S, int e, const double* 
   }
 }
 
-static __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
+template <bool POLY>
+__global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
   const SnapDev& S = A.S;
   extern __shared__ __align__(16) double su_smem[];
   double* xs = su_smem;                       // nx sums
   double* tab = su_smem + ((S.nx + 1) & ~1);  // 32 rows
   const int al = blockIdx.x, lane = threadIdx.x;
-  const int cols = su_stride(S.cols), n = A.cnt[al];
-  const int2* __restrict__ xsum = S.xsum;
+  const int cols = POLY ? su_pcols(S.twojmax) : su_stride(S.cols), n = A.cnt[al];
+  const int2* __restrict__ xsum = POLY ? S.psum : S.xsum;
   const size_t np = size_t(A.n) * A.cap;
   const double* pd = A.pd + size_t(al) * A.cap;
   for (int n0 = 0; n0 < max(n, 1); n0 += 32) {
     const int m = min(32, n - n0);
     if (lane < m) {
       const double* q = pd + n0 + lane;
-      su_row(S.twojmax, tab + lane * cols, q[PD_AR * np], q[PD_AI * np], q[PD_BR * np], q[PD_BI * np], q[PD_SF * np]);
+      const double ar = q[PD_AR * np], ai = q[PD_AI * np], br = q[PD_BR * np], bi = q[PD_BI * np], w = q[PD_SF * np];
+      if (POLY) su_row_p(S, tab + lane * cols, ar, ai, br, bi, w);
+      else su_row(S.twojmax, tab + lane * cols, ar, ai, br, bi, w);
     }
     __syncwarp();
     for (int r0 = 0; r0 < S.nx; r0 += 96) {  // three sums per lane at once
@@ -472,7 +533,7 @@ static __global__ void __launch_bounds__(32) k_snap_u(SnapArgs A) {
     __syncwarp();
   }
   Cplx<double>* U = static_cast<Cplx<double>*>(A.U) + size_t(al) * S.nh;
-  for (int e = lane; e < S.ne; e += 32) su_store(S, __ldg(S.eord + e), xs, S.wself, U);
+  for (int e = lane; e < S.ne; e += 32) su_store<POLY>(S, __ldg(S.eord + e), xs, S.wself, U);
 }
 
 // ------------------------------------------------------------------- Z, Y
@@ -1300,7 +1361,7 @@ static __global__ void __launch_bounds__(32) k_snap_dt(SnapArgs A) {
     }
     __syncwarp();
   }
-  for (int e = lane; e < S.ne; e += 32) su_store(S, __ldg(S.eord + e), xs, 0.0, A.D + size_t(al) * S.nh);
+  for (int e = lane; e < S.ne; e += 32) su_store<false>(S, __ldg(S.eord + e), xs, 0.0, A.D + size_t(al) * S.nh);
 }
 
 // half-grid elements of U and D, weighted (2, or 1 for the self-inverse ones,
@@ -1378,11 +1439,17 @@ void launch_y32(const SnapArgs& A, cudaStream_t s) {
   }
 }
 
-inline void launch_u(const SnapArgs& A, cudaStream_t s) {
-  const size_t smem = sizeof(double) * (size_t((A.S.nx + 1) & ~1) + 32 * size_t(su_stride(A.S.cols)));
-  allow_dyn_smem(k_snap_u);
-  k_snap_u<<<A.n, 32, smem, s>>>(A);
+template <bool POLY>
+void launch_u(const SnapArgs& A, cudaStream_t s) {
+  const size_t cols = size_t(POLY ? su_pcols(A.S.twojmax) : su_stride(A.S.cols));
+  const size_t smem = sizeof(double) * (size_t((A.S.nx + 1) & ~1) + 32 * cols);
+  allow_dyn_smem(k_snap_u<POLY>);
+  k_snap_u<POLY><<<A.n, 32, smem, s>>>(A);
   EMD_CHECK_LAUNCH();
+}
+inline void launch_u(const SnapArgs& A, cudaStream_t s) {
+  if (A.S.twojmax > SU_POWERS) launch_u<true>(A, s);
+  else launch_u<false>(A, s);
 }
 
 template <typename R, int JC>

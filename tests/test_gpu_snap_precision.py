@@ -55,3 +55,21 @@ def test_mixed_repulsion_is_fp64(cells, a):
     n = near.sum(axis=1)
     tol = 2.0 ** -53 * (20 + 2 * n) * 2 * pair
     assert np.all(np.abs(got - ref).max(axis=1) <= tol)
+
+
+@pytest.mark.parametrize("J", [10, 12, 14])
+def test_bispectrum_of_large_twojmax(J):
+    """The bispectrum summed over the atoms (the adjoint's energy part) against the
+    oracle's layer recursion, whose own RMS relative error against long double is up to
+    1.1e-15 on these systems; twice that is allowed between the two."""
+    from examinimd_gb300 import Context
+    from oracle.orc import Oracle
+    st, state = _deck(J, (3, 3, 3), 2.3, seed=J)
+    n = len(state["x"])
+    gpu, orc = Context(0), Oracle(4)
+    mdloop.init(gpu, st, state)
+    mdloop.init(orc, st, state)
+    got = gpu.snap_adjoint(np.zeros((n, 3)), 1.0, 1, len(st.elements[0]["beta"])).ravel()[1:]
+    ref = orc.snap_bispectrum().sum(axis=0)
+    gpu.close()
+    assert np.sqrt(np.mean((got / ref - 1.0) ** 2)) <= 2.2e-15
