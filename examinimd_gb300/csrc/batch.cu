@@ -195,12 +195,13 @@ __device__ void build_row(const BArgs& A, const BSys& S, int i) {
 }
 
 // floor(x / w), the division only where FP32 leaves it open: one CTA bins a whole
-// system, and three FP64 divisions a particle took most of the rebuild
-__device__ __noinline__ int bin_fp64(double x, double w) { return int(floor(x / w)); }
-__device__ __forceinline__ int bin_of(double x, double w, float winv) {
+// system, and three FP64 divisions a particle took most of the rebuild.  Within [lo, hi]
+// whatever x is: conversions saturate, and f32_bits makes an infinity of a NaN
+__device__ __noinline__ int bin_fp64(double x, double w) { return __double2int_rd(x / w); }
+__device__ __forceinline__ int bin_of(double x, double w, float winv, int lo, int hi) {
   const float t = f32_bits(x) * winv;  // within 2.5e-7 |t|
   const float b = floorf(t), r = t - b, e = 4e-7f * (fabsf(t) + 1.f);
-  return r < e || r > 1.f - e ? bin_fp64(x, w) : int(b);
+  return min(max(r < e || r > 1.f - e ? bin_fp64(x, w) : __float2int_rz(b), lo), hi);
 }
 
 // a double's order as an integer's (the integer pipe compares 8 times as fast here)
@@ -270,7 +271,10 @@ __device__ void rebuild(const BArgs& A, const BSys& S, int* sh, int* hist) {
   bool over = false;
   for (int d = 0; d < 3; ++d) {
     const int cur = min(n + ng, S.cap);
-    const long long klo = order_key(A.cut_nb), khi = order_key(S.L[d] - A.cut_nb);
+    // in the lower face's range [-inf, cut_nb), the upper one's [L - cut_nb, inf]: a NaN is in neither
+    constexpr long long kinf = 0x7ff0000000000000LL, kninf = -0x7ff0000000000001LL;
+    const long long khi = order_key(S.L[d] - A.cut_nb);
+    const unsigned long long nlo = order_key(A.cut_nb) - kninf, nhi = kinf - khi;
     // four candidates a thread and scan: a scan's barriers cost more than its sweep
     for (int c0 = 0; c0 < cur; c0 += 4 * T) {
       const int c1 = c0 + 4 * tid;
@@ -279,7 +283,8 @@ __device__ void rebuild(const BArgs& A, const BSys& S, int* sh, int* hist) {
       for (int k = 0; k < 4; ++k)
         if (c1 + k < cur) {
           const long long key = order_key((&x[c1 + k].x)[d]);
-          faces |= (key < klo ? 1 << (2 * k) : 0) | (key >= khi ? 2 << (2 * k) : 0);
+          faces |= ((unsigned long long)key - kninf < nlo ? 1 << (2 * k) : 0) |
+                   ((unsigned long long)key - khi <= nhi ? 2 << (2 * k) : 0);
         }
       int tot;
       int g = n + ng + block_excl(__popc(faces), sh, tot);
@@ -315,9 +320,9 @@ __device__ void rebuild(const BArgs& A, const BSys& S, int* sh, int* hist) {
     const double4_32a q = x[p];
     // owned atoms stay in the interior bins, also one that rounds onto the upper face
     const int o = p < n ? 1 : 0;
-    const int bx = min(max(bin_of(q.x, S.w[0], wi[0]) + 1, o), S.nb[0] + 1 - o);
-    const int by = min(max(bin_of(q.y, S.w[1], wi[1]) + 1, o), S.nb[1] + 1 - o);
-    const int bz = min(max(bin_of(q.z, S.w[2], wi[2]) + 1, o), S.nb[2] + 1 - o);
+    const int bx = bin_of(q.x, S.w[0], wi[0], o - 1, S.nb[0] - o) + 1;
+    const int by = bin_of(q.y, S.w[1], wi[1], o - 1, S.nb[1] - o) + 1;
+    const int bz = bin_of(q.z, S.w[2], wi[2], o - 1, S.nb[2] - o) + 1;
     const int b = (bx * (S.nb[1] + 2) + by) * (S.nb[2] + 2) + bz;
     binof[p] = b;
     const ushort4 c = make_ushort4(bx, by, bz, img[p]);

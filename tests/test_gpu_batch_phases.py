@@ -45,3 +45,35 @@ def test_phased_equals_persistent(systems, runs):
     assert np.all(np.isfinite(out[0][0]))
     for p, q in zip(*out):
         np.testing.assert_array_equal(p, q)
+
+
+@pytest.mark.parametrize("spl", [7, 0])
+@pytest.mark.parametrize("what", ["one_nan", "all_nan", "far", "inf"])
+def test_a_blown_up_system_leaves_the_others_alone(spl, what):
+    """NaN, infinite and far positions stay in their bins and images' bounds: the run
+    goes on, and the other systems' bits are those of a run beside a sound system."""
+    from examinimd_gb300 import Batch
+    rng = np.random.default_rng(12)
+    parts = [_system(c, rng) for c in ((5, 4, 4), (5, 5, 4), (4, 4, 4))]
+    ns, boxes = [len(p[0]) for p in parts], np.array([p[2] for p in parts])
+    x = np.concatenate([p[0] for p in parts])
+    o = np.concatenate([[0], np.cumsum(ns)])
+    out = []
+    for bad in (False, True):
+        v = np.concatenate([p[1] for p in parts])
+        if bad and what == "one_nan":
+            v[o[1] + 7] = np.nan
+        elif bad and what == "all_nan":
+            v[o[1]:o[2]] = -np.nan if spl else np.nan
+        elif bad:
+            v[o[1] + 7] = [1e300, -1e300, 1e25] if what == "inf" else [1e6, -1e6, 1e12]
+        b = Batch(ns, boxes, x, v, dt=0.0005)
+        b.set_shape(256, spl)
+        b.run(45)
+        out.append(b.get())
+        b.close()
+    for p, q in zip(*out):
+        np.testing.assert_array_equal(p[:o[1]], q[:o[1]])
+        np.testing.assert_array_equal(p[o[2]:], q[o[2]:])
+    if what == "all_nan":
+        assert np.all(np.isnan(out[1][0][o[1]:o[2]]))
