@@ -812,7 +812,7 @@ emd_status emd_batch_create(emd_batch** out, int device, int nsys, const int* na
   require(slot < (1LL << 25), EMD_ERR_ARG, "emd_batch_create: packed rows need fewer than 2^25 slots per system");
   b->smem = sizeof(int) * size_t(max_bins);
   require(b->smem <= 200 * 1024, EMD_ERR_ARG, "emd_batch_create: a system's bin grid exceeds shared memory");
-  EMD_CUDA(cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, int(b->smem)));
+  allow_dyn_smem(k_batch);
   const size_t ns = size_t(slot);
   b->slots = ns;
   b->x.reserve(ns, b->stream);

@@ -77,3 +77,26 @@ def test_a_blown_up_system_leaves_the_others_alone(spl, what):
         np.testing.assert_array_equal(p[o[2]:], q[o[2]:])
     if what == "all_nan":
         assert np.all(np.isnan(out[1][0][o[1]:o[2]]))
+
+
+def test_a_small_batch_leaves_a_large_one_its_shared_memory():
+    """24^3 bins take 55 KB of shared memory, more than a kernel gets unasked; a batch
+    with few bins, created in between, does not lower the limit."""
+    from examinimd_gb300 import Batch
+    rng = np.random.default_rng(13)
+    box, n = 62.0, 8000
+    g = np.stack(np.meshgrid(*[np.arange(20)] * 3, indexing="ij"), -1).reshape(-1, 3) * (box / 20)
+    x, v = np.mod(g + 0.1 * rng.standard_normal((n, 3)), box), rng.standard_normal((n, 3))
+    out = []
+    for between in (False, True):
+        b = Batch([n], np.full((1, 3), box), x, v)
+        b.set_shape(512, 0)
+        if between:
+            xs, vs, bs = _system((4, 4, 4), rng)
+            small = Batch([len(xs)], bs[None], xs, vs)
+        b.run(25)
+        out.append(b.get())
+        b.close()
+    small.close()
+    for p, q in zip(*out):
+        np.testing.assert_array_equal(p, q)

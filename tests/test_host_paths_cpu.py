@@ -1,0 +1,53 @@
+"""Host paths of the library on a CUDA runtime without a GPU (fake_cudart.cpp): what
+the calls do with devices, limits and failing allocations.  No kernel runs."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from tests.conftest import ROOT
+
+PRELUDE = """
+import ctypes, numpy as np
+from examinimd_gb300 import Batch, Context, EmdError, EMD_PREC_MIXED
+from tests import mdloop
+fake = ctypes.CDLL({so!r})
+fake.fake_set_budget.argtypes = [ctypes.c_size_t]
+fake.fake_held.restype = ctypes.c_size_t
+def current():
+    d = ctypes.c_int()
+    fake.cudaGetDevice(ctypes.byref(d))
+    return d.value
+def batch(n=(40, 30), box=9.0, device=0, **kw):
+    x = np.random.default_rng(1).uniform(0.0, box, (sum(n), 3))
+    return Batch(list(n), np.full((len(n), 3), box), x, 0.0 * x, device=device, **kw)
+"""
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    """run(code): the code in a process of its own, on the fake runtime."""
+    from examinimd_gb300 import build
+    cuda = build._cuda_home(build._nvcc())
+    build.build()
+    so = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(cuda, "include"), "-o", so,
+                    os.path.join(ROOT, "tests", "fake_cudart.cpp")], check=True)
+
+    def go(code):
+        r = subprocess.run([sys.executable, "-c", PRELUDE.format(so=so) + code], cwd=ROOT, capture_output=True, text=True,
+                           env=dict(os.environ, LD_PRELOAD=so), timeout=120)
+        assert r.returncode == 0, r.stderr[-2000:]
+    return go
+
+
+def test_a_batch_keeps_its_shared_memory_limit(run):
+    """24^3 bins take 55 KB; the limit belongs to the kernel, not to the batch."""
+    run("""
+big = batch(box=62.0)
+small = batch(box=9.0)
+big.set_shape(512, 0)
+for b in (big, small, big):
+    b.run(40)
+""")
