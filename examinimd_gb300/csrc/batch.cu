@@ -950,6 +950,7 @@ const char* emd_batch_last_error(const emd_batch* b) { return b ? b->last_error.
 
 emd_status emd_batch_run(emd_batch* b, int nsteps) {
   BATCH_BEGIN
+  const DeviceGuard device(b->device);
   require(nsteps >= 0, EMD_ERR_ARG, "emd_batch_run: nsteps");
   if (nsteps == 0) return EMD_OK;
   batch_run(b, nsteps, b->threads, b->steps_per_launch, b->phased);
@@ -970,6 +971,7 @@ emd_status emd_batch_set_shape(emd_batch* b, int threads, int steps_per_launch) 
 
 emd_status emd_batch_tune(emd_batch* b, int trial_steps, int* threads_out, int* spl_out) {
   BATCH_BEGIN
+  const DeviceGuard device(b->device);
   require(trial_steps >= 1, EMD_ERR_ARG, "emd_batch_tune: trial_steps");
   // every candidate runs the same trial from the same state, which is then restored
   const size_t ns = b->slots;
@@ -1039,6 +1041,7 @@ emd_status emd_batch_tune(emd_batch* b, int trial_steps, int* threads_out, int* 
 // host (1.36 million atoms: 23.7 ms with the slots copied, 4.4 packed).
 emd_status emd_batch_get(emd_batch* b, double* x, double* v, double* f) {
   BATCH_BEGIN
+  const DeviceGuard device(b->device);
   const size_t n3 = 3 * size_t(b->atoms);
   b->pack.reserve(n3, b->stream);
   auto get = [&](double* out, const double* src, int stride) {
@@ -1056,6 +1059,7 @@ emd_status emd_batch_get(emd_batch* b, double* x, double* v, double* f) {
 
 emd_status emd_batch_thermo(emd_batch* b, double* mv2, double* pe) {
   BATCH_BEGIN
+  const DeviceGuard device(b->device);
   k_batch_thermo<<<b->nsys, 256, 0, b->stream>>>(b->a, b->mass, b->lj1, b->lj2, b->cutsq, b->thermo.p);
   EMD_CHECK_LAUNCH();
   std::vector<double> h(2 * size_t(b->nsys));

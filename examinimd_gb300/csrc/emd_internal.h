@@ -40,6 +40,23 @@ inline void require(bool ok, emd_status code, const char* msg) {
   if (!ok) throw Error(code, msg);
 }
 
+// Makes a device current for a call, and the caller's own again after it.
+struct DeviceGuard {
+  int before = 0;
+  bool changed = false;
+  explicit DeviceGuard(int device) {
+    EMD_CUDA(cudaGetDevice(&before));
+    if (before == device) return;
+    EMD_CUDA(cudaSetDevice(device));
+    changed = true;
+  }
+  ~DeviceGuard() {
+    if (changed) cudaSetDevice(before);
+  }
+  DeviceGuard(const DeviceGuard&) = delete;
+  DeviceGuard& operator=(const DeviceGuard&) = delete;
+};
+
 // Every device allocation of the library goes through device_malloc, which
 // counts it (emd_device_allocations), so callers and tests can check that a
 // call allocated nothing.

@@ -51,3 +51,20 @@ big.set_shape(512, 0)
 for b in (big, small, big):
     b.run(40)
 """)
+
+
+@pytest.mark.parametrize("spl", [0, 20])
+def test_a_batch_works_on_its_own_device(run, spl):
+    """Whatever the calling thread's current device is, which stays as it was."""
+    run(f"""
+b = batch(device=1)
+b.set_shape(512, {spl})
+fake.cudaSetDevice(0)
+b.get(); b.run(45); b.thermo(); b.tune(20); b.run(3); b.get(); b.info()
+assert current() == 0 and fake.fake_wrong_device() == 0
+held = fake.fake_held()
+b.run(5); b.get()
+assert fake.fake_held() == held
+b.close()
+assert fake.fake_held() == 0 and current() == 0
+""")
