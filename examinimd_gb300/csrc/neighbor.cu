@@ -234,6 +234,7 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
 emd_status emd_neigh_get(emd_ctx* ctx, int* num_neighs, int* entries) {
   EMD_API_BEGIN
   require(c.neigh_ready, EMD_ERR_STATE, "emd_neigh_get: no neighbour list");
+  const DeviceGuard device(c.device);
   const int n = c.neigh_rows;
   neigh_total(c);
   if (num_neighs && n > 0)

@@ -68,3 +68,16 @@ assert fake.fake_held() == held
 b.close()
 assert fake.fake_held() == 0 and current() == 0
 """)
+
+
+def test_a_list_is_read_from_its_own_device(run):
+    """The row starts of a list built without its total are formed when it is read."""
+    run("""
+setup = mdloop.LJSetup(4)
+c = Context(1)
+mdloop.init(c, setup, mdloop.make_lattice(setup))
+assert c.lib.emd_neigh_create(c.h, 0, None) == 0
+fake.cudaSetDevice(0)
+c.neigh_get()
+assert current() == 0 and fake.fake_wrong_device() == 0
+""")
