@@ -282,7 +282,7 @@ emd_status emd_binning_create(emd_ctx* ctx, double dx_in, double dy_in, double d
                                                             c.bincount.p, c.xl_bin.p, c.d_status);
       EMD_CHECK_LAUNCH();
     }
-    exclusive_scan_int(c, c.bincount.p, c.binoffsets.p, nbins, nullptr);
+    exclusive_scan_int(c, c.bincount.p, c.binoffsets.p, nbins);
     if (n > 0) {
       {
         TimedLaunch t(c, "bin_scatter");

@@ -69,11 +69,9 @@ __device__ __forceinline__ int warp_incl_scan(int v) {
   return v;
 }
 
-// Exclusive scan of one tile per block; block totals to sums[blockIdx.x] (and a
-// zero after them, whose exclusive scan is the total), the total of a single tile
-// to *total.
+// Exclusive scan of one tile per block; block totals to sums[blockIdx.x].
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(const int* __restrict__ in, int* __restrict__ out,
-                                                              int n, int* __restrict__ sums, int* total) {
+                                                              int n, int* __restrict__ sums) {
   __shared__ int warp_tot[SCAN_THREADS / 32];
   const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_PER_THREAD;
   int vals[SCAN_PER_THREAD];
@@ -101,20 +99,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(const int* __restri
     if (idx < n) out[idx] = run;
     run += vals[k];
   }
-  if (threadIdx.x == SCAN_THREADS - 1) {
-    if (gridDim.x > 1) {
-      sums[blockIdx.x] = run;
-      if (blockIdx.x == 0) sums[gridDim.x] = 0;
-    } else if (total) {
-      *total = run;
-    }
-  }
+  if (threadIdx.x == SCAN_THREADS - 1) sums[blockIdx.x] = run;
 }
 
-__global__ void k_scan_add(int* __restrict__ out, int n, const int* __restrict__ offs, int tiles, int* total) {
+__global__ void k_scan_add(int* __restrict__ out, int n, const int* __restrict__ offs) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] += offs[i / SCAN_TILE];
-  if (i == 0 && total) *total = offs[tiles];
 }
 
 // Deterministic FP64 sum: fixed grid, fixed per-thread partition.
@@ -153,32 +143,29 @@ __global__ void __launch_bounds__(SUM_THREADS) k_sum_short(const double* __restr
 }
 }  // namespace
 
-static void scan_rec(Ctx& c, const int* in, int* out, int n, int level, int* total) {
+static void scan_rec(Ctx& c, const int* in, int* out, int n, int level) {
   const int tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
   require(level < (int)c.scan_levels.size(), EMD_ERR_ARG, "scan: too many levels");
   DevBuf<int>& sums = c.scan_levels[level];
   sums.reserve(size_t(tiles) + 1, c.stream);
   {
     TimedLaunch t(c, "scan_tiles");
-    k_scan_tiles<<<tiles, SCAN_THREADS, 0, c.stream>>>(in, out, n, sums.p, total);
+    k_scan_tiles<<<tiles, SCAN_THREADS, 0, c.stream>>>(in, out, n, sums.p);
     EMD_CHECK_LAUNCH();
   }
   if (tiles > 1) {
-    scan_rec(c, sums.p, sums.p, tiles + 1, level + 1, nullptr);
+    scan_rec(c, sums.p, sums.p, tiles, level + 1);
     TimedLaunch t(c, "scan_add");
-    k_scan_add<<<blocks_for(n, 256), 256, 0, c.stream>>>(out, n, sums.p, tiles, total);
+    k_scan_add<<<blocks_for(n, 256), 256, 0, c.stream>>>(out, n, sums.p);
     EMD_CHECK_LAUNCH();
   }
 }
 
-void exclusive_scan_int(Ctx& c, const int* d_in, int* d_out, int n, int* d_total) {
-  if (n <= 0) {
-    if (d_total) EMD_CUDA(cudaMemsetAsync(d_total, 0, sizeof(int), c.stream));
-    return;
-  }
+void exclusive_scan_int(Ctx& c, const int* d_in, int* d_out, int n) {
+  if (n <= 0) return;
   // levels are sized once so references into the vector stay valid
   if (c.scan_levels.size() < 6) c.scan_levels.resize(6);
-  scan_rec(c, d_in, d_out, n, 0, d_total);
+  scan_rec(c, d_in, d_out, n, 0);
 }
 
 double device_sum(Ctx& c, const double* d_vals, int n) {
@@ -361,7 +348,7 @@ void emd_destroy(emd_ctx* ctx) {
     b->release();
   for (auto* b : {&c.type, &c.id, &c.stage_i, &c.pack, &c.ghost_owner, &c.ghost_img, 
                   &c.bincount, &c.binoffsets, &c.permute, &c.binof, &c.bin_slot, &c.perm_tmp, &c.num_neighs,
-                  &c.neigh_offsets, &c.neighs, &c.resize_flag, &c.abin})
+                  &c.neighs, &c.resize_flag, &c.abin})
     b->release();
   for (auto& b : c.stage_up) b.release();
   c.x4.release();
@@ -373,6 +360,8 @@ void emd_destroy(emd_ctx* ctx) {
   c.ctr_tab.release();
   c.bin_ctab.release();
   c.neigh_rows2d.release();
+  c.neigh_starts.release();
+  c.neigh_tiles.release();
   c.lj_params_f.release();
   for (auto& b : c.scan_levels) b.release();
   c.halo_state.release();

@@ -192,7 +192,8 @@ struct Ctx {
   long long neigh_total = 0;
   int maxneighs = 16;       // 2D stride
   int neigh_stride = 0;     // 2D: rows (column-major leading dimension)
-  DevBuf<int> num_neighs, neigh_offsets, neighs;
+  DevBuf<int> num_neighs, neighs;
+  DevBuf<long long> neigh_starts, neigh_tiles;  // row starts in their tile, the tiles' (neigh_total)
   DevBuf<int> resize_flag;  // [0] = resize, [1] = new max
   int neigh_packed = 0;     // entries are (j << 5) | stencil code
   int neigh_maxrow = 0;     // longest row of the current list
@@ -290,9 +291,8 @@ inline int blocks_for(long long n, int threads) {
   return int(b < 1 ? 1 : b);
 }
 
-// exclusive scan of n ints in d_in into d_out (may alias); returns total via
-// *d_total (device int) when non-null.  Uses ctx scratch.
-void exclusive_scan_int(Ctx& c, const int* d_in, int* d_out, int n, int* d_total);
+// exclusive scan of n ints in d_in into d_out (may alias).  Uses ctx scratch.
+void exclusive_scan_int(Ctx& c, const int* d_in, int* d_out, int n);
 // deterministic FP64 sum of n doubles (device) -> host value
 double device_sum(Ctx& c, const double* d_vals, int n);
 // the same two reduction kernels on caller-provided device scratch of

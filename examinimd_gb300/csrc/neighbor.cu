@@ -82,14 +82,61 @@ __global__ void k_zero_rows(int* num, int n, int* flags) {
   if (i < 1 + NB_SLOTS) flags[i] = 0;
 }
 
-// column-major rows -> CSR rows at offs[i]
+// Row starts (NeighListCSR::row_map) in 64 bits: a list of 28 million liquid atoms has
+// more than 2^31 entries.  Each tile of rows is scanned by one CTA, then the tiles'
+// totals by one, which leaves the number of entries behind the last.
+constexpr int RS_TILE = 1024;
+__device__ __forceinline__ long long row_scan(long long v, long long& total) {
+  __shared__ long long sh[RS_TILE / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  long long x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long y = __shfl_up_sync(FULL_MASK, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) sh[w] = x;
+  __syncthreads();
+  long long before = 0;
+  total = 0;
+  for (int k = 0; k < RS_TILE / 32; ++k) {
+    before += k < w ? sh[k] : 0;
+    total += sh[k];
+  }
+  __syncthreads();
+  return before + x - v;
+}
+__global__ void __launch_bounds__(RS_TILE) k_row_starts(const int* __restrict__ num, int n,
+                                                        long long* __restrict__ starts,
+                                                        long long* __restrict__ tiles) {
+  const int i = blockIdx.x * RS_TILE + threadIdx.x;
+  long long total;
+  const long long s = row_scan(i < n ? num[i] : 0, total);
+  if (i < n) starts[i] = s;
+  if (threadIdx.x == 0) tiles[blockIdx.x] = total;
+}
+__global__ void __launch_bounds__(RS_TILE) k_row_tiles(long long* tiles, int nt) {
+  long long run = 0;
+  for (int t0 = 0; t0 < nt; t0 += RS_TILE) {
+    const int t = t0 + threadIdx.x;
+    long long total;
+    const long long s = row_scan(t < nt ? tiles[t] : 0, total);
+    if (t < nt) tiles[t] = run + s;
+    run += total;
+  }
+  if (threadIdx.x == 0) tiles[nt] = run;
+}
+
+// column-major rows -> CSR rows
 __global__ void __launch_bounds__(256) k_rows_to_csr(const int* __restrict__ rows, int stride,
-                                                     const int* __restrict__ num, const int* __restrict__ offs, int n,
+                                                     const int* __restrict__ num, const long long* __restrict__ starts,
+                                                     const long long* __restrict__ tiles, int n,
                                                      int* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int m = num[i], o = offs[i];
-  for (int k = 0; k < m; ++k) out[o + k] = rows[quad_index(i, k, stride)];
+  const int m = num[i];
+  out += starts[i] + tiles[i / RS_TILE];
+  for (int k = 0; k < m; ++k) out[k] = rows[quad_index(i, k, stride)];
 }
 
 // packed entries -> plain j (for emd_neigh_get)
@@ -103,16 +150,23 @@ __global__ void k_unpack(int* __restrict__ e, long long n) {
 
 using namespace emd;
 
-// row starts (NeighListCSR::row_map) and number of entries of the current list
+// number of entries of the current list; forms the row starts
 static long long neigh_total(Ctx& c) {
   if (c.neigh_total >= 0) return c.neigh_total;
-  const int n = c.neigh_rows;
-  c.neigh_offsets.reserve(size_t(n) + 2, c.stream);
-  exclusive_scan_int(c, c.num_neighs.p, c.neigh_offsets.p, n, c.neigh_offsets.p + n);
-  EMD_CUDA(cudaMemcpyAsync(c.h_int, c.neigh_offsets.p + n, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  const int n = c.neigh_rows, nt = (n + RS_TILE - 1) / RS_TILE;
+  if (n == 0) return c.neigh_total = 0;
+  c.neigh_starts.reserve(size_t(n), c.stream);
+  c.neigh_tiles.reserve(size_t(nt) + 1, c.stream);
+  {
+    TimedLaunch t(c, "neigh_row_starts");
+    k_row_starts<<<nt, RS_TILE, 0, c.stream>>>(c.num_neighs.p, n, c.neigh_starts.p, c.neigh_tiles.p);
+    EMD_CHECK_LAUNCH();
+    k_row_tiles<<<1, RS_TILE, 0, c.stream>>>(c.neigh_tiles.p, nt);
+    EMD_CHECK_LAUNCH();
+  }
+  EMD_CUDA(cudaMemcpyAsync(c.h_ll, c.neigh_tiles.p + nt, sizeof(long long), cudaMemcpyDeviceToHost, c.stream));
   EMD_CUDA(cudaStreamSynchronize(c.stream));
-  c.neigh_total = n > 0 ? c.h_int[0] : 0;
-  return c.neigh_total;
+  return c.neigh_total = c.h_ll[0];
 }
 
 extern "C" {
@@ -243,7 +297,7 @@ emd_status emd_neigh_get(emd_ctx* ctx, int* num_neighs, int* entries) {
     DevBuf<int> tmp;
     tmp.reserve(size_t(c.neigh_total), c.stream);
     k_rows_to_csr<<<blocks_for(n, 256), 256, 0, c.stream>>>(neigh_rows(c), c.neigh_stride, c.num_neighs.p,
-                                                            c.neigh_offsets.p, n, tmp.p);
+                                                            c.neigh_starts.p, c.neigh_tiles.p, n, tmp.p);
     EMD_CHECK_LAUNCH();
     if (c.neigh_packed) {
       k_unpack<<<blocks_for(c.neigh_total, 256), 256, 0, c.stream>>>(tmp.p, c.neigh_total);
