@@ -277,6 +277,7 @@ __device__ __forceinline__ int rows_of_bin(const RowArgs& a, RowStage& st, int b
           st.w[lane] = w;
         }
         st.self[lane] = at >= full ? at - full : -1;
+        __syncwarp();  // the next candidates' lanes write self too
         m = rest;
       }
     }

@@ -64,3 +64,18 @@ def test_reverse_forces(n, box):
         out.append(mdloop.by_id(b.get(0, n))["f"])
     scale = np.abs(out[1]).max()
     assert np.abs(out[0] - out[1]).max() <= 1e-12 * scale
+
+
+@pytest.mark.parametrize("half,prec", [(False, 0), (True, 0), (False, 1)])
+def test_rows_of_crowded_bins(half, prec):
+    """90 atoms a bin: every chunk of 32 centre atoms stages some 900 candidates, 256 at a
+    time, and finds its own atoms among those carried over."""
+    from examinimd_gb300 import Context
+    from oracle.orc import Oracle
+    st, state = _gas(3000, 9.0, 21, half=half)
+    gpu, orc = Context(0), Oracle(4)
+    tg, to = mdloop.init(gpu, st, state, precision=prec), mdloop.init(orc, st, state)
+    assert tg == to
+    for p, q in zip(gpu.neigh_get(tg), orc.neigh_get(to)):
+        np.testing.assert_array_equal(p, q)
+    gpu.close()
