@@ -15,6 +15,9 @@
 // Bound by instruction issue: about 7 instructions per candidate and lane and 13
 // per listed pair (tests, order rule and append for every candidate took 20).
 // Full lists, packed, 4,000,000 particles: 2.26 ms with one loop, 1.81 with masks.
+// A gas's build is bound by the latency of its many short warps: an empty bin leaves
+// first, and up to eight candidates take a quarter of the mask (256,000 particles, 0.2 / 0.5 / 1.1 a
+// bin: 395 / 253 / 132 us with one loop, 411 / 286 / 155 with whole masks, 366 / 249 / 137 so).
 #pragma once
 #include "emd_device.cuh"
 #include "emd_internal.h"
@@ -78,8 +81,9 @@ __device__ __noinline__ bool above_fp64(const double4_32a* __restrict__ x4, int 
   return (jx > ix) || ((jx == ix) && ((jy > iy) || ((jy == iy) && (jz > iz))));
 }
 
-// bit 31 - k: candidate k of the 32 from `b` on is within the cutoff of xi
-__device__ __forceinline__ unsigned row_mask(const RowArgs& a, const RowStage& st, int b, const float4& xi, int i,
+// bit 31 - k: candidate k of the n <= 32 from `b` on is within the cutoff of xi (the
+// first eight alone where there are no more: a gas's bins)
+__device__ __forceinline__ unsigned row_mask(const RowArgs& a, const RowStage& st, int b, int n, const float4& xi, int i,
                                              bool packed) {
   const float2 m1 = make_float2(-1.f, -1.f);
   const float2 xx = make_float2(xi.x, xi.x), yy = make_float2(xi.y, xi.y), zz = make_float2(xi.z, xi.z);
@@ -97,6 +101,10 @@ __device__ __forceinline__ unsigned row_mask(const RowArgs& a, const RowStage& s
   };
 #pragma unroll
   for (int k = 0; k < 32; k += 4) {
+    if (k == 8 && n <= 8) {
+      mask <<= 24;
+      break;
+    }
     const float4 x = *reinterpret_cast<const float4*>(st.x + b + k);
     const float4 y = *reinterpret_cast<const float4*>(st.y + b + k);
     const float4 z = *reinterpret_cast<const float4*>(st.z + b + k);
@@ -128,6 +136,8 @@ __device__ __forceinline__ int rows_of_bin(const RowArgs& a, RowStage& st, int b
     const int dbx = lane / 9 - 1, dby = (lane / 3) % 3 - 1, dbz = lane % 3 - 1;
     cntb = bin(((bx + dbx) * a.nby + (by + dby)) * a.nbz + (bz + dbz), offb);
   }
+  const int nc = __shfl_sync(FULL_MASK, cntb, 13), oc = __shfl_sync(FULL_MASK, offb, 13);
+  if (nc == 0) return 0;
   // inclusive scan of the 27 stencil counts over the lanes
   int inc = cntb;
 #pragma unroll
@@ -142,7 +152,6 @@ __device__ __forceinline__ int rows_of_bin(const RowArgs& a, RowStage& st, int b
   if (lane == 0) st.pre[0] = 0;
   __syncwarp();
   const int M = st.pre[27];
-  const int nc = __shfl_sync(FULL_MASK, cntb, 13), oc = __shfl_sync(FULL_MASK, offb, 13);
   int mx = 0;
   // Candidates farther than the cutoff from every centre atom of the chunk
   // are dropped while staging, once per warp: the squared FP32 distance to the
@@ -185,8 +194,8 @@ __device__ __forceinline__ int rows_of_bin(const RowArgs& a, RowStage& st, int b
       rp += (cnt & 3) == 3 ? jump : 1;
       ++cnt;
     };
-    auto append = [&](int b) {  // the 32 candidates from b on
-      unsigned mask = row_mask(a, st, b, xi, i, PACKED);
+    auto append = [&](int b, int n) {  // the n <= 32 candidates from b on
+      unsigned mask = row_mask(a, st, b, n, xi, i, PACKED);
       if (unsigned(at - b) < 32u) mask &= ~(0x80000000u >> (at - b));
       if (HALF) {
         // neighbor_csr.h:287-291: skip unless j is "above" i
@@ -260,7 +269,7 @@ __device__ __forceinline__ int rows_of_bin(const RowArgs& a, RowStage& st, int b
         __syncwarp();
         at = st.self[lane];
         if (own)
-          for (int b = 0; b < full; b += 32) append(b);
+          for (int b = 0; b < full; b += 32) append(b, m - b);
         __syncwarp();
         const int rest = last ? 0 : m - full;
         if (lane < rest) {

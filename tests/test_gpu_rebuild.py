@@ -79,3 +79,18 @@ def test_rows_of_crowded_bins(half, prec):
     for p, q in zip(gpu.neigh_get(tg), orc.neigh_get(to)):
         np.testing.assert_array_equal(p, q)
     gpu.close()
+
+
+@pytest.mark.parametrize("half,prec", [(False, 0), (True, 0), (False, 1)])
+@pytest.mark.parametrize("n,box", [(1, 9.0), (300, 30.0), (2500, 30.0), (8000, 35.0)])
+def test_rows_of_a_gas(n, box, half, prec):
+    """Empty bins, and bins with up to eight, nine and 32 candidates (0.2, 1.7 and 4 atoms a bin)."""
+    from examinimd_gb300 import Context
+    from oracle.orc import Oracle
+    st, state = _gas(n, box, 5 * n, half=half)
+    gpu, orc = Context(0), Oracle(4)
+    tg, to = mdloop.init(gpu, st, state, precision=prec), mdloop.init(orc, st, state)
+    assert tg == to
+    for p, q in zip(gpu.neigh_get(tg), orc.neigh_get(to)):
+        np.testing.assert_array_equal(p, q)
+    gpu.close()
