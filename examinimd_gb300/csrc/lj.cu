@@ -51,8 +51,22 @@ int lj_tile_rows(int n, bool half) {
 // the sum depends on the atom count only and its scratch is bounded
 constexpr int LJE_BLOCKS = 152 * 6;
 
+// A gas's rows: a tile's warp takes a trip to memory for each of them, however short, a
+// thread per row one for 32.  Measured on a random gas (us, thread / tile): 256,000 atoms,
+// 0.5, 1.8 and 3.7 entries a row (longest 6, 10, 16), force 44 / 82, 82 / 98, 121 / 105;
+// 32,000, longest 5 and 9, 12 / 17 and 18 / 21; 16,000, 9 / 10 and 14 / 12; 2,000, 8 / 6 and 12 / 7:
+// there the chip is not full and the tiles' warps run side by side.  Energy, longest
+// 9 or 10: 97 / 127, 41 / 46, 38 / 38 and 36 / 39.
+bool lj_short_rows(const LJTile& T, bool energy) { return T.longest <= 9 && (energy || T.n > 16384); }
+
 template <int MODE, bool UNI, bool IDIAL = false, bool ZERO = false>
 void launch_lj_fp64(LJTile T, cudaStream_t s) {
+  if (lj_short_rows(T, MODE == LJ_ENERGY)) {
+    k_lj_fp64_rows<MODE, UNI, IDIAL, ZERO>
+        <<<MODE == LJ_ENERGY ? LJE_BLOCKS : blocks_for(T.n, LJR_THREADS), LJR_THREADS, 0, s>>>(T);
+    EMD_CHECK_LAUNCH();
+    return;
+  }
   T.rows = lj_tile_rows(T.n, T.half);
   T.cap = ljt_cap(T.rows, T.half);
   const size_t smem = LJT_WARPS * ljt_warp_bytes(T.cap, T.half, UNI);
@@ -139,6 +153,7 @@ static LJTile lj_tile(Ctx& c) {
   T.n = c.N_local;
   T.half = c.lj_half;
   T.packed = c.neigh_packed;
+  T.longest = c.neigh_maxrow;
   return T;
 }
 

@@ -84,6 +84,7 @@ struct LJTile {
   int n, rows, cap;  // owned atoms, rows per warp, slots of its list
   int half;        // the list is a half list
   int packed;      // entries are (j << 6) | code
+  int longest;     // longest row
   double* part;    // energy: one partial per CTA
 };
 
@@ -281,6 +282,66 @@ __global__ void __launch_bounds__(LJT_THREADS) k_lj_fp64(LJTile T) {
   }
   if constexpr (MODE == LJ_ENERGY) {
     __shared__ double sh[LJT_WARPS];
+    const double t = block_sum(esum, sh);
+    if (threadIdx.x == 0) T.part[blockIdx.x] = t;
+  }
+}
+
+// A thread per row, for short rows (lj_short_rows): the same operations in the same
+// order.  Energy: a fixed number of CTAs, one partial each, as above.
+constexpr int LJR_THREADS = 128;
+template <int MODE, bool UNI, bool IDIAL, bool ZERO>
+__global__ void __launch_bounds__(LJR_THREADS) k_lj_fp64_rows(LJTile T) {
+  double esum = 0.0;
+  const int step = MODE == LJ_ENERGY ? gridDim.x * LJR_THREADS : T.n;
+  for (int i = blockIdx.x * LJR_THREADS + threadIdx.x; i < T.n; i += step) {
+    const double4_32a xi = T.x4[i];
+    const Row row(T.L, i);
+    const int ti = UNI ? 0 : T.P.type[i] * T.P.ntypes;
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    for (int k = 0; k < row.n; ++k) {
+      int j = row[k];
+      if (T.packed) j >>= 6;
+      const double4_32a xj = T.x4[j];
+      const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+      const double rsq = dx * dx + dy * dy + dz * dz;
+      const int tp = UNI ? 0 : ti + __ldg(T.P.type + j);
+      const double cutsq = UNI ? T.P.cutsq_0 : __ldg(T.P.cutsq + tp);
+      if (!(rsq < cutsq)) continue;
+      const double lj1 = UNI ? T.P.lj1_0 : __ldg(T.P.lj1 + tp), lj2 = UNI ? T.P.lj2_0 : __ldg(T.P.lj2 + tp);
+      if constexpr (MODE == LJ_ENERGY) {
+        const double r2inv = recip_rn(rsq), r6inv = r2inv * r2inv * r2inv;
+        const double r2c = 1.0 / cutsq, r6c = r2c * r2c * r2c, c12 = lj1 / 12.0, c6 = lj2 / 6.0;
+        esum += (T.half && j < T.n ? 1.0 : 0.5) * (r6inv * (c12 * r6inv - c6) - r6c * (c12 * r6c - c6));
+      } else {
+        const double fpair = lj_fpair<IDIAL>(rsq, lj1, lj2, IDIAL ? __ldg(T.P.intensity + tp) : 1.0);
+        const double px = dx * fpair, py = dy * fpair, pz = dz * fpair;
+        fx += px;
+        fy += py;
+        fz += pz;
+        if (MODE == LJ_HALF && (!IDIAL || j < T.n)) {
+          double* fj = T.f + 3 * size_t(j);
+          atomicAdd(fj, -px);
+          atomicAdd(fj + 1, -py);
+          atomicAdd(fj + 2, -pz);
+        }
+      }
+    }
+    if constexpr (MODE != LJ_ENERGY) {
+      double* fi = T.f + 3 * size_t(i);
+      if (MODE == LJ_HALF) {
+        atomicAdd(fi, fx);
+        atomicAdd(fi + 1, fy);
+        atomicAdd(fi + 2, fz);
+      } else {  // ZERO: the pending deep_copy(f, 0) folded into the store
+        fi[0] = (ZERO ? 0.0 : fi[0]) + fx;
+        fi[1] = (ZERO ? 0.0 : fi[1]) + fy;
+        fi[2] = (ZERO ? 0.0 : fi[2]) + fz;
+      }
+    }
+  }
+  if constexpr (MODE == LJ_ENERGY) {
+    __shared__ double sh[LJR_THREADS / 32];
     const double t = block_sum(esum, sh);
     if (threadIdx.x == 0) T.part[blockIdx.x] = t;
   }

@@ -87,3 +87,48 @@ def test_filter_far_from_the_origin(shift):
         b.lj_compute()
         f.append(b.get(0, n)["f"])
     assert np.array_equal(f[0], f[1])
+
+
+@pytest.mark.parametrize("n", [300, 16384, 16385, 30000])
+@pytest.mark.parametrize("ntypes", [1, 13])
+@pytest.mark.parametrize("half", [False, True])
+def test_gas_with_short_rows(n, ntypes, half):
+    """One entry a row on average, none above nine: a thread per row for the energy, and
+    for the forces of more than 16,384 atoms."""
+    from examinimd_gb300 import Context
+    from oracle.orc import Oracle
+    st, state = _gas(n, (n / 0.011) ** (1.0 / 3.0), ntypes, n, half, 0)
+    gpu, orc = Context(0), Oracle()
+    total = mdloop.init(gpu, st, state)
+    mdloop.init(orc, st, state)
+    assert 0 < gpu.neigh_get(total)[0].max() <= 9
+    a, b = gpu.get(0, n), orc.get(0, n)
+    for again in range(2):  # the second time on top of the first one's forces
+        if half:
+            assert np.abs(a["f"] - b["f"]).max() <= 1e-12 * np.abs(b["f"]).max()
+        else:
+            assert np.array_equal(a["f"], b["f"])
+        gpu.lj_compute()
+        orc.lj_compute()
+        a, b = gpu.get(0, n), orc.get(0, n)
+    eg, eo = gpu.lj_energy(), orc.lj_energy()
+    assert abs(eg - eo) <= 1e-12 * max(abs(eo), float(n))
+    assert gpu.lj_energy_noalloc() == eg
+    gpu.close()
+
+
+def test_intensity_dial_with_short_rows():
+    """One evaluation per pair is the plain force, divided by one."""
+    import ctypes
+    from examinimd_gb300 import Context
+    n = 20000
+    st, state = _gas(n, (n / 0.011) ** (1.0 / 3.0), 1, 9, False, 0)
+    gpu = Context(0)
+    mdloop.init(gpu, st, state)
+    f = gpu.get(0, n)["f"]
+    one = np.ones(1)
+    assert gpu.lib.emd_lj_set_intensity(gpu.h, one.ctypes.data_as(ctypes.c_void_p)) == 0
+    gpu.zero_forces()
+    gpu.lj_compute()
+    assert np.array_equal(gpu.get(0, n)["f"], f) and np.abs(f).max() > 0.0
+    gpu.close()
