@@ -286,10 +286,11 @@ __global__ void k_halo_force(double* __restrict__ f, const int* __restrict__ pac
 }
 
 // The six phases in order by one CTA, or one cluster of eight, which goes past L1
-// because a phase reads what another CTA wrote (a launch per phase costs more than
-// its additions up to here): 400 ghosts 36 -> 10 us, 7,000 36 -> 20 (the cluster
-// takes as long), 48,000 39 -> 26.
-constexpr int HALO_FORCE_MAX = 200000, HALO_FORCE_ONE = 8192, HALO_FORCE_CTAS = 8, HALO_FORCE_THREADS = 1024;
+// because a phase reads what another CTA wrote.  Six launches take 24.8 us whatever their
+// additions, up to 250,000 ghosts; one CTA 14.5 for 5,841 ghosts, the cluster 18.6 for 13,275
+// and 19.4 for 42,381, but 24.8 for 50,760, 30.9 for 59,895 and 53.4 for 160,191: eight
+// SMs, so the launches take over at 50,000.
+constexpr int HALO_FORCE_MAX = 50000, HALO_FORCE_ONE = 8192, HALO_FORCE_CTAS = 8, HALO_FORCE_THREADS = 1024;
 struct HaloPhases {
   int pack[6], count[6], ghost[6];
 };

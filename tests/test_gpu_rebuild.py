@@ -94,3 +94,18 @@ def test_rows_of_a_gas(n, box, half, prec):
     for p, q in zip(gpu.neigh_get(tg), orc.neigh_get(to)):
         np.testing.assert_array_equal(p, q)
     gpu.close()
+
+
+@pytest.mark.parametrize("n,lo,hi", [(140000, 42000, 50000), (170000, 50001, 60000)])
+def test_reverse_forces_on_either_side_of_the_cluster(n, lo, hi):
+    """Up to 50,000 ghosts one cluster, beyond a launch per phase (tolerance as above)."""
+    from examinimd_gb300 import Context
+    from oracle.orc import Oracle
+    st, state = _gas(n, (n / 0.8442) ** (1.0 / 3.0), n, half=True)
+    out = []
+    for b in (Context(0), Oracle(8)):
+        mdloop.init(b, st, state)
+        assert lo <= b.info()[1] <= hi
+        out.append(mdloop.by_id(b.get(0, n))["f"])
+    scale = np.abs(out[1]).max()
+    assert np.abs(out[0] - out[1]).max() <= 1e-12 * scale
