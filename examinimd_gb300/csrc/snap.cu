@@ -27,10 +27,11 @@ struct SnapTables;
 struct SnapHost {
   SnapDev d{};
   const int* tmask = nullptr;  // k_snap_force: groups of T
+  const int4* zsrc = nullptr;  // the FP32 stream's products (SnapTables::src)
   const SnapTables* tab = nullptr;
   int precision = EMD_PREC_FP64;
   DevBuf<unsigned char> tables;  // every constant table, one allocation and copy
-  DevBuf<double> cY, beta0;
+  DevBuf<double> coef;  // cY, then beta_0 of every element
   DevBuf<uint4> zs;
   // per-chunk work arrays
   DevBuf<double> pd, pr_f, U, Y, zk;
@@ -111,10 +112,7 @@ struct SnapTables {
   std::vector<double> zc, AB, monod;
   std::vector<ZGrp> grp;
   std::vector<unsigned> words;  // the FP32 stream without its coefficients
-  struct Src {
-    int word, c0, t0, nj;  // of a product: its words, coefficients and highest triple
-  };
-  std::vector<Src> src;
+  std::vector<int4> src;  // of a product in it: first word, coefficient, highest triple, number of j
   int nz = 0, nh = 0, ny = 0;
   // cost of the busiest of k + 1 CTAs that share a tile's tasks: FP64 in cycles,
   // mixed in instructions of the busiest of 12 or 16 warps
@@ -312,7 +310,7 @@ struct SnapTables {
         }
         for (int i = 0; i < z.np; ++i) {
           const int2 u = prod[size_t(z.p0 + i)];
-          src.push_back(Src{int(words.size()), z.c0 + i * z.nj, z.t0, z.nj});
+          src.push_back(int4{int(words.size()), z.c0 + i * z.nj, z.t0, z.nj});
           words.push_back(unsigned(u.x) | unsigned(u.y) << 16);
           words.resize(words.size() + size_t(nw) - 1, 0u);
         }
@@ -373,6 +371,16 @@ const SnapTables& snap_tables(int J, const std::vector<int>& trip) {
   return *tables[J];
 }
 
+// the FP32 stream's coefficients: the Clebsch-Gordan products times cY
+__global__ void __launch_bounds__(256) k_zs_fill(SnapDev S, const int4* __restrict__ src, int n, unsigned* zs) {
+  const int k = blockIdx.x * 256 + threadIdx.x, e = blockIdx.y;
+  if (k >= n) return;
+  const int4 p = src[k];
+  const double* c = S.cY + size_t(e) * S.nfull + p.z;
+  unsigned* w = zs + size_t(e) * S.zs_n * 4 + p.x + 1;
+  for (int j = 0; j < p.w; ++j) w[j] = __float_as_uint(float(S.zc[p.y + j] * c[-j]));
+}
+
 // per-element column sums of the adjoint's per-atom outputs (fixed order)
 __global__ void __launch_bounds__(256) k_adj_reduce(const double* __restrict__ adj, int n, int ncols,
                                                     const int* __restrict__ type, const int* __restrict__ map,
@@ -397,7 +405,7 @@ void free_snap(Ctx& c) {
   h->D.release();
   h->H.release();
   for (auto* b : {&h->pj, &h->cnt}) b->release();
-  for (auto* b : {&h->cY, &h->beta0, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk, &h->eatom, &h->adj, &h->adj_sum, &h->adj_g,
+  for (auto* b : {&h->coef, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk, &h->eatom, &h->adj, &h->adj_sum, &h->adj_g,
                   &h->keep_u, &h->keep_z})
     b->release();
   delete h;
@@ -410,35 +418,24 @@ static void upload(Ctx& c, DevBuf<T>& b, const std::vector<T>& v) {
   EMD_CUDA(cudaMemcpyAsync(b.p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, c.stream));
 }
 
-// the FP32 stream of every element: the tables' words with coefficients times cY
-static void upload_stream(Ctx& c, SnapHost* h, const SnapTables& tab, const std::vector<double>& cY) {
-  const SnapDev& S = h->d;
-  const size_t n = tab.words.size();
-  std::vector<unsigned> w(n * size_t(S.nelem));
-  for (int e = 0; e < S.nelem; ++e) {
-    std::copy(tab.words.begin(), tab.words.end(), w.begin() + long(n) * e);
-    const double* ce = &cY[size_t(e) * S.nfull];
-    for (const auto& p : tab.src)
-      for (int j = 0; j < p.nj; ++j) {
-        const float v = float(tab.zc[size_t(p.c0 + j)] * ce[p.t0 - j]);
-        std::memcpy(&w[n * size_t(e) + size_t(p.word + 1 + j)], &v, sizeof v);
-      }
-  }
-  h->zs.reserve(w.size() / 4 + 1, c.stream);
-  EMD_CUDA(cudaMemcpyAsync(h->zs.p, w.data(), w.size() * sizeof(unsigned), cudaMemcpyHostToDevice, c.stream));
-  EMD_CUDA(cudaStreamSynchronize(c.stream));
+// the coefficients' part of the FP32 stream, where the form has one
+static void fill_stream(Ctx& c, SnapHost* h) {
+  if (h->precision != EMD_PREC_MIXED) return;
+  const int n = int(h->tab->src.size());
+  TimedLaunch t(c, "snap_stream");
+  k_zs_fill<<<dim3(blocks_for(n, 256), h->d.nelem), 256, 0, c.stream>>>(h->d, h->zsrc, n,
+                                                                        reinterpret_cast<unsigned*>(h->zs.p));
+  EMD_CHECK_LAUNCH();
 }
 
 // Y's coefficients: beta_k folded onto the full triples of compute_dbidrj's
-// three terms (sna_impl.hpp:330-570), per element, with beta_0 apart
-void snap_fold_beta(const SnapHost& h, int nfull, int nelem, int ncoeffall, const double* beta,
-                    std::vector<double>& cY, std::vector<double>& beta0) {
-  cY.assign(size_t(nelem) * nfull, 0.0);
-  beta0.assign(static_cast<size_t>(nelem), 0.0);
+// three terms (sna_impl.hpp:330-570), per element, then every element's beta_0
+std::vector<double> snap_fold_beta(const SnapHost& h, int nfull, int nelem, int ncoeffall, const double* beta) {
+  std::vector<double> c(size_t(nelem) * (nfull + 1), 0.0);
   for (int e = 0; e < nelem; ++e) {
     const double* be = beta + size_t(e) * ncoeffall;
-    beta0[size_t(e)] = be[0];
-    double* ce = &cY[size_t(e) * nfull];
+    c[size_t(nelem) * nfull + size_t(e)] = be[0];
+    double* ce = &c[size_t(e) * nfull];
     for (size_t k = 0; k < h.k_t1.size(); ++k) {
       const int j1 = h.k_j[3 * k], j2 = h.k_j[3 * k + 1], j = h.k_j[3 * k + 2];
       const double bk = be[k + 1];
@@ -447,6 +444,7 @@ void snap_fold_beta(const SnapHost& h, int nfull, int nelem, int ncoeffall, cons
       ce[h.k_t3[k]] += bk * (j + 1) / (j2 + 1.0);
     }
   }
+  return c;
 }
 
 // Atoms are worked on in chunks so that the work arrays stay bounded: at most
@@ -764,8 +762,7 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
     h->k_f3.push_back((j + 1) / (j2 + 1.0));
     h->k_j.insert(h->k_j.end(), {j1, j2, j});
   }
-  std::vector<double> cY, beta0;
-  snap_fold_beta(*h, S.nfull, nelem, ncoeffall, beta, cY, beta0);
+  const std::vector<double> coef = snap_fold_beta(*h, S.nfull, nelem, ncoeffall, beta);
   double rcutmax = 0.0;
   for (int e = 0; e < nelem; e++) rcutmax = std::max(2.0 * radelem[e] * rcutfac, rcutmax);
   S.rfac0 = rfac0;
@@ -824,17 +821,23 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   put(S.wj32, wj32);
   put(S.wjelem, std::vector<double>(wjelem, wjelem + nelem));
   put(S.map, std::vector<int>(map, map + ntypes));
+  if (precision == EMD_PREC_MIXED) put(h->zsrc, tab.src);
   upload(c, h->tables, bytes);
   for (auto& f : place) f(h->tables.p);
-  upload(c, h->cY, cY);
-  upload(c, h->beta0, beta0);
-  EMD_CUDA(cudaStreamSynchronize(c.stream));
-  S.cY = h->cY.p;
-  S.beta0 = h->beta0.p;
+  upload(c, h->coef, coef);
+  S.cY = h->coef.p;
+  S.beta0 = h->coef.p + size_t(nelem) * S.nfull;
   S.zs_n = int(tab.words.size() / 4);
   h->tab = &tab;
-  if (precision == EMD_PREC_MIXED) upload_stream(c, h, tab, cY);
+  std::vector<unsigned> w;
+  if (precision == EMD_PREC_MIXED) {
+    for (int e = 0; e < nelem; ++e) w.insert(w.end(), tab.words.begin(), tab.words.end());
+    h->zs.reserve(w.size() / 4, c.stream);
+    EMD_CUDA(cudaMemcpyAsync(h->zs.p, w.data(), w.size() * sizeof(unsigned), cudaMemcpyHostToDevice, c.stream));
+  }
   S.zs = h->zs.p;
+  fill_stream(c, h);
+  EMD_CUDA(cudaStreamSynchronize(c.stream));
   EMD_API_END
 }
 
@@ -865,12 +868,9 @@ emd_status emd_snap_set_beta(emd_ctx* ctx, const double* beta) {
   SnapHost* h = static_cast<SnapHost*>(c.snap);
   require(h != nullptr, EMD_ERR_STATE, "emd_snap_set_beta: SNAP not initialised");
   require(beta != nullptr, EMD_ERR_ARG, "emd_snap_set_beta: null beta");
-  std::vector<double> cY, beta0;
-  snap_fold_beta(*h, h->d.nfull, h->d.nelem, h->d.ncoeffall, beta, cY, beta0);
-  EMD_CUDA(cudaMemcpyAsync(h->cY.p, cY.data(), sizeof(double) * cY.size(), cudaMemcpyHostToDevice, c.stream));
-  if (h->precision == EMD_PREC_MIXED) upload_stream(c, h, *h->tab, cY);
-  EMD_CUDA(cudaMemcpyAsync(h->beta0.p, beta0.data(), sizeof(double) * beta0.size(), cudaMemcpyHostToDevice,
-                           c.stream));
+  const std::vector<double> coef = snap_fold_beta(*h, h->d.nfull, h->d.nelem, h->d.ncoeffall, beta);
+  EMD_CUDA(cudaMemcpyAsync(h->coef.p, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice, c.stream));
+  fill_stream(c, h);
   EMD_CUDA(cudaStreamSynchronize(c.stream));
   EMD_API_END
 }

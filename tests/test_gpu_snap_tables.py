@@ -123,3 +123,28 @@ def test_threads_with_systems_of_different_size():
         for ref, got in zip(alone, ex.map(force, decks)):
             for f in got:
                 assert np.abs(f - ref).max() <= 1e-13 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("J,nelem", [(0, 1), (4, 3), (8, 2), (10, 1)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_new_coefficients_are_those_of_a_new_potential(J, nelem, precision):
+    """emd_snap_set_beta against emd_snap_init with the same coefficients: the same
+    forces to the scatter's order of adds, the same energy."""
+    from examinimd_gb300 import Context
+    st, state = _deck(J, (3, 3, 3), 3.1803, nelem=nelem, seed=J)
+    n = len(state["x"])
+    new = np.array([[b * (1.0 + 0.3 * k) + 0.01 for b in e["beta"]] for k, e in enumerate(st.elements)])
+    a, b = Context(0), Context(0)
+    mdloop.init(a, st, state, precision=precision)
+    a.snap_set_beta(new)
+    for e, row in zip(st.elements, new):
+        e["beta"] = list(row)
+    mdloop.init(b, st, state, precision=precision)
+    a.zero_forces()
+    a.snap_compute()
+    a.comm_update_force()
+    fa, fb = a.get(0, n)["f"], b.get(0, n)["f"]
+    assert np.abs(fa - fb).max() <= 1e-13 * np.abs(fb).max()
+    assert a.snap_energy() == b.snap_energy()
+    a.close()
+    b.close()
