@@ -2,6 +2,7 @@
 // (force_snap_neigh_impl.h:160-724, sna_impl.hpp).  The kernel is in
 // snap_kernel.cuh; the mixed-form instantiation is compiled in snap_mixed.cu.
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <functional>
@@ -55,10 +56,15 @@ struct SnapHost {
 
 
 // ---------------------------------------------------------------- host tables
+constexpr int kFactorials = 32;  // the largest: 3 / 2 twojmax + 1 = 22
 double factorial(int n) {
-  double r = 1.0;
-  for (int i = 1; i <= n; i++) r *= 1.0 * i;
-  return r;
+  static const std::array<double, kFactorials> table = [] {
+    std::array<double, kFactorials> t{};
+    t[0] = 1.0;
+    for (int i = 1; i < kFactorials; i++) t[size_t(i)] = t[size_t(i - 1)] * i;
+    return t;
+  }();
+  return table[size_t(n)];
 }
 double deltacg(int j1, int j2, int j) {
   const double s = factorial((j1 + j2 + j) / 2 + 1);
