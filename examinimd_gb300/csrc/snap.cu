@@ -38,6 +38,12 @@ struct SnapHost {
   DevBuf<double> pd, pr_f, U, Y, zk;
   DevBuf<int> pj, cnt;
   DevBuf<Cplx<double>> D, H;
+  int fits = 1 << 30;  // atoms that memory had room for when it was short (snap_chunks)
+  void release_work() {
+    for (auto* b : {&pd, &pr_f, &U, &Y, &zk}) b->release();
+    for (auto* b : {&pj, &cnt}) b->release();
+    for (auto* b : {&D, &H}) b->release();
+  }
   DevBuf<double> eatom;
   // adjoint: per-atom columns, their per-element sums, the loss gradient dL/dF
   DevBuf<double> adj, adj_sum, adj_g;
@@ -406,14 +412,10 @@ __global__ void __launch_bounds__(256) k_adj_reduce(const double* __restrict__ a
 void free_snap(Ctx& c) {
   if (!c.snap) return;
   SnapHost* h = static_cast<SnapHost*>(c.snap);
+  h->release_work();
   h->tables.release();
   h->zs.release();
-  h->D.release();
-  h->H.release();
-  for (auto* b : {&h->pj, &h->cnt}) b->release();
-  for (auto* b : {&h->coef, &h->pd, &h->pr_f, &h->U, &h->Y, &h->zk, &h->eatom, &h->adj, &h->adj_sum, &h->adj_g,
-                  &h->keep_u, &h->keep_z})
-    b->release();
+  for (auto* b : {&h->coef, &h->eatom, &h->adj, &h->adj_sum, &h->adj_g, &h->keep_u, &h->keep_z}) b->release();
   delete h;
   c.snap = nullptr;
 }
@@ -464,6 +466,25 @@ static int snap_chunk(int n, int cap, bool adjoint_z, const SnapDev& S) {
   const size_t most = std::max<size_t>(32, std::min<size_t>(kChunk, kChunkBytes / per));
   const int chunks = int((size_t(n) + most - 1) / most);
   return std::min(n, ((n + chunks - 1) / chunks + 31) & ~31);
+}
+
+// work(first, n) for all atoms, `chunk` at a time.  It reserves its work arrays before its
+// first launch; where they do not fit, they are given back and half as many atoms are
+// taken (multiples of 32, the tiles of what an adjoint keeps), by later calls too.
+template <typename Work>
+static void snap_chunks(Ctx& c, SnapHost* h, int n, int chunk, Work&& work) {
+  for (int first = 0; first < n;) {
+    const int m = std::min({chunk, h->fits, n - first});
+    try {
+      work(first, m);
+      first += m;
+    } catch (const Error& e) {
+      if (e.code != EMD_ERR_NOMEM || m <= 32) throw;
+      EMD_CUDA(cudaStreamSynchronize(c.stream));
+      h->release_work();
+      h->fits = (m / 2 + 31) & ~31;
+    }
+  }
 }
 
 // Atoms per tile of k_snap_y and CTAs that share a tile's tasks: the smallest
@@ -583,8 +604,8 @@ static void snap_launch(Ctx& c, bool energy) {
     h->keep_z.reserve(2 * size_t(S.nz) * ((size_t(n) + 31) & ~size_t(31)), c.stream);
   }
   const int chunk = snap_chunk(n, std::max(1, c.neigh_maxrow), false, S);
-  for (int first = 0; first < n; first += chunk) {
-    SnapArgs A = snap_args(c, h, first, std::min(chunk, n - first), fp64, fp64 && h->keep_on);
+  snap_chunks(c, h, n, chunk, [&](int first, int m) {
+    SnapArgs A = snap_args(c, h, first, m, fp64, fp64 && h->keep_on);
     if (keep) {
       A.U = h->keep_u.p + 2 * size_t(S.nh) * first;
       A.zkeep = h->keep_z.p + 2 * size_t(S.nz) * first;
@@ -599,7 +620,7 @@ static void snap_launch(Ctx& c, bool energy) {
       k_snap_energy<<<(A.n + 3) / 4, 128, 0, c.stream>>>(A);
       EMD_CHECK_LAUNCH();
     }
-    if (energy) continue;
+    if (energy) return;
     // Eight atoms pool about 208 pairs for 256 lanes; a small system takes one
     // atom per CTA and spreads the T of a pair over four warps
     A.apc = std::max(1, std::min(SF_ATOMS, A.n / 152));
@@ -608,7 +629,7 @@ static void snap_launch(Ctx& c, bool energy) {
     TimedLaunch t(c, fp64 ? "snap_force_fp64" : "snap_force_mixed");
     if (!fp64) snap_mixed_force(A, threads, c.stream);
     else launch_force<double>(A, threads, c.stream);
-  }
+  });
   if (fused) {
     c.snap_pe_fused_valid = true;
     c.snap_pe_fused_version = c.x_version;
@@ -640,9 +661,11 @@ static void snap_adjoint(Ctx& c, const double* dL_dF, double dL_dE, double* grad
     const bool kept = h->keep_on && h->keep_valid && h->keep_xver == c.x_version && h->keep_builds == c.neigh_builds &&
                       h->keep_n == n;
     const int chunk = snap_chunk(n, std::max(1, c.neigh_maxrow), true, S);
-    for (int first = 0; first < n; first += chunk) {
-      SnapArgs A = snap_args(c, h, first, std::min(chunk, n - first), true, true);
+    snap_chunks(c, h, n, chunk, [&](int first, int m) {
+      SnapArgs A = snap_args(c, h, first, m, true, true);
       const int tiles = (A.n + 31) / 32;
+      h->D.reserve(size_t(S.nh) * A.n, c.stream);
+      h->H.reserve(size_t(tiles) * 2 * S.nh * 32, c.stream);
       if (kept) {
         A.U = h->keep_u.p + 2 * size_t(S.nh) * first;
         A.zkeep = h->keep_z.p + 2 * size_t(S.nz) * first;
@@ -655,8 +678,6 @@ static void snap_adjoint(Ctx& c, const double* dL_dF, double dL_dE, double* grad
         A.zkeep = h->zk.p;
         snap_uy(c, A, true);
       }
-      h->D.reserve(size_t(S.nh) * A.n, c.stream);
-      h->H.reserve(size_t(tiles) * 2 * S.nh * 32, c.stream);
       A.D = h->D.p;
       A.H = h->H.p;
       A.g = h->adj_g.p;
@@ -676,7 +697,7 @@ static void snap_adjoint(Ctx& c, const double* dL_dF, double dL_dE, double* grad
       EMD_CHECK_LAUNCH();
       k_snap_pq<<<dim3(tiles, (S.nfull + 7) / 8), 256, 0, c.stream>>>(A);
       EMD_CHECK_LAUNCH();
-    }
+    });
     {
       TimedLaunch t(c, "snap_adjoint_reduce");
       k_adj_reduce<<<dim3(ncols, nelem), 256, 0, c.stream>>>(h->adj.p, n, ncols, c.type.p, S.map, h->adj_sum.p);

@@ -81,3 +81,49 @@ fake.cudaSetDevice(0)
 c.neigh_get()
 assert current() == 0 and fake.fake_wrong_device() == 0
 """)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_snap_works_in_smaller_chunks_where_memory_is_short(run, precision):
+    """Work arrays for all atoms at once do not fit what is left: a call takes fewer atoms
+    at a time, and fails only when those of 32 do not fit."""
+    run(f"""
+from tests.test_gpu_snap_tables import _deck
+st, state = _deck(8, (28, 28, 28), 3.1803)
+n, ncoeffall = len(state["x"]), len(st.elements[0]["beta"])
+def held(compute):
+    if not compute:
+        st.force_compute = lambda b: None
+    c = Context(0)
+    mdloop.init(c, st, state, precision={precision})
+    return c, fake.fake_held()
+c, full = held(True)
+c.close()
+assert fake.fake_held() == 0
+c, bare = held(False)
+work = full - bare
+assert work > 2000 * n
+whole = int(1.25 * n * 8 * (1 + 3 + 2 * 125 + 1)) + 10000   # energies, dL/dF and the adjoint's sums of every atom
+launches = []
+for part in (1.2, 0.3, 0.1, 0.02):
+    fake.fake_set_budget(int(bare + whole + part * work))
+    l = fake.fake_launches()
+    c.snap_compute()
+    launches.append(fake.fake_launches() - l)
+    c.snap_energy()
+    if {precision} == 0:
+        c.snap_adjoint(np.zeros((n, 3)), 1.0, 1, ncoeffall)
+assert launches == sorted(launches) and launches[-1] > launches[0]
+c.close()
+c, bare = held(False)
+fake.fake_set_budget(bare)
+try:
+    c.snap_compute()
+    raise SystemExit("ran without memory")
+except EmdError as e:
+    assert "device allocation failed" in str(e)
+fake.fake_set_budget(full)
+c.snap_compute()
+c.close()
+assert fake.fake_held() == 0
+""")
