@@ -100,3 +100,26 @@ def test_a_small_batch_leaves_a_large_one_its_shared_memory():
     small.close()
     for p, q in zip(*out):
         np.testing.assert_array_equal(p, q)
+
+
+def test_bins_of_more_than_64_particles():
+    """Bins of about 90: put in ascending order by one lane, so that no sum depends on
+    the order in which the particles arrived (other CTA sizes, either form)."""
+    from examinimd_gb300 import Batch
+    rng = np.random.default_rng(14)
+    a = 1.0  # fcc, four atoms per unit volume
+    g = np.stack(np.meshgrid(*[np.arange(9)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    x = ((g[:, None, :] + BASIS[None]) * a).reshape(-1, 3)
+    x = np.mod(x + 0.02 * rng.standard_normal(x.shape), 9 * a)
+    v = rng.standard_normal(x.shape)
+    out = []
+    for threads, spl in ((256, 0), (1024, 0), (256, 10), (1024, 10)):
+        b = Batch([len(x)], np.full((1, 3), 9 * a), x, v, dt=1e-7, max_neigh=512, every=2)
+        b.set_shape(threads, spl)
+        b.run(9)
+        out.append(b.get())
+        b.close()
+    assert np.all(np.isfinite(out[0][2]))
+    for o in out[1:]:
+        for p, q in zip(out[0], o):
+            np.testing.assert_array_equal(p, q)
