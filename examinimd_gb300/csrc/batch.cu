@@ -713,7 +713,12 @@ void batch_run(emd_batch* b, int nsteps, int threads, int spl, bool phased) {
     b->a.xn = b->a.x == b->x.p ? b->x2.p : b->x.p;
     b->a.xln = b->a.xl == b->xl.p ? b->xl2.p : b->xl.p;
   }
+  auto clean = [&] {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+  };
   EMD_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+  bool capturing = true;
   try {
     if (phased) {
       batch_phase<BP_NVE_INITIAL>(b);
@@ -722,19 +727,17 @@ void batch_run(emd_batch* b, int nsteps, int threads, int spl, bool phased) {
       for (int s = 0; s < nsteps; s += spl)
         batch_launch(b, int(b->steps_done + s), std::min(spl, nsteps - s), threads);
     }
+    capturing = false;
+    EMD_CUDA(cudaStreamEndCapture(b->stream, &graph));
+    EMD_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+    EMD_CUDA(cudaGraphLaunch(exec, b->stream));
   } catch (...) {
-    cudaStreamEndCapture(b->stream, &graph);
-    if (graph) cudaGraphDestroy(graph);
-    b->a = before;
+    if (capturing) cudaStreamEndCapture(b->stream, &graph);
+    clean();
+    b->a = before;  // nothing has run: the buffers did not change places
     throw;
   }
-  EMD_CUDA(cudaStreamEndCapture(b->stream, &graph));
-  cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
-  if (e == cudaSuccess) e = cudaGraphLaunch(exec, b->stream);
-  if (exec) cudaGraphExecDestroy(exec);
-  cudaGraphDestroy(graph);
-  if (e != cudaSuccess) b->a = before;
-  EMD_CUDA(e);
+  clean();
   b->steps_done += nsteps;
 }
 

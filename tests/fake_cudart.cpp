@@ -9,6 +9,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <string>
 
 namespace {
 struct Fake {
@@ -18,6 +19,10 @@ struct Fake {
   size_t held = 0, budget = ~size_t(0);
   int wrong_device = 0, launches = 0, fail_end_capture = 0;
   cudaError_t last = cudaSuccess;
+  std::map<const void*, std::string> names;
+  std::string watched;       // argument `arg` of the last launch of the kernel of this name
+  int arg = 0;
+  unsigned long long seen = 0;
 } F;
 thread_local int device = 0;
 thread_local struct {
@@ -30,7 +35,7 @@ cudaError_t err(cudaError_t e) {
   return e;
 }
 int device_of(cudaStream_t s) { return s ? *reinterpret_cast<int*>(s) : device; }
-cudaError_t launch(const void* k, dim3 g, dim3 b, size_t sm, cudaStream_t s) {
+cudaError_t launch(const void* k, dim3 g, dim3 b, void** args, size_t sm, cudaStream_t s) {
   std::lock_guard<std::mutex> l(F.mu);
   if (device_of(s) != device) {
     F.wrong_device++;
@@ -40,6 +45,7 @@ cudaError_t launch(const void* k, dim3 g, dim3 b, size_t sm, cudaStream_t s) {
   const size_t most = it == F.limit.end() ? 48 * 1024 : size_t(it->second);
   if (sm > most || g.x == 0 || b.x * b.y * b.z > 1024) return err(cudaErrorInvalidValue);
   F.launches++;
+  if (!F.watched.empty() && F.names[k].find(F.watched) != std::string::npos) memcpy(&F.seen, args[F.arg], sizeof F.seen);
   return cudaSuccess;
 }
 }  // namespace
@@ -49,6 +55,8 @@ void fake_set_budget(size_t bytes) { F.budget = bytes; }
 size_t fake_held() { return F.held; }
 int fake_wrong_device() { return F.wrong_device; }
 int fake_launches() { return F.launches; }
+void fake_watch(const char* kernel, int arg) { F.watched = kernel, F.arg = arg; }
+unsigned long long fake_seen() { return F.seen; }
 void fake_fail_end_capture(int n) { F.fail_end_capture = n; }
 
 cudaError_t cudaGetDeviceCount(int* n) { return *n = 2, cudaSuccess; }
@@ -138,14 +146,14 @@ cudaError_t __cudaGetKernel(cudaKernel_t* k, const void* f) {
   *k = reinterpret_cast<cudaKernel_t>(const_cast<void*>(f));
   return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3 b, void**, size_t sm, cudaStream_t s) {
-  return launch(k, g, b, sm, s);
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3 b, void** a, size_t sm, cudaStream_t s) {
+  return launch(k, g, b, a, sm, s);
 }
-cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void**, size_t sm, cudaStream_t s) {
-  return launch(f, g, b, sm, s);
+cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void** a, size_t sm, cudaStream_t s) {
+  return launch(f, g, b, a, sm, s);
 }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
-  return launch(f, c->gridDim, c->blockDim, c->dynamicSmemBytes, c->stream);
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** a) {
+  return launch(f, c->gridDim, c->blockDim, a, c->dynamicSmemBytes, c->stream);
 }
 void** __cudaRegisterFatBinary(void*) {
   static void* h;
@@ -153,6 +161,8 @@ void** __cudaRegisterFatBinary(void*) {
 }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
-void __cudaRegisterFunction(void**, const char*, char*, const char*, int, uint3*, uint3*, dim3*, dim3*, int*) {}
+void __cudaRegisterFunction(void**, const char* f, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*) {
+  F.names[f] = name;
+}
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
 }

@@ -15,6 +15,7 @@ from tests import mdloop
 fake = ctypes.CDLL({so!r})
 fake.fake_set_budget.argtypes = [ctypes.c_size_t]
 fake.fake_held.restype = ctypes.c_size_t
+fake.fake_seen.restype = ctypes.c_ulonglong
 def current():
     d = ctypes.c_int()
     fake.cudaGetDevice(ctypes.byref(d))
@@ -126,4 +127,27 @@ fake.fake_set_budget(full)
 c.snap_compute()
 c.close()
 assert fake.fake_held() == 0
+""")
+
+
+def test_a_batch_run_that_could_not_be_captured_changes_nothing(run):
+    """The phased form's buffers alternate while a run is captured: if that fails, the
+    positions are still where they were."""
+    run("""
+b = batch()
+b.set_shape(512, 0)
+fake.fake_watch(b"k_batch_pack", 2)
+def positions():
+    b.lib.emd_batch_get(b.h, np.empty(3 * 70).ctypes.data_as(ctypes.POINTER(ctypes.c_double)), None, None)
+    return fake.fake_seen()
+p = positions()
+fake.fake_fail_end_capture(1)
+try:
+    b.run(2)
+    raise SystemExit("captured")
+except EmdError:
+    pass
+assert positions() == p and b.info()["steps_done"] == 0
+b.run(2)
+assert positions() != p and b.info()["steps_done"] == 2
 """)
