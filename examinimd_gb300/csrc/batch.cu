@@ -701,15 +701,33 @@ void batch_phased_step(emd_batch* b, long long step, int threads, bool last) {
   std::swap(b->a.xl, b->a.xln);
 }
 
+// f() unless device memory is short
+template <typename F>
+bool batch_fits(F&& f) {
+  try {
+    f();
+  } catch (const Error& e) {
+    if (e.code != EMD_ERR_NOMEM) throw;
+    return false;
+  }
+  return true;
+}
+
 // runs nsteps in one CUDA graph: ceil(nsteps / spl) persistent launches, or
-// the phased form's launches per step
+// the phased form's launches per step; without room for its second set of buffers
+// the persistent form, which gives the same bits
 void batch_run(emd_batch* b, int nsteps, int threads, int spl, bool phased) {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   const BArgs before = b->a;
+  if (phased && !batch_fits([&] {
+        b->x2.reserve(b->slots, b->stream);
+        b->xl2.reserve(b->slots, b->stream);
+      })) {
+    b->x2.release();  // not in use: the buffers have not changed places yet
+    phased = false;
+  }
   if (phased) {
-    b->x2.reserve(b->slots, b->stream);
-    b->xl2.reserve(b->slots, b->stream);
     b->a.xn = b->a.x == b->x.p ? b->x2.p : b->x.p;
     b->a.xln = b->a.xl == b->xl.p ? b->xl2.p : b->xl.p;
   }
@@ -1046,9 +1064,16 @@ emd_status emd_batch_get(emd_batch* b, double* x, double* v, double* f) {
   BATCH_BEGIN
   const DeviceGuard device(b->device);
   const size_t n3 = 3 * size_t(b->atoms);
-  b->pack.reserve(n3, b->stream);
+  const bool room = batch_fits([&] { b->pack.reserve(n3, b->stream); });
   auto get = [&](double* out, const double* src, int stride) {
     if (!out) return;
+    if (!room) {  // system by system
+      for (const BSys& S : b->sys)
+        EMD_CUDA(cudaMemcpy2DAsync(out + 3 * S.out, 3 * sizeof(double), src + size_t(S.base) * stride,
+                                   stride * sizeof(double), 3 * sizeof(double), size_t(S.n), cudaMemcpyDeviceToHost,
+                                   b->stream));
+      return;
+    }
     k_batch_pack<<<b->n_chunks, BP_THREADS, 0, b->stream>>>(b->a, b->d_chunks, src, stride, b->pack.p);
     EMD_CHECK_LAUNCH();
     EMD_CUDA(cudaMemcpyAsync(out, b->pack.p, sizeof(double) * n3, cudaMemcpyDeviceToHost, b->stream));

@@ -93,6 +93,11 @@ cudaError_t cudaFreeHost(void* p) { return free(p), cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
   return memmove(d, s, n), cudaSuccess;
 }
+cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size_t w, size_t h, cudaMemcpyKind,
+                              cudaStream_t) {
+  for (size_t i = 0; i < h; ++i) memmove(static_cast<char*>(d) + i * dp, static_cast<const char*>(s) + i * sp, w);
+  return cudaSuccess;
+}
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { return memset(d, v, n), cudaSuccess; }
 
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {

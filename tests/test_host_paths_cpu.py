@@ -151,3 +151,26 @@ assert positions() == p and b.info()["steps_done"] == 0
 b.run(2)
 assert positions() != p and b.info()["steps_done"] == 2
 """)
+
+
+def test_a_batch_without_room_for_more(run):
+    """The phased form's second set of buffers and the packed read-back are extra: without
+    room for them a run takes the persistent form, which gives the same bits, and the
+    read-back copies system by system."""
+    run("""
+b = batch(n=(300, 200))
+ref = b.get()
+b.close()
+b = batch(n=(300, 200))
+b.set_shape(512, 0)
+fake.fake_set_budget(fake.fake_held())
+b.run(25)
+got = b.get()
+assert b.info()["steps_done"] == 25 and b.info()["steps_per_launch"] == 0
+x = np.random.default_rng(1).uniform(0.0, 9.0, (500, 3))
+np.testing.assert_array_equal(got[0], x)   # no kernel ran: what was put in
+np.testing.assert_array_equal(got[1], 0.0 * x)
+fake.fake_set_budget(2 ** 40)
+b.run(25)
+assert b.info()["steps_done"] == 50
+""")
