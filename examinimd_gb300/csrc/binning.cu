@@ -253,6 +253,7 @@ emd_status emd_binning_create(emd_ctx* ctx, double dx_in, double dy_in, double d
   const double key[9] = {double(nb[0]), double(nb[1]), double(nb[2]), c.bmin[0], c.bmin[1],
                          c.bmin[2],     c.bmax[0],     c.bmax[1],     c.bmax[2]};
   if (size_t(ntab) > c.bin_ctab.cap || !std::equal(key, key + 9, c.bin_ctab_key)) {
+    c.bin_ctab_key[0] = 0;  // no box's, should the launch fail
     c.bin_ctab.reserve(size_t(ntab), c.stream);
     TimedLaunch t(c, "bin_ctab");
     k_bin_ctab<<<blocks_for(ntab, 256), 256, 0, c.stream>>>(

@@ -21,8 +21,9 @@ struct Fake {
   cudaError_t last = cudaSuccess;
   std::map<const void*, std::string> names;
   std::string watched;       // argument `arg` of the last launch of the kernel of this name
-  int arg = 0;
+  int arg = 0, count = 0;
   unsigned long long seen = 0;
+  std::string failing;       // the kernel whose next launch fails
 } F;
 thread_local int device = 0;
 thread_local struct {
@@ -44,8 +45,16 @@ cudaError_t launch(const void* k, dim3 g, dim3 b, void** args, size_t sm, cudaSt
   const auto it = F.limit.find(k);
   const size_t most = it == F.limit.end() ? 48 * 1024 : size_t(it->second);
   if (sm > most || g.x == 0 || b.x * b.y * b.z > 1024) return err(cudaErrorInvalidValue);
+  const std::string& name = F.names[k];
+  if (!F.failing.empty() && name.find(F.failing) != std::string::npos) {
+    F.failing.clear();
+    return err(cudaErrorLaunchOutOfResources);
+  }
   F.launches++;
-  if (!F.watched.empty() && F.names[k].find(F.watched) != std::string::npos) memcpy(&F.seen, args[F.arg], sizeof F.seen);
+  if (!F.watched.empty() && name.find(F.watched) != std::string::npos) {
+    memcpy(&F.seen, args[F.arg], sizeof F.seen);
+    F.count++;
+  }
   return cudaSuccess;
 }
 }  // namespace
@@ -55,7 +64,9 @@ void fake_set_budget(size_t bytes) { F.budget = bytes; }
 size_t fake_held() { return F.held; }
 int fake_wrong_device() { return F.wrong_device; }
 int fake_launches() { return F.launches; }
-void fake_watch(const char* kernel, int arg) { F.watched = kernel, F.arg = arg; }
+void fake_watch(const char* kernel, int arg) { F.watched = kernel, F.arg = arg, F.count = 0; }
+int fake_count() { return F.count; }
+void fake_fail_launch(const char* kernel) { F.failing = kernel; }
 unsigned long long fake_seen() { return F.seen; }
 void fake_fail_end_capture(int n) { F.fail_end_capture = n; }
 

@@ -174,3 +174,25 @@ fake.fake_set_budget(2 ** 40)
 b.run(25)
 assert b.info()["steps_done"] == 50
 """)
+
+
+def test_bin_centres_after_a_failed_launch(run):
+    """A box binned as before keeps its table of bin centres, unless the table was being
+    replaced when the call failed."""
+    run("""
+c = Context(0)
+setup = mdloop.LJSetup(4)
+mdloop.init(c, setup, mdloop.make_lattice(setup))
+fake.fake_watch(b"k_bin_ctab", 0)
+def bins(width):
+    c.binning_create(width, width, width, 1, True, True, False)
+    return fake.fake_count()
+assert bins(2.8) == 0 and bins(2.0) == 1 and bins(2.8) == 2 and bins(2.8) == 2
+fake.fake_fail_launch(b"k_bin_ctab")
+try:
+    bins(0.5)
+    raise SystemExit("launched")
+except EmdError:
+    pass
+assert bins(2.8) == 3
+""")
