@@ -409,14 +409,16 @@ __global__ void __launch_bounds__(256) k_adj_reduce(const double* __restrict__ a
 
 }  // namespace
 
-void free_snap(Ctx& c) {
-  if (!c.snap) return;
-  SnapHost* h = static_cast<SnapHost*>(c.snap);
+static void drop_snap(SnapHost* h) {
   h->release_work();
   h->tables.release();
   h->zs.release();
   for (auto* b : {&h->coef, &h->eatom, &h->adj, &h->adj_sum, &h->adj_g, &h->keep_u, &h->keep_z}) b->release();
   delete h;
+}
+void free_snap(Ctx& c) {
+  c.snap_pe_fused_valid = false;
+  if (c.snap) drop_snap(static_cast<SnapHost*>(c.snap));
   c.snap = nullptr;
 }
 
@@ -741,8 +743,8 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   for (int t = 0; t < ntypes; ++t)
     require(map[t] >= 0 && map[t] < nelem, EMD_ERR_ARG, "emd_snap_init: every type must map to an element");
   free_snap(c);
-  SnapHost* h = new SnapHost();
-  c.snap = h;
+  std::unique_ptr<SnapHost, void (*)(SnapHost*)> made(new SnapHost(), drop_snap);  // the context's once it is complete
+  SnapHost* h = made.get();
   h->precision = precision;
   SnapDev& S = h->d;
   S.twojmax = twojmax;
@@ -865,6 +867,7 @@ emd_status emd_snap_init(emd_ctx* ctx, int twojmax, double rfac0, double rmin0, 
   S.zs = h->zs.p;
   fill_stream(c, h);
   EMD_CUDA(cudaStreamSynchronize(c.stream));
+  c.snap = made.release();
   EMD_API_END
 }
 

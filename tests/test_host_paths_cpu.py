@@ -196,3 +196,36 @@ except EmdError:
     pass
 assert bins(2.8) == 3
 """)
+
+
+@pytest.mark.parametrize("how", ["arguments", "memory"])
+def test_a_failed_snap_init_leaves_no_potential(run, how):
+    """emd_snap_init that fails half way: later calls say so."""
+    run(f"""
+from tests.test_gpu_snap_tables import _deck
+st, state = _deck(4, (3, 3, 3), 3.1803)
+c = Context(0)
+mdloop.init(c, st, state)
+if {how!r} == "memory":
+    fake.fake_set_budget(0)
+else:
+    st.elements[0]["beta"] = st.elements[0]["beta"][:-1]
+try:
+    st.force_init(c)
+    raise SystemExit("initialised")
+except EmdError:
+    pass
+fake.fake_set_budget(2 ** 40)
+calls = [c.snap_compute, c.snap_energy, lambda: c.snap_adjoint(np.zeros((54, 3)), 1.0, 1, 15), c.snap_info]
+for call in calls:
+    try:
+        call()
+        raise SystemExit("went on")
+    except EmdError as e:
+        assert "not initialised" in str(e), e
+st, state = _deck(4, (3, 3, 3), 3.1803)
+st.force_init(c)
+c.snap_compute()
+c.close()
+assert fake.fake_held() == 0
+""")
