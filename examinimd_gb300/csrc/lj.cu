@@ -51,17 +51,29 @@ int lj_tile_rows(int n, bool half) {
 // the sum depends on the atom count only and its scratch is bounded
 constexpr int LJE_BLOCKS = 152 * 6;
 
+// Where a thread per row is faster than a tile.
 // A gas's rows: a tile's warp takes a trip to memory for each of them, however short, a
 // thread per row one for 32.  Measured on a random gas (us, thread / tile): 256,000 atoms,
 // 0.5, 1.8 and 3.7 entries a row (longest 6, 10, 16), force 44 / 82, 82 / 98, 121 / 105;
 // 32,000, longest 5 and 9, 12 / 17 and 18 / 21; 16,000, 9 / 10 and 14 / 12; 2,000, 8 / 6 and 12 / 7:
 // there the chip is not full and the tiles' warps run side by side.  Energy, longest
 // 9 or 10: 97 / 127, 41 / 46, 38 / 38 and 36 / 39.
-bool lj_short_rows(const LJTile& T, bool energy) { return T.longest <= 9 && (energy || T.n > 16384); }
+// Rows of hundreds of entries: few fit a warp's list at once, and a row's sums, in order,
+// keep three lanes.  fcc at liquid density, full lists, longest 202, 309, 394 and 688: 256,000
+// atoms 2633 / 2667, 3957 / 4480, 5137 / 7202, 9031 / 14413; 32,000: 384 / 370, 575 / 616, 746 / 919,
+// 1309 / 1884; 16,384: 226 / 192, 338 / 313, 436 / 489, 761 / 964; 8,788: 759 / 566 at 687.  Half lists,
+// longest 117, 168, 217 and 373: 256,000 1703 / 1409, 2411 / 2251, 3236 / 3560, 5591 / 8067; 32,000:
+// 254 / 245, 354 / 388, 475 / 585, 816 / 1483; 16,384: 157 / 104, 217 / 160, 289 / 249, 493 / 531.
+// The energy, which has no sums in order, is faster by tiles throughout.
+bool lj_by_rows(const LJTile& T, bool energy) {
+  if (T.longest <= 9) return energy || T.n > 16384;
+  if (energy) return false;
+  return (T.n > 20000 && T.longest > (T.half ? 160 : 250)) || (T.n > 12000 && T.longest > (T.half ? 300 : 350));
+}
 
 template <int MODE, bool UNI, bool IDIAL = false, bool ZERO = false>
 void launch_lj_fp64(LJTile T, cudaStream_t s) {
-  if (lj_short_rows(T, MODE == LJ_ENERGY)) {
+  if (lj_by_rows(T, MODE == LJ_ENERGY)) {
     k_lj_fp64_rows<MODE, UNI, IDIAL, ZERO>
         <<<MODE == LJ_ENERGY ? LJE_BLOCKS : blocks_for(T.n, LJR_THREADS), LJR_THREADS, 0, s>>>(T);
     EMD_CHECK_LAUNCH();

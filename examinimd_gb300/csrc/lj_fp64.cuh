@@ -287,8 +287,8 @@ __global__ void __launch_bounds__(LJT_THREADS) k_lj_fp64(LJTile T) {
   }
 }
 
-// A thread per row, for short rows (lj_short_rows): the same operations in the same
-// order.  Energy: a fixed number of CTAs, one partial each, as above.
+// A thread per row, for very short and very long rows (lj_by_rows): the same operations
+// in the same order.  Energy: a fixed number of CTAs, one partial each, as above.
 constexpr int LJR_THREADS = 128;
 template <int MODE, bool UNI, bool IDIAL, bool ZERO>
 __global__ void __launch_bounds__(LJR_THREADS) k_lj_fp64_rows(LJTile T) {

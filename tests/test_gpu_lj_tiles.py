@@ -132,3 +132,34 @@ def test_intensity_dial_with_short_rows():
     gpu.lj_compute()
     assert np.array_equal(gpu.get(0, n)["f"], f) and np.abs(f).max() > 0.0
     gpu.close()
+
+
+@pytest.mark.parametrize("n,cut,half,by_rows", [(20000, 5.0, False, False), (20004, 5.0, False, True),
+                                                (12500, 6.0, False, True), (20004, 5.0, True, True), (12500, 6.6, True, True)])
+def test_rows_of_hundreds_of_entries(n, cut, half, by_rows):
+    """Either side of the rule for long rows (full lists: above 250 entries from 20,001
+    atoms, above 350 from 12,001; half lists above 160 and 300)."""
+    from examinimd_gb300 import Context
+    from oracle.orc import Oracle
+    rng = np.random.default_rng(n)
+    st = mdloop.LJSetup(1, half=half, newton=half, cut=cut - 0.3)
+    st.nx = st.ny = st.nz = 1
+    m = int(np.ceil(n ** (1.0 / 3.0)))
+    st.a = m * 1.18  # a simple cubic lattice at about 0.6 of the volume's atoms, displaced
+    g = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    x = np.mod((g + 0.5) * 1.18 + 0.05 * rng.standard_normal((n, 3)), st.a)
+    state = dict(x=x, v=np.zeros((n, 3)), id=np.arange(1, n + 1, dtype=np.int32), type=np.zeros(n, np.int32))
+    gpu, orc = Context(0), Oracle(8)
+    total = mdloop.init(gpu, st, state)
+    mdloop.init(orc, st, state)
+    longest = gpu.neigh_get(total)[0].max()
+    lo = (160 if half else 250) if n > 20000 else (300 if half else 350)
+    assert (longest > lo) == by_rows
+    a, b = gpu.get(0, n), orc.get(0, n)
+    if half:
+        assert np.abs(a["f"] - b["f"]).max() <= 1e-12 * np.abs(b["f"]).max()
+    else:
+        assert np.array_equal(a["f"], b["f"])
+    eg, eo = gpu.lj_energy(), orc.lj_energy_compensated()  # ten million terms: a serial sum is off by 1e-10
+    assert abs(eg - eo) <= 1e-12 * max(abs(eo), float(n))
+    gpu.close()
