@@ -1059,17 +1059,22 @@ emd_status emd_batch_tune(emd_batch* b, int trial_steps, int* threads_out, int* 
 
 // The slots also hold ghosts, in the device's order of systems: packed on the
 // device, a third of the bytes goes over the link and nothing is moved on the
-// host (1.36 million atoms: 23.7 ms with the slots copied, 4.4 packed).
+// host (1.36 million atoms: 23.7 ms with the slots copied, 4.4 packed).  One system is
+// copied as it lies (256 atoms: 53 us packed, 38 so).
 emd_status emd_batch_get(emd_batch* b, double* x, double* v, double* f) {
   BATCH_BEGIN
   const DeviceGuard device(b->device);
   const size_t n3 = 3 * size_t(b->atoms);
-  const bool room = batch_fits([&] { b->pack.reserve(n3, b->stream); });
+  const bool pack = b->nsys > 1 && batch_fits([&] { b->pack.reserve(n3, b->stream); });
   auto get = [&](double* out, const double* src, int stride) {
     if (!out) return;
-    if (!room) {  // system by system
+    if (!pack) {  // system by system
       for (const BSys& S : b->sys)
-        EMD_CUDA(cudaMemcpy2DAsync(out + 3 * S.out, 3 * sizeof(double), src + size_t(S.base) * stride,
+        if (stride == 3)
+          EMD_CUDA(cudaMemcpyAsync(out + 3 * S.out, src + 3 * size_t(S.base), sizeof(double) * 3 * size_t(S.n),
+                                   cudaMemcpyDeviceToHost, b->stream));
+        else
+          EMD_CUDA(cudaMemcpy2DAsync(out + 3 * S.out, 3 * sizeof(double), src + size_t(S.base) * stride,
                                    stride * sizeof(double), 3 * sizeof(double), size_t(S.n), cudaMemcpyDeviceToHost,
                                    b->stream));
       return;
