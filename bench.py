@@ -388,11 +388,14 @@ def run_gpu_arm(a, ws, rank, local):
     mean_row = float(md_row_mean(ctx, nl))
     peaks = load_peaks()
     if snap:
-        # bound by the FP64 pipe (the Wigner-U recursion stays FP64 in both
-        # forms); no measured FP64 peak exists to divide by
-        roof = {"kernel": kname, "bound": "fp64", "achieved": None, "peak": None, "unit": "GFLOP/s",
-                "frac": None, "traffic": None, "mean_row": mean_row, "launch_ms": (kms / kn) if kn else None,
-                "note": "FP64-pipe bound (ncu sm__inst_executed_pipe_fp64); DRAM traffic negligible"}
+        # the FP64 form is bound by the FP64 pipe; the mixed form's Y by the
+        # shared-memory reads of its operands, the rest of it by issue; no measured
+        # peak of either exists to divide by
+        roof = {"kernel": kname, "bound": "fp64" if a.precision == "fp64" else "shared memory", "achieved": None,
+                "peak": None, "unit": "GFLOP/s", "frac": None, "traffic": None, "mean_row": mean_row,
+                "launch_ms": (kms / kn) if kn else None,
+                "note": ("FP64-pipe bound (ncu sm__inst_executed_pipe_fp64)" if a.precision == "fp64" else
+                         "shared-memory wavefronts and instruction issue") + "; DRAM traffic negligible"}
     else:
         bytes_launch = algorithmic_bytes_per_atom(a.precision, mean_row) * nl
         achieved = bytes_launch / (kms / kn * 1e-3) / 1e9 if kn else None

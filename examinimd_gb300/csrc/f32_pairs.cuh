@@ -1,5 +1,6 @@
 // Sums of products in FP32 pairs (high and low part, 48 bits) on the FP32 pipe,
-// which issues 76 times as many lane operations as the FP64 one here.
+// which issues 76 times as many lane operations as the FP64 one here.  Built from
+// Knuth's two-sum and Dekker's product (here a fused multiply-add's remainder).
 #pragma once
 #include "emd_device.cuh"
 
@@ -25,8 +26,8 @@ __device__ __forceinline__ F2 f2_two_sum(float a, float b) {
   return F2{t, add_rn(sub_rn(a, sub_rn(t, y)), sub_rn(b, y))};
 }
 
-// 1.5 times a power of two at least four times as large as b: sums below 2 b in
-// magnitude leave it within one binade
+// 1.5 times the power of two that is four times b's own (more than twice b): sums up
+// to b in magnitude leave it within one binade
 __device__ __forceinline__ float f2_base(float b) {
   const unsigned e = min(max((__float_as_uint(b) >> 23) & 0xffu, 67u), 250u) + 2u;
   return __uint_as_float((e << 23) | 0x400000u);

@@ -187,6 +187,7 @@ static void launch_lj_energy(Ctx& c, double* part) {
 // earlier in that same call.  The array is one per device and per process, so
 // calls that can overlap on one device (two contexts, two host threads, two
 // streams) race on it and must be serialised by the caller.
+// Its size and the call's atom limit date from one partial per 256 atoms, and stay.
 constexpr int kNoAllocBlocks = EMD_LJ_ENERGY_NOALLOC_MAX_LOCAL / 256;  // 16,384 doubles
 static_assert(kNoAllocBlocks >= LJE_BLOCKS, "room for every CTA's partial");
 constexpr int kNoAllocDoubles = kNoAllocBlocks + kSumScratchDoubles;  // 133,512 bytes

@@ -26,10 +26,10 @@
 // directional derivative of X) and k_snap_pq.
 //
 // Precision forms: FP64 (the drop-in; snap.cu, -fmad=false) and mixed
-// (snap_mixed.cu), where the pair scalars are FP64, the sums of U_tot are formed
-// from FP32 pairs of 48 bits and rounded to FP32, and k_snap_y and the sums of
-// k_snap_force run in FP32, with FP64 force sums.  The recurrences and
-// contractions use explicit fused multiply-adds in both forms.
+// (snap_mixed.cu), where the pair scalars and the sums of U_tot are formed in FP32
+// pairs of 48 bits and rounded to FP32, k_snap_y and the sums of k_snap_force run in
+// FP32, and the cutoff test, the r^-14 repulsion and the force sums in FP64.  The
+// recurrences and contractions use explicit fused multiply-adds in both forms.
 #pragma once
 #include <algorithm>
 #include <cmath>
@@ -720,7 +720,7 @@ __global__ void __launch_bounds__(SY_THREADS) k_snap_y(SnapArgs A) {
 // FP32.  Here the FP64 pipe's slow cadence does not hide the rest, so
 //  - the products of a task with equal nj and d form one group, whatever their
 //    (j1, j2): cY is folded into the coefficients, Y is summed directly and the
-//    255 groups (at twojmax 8) replace 1,285 records;
+//    309 groups (at twojmax 8) replace 1,285 records;
 //  - the tables (200 KB) do not fit what the tile leaves of L1, so a task's
 //    entries come as one stream through a shared buffer of the warp's own:
 //    while one KB is worked on the next is on its way in registers;
@@ -890,11 +890,12 @@ __global__ void __launch_bounds__(sy32_threads(NA), NA == 2 ? 1 : 2) k_snap_y32(
 //
 // With twojmax a constant (2, 4, 6, 8) every loop is unrolled and the recurrences'
 // constants are operands; other twojmax take the loops.  The mixed form forms the
-// powers of a and b from their 48-bit values and keeps what the sum over T rounds
-// off, 1,000 operations more, half of the FP32 error (rms against the FP64 form, W
-// bcc 2,000 atoms at 0.05 A: 7.5e-6 -> 5.5e-6 eV/A, of which 3.3e-6 are Y's).
+// powers of a and b from their 48-bit values, keeps what the sum over T rounds off,
+// sums even and odd q apart and takes the gradient's radial part off: 1,000 operations
+// more (rms error against the FP64 form, W bcc 2,000 atoms at 0.05 A: 7.5e-6 eV/A without,
+// 5.5e-6 with the first two, 4.9e-6 with all; U and Y alone account for a third).
 // Bound by instruction issue and the latency of the phases; per 128,000 atoms
-// mixed 0.88 ms as loops, 0.50 unrolled with the extra operations; 8,160 atoms FP64
+// mixed 0.88 ms as loops, 0.51 unrolled with the extra operations; 8,160 atoms FP64
 // 0.64 and 0.55 (0.50 of FP64 issue).
 constexpr int SF_THREADS = 256;
 constexpr int SF_ATOMS = 8;

@@ -1,7 +1,7 @@
-// The mixed form's SNAP kernels (snap_kernel.cuh, snap_split.cuh): pair scalars in
-// FP64, U_tot from FP32 pairs, Z, Y and the pair forces in FP32.  Compiled apart from snap.cu so
-// that the pair scalars may use fused multiply-adds; the FP64 drop-in keeps
-// -fmad=false.
+// The mixed form's SNAP kernels (snap_kernel.cuh, snap_split.cuh): pair scalars and
+// U_tot in FP32 pairs of 48 bits, Z, Y and the pair forces in FP32.  Compiled apart from
+// snap.cu so that plain FP32 expressions may use fused multiply-adds; the FP64 drop-in
+// keeps -fmad=false.
 #include "snap_kernel.cuh"
 #include "snap_split.cuh"
 

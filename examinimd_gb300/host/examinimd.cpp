@@ -48,7 +48,7 @@ struct PhaseClock {
     marks[bucket].push_back({last, e});
     last = e;
   }
-  // seconds per bucket; the events go back to the pool
+  // seconds per bucket; the events may be recorded again
   void collect(double out[4]) {
     for (int b = 0; b < 4; ++b) {
       double t = 0;

@@ -213,8 +213,8 @@ emd_status emd_lj_request_energy(emd_ctx* ctx);
 emd_status emd_lj_force_energy(emd_ctx* ctx, double* pe, int* available);
 /* The same mixed-precision energy kernel on its own, for the current
  * positions and list, without a force call (compute_energy in the mixed
- * form, force_lj_neigh_impl.h:129-156; about 20x cheaper than the FP64 pass
- * of emd_lj_energy at LJ-4M, within 1e-11 relative of it).  *available = 0
+ * form, force_lj_neigh_impl.h:129-156; 1.5 ms at LJ-4M where the FP64 pass of
+ * emd_lj_energy takes 10.4, within 1e-11 relative of it).  *available = 0
  * (and nothing launched) unless the context runs the mixed form with one type
  * pair on a current full list. */
 emd_status emd_lj_energy_mixed(emd_ctx* ctx, double* pe, int* available);
@@ -239,7 +239,8 @@ emd_status emd_lj_adjoint(emd_ctx* ctx, const double* dL_dF, double dL_dE, doubl
  *   device's primary context): a later call under another context (after
  *   cudaDeviceReset, or with the caller's own context current) looks it up
  *   again.
- * - More than EMD_LJ_ENERGY_NOALLOC_MAX_LOCAL owned atoms: EMD_ERR_ARG.
+ * - More than EMD_LJ_ENERGY_NOALLOC_MAX_LOCAL owned atoms: EMD_ERR_ARG (a limit of
+ *   the call, kept; the scratch holds one partial per CTA at any atom count).
  * - Nothing has to be zeroed beforehand.
  * - One array per device and process: calls that can overlap on a device
  *   (two contexts, threads or streams) race and must be serialised. */
