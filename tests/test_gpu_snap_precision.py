@@ -73,3 +73,34 @@ def test_bispectrum_of_large_twojmax(J):
     ref = orc.snap_bispectrum().sum(axis=0)
     gpu.close()
     assert np.sqrt(np.mean((got / ref - 1.0) ** 2)) <= 2.2e-15
+
+
+def test_mixed_forces_of_tungsten():
+    """bcc tungsten, 2,000 atoms displaced by 0.05 A, coefficients of the benchmark: RMS
+    error in eV/A below the 5.9e-6 of FP64 recursions."""
+    from tests.golden.decks import snap_w_synthetic
+    n = 10
+    st = mdloop.SnapSetup(n, n, n, snap_w_synthetic(), lattice_style=2)
+    g = np.stack(np.meshgrid(*[np.arange(n)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    x = ((g[:, None, :] + np.array([[0, 0, 0], [0.5, 0.5, 0.5]])[None]) * st.a).reshape(-1, 3)
+    x = np.mod(x + np.random.default_rng(8).normal(0.0, 0.05, x.shape), st.domain)
+    state = dict(x=x, v=np.zeros_like(x), id=np.arange(1, len(x) + 1, dtype=np.int32), type=np.zeros(len(x), np.int32))
+    from examinimd_gb300 import EMD_PREC_MIXED
+    d = _forces(st, state, EMD_PREC_MIXED) - _forces(st, state, 0)
+    assert np.sqrt(np.mean(np.sum(d * d, axis=1))) <= 5.9e-6
+
+
+@pytest.mark.parametrize("J", [11, 12, 13, 14])
+@pytest.mark.parametrize("a", [3.1803, 2.3])
+def test_forces_of_the_largest_twojmax(J, a):
+    """FP64 against the oracle (four times 1e-12, as for 9 and 10) and mixed against FP64."""
+    from examinimd_gb300 import EMD_PREC_MIXED
+    from oracle.orc import Oracle
+    st, state = _deck(J, (3, 3, 3), a, seed=J)
+    orc = Oracle(8)
+    mdloop.init(orc, st, state)
+    ref = mdloop.by_id(orc.get(0, len(state["x"])))["f"]
+    got, mixed = _forces(st, state, 0), _forces(st, state, EMD_PREC_MIXED)
+    rms = np.sqrt(np.mean(ref * ref))
+    assert np.abs(got - ref).max() <= 4e-12 * rms
+    assert np.sqrt(np.mean((mixed - got) ** 2)) <= 1e-5 * rms
