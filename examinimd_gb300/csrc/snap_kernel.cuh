@@ -270,6 +270,12 @@ __global__ void __launch_bounds__(64) k_snap_pairs(SnapArgs A) {
         const F2 x2 = in ? f2_split(x) : zero, y2 = in ? f2_split(y) : zero, z2 = in ? f2_split(z) : zero;
         F2 sn, cs, sf = w32, dsf = zero;
         f2_sincos(f2_mul(d, scale), sn, cs);
+        // r0inv is a positive root: beyond theta0 = pi (a pair past its own cutoff, inside
+        // the common one, without switching) it is -s / r, and a, b change sign
+        if (sn.h < 0.f) {
+          sn = F2{-sn.h, -sn.l};
+          cs = F2{-cs.h, -cs.l};
+        }
         if (S.switchflag != 0 && d.h > 0.f) {
           F2 ss, cc;
           f2_sincos(f2_mul(d, slope), ss, cc);

@@ -104,3 +104,14 @@ def test_forces_of_the_largest_twojmax(J, a):
     rms = np.sqrt(np.mean(ref * ref))
     assert np.abs(got - ref).max() <= 4e-12 * rms
     assert np.sqrt(np.mean((mixed - got) ** 2)) <= 1e-5 * rms
+
+
+@pytest.mark.parametrize("J", [1, 4, 7, 8, 9])
+def test_mixed_pairs_past_their_own_cutoff(J):
+    """Without switching a pair of the smaller element counts up to the larger one's cutoff,
+    where theta0 exceeds pi; RMS force error of the mixed form."""
+    from examinimd_gb300 import EMD_PREC_MIXED
+    st, state = _deck(J, (3, 3, 3), 3.1803, nelem=2, switchflag=0, seed=J)
+    st.elements[1]["radius"] = 0.38
+    ref, got = _forces(st, state, 0), _forces(st, state, EMD_PREC_MIXED)
+    assert np.sqrt(np.mean((got - ref) ** 2)) <= 1e-5 * np.sqrt(np.mean(ref ** 2))
