@@ -1178,12 +1178,20 @@ __global__ void __launch_bounds__(SF_THREADS, sizeof(R) == 4 ? 3 : 2) k_snap_for
       const R gx2 = gx.value() + gx.value();
       R ga = fma(ar, gx2, gar.value()), gb = fma(ai, gx2, gai.value());
       R gc = fma(-br, gx2, gbr.value()), gd = fma(-bi, gx2, gbi.value());
-      if constexpr (!kF64) {
-        // |a|^2 + |b|^2 = 1, so the gradient's part along (a, b), which is the larger
-        // one (a degree j times Phi), drops out of the force below; rounded with it, it
-        // left a third of the error.  Taken off before the last roundings: ga = ar (gx2
-        // - rho) + gar, gc = -br (gx2 + rho) + gbr
-        const R rho = fma(ar, ga, fma(ai, gb, fma(br, gc, bi * gd)));
+      // |a|^2 + |b|^2 = 1, so the gradient's part along (a, b), which is the larger one (a
+      // degree j times Phi), drops out of the force below. Rounded with the rest it left a
+      // third of the mixed form's error; in the FP64 form it meets the rounding of the
+      // reference's derivatives, large where theta0 nears pi (no switching: 1e-12 to 1e-11
+      // of the RMS force, the layer recursion too; 1e-14 without it). Taken off before the
+      // last roundings: ga = ar (gx2 - rho) + gar, gc = -br (gx2 + rho) + gbr
+      const R rho = fma(ar, ga, fma(ai, gb, fma(br, gc, bi * gd)));
+      if constexpr (kF64) {
+        const R wa = gx2 - rho, wb = -gx2 - rho;
+        ga = fma(ar, wa, gar.s);
+        gb = fma(ai, wa, gai.s);
+        gc = fma(br, wb, gbr.s);
+        gd = fma(bi, wb, gbi.s);
+      } else {
         const F2 wa = f2_two_sum(gx.s + gx.s, -rho), wb = f2_two_sum(-gx.s - gx.s, -rho);
         const R la = wa.l + (gx.c + gx.c), lb = wb.l - (gx.c + gx.c);
         ga = fma(ar, wa.h, gar.s) + fma(ar, la, gar.c);

@@ -115,3 +115,35 @@ def test_mixed_pairs_past_their_own_cutoff(J):
     st.elements[1]["radius"] = 0.38
     ref, got = _forces(st, state, 0), _forces(st, state, EMD_PREC_MIXED)
     assert np.sqrt(np.mean((got - ref) ** 2)) <= 1e-5 * np.sqrt(np.mean(ref ** 2))
+
+
+@pytest.mark.parametrize("J", [2, 5, 8, 9])
+def test_pairs_near_theta0_pi(J):
+    """A pair of the smaller element where theta0 is within 1e-5 of pi (no switching): the
+    reference's derivatives of (a, b) are differences of terms 1e5 times as large, off
+    by some 1e-11 along (a, b), which the force does not depend on.  The force is smooth
+    in the pair's distance, so over steps of 1e-9 of it second differences are
+    roundings: four times 2^-53 of each of some 200 terms."""
+    worst = 0.0
+    for seed in range(4):
+        rng = np.random.default_rng(100 * J + seed)
+        st, _ = _deck(J, (6, 6, 6), 3.1803, nelem=2, switchflag=0, seed=J)
+        st.elements[1]["radius"] = 0.46
+        rcut = 2 * 0.46 * st.rcutfac
+        u = rng.normal(size=3)
+        pair = rcut / st.rfac0 * (1.0 + 1e-5 / np.pi * rng.choice([-1, 1])) * u / np.linalg.norm(u)
+        x = [np.full(3, 9.0), 9.0 + pair]
+        while len(x) < 14:
+            y = rng.uniform(4.0, 15.0, 3)
+            if min(np.linalg.norm(y - z) for z in x) > 2.4:
+                x.append(y)
+        n = len(x)
+        types = np.where(np.arange(n) < 2, 1, rng.integers(0, 2, n)).astype(np.int32)
+        f = []
+        for k in range(-4, 5):
+            x[1] = 9.0 + pair * (1.0 + 1e-9 * k)
+            f.append(_forces(st, dict(x=np.array(x), v=np.zeros((n, 3)), id=np.arange(1, n + 1, dtype=np.int32),
+                                      type=types), 0))
+        f = np.array(f)
+        worst = max(worst, np.abs(f[2:] - 2.0 * f[1:-1] + f[:-2]).max() / np.sqrt(np.mean(f[4] ** 2)))
+    assert worst <= 1e-13
