@@ -913,7 +913,7 @@ def batch_measure(local: int, steps: int, loop_sample: int, loop_steps: int) -> 
     loop_rate = loop_atoms / (loop_ms * 1e-3)
     return {"value": value, "unit": METRIC, "systems": int(len(ns)), "atoms": total, "steps": steps,
             "ms": ms, "atoms_min": int(ns.min()), "atoms_max": int(ns.max()),
-            "shape": {"form": "phased (one launch per phase over all systems)" if spl == 0 else
+            "shape": {"form": "phased (two launches a step over all systems)" if spl == 0 else
                       "persistent (one CTA per system)", "threads_per_cta": threads, "steps_per_launch": spl,
                       "chosen_by": "emd_batch_tune (40 steps)"},
             "create_s": t_create, "energy_drift_rel_per_1000_max": float(drift.max()),

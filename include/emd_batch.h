@@ -7,7 +7,7 @@
  * sigma with a fixed cutoff, and NVE velocity-Verlet.  Every `every` steps
  * its halo and full neighbour list (cutoff + skin) are rebuilt.  Two forms:
  * persistent (one CTA advances one system for a whole launch) and phased
- * (one launch per phase over all systems; the per-system rebuild on one CTA
+ * (two launches a step over all systems; the per-system rebuild on one CTA
  * each).  A run's launches are captured in one CUDA graph, and
  * emd_batch_tune times the forms, CTA sizes and steps per launch on the
  * ensemble itself.
@@ -36,11 +36,14 @@ emd_status emd_batch_create(emd_batch** out, int device, int nsys, const int* na
 void emd_batch_destroy(emd_batch* b);
 const char* emd_batch_last_error(const emd_batch* b);
 /* Advances every system nsteps (one CUDA graph of ceil(nsteps /
- * steps_per_launch) launches). */
+ * steps_per_launch) launches, or of the phased form's).  This and the calls below
+ * work on the batch's device whatever the thread's current one is. */
 emd_status emd_batch_run(emd_batch* b, int nsteps);
 /* CTA size (multiple of 32, 64..1024) and steps per persistent launch; 0
- * steps per launch selects the phased form: one launch per phase over every
- * system (128-atom chunks), the per-system rebuild on `threads`-thread CTAs. */
+ * steps per launch selects the phased form: two launches a step over 128-atom
+ * chunks of every system, the per-system rebuild on `threads`-thread CTAs.  It
+ * needs a second set of position buffers; without room for it a run takes the
+ * persistent form, whose results have the same bits. */
 emd_status emd_batch_set_shape(emd_batch* b, int threads, int steps_per_launch);
 /* Times every candidate shape (persistent and phased) on trial_steps steps
  * from the current state (restored after each trial), keeps the fastest and
