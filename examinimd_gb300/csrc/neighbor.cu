@@ -192,6 +192,8 @@ emd_status emd_neigh_create(emd_ctx* ctx, int half_neigh, long long* total_out) 
   require(!c.bin_sorted, EMD_ERR_STATE,
           "emd_neigh_create: the last binning re-sorted the particles, so its permutation no longer refers to "
           "them; bin owned and ghost particles again without sorting first (as ExaMiniMD does)");
+  require(c.nhalo >= 1, EMD_ERR_STATE,
+          "emd_neigh_create: the binning has no halo bins; rows read the 27 bins around each interior one");
   const int n = c.N_local;
   c.half_neigh = half_neigh ? 1 : 0;
   const int packed = (c.lj_ready && c.lj_prec == EMD_PREC_MIXED) ? 1 : 0;

@@ -229,3 +229,21 @@ c.snap_compute()
 c.close()
 assert fake.fake_held() == 0
 """)
+
+
+def test_no_list_from_bins_without_a_halo_layer(run):
+    """Rows read the 27 bins around each interior bin: without a layer of halo bins those
+    of the outer ones do not exist."""
+    run("""
+c = Context(0)
+setup = mdloop.LJSetup(4)
+mdloop.init(c, setup, mdloop.make_lattice(setup))
+c.binning_create(2.8, 2.8, 2.8, 0, True, True, False)
+try:
+    c.neigh_create(False)
+    raise SystemExit("built")
+except EmdError as e:
+    assert "halo" in str(e)
+c.binning_create(2.8, 2.8, 2.8, 1, True, True, False)
+c.neigh_create(False)
+""")
